@@ -31,7 +31,6 @@
 
 #include <algorithm>
 #include <map>
-#include <tuple>
 #include <vector>
 
 #include "jk_internal.h"
@@ -42,51 +41,21 @@
         if (e_ != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e_));    \
     } while (0)
 
-struct JKDmCond {
-    const double* dm;
-    const int* gao;  // group AO offsets (device)
-    double* out;     // ngroups x ngroups
-    int nao, n_dm, ngroups;
-};
-
 struct JKSym {
     const double* in;
     double* out;
     int nao, n_dm;
 };
 
-struct JKBatchKey {
-    int cls, np_ij, np_kl;                  // np_* = -1: any primitive count
-    std::vector<std::pair<int, int>> segs;  // (molecule, class quartet)
-    std::vector<long long> seg_tasks;       // unscreened tasks of each segment
-    long long max_tasks = 0;
-    JKBatchCfg cfg[2] = {{nullptr, 0, 1}, {nullptr, 0, 1}};  // FP64 part, FP32 part (queue set at launch)
-    float tuned_ms[2] = {-1.f, -1.f};
-};
-
-// a class quartet launched on its own (see the top of the file)
-struct JKSolo {
-    int mol, cq, cls;
-    long long tasks;  // unscreened
-    JKSeg s64, s32;   // FP64 and FP32 parts, filled with the segment tables
-};
-
 struct jk_batch {
-    int device = 0, nsm = 148, nmol = 0, max_groups = 0;
-    long long solo_tasks = JK_BATCH_SOLO_TASKS;
+    int device = 0, nsm = 148, nmol = 0, max_groups = 0, max_nao = 0;
     std::vector<jk_basis*> mols;
-    std::vector<JKBatchKey> keys;
-    std::vector<JKSolo> solo;
-    std::vector<int> key_off;  // nkeys + 1 segment offsets
-    int nseg = 0;
+    JKPlan* plan = nullptr;  // merged keys, then the class quartets launched on their own
+    int nmerged = 0;         // merged keys
     JKScreenCQ* d_cq = nullptr;
     int ncq = 0;
     JKDmCond* d_dmc = nullptr;
     std::vector<JKDmCond> h_dmc;
-    JKSeg *d_seg64 = nullptr, *d_seg32 = nullptr;
-    long long *d_segt64 = nullptr, *d_segt32 = nullptr;
-    const long long **d_cnt64 = nullptr, **d_cnt32 = nullptr;
-    int* d_key_off = nullptr;
     // pointer set the segment tables were built for
     std::vector<const double*> seg_dm;
     std::vector<double*> seg_vj, seg_vk;
@@ -101,7 +70,6 @@ struct jk_batch {
     // captured graph
     cudaGraphExec_t graph = nullptr;
     JKFanout fan;  // side streams of the class launches
-    unsigned long long* d_queue = nullptr;  // 2 work counters per key (persistent launches)
     // pair-packed J side: every molecule's packed densities, then every
     // molecule's packed J accumulators (one memset clears them all)
     double* d_pk = nullptr;
@@ -110,48 +78,6 @@ struct jk_batch {
     long long pk_max = 0;          // largest per-molecule packed size
     bool packed = false;
 };
-
-// per (molecule, gi, gj): max |D| over the group block (blockIdx.z = molecule)
-__global__ void jk_dm_cond_batch_kernel(const JKDmCond* __restrict__ t) {
-    const JKDmCond m = t[blockIdx.z];
-    int gi = blockIdx.x, gj = blockIdx.y;
-    if (gi >= m.ngroups || gj >= m.ngroups) return;
-    int p0 = m.gao[gi], p1 = m.gao[gi + 1], q0 = m.gao[gj], q1 = m.gao[gj + 1];
-    int np = p1 - p0, nq = q1 - q0;
-    double mx = 0;
-    long long n = (long long)np * nq * m.n_dm;
-    for (long long e = threadIdx.x; e < n; e += blockDim.x) {
-        int idm = (int)(e / ((long long)np * nq));
-        int rem = (int)(e - (long long)idm * np * nq);
-        int p = p0 + rem / nq, q = q0 + rem % nq;
-        mx = fmax(mx, fabs(m.dm[(size_t)idm * m.nao * m.nao + (size_t)p * m.nao + q]));
-    }
-    __shared__ double red[256];
-    red[threadIdx.x] = mx;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) m.out[gi * m.ngroups + gj] = red[0];
-}
-
-// exclusive prefix of the per-segment task counts of every key
-// (blockIdx.x = key); key k's prefix lives at segt[key_off[k] + k], n_k + 1 entries
-__global__ void jk_seg_prefix_kernel(const long long* const* __restrict__ cnt, const int* __restrict__ key_off,
-                                     long long* __restrict__ segt) {
-    int k = blockIdx.x;
-    int s0 = key_off[k], n = key_off[k + 1] - s0;
-    long long* out = segt + s0 + k;
-    if (threadIdx.x == 0) {
-        long long acc = 0;
-        out[0] = 0;
-        for (int i = 0; i < n; i++) {
-            acc += *cnt[s0 + i];
-            out[i + 1] = acc;
-        }
-    }
-}
 
 // J = 2 (V + V^T), K = V + V^T per molecule (blockIdx.y = molecule)
 __global__ void jk_symmetrize_batch_kernel(const JKSym* __restrict__ t, double fac) {
@@ -175,14 +101,7 @@ static void free_batch(jk_batch* t) {
     cudaFree(t->d_pmol);
     cudaFree(t->d_cq);
     cudaFree(t->d_dmc);
-    cudaFree(t->d_seg64);
-    cudaFree(t->d_seg32);
-    cudaFree(t->d_segt64);
-    cudaFree(t->d_segt32);
-    cudaFree((void*)t->d_cnt64);
-    cudaFree((void*)t->d_cnt32);
-    cudaFree(t->d_key_off);
-    cudaFree(t->d_queue);
+    jk_plan_free(t->plan);
     cudaFree(t->d_work);
     cudaFree(t->d_sym);
     if (t->blas) cublasDestroy(t->blas);
@@ -190,103 +109,35 @@ static void free_batch(jk_batch* t) {
 }
 
 static int batch_create(jk_basis_t* const* bases, int nmol, long long solo_tasks, jk_batch* t) {
-    t->solo_tasks = solo_tasks;
     BCUDA(cudaGetDevice(&t->device));
     BCUDA(cudaDeviceGetAttribute(&t->nsm, cudaDevAttrMultiProcessorCount, t->device));
     BCUDA(t->fan.init());
     t->nmol = nmol;
+    t->plan = new JKPlan();
     std::vector<JKScreenCQ> cqs;
-    std::map<std::tuple<int, int, int>, int> kidx;
     for (int m = 0; m < nmol; m++) {
         jk_basis* b = bases[m];
         if (!b) return jk_internal_set_err(JK_ERR_ARG, "jk_batch_create: null basis");
         if (b->device != t->device) return jk_internal_set_err(JK_ERR_ARG, "jk_batch_create: bases on other devices");
         t->mols.push_back(b);
         t->max_groups = std::max(t->max_groups, b->ngroups);
+        t->max_nao = std::max(t->max_nao, b->nao);
         for (int c = 0; c < b->ncq; c++) {
             const JKScreenCQ& cq = b->h_cq[c];
             cqs.push_back(cq);
-            int cls = jk_internal_class_index(b, cq.cp_ij, cq.cp_kl);
             const long long n = cq.cp_ij == cq.cp_kl ? (long long)cq.n_ij * (cq.n_ij + 1) / 2
                                                      : (long long)cq.n_ij * cq.n_kl;
-            if (solo_tasks > 0 && n >= solo_tasks) {
-                JKSolo so{};
-                so.mol = m;
-                so.cq = c;
-                so.cls = cls;
-                so.tasks = n;
-                t->solo.push_back(so);
-                continue;
-            }
-            int np_ij = b->h_group_nprim[cq.gi] * b->h_group_nprim[cq.gj];
-            int np_kl = b->h_group_nprim[cq.gk] * b->h_group_nprim[cq.gl];
-            if (!jk_internal_class_team(cls)) np_ij = np_kl = -1;
-            auto key = std::make_tuple(cls, np_ij, np_kl);
-            auto it = kidx.find(key);
-            if (it == kidx.end()) {
-                kidx[key] = (int)t->keys.size();
-                JKBatchKey k;
-                k.cls = cls;
-                k.np_ij = np_ij;
-                k.np_kl = np_kl;
-                t->keys.push_back(k);
-                it = kidx.find(key);
-            }
-            JKBatchKey& k = t->keys[it->second];
-            k.segs.push_back({m, c});
-            k.seg_tasks.push_back(n);
-            k.max_tasks += n;
+            int rc = jk_plan_add(t->plan, b, m, c, solo_tasks > 0 && n >= solo_tasks);
+            if (rc) return rc;
         }
     }
-    // longest first within every key (stable: ties keep molecule order)
-    for (auto& k : t->keys) {
-        std::vector<int> ord(k.segs.size());
-        for (size_t i = 0; i < ord.size(); i++) ord[i] = (int)i;
-        std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return k.seg_tasks[a] > k.seg_tasks[b]; });
-        std::vector<std::pair<int, int>> segs(ord.size());
-        std::vector<long long> tasks(ord.size());
-        for (size_t i = 0; i < ord.size(); i++) {
-            segs[i] = k.segs[ord[i]];
-            tasks[i] = k.seg_tasks[ord[i]];
-        }
-        k.segs.swap(segs);
-        k.seg_tasks.swap(tasks);
-    }
-    for (auto& k : t->keys)
-        if (!jk_internal_batch_launcher(k.cls, 0))
-            return jk_internal_set_err(JK_ERR_UNSUPPORTED, "jk_batch_create: class without kernel");
-    for (auto& so : t->solo)
-        if (!jk_internal_batch_launcher(so.cls, 0))
-            return jk_internal_set_err(JK_ERR_UNSUPPORTED, "jk_batch_create: class without kernel");
+    int rc = jk_plan_finish(t->plan, t->mols);
+    if (rc) return rc;
+    for (const auto& k : t->plan->keys) t->nmerged += !k.solo;
     t->ncq = (int)cqs.size();
-    t->key_off.push_back(0);
-    std::vector<const long long*> c64, c32;
-    for (auto& k : t->keys) {
-        for (auto& sgi : k.segs) {
-            const JKScreenCQ& cq = t->mols[sgi.first]->h_cq[sgi.second];
-            c64.push_back(cq.task0 + 1);
-            c32.push_back(cq.task032 + 1);
-        }
-        t->key_off.push_back(t->key_off.back() + (int)k.segs.size());
-    }
-    t->nseg = t->key_off.back();
-    int nkeys = (int)t->keys.size();
     BCUDA(cudaMalloc(&t->d_cq, sizeof(JKScreenCQ) * std::max(1, t->ncq)));
     if (t->ncq) BCUDA(cudaMemcpy(t->d_cq, cqs.data(), sizeof(JKScreenCQ) * t->ncq, cudaMemcpyHostToDevice));
     BCUDA(cudaMalloc(&t->d_dmc, sizeof(JKDmCond) * nmol));
-    BCUDA(cudaMalloc(&t->d_seg64, sizeof(JKSeg) * std::max(1, t->nseg)));
-    BCUDA(cudaMalloc(&t->d_seg32, sizeof(JKSeg) * std::max(1, t->nseg)));
-    BCUDA(cudaMalloc(&t->d_segt64, sizeof(long long) * (t->nseg + nkeys + 1)));
-    BCUDA(cudaMalloc(&t->d_segt32, sizeof(long long) * (t->nseg + nkeys + 1)));
-    BCUDA(cudaMalloc((void**)&t->d_cnt64, sizeof(long long*) * std::max(1, t->nseg)));
-    BCUDA(cudaMalloc((void**)&t->d_cnt32, sizeof(long long*) * std::max(1, t->nseg)));
-    BCUDA(cudaMalloc(&t->d_key_off, sizeof(int) * (nkeys + 1)));
-    BCUDA(cudaMalloc(&t->d_queue, sizeof(unsigned long long) * 2 * std::max(1, nkeys)));
-    if (t->nseg) {
-        BCUDA(cudaMemcpy((void*)t->d_cnt64, c64.data(), sizeof(long long*) * t->nseg, cudaMemcpyHostToDevice));
-        BCUDA(cudaMemcpy((void*)t->d_cnt32, c32.data(), sizeof(long long*) * t->nseg, cudaMemcpyHostToDevice));
-    }
-    BCUDA(cudaMemcpy(t->d_key_off, t->key_off.data(), sizeof(int) * (nkeys + 1), cudaMemcpyHostToDevice));
     return JK_OK;
 }
 
@@ -330,7 +181,7 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
         size_t tot = 0;
         for (int m = 0; m < t->nmol; m++) {
             dp_off[m] = tot;
-            tot += (size_t)n_dm * t->mols[m]->pack_total;
+            tot += 2 * (size_t)n_dm * t->mols[m]->pack_total;
             t->pk_max = std::max(t->pk_max, t->mols[m]->pack_total);
         }
         t->pk_jp = tot;
@@ -342,59 +193,41 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
         }
         std::vector<JKPackMol> pm(t->nmol);
         for (int m = 0; m < t->nmol; m++) {
-            const jk_basis* b = t->mols[m];
-            pm[m] = JKPackMol{b->d_pack, b->ncp, b->pack_total, b->d_pair2bra, b->d_pair2ket, b->d_ao_loc,
-                              dms[m], b->nao, n_dm, t->d_pk + dp_off[m], t->d_pk + tot + dp_off[m], vjs[m]};
+            pm[m] = jk_internal_pack_mol(t->mols[m], dms[m], n_dm, t->d_pk + dp_off[m], t->d_pk + tot + dp_off[m],
+                                         vjs[m]);
         }
         if (!t->d_pmol) BCUDA(cudaMalloc(&t->d_pmol, sizeof(JKPackMol) * t->nmol));
         BCUDA(cudaMemcpy(t->d_pmol, pm.data(), sizeof(JKPackMol) * t->nmol, cudaMemcpyHostToDevice));
     }
-    // pair-packed J side of molecule m's class quartet c in both parts
-    auto set_packed = [&](int m, int c, JKSeg* a, JKSeg* b2) {
-        if (!t->packed) return;
-        const jk_basis* b = t->mols[m];
-        const JKScreenCQ& cq = b->h_cq[c];
-        const JKPackCls &ki = b->h_pack[cq.cp_ij], &kk = b->h_pack[cq.cp_kl];
-        double* dp = t->d_pk + dp_off[m];
-        double* jp = t->d_pk + t->pk_jp + dp_off[m];
-        for (JKSeg* sg : {a, b2}) {
-            sg->dp_ij = dp + ki.off;
-            sg->dp_kl = dp + kk.off;
-            sg->jp_ij = jp + ki.off;
-            sg->jp_kl = jp + kk.off;
-            sg->np_ij = ki.np;
-            sg->np_kl = kk.np;
-            sg->pk_stride = b->pack_total;
-        }
-    };
-    for (auto& so : t->solo) {
-        const int m = so.mol;
-        jk_internal_fill_seg_batch(t->mols[m], so.cq, dms[m], n_dm, vjs ? vjs[m] : nullptr, vks ? vks[m] : nullptr, 0,
-                                   &so.s64);
-        jk_internal_fill_seg_batch(t->mols[m], so.cq, dms[m], n_dm, vjs ? vjs[m] : nullptr, vks ? vks[m] : nullptr, 1,
-                                   &so.s32);
-        set_packed(m, so.cq, &so.s64, &so.s32);
-    }
-    std::vector<JKSeg> s64(std::max(1, t->nseg)), s32(std::max(1, t->nseg));
-    int i = 0;
-    for (auto& k : t->keys) {
-        for (auto& sgi : k.segs) {
-            int m = sgi.first;
-            jk_internal_fill_seg_batch(t->mols[m], sgi.second, dms[m], n_dm, vjs ? vjs[m] : nullptr,
-                                       vks ? vks[m] : nullptr, 0, &s64[i]);
-            jk_internal_fill_seg_batch(t->mols[m], sgi.second, dms[m], n_dm, vjs ? vjs[m] : nullptr,
-                                       vks ? vks[m] : nullptr, 1, &s32[i]);
-            set_packed(m, sgi.second, &s64[i], &s32[i]);
-            i++;
-        }
+    JKPlan* p = t->plan;
+    std::vector<JKSeg> seg(std::max(1, p->nseg));
+    for (int part = 0; part < 2; part++) {
+        int i = 0;
+        for (auto& k : p->keys)
+            for (auto& sgi : k.segs) {
+                const int m = sgi.first;
+                JKSeg& s = seg[i++];
+                jk_internal_fill_seg_cq(t->mols[m], sgi.second, part, &s);
+                s.dm = dms[m];
+                s.vj = vjs ? vjs[m] : nullptr;
+                s.vk = vks ? vks[m] : nullptr;
+                s.n_dm = n_dm;
+                if (t->packed) {
+                    const size_t n = (size_t)n_dm * t->mols[m]->pack_total;
+                    s.dp = t->d_pk + dp_off[m];
+                    s.dpb = s.dp + n;
+                    s.jp = t->d_pk + t->pk_jp + dp_off[m];
+                    s.jpb = s.jp + n;
+                }
+            }
+        BCUDA(cudaMemcpy(p->d_seg[part], seg.data(), sizeof(JKSeg) * p->nseg, cudaMemcpyHostToDevice));
     }
     t->h_dmc.resize(t->nmol);
     for (int m = 0; m < t->nmol; m++) {
         jk_basis* b = t->mols[m];
-        t->h_dmc[m] = JKDmCond{dms[m], b->d_group_ao, b->d_dm_cond, b->nao, n_dm, b->ngroups};
+        t->h_dmc[m] = JKDmCond{dms[m],     b->d_group_ao, b->d_dm_cond, b->nao, n_dm,
+                               b->ngroups, (unsigned long long*)b->d_zero, (int)(b->zero_bytes / 8)};
     }
-    BCUDA(cudaMemcpy(t->d_seg64, s64.data(), sizeof(JKSeg) * t->nseg, cudaMemcpyHostToDevice));
-    BCUDA(cudaMemcpy(t->d_seg32, s32.data(), sizeof(JKSeg) * t->nseg, cudaMemcpyHostToDevice));
     BCUDA(cudaMemcpy(t->d_dmc, t->h_dmc.data(), sizeof(JKDmCond) * t->nmol, cudaMemcpyHostToDevice));
     t->seg_dm.assign(dms, dms + t->nmol);
     t->seg_vj.assign(t->nmol, nullptr);
@@ -417,41 +250,16 @@ static int batch_prepare(jk_batch* t, const double* const* dms, double* const* v
     int nbins = opts && opts->nbins > 0 ? opts->nbins : 10;
     int prescreen = opts ? opts->prescreen : 1;
     double fp32_cutoff = opts ? opts->fp32_cutoff : 0.;
-    dim3 g(t->max_groups, t->max_groups, t->nmol);
-    jk_dm_cond_batch_kernel<<<g, 256, 0, st>>>(t->d_dmc);
-    BCUDA(cudaGetLastError());
-    if (t->ncq == 0) return JK_OK;
+    rc = jk_internal_dm_cond(t->d_dmc, t->nmol, t->max_groups, t->max_nao, st);
+    if (rc || t->ncq == 0) return rc;
     rc = jk_internal_screen(t->d_cq, t->ncq, tol, nbins, prescreen, fp32_cutoff, st);
+    if (!rc) rc = jk_plan_prefix(t->plan, fp32_cutoff > 0, st);
     if (rc) return rc;
-    int nkeys = (int)t->keys.size();
-    if (nkeys > 0) {
-        jk_seg_prefix_kernel<<<nkeys, 32, 0, st>>>(t->d_cnt64, t->d_key_off, t->d_segt64);
-        BCUDA(cudaGetLastError());
-    }
-    if (fp32_cutoff > 0 && nkeys > 0) {
-        jk_seg_prefix_kernel<<<nkeys, 32, 0, st>>>(t->d_cnt32, t->d_key_off, t->d_segt32);
-        BCUDA(cudaGetLastError());
-    }
     if (t->packed) {
         rc = jk_internal_pack_batch(t->d_pmol, t->nmol, t->pk_max, 0, st);
         if (rc) return rc;
         BCUDA(cudaMemsetAsync(t->d_pk + t->pk_jp, 0, sizeof(double) * t->pk_jp, st));
     }
-    return JK_OK;
-}
-
-// the class launch of key k, part 0 (FP64) or 1 (FP32), with shape cfg
-static int batch_launch_key(jk_batch* t, int k, int part, const JKBatchCfg& cfg, cudaStream_t st) {
-    const JKBatchKey& key = t->keys[k];
-    int off = t->key_off[k], n = t->key_off[k + 1] - off;
-    jk_launch_batch_fn f = jk_internal_batch_launcher(key.cls, part);
-    if (!f) return jk_internal_set_err(JK_ERR_UNSUPPORTED, "no kernel for a class of the batch");
-    JKBatchCfg c = cfg;
-    if (c.grab > 0) c.queue = t->d_queue + 2 * k + part;
-    else c.queue = nullptr;
-    const JKSeg* segs = (part ? t->d_seg32 : t->d_seg64) + off;
-    const long long* segt = (part ? t->d_segt32 : t->d_segt64) + off + k;
-    BCUDA(f(segs, segt, n, key.max_tasks, t->nsm, c, st));
     return JK_OK;
 }
 
@@ -463,26 +271,17 @@ extern "C" int jk_batch_build(jk_batch_t* t, const double* const* dms, double* c
     int rc = batch_prepare(t, dms, vjs, vks, n_dm, opts, st);
     if (rc || t->ncq == 0) return rc;
     const bool mixed = opts && opts->fp32_cutoff > 0;
-    int nkeys = (int)t->keys.size();
+    const int nkeys = (int)t->plan->keys.size();
     // work counters of the persistent launches start at zero every build
-    BCUDA(cudaMemsetAsync(t->d_queue, 0, sizeof(unsigned long long) * 2 * nkeys, st));
+    BCUDA(cudaMemsetAsync(t->plan->d_queue, 0, sizeof(unsigned long long) * 2 * nkeys, st));
     BCUDA(t->fan.begin(st));
-    int lane = 0;  // FP64 parts on the even side streams, FP32 parts on the odd ones
-    for (const JKSolo& so : t->solo) {
-        const JKScreenCQ& cq = t->mols[so.mol]->h_cq[so.cq];
-        rc = jk_internal_launch_part(so.cls, 0, so.s64, cq.task0, so.tasks, t->nsm, t->fan.pick(2 * lane));
-        if (rc) return rc;
-        if (mixed) {
-            rc = jk_internal_launch_part(so.cls, 1, so.s32, cq.task032, so.tasks, t->nsm, t->fan.pick(2 * lane + 1));
-            if (rc) return rc;
-        }
-        lane++;
-    }
-    for (int k = 0; k < nkeys; k++, lane++) {
-        rc = batch_launch_key(t, k, 0, t->keys[k].cfg[0], t->fan.pick(2 * lane));
-        if (rc) return rc;
-        if (mixed) {
-            rc = batch_launch_key(t, k, 1, t->keys[k].cfg[1], t->fan.pick(2 * lane + 1));
+    // class quartets on their own first; FP64 parts on the even side streams,
+    // FP32 parts on the odd ones
+    for (int lane = 0; lane < nkeys; lane++) {
+        const int k = (t->nmerged + lane) % nkeys;
+        for (int part = 0; part < (mixed ? 2 : 1); part++) {
+            rc = jk_plan_launch(t->plan, k, part, t->plan->keys[k].cfg[part], n_dm, t->nsm,
+                                t->fan.pick(2 * lane + part));
             if (rc) return rc;
         }
     }
@@ -499,25 +298,19 @@ extern "C" int jk_batch_build(jk_batch_t* t, const double* const* dms, double* c
 // launch shapes are timed on this batch with CUDA events, each launch alone
 // on the caller's stream after the bookkeeping of a real build, and the
 // fastest is kept.  Candidates: static chunks; the persistent mode at one
-// resident grid with three grab sizes (tasks per warp for the thread
-// kernels, per team for the team kernels, per block for the generic kernel)
+// resident grid with three grab sizes (items per warp for the run kernels,
+// tasks per team for the team kernels, per block for the generic kernel)
 // and at two resident grids with the middle one.  A cache file keeps the
 // choices per (class, primitive counts, part, log2 of the task count); keys
 // found there are not timed again.
 // ---------------------------------------------------------------------------
-static bool class_is_generic(int cls) {
-    const int ll = cls % 7, lk = (cls / 7) % 7, lj = (cls / 49) % 7, li = cls / 343;
-    return li > JK_LMAX || lj > JK_LMAX || lk > JK_LMAX || ll > JK_LMAX;
-}
-
 static int cand_grabs(int cls, int* g) {
     if (jk_internal_class_team(cls)) { g[0] = 2; g[1] = 8; g[2] = 32; }
-    else if (class_is_generic(cls)) { g[0] = 1; g[1] = 4; g[2] = 16; }
-    else { g[0] = 64; g[1] = 256; g[2] = 1024; }
+    else { g[0] = 1; g[1] = 4; g[2] = 16; }
     return 3;
 }
 
-static std::string tune_key_str(const JKBatchKey& k, int part) {
+static std::string tune_key_str(const JKPlanKey& k, int part) {
     int b = 0;
     for (long long x = k.max_tasks; x > 1; x >>= 1) b++;
     char buf[96];
@@ -530,7 +323,7 @@ extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* co
     if (!t || !dms || n_dm <= 0 || (!vjs && !vks))
         return jk_internal_set_err(JK_ERR_ARG, "jk_batch_tune: invalid arguments");
     cudaStream_t st = (cudaStream_t)stream;
-    int nkeys = (int)t->keys.size();
+    const int nkeys = t->nmerged;
     const bool mixed = opts && opts->fp32_cutoff > 0;
     // cached choices: "cls np_ij np_kl part log2tasks mode grab grid_mul ms"
     std::map<std::string, std::pair<JKBatchCfg, float>> cache;
@@ -555,7 +348,7 @@ extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* co
     BCUDA(cudaEventCreate(&e0));
     BCUDA(cudaEventCreate(&e1));
     for (int k = 0; k < nkeys && t->ncq; k++) {
-        JKBatchKey& key = t->keys[k];
+        JKPlanKey& key = t->plan->keys[k];
         for (int part = 0; part < (mixed ? 2 : 1); part++) {
             const std::string ks = tune_key_str(key, part);
             auto hit = cache.find(ks);
@@ -570,16 +363,16 @@ extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* co
             for (int i = 0; i < 3; i++) cands.push_back({nullptr, g[i], 1});
             cands.push_back({nullptr, g[1], 2});
             // untimed first launch (attributes, instruction cache)
-            BCUDA(cudaMemsetAsync(t->d_queue, 0, sizeof(unsigned long long) * 2 * nkeys, st));
-            rc = batch_launch_key(t, k, part, cands[0], st);
+            BCUDA(cudaMemsetAsync(t->plan->d_queue, 0, sizeof(unsigned long long) * 2 * nkeys, st));
+            rc = jk_plan_launch(t->plan, k, part, cands[0], n_dm, t->nsm, st);
             if (rc) return rc;
             float best = -1.f;
             for (const JKBatchCfg& c : cands) {
                 float tmin = -1.f;
                 for (int rep = 0; rep < 1; rep++) {
-                    BCUDA(cudaMemsetAsync(t->d_queue, 0, sizeof(unsigned long long) * 2 * nkeys, st));
+                    BCUDA(cudaMemsetAsync(t->plan->d_queue, 0, sizeof(unsigned long long) * 2 * nkeys, st));
                     BCUDA(cudaEventRecord(e0, st));
-                    rc = batch_launch_key(t, k, part, c, st);
+                    rc = jk_plan_launch(t->plan, k, part, c, n_dm, t->nsm, st);
                     if (rc) return rc;
                     BCUDA(cudaEventRecord(e1, st));
                     BCUDA(cudaEventSynchronize(e1));
@@ -619,7 +412,7 @@ extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* co
 
 extern "C" int jk_batch_nsolo(const jk_batch_t* t, int* nsolo) {
     if (!t || !nsolo) return jk_internal_set_err(JK_ERR_ARG, "jk_batch_nsolo: invalid arguments");
-    *nsolo = (int)t->solo.size();
+    *nsolo = (int)t->plan->keys.size() - t->nmerged;
     return JK_OK;
 }
 
@@ -628,10 +421,10 @@ extern "C" int jk_batch_nsolo(const jk_batch_t* t, int* nsolo) {
 // not tuned); out holds 12 ints per key
 extern "C" int jk_batch_info(const jk_batch_t* t, int* nkeys, int* out) {
     if (!t || !nkeys) return jk_internal_set_err(JK_ERR_ARG, "jk_batch_info: invalid arguments");
-    *nkeys = (int)t->keys.size();
+    *nkeys = t->nmerged;
     if (!out) return JK_OK;
-    for (size_t k = 0; k < t->keys.size(); k++) {
-        const JKBatchKey& key = t->keys[k];
+    for (int k = 0; k < t->nmerged; k++) {
+        const JKPlanKey& key = t->plan->keys[k];
         int* o = out + 12 * k;
         o[0] = key.cls;
         o[1] = key.np_ij;

@@ -39,41 +39,82 @@
 // (cuobc/lib/gint/rys_roots.cu:1214-2176).
 //   n = 1:  w = F0(x), s = F1(x)/F0(x) from the Boys function itself
 //           (a Taylor series below x = 0.75, erf/exp above);
-//   n > 1:  the generated Chebyshev tables (uniform intervals of width 2 up
-//           to rys_xmax[n], Gauss-Hermite limit beyond), evaluated from a
-//           copy of the n-root table in shared memory.  Lanes of a warp
-//           read the intervals of their own x; the copy's interval stride is
-//           odd in doubles so that different intervals start in different
-//           banks.
+//   n > 1:  the generated tables (power series in t on uniform intervals of
+//           width 2 up to rys_xmax[n], Gauss-Hermite limit beyond), evaluated
+//           by Horner's rule from a copy of the n-root table in shared memory
+//           (the run kernels take n = 1 from its table too: one series of 14
+//           terms for all lanes instead of three branches of erf and exp).
+//           Lanes of a warp read the intervals of their own x, two
+//           coefficients per 16-byte load; the copy's interval stride is an
+//           odd number of 16-byte words, so that different intervals start in
+//           different banks.  Clenshaw's rule on the Chebyshev form, as
+//           before, took twice the FP64 operations and 8-byte loads.
 // ---------------------------------------------------------------------------
 template <int N>
 struct RysS {
     static constexpr int NS = 2 * N;                 // series per interval
-    static constexpr int STRIDE = NS * RYS_NC + 1;   // doubles per interval
+    static constexpr int STRIDE = NS * RYS_NC + 2;   // elements per interval
     static constexpr int NINT = rys_nint_c(N);
     static constexpr int HERM = NINT * STRIDE;       // Gauss-Hermite nodes, then weights
-    static constexpr int WORDS = N == 1 ? 0 : HERM + NS;  // doubles in shared memory
+    static constexpr int TWORDS = HERM + NS;         // the whole copy
+    static constexpr int WORDS = N == 1 ? 0 : TWORDS;  // without the n = 1 table
     static constexpr double XMAX = rys_xmax_c(N);
 };
 
 // block-cooperative copy of the n-root table into shared memory (layout
-// [interval][k][series], series f < N nodes, f >= N weights)
+// [interval][series][k], series f < N nodes, f >= N weights)
 template <int N>
-__device__ __forceinline__ void rys_table_to_smem(const double* __restrict__ g, double* __restrict__ tab) {
+__device__ __forceinline__ void rys_table_copy(const double* __restrict__ g, double* __restrict__ tab) {
     using S = RysS<N>;
-    if (N == 1) return;
     const double* src = g + rys_off_c(N);
     for (int e = threadIdx.x; e < S::NINT * S::NS * RYS_NC; e += blockDim.x) {
-        int m = e / (S::NS * RYS_NC);
-        int rem = e - m * (S::NS * RYS_NC);
-        int f = rem / RYS_NC, k = rem - f * RYS_NC;
-        tab[m * S::STRIDE + k * S::NS + f] = __ldg(src + e);
+        const int m = e / (S::NS * RYS_NC);
+        tab[e + 2 * m] = __ldg(src + e);
     }
     for (int r = threadIdx.x; r < N; r += blockDim.x) {
         tab[S::HERM + r] = rys_herm_r[N * (N - 1) / 2 + r];
         tab[S::HERM + N + r] = rys_herm_w[N * (N - 1) / 2 + r];
     }
 }
+template <int N>
+__device__ __forceinline__ void rys_table_to_smem(const double* __restrict__ g, double* __restrict__ tab) {
+    if (N > 1) rys_table_copy<N>(g, tab);
+}
+
+// sum_k c_k t^k of one series (16-byte aligned doubles in shared memory)
+__device__ __forceinline__ double rys_series(const double* __restrict__ c, double t) {
+    const double2* c2 = reinterpret_cast<const double2*>(c);
+    double2 p = c2[RYS_NC / 2 - 1];
+    double v = fma(p.y, t, p.x);
+#pragma unroll
+    for (int k = RYS_NC / 2 - 2; k >= 0; k--) {
+        p = c2[k];
+        v = fma(fma(v, t, p.y), t, p.x);
+    }
+    return v;
+}
+// the same from the global table (8-byte aligned)
+__device__ __forceinline__ double rys_series_g(const double* __restrict__ c, double t) {
+    double v = __ldg(c + RYS_NC - 1);
+#pragma unroll
+    for (int k = RYS_NC - 2; k >= 0; k--) v = fma(v, t, __ldg(c + k));
+    return v;
+}
+// the same in single precision (8-byte aligned); the terms from t^10 on are
+// below 1e-8 of the sum, under half a unit in the last place of a float
+#define RYS_NCF 10
+__device__ __forceinline__ float rys_series_f(const float* __restrict__ c, float t) {
+    const float2* c2 = reinterpret_cast<const float2*>(c);
+    float2 p = c2[RYS_NCF / 2 - 1];
+    float v = fmaf(p.y, t, p.x);
+#pragma unroll
+    for (int k = RYS_NCF / 2 - 2; k >= 0; k--) {
+        p = c2[k];
+        v = fmaf(fmaf(v, t, p.y), t, p.x);
+    }
+    return v;
+}
+static_assert(RYS_NC % 2 == 0, "the series are read in pairs of coefficients");
 
 // F0 and F1 of the Boys function
 __device__ __forceinline__ void boys01(double x, double& f0, double& f1) {
@@ -119,33 +160,42 @@ __device__ __forceinline__ void rys_root_rt(const double* __restrict__ rys, int 
     }
     if (x >= rys_xmax_c(N)) {
         const int b = N * (N - 1) / 2 + r;
-        const double rx = 1. / x;
-        s = rys_herm_r[b] * rx;
-        w = rys_herm_w[b] * sqrt(rx);
+        const double rx = rsqrt(x);
+        s = rys_herm_r[b] * (rx * rx);
+        w = rys_herm_w[b] * rx;
         return;
     }
     const int m = (int)(x * 0.5);
-    const double t = x - (2 * m + 1), tt = t + t;
+    const double t = x - (2 * m + 1);
     const double* c = rys + rys_off_c(N) + (size_t)(m * 2 * N) * RYS_NC;
-    const double* cs = c + r * RYS_NC;
-    const double* cw = c + (N + r) * RYS_NC;
-    double b1 = 0., b2 = 0., v1 = 0., v2 = 0.;
-    for (int k = RYS_NC - 1; k >= 1; k--) {
-        double b0 = fma(tt, b1, __ldg(cs + k) - b2);
-        b2 = b1;
-        b1 = b0;
-        b0 = fma(tt, v1, __ldg(cw + k) - v2);
-        v2 = v1;
-        v1 = b0;
-    }
-    s = fma(t, b1, __ldg(cs) - b2);
-    w = fma(t, v1, __ldg(cw) - v2);
+    s = rys_series_g(c + r * RYS_NC, t);
+    w = rys_series_g(c + (N + r) * RYS_NC, t);
 }
 
 // all N roots at x from the shared-memory table
 template <int N>
-__device__ __forceinline__ void rys_roots_all(const double* __restrict__ tab, double x, double* s, double* w) {
+__device__ __forceinline__ void rys_table_all(const double* __restrict__ tab, double x, double* s, double* w) {
     using S = RysS<N>;
+    if (x >= S::XMAX) {
+        const double rx = rsqrt(x), rx2 = rx * rx;
+#pragma unroll
+        for (int r = 0; r < N; r++) {
+            s[r] = tab[S::HERM + r] * rx2;
+            w[r] = tab[S::HERM + N + r] * rx;
+        }
+        return;
+    }
+    const int m = (int)(x * 0.5);
+    const double t = x - (2 * m + 1);
+    const double* c = tab + m * S::STRIDE;
+#pragma unroll
+    for (int r = 0; r < N; r++) {
+        s[r] = rys_series(c + r * RYS_NC, t);
+        w[r] = rys_series(c + (N + r) * RYS_NC, t);
+    }
+}
+template <int N>
+__device__ __forceinline__ void rys_roots_all(const double* __restrict__ tab, double x, double* s, double* w) {
     if (N == 1) {
         double f0, f1;
         boys01(x, f0, f1);
@@ -153,35 +203,7 @@ __device__ __forceinline__ void rys_roots_all(const double* __restrict__ tab, do
         s[0] = f1 / f0;
         return;
     }
-    if (x >= S::XMAX) {
-        double rx = 1. / x, srx = sqrt(rx);
-#pragma unroll
-        for (int r = 0; r < N; r++) {
-            s[r] = tab[S::HERM + r] * rx;
-            w[r] = tab[S::HERM + N + r] * srx;
-        }
-        return;
-    }
-    int m = (int)(x * 0.5);
-    double t = x - (2 * m + 1), t2 = t + t;
-    const double* c = tab + m * S::STRIDE;
-    double b1[S::NS], b2[S::NS];
-#pragma unroll
-    for (int f = 0; f < S::NS; f++) b1[f] = b2[f] = 0.;
-#pragma unroll
-    for (int k = RYS_NC - 1; k >= 1; k--) {
-#pragma unroll
-        for (int f = 0; f < S::NS; f++) {
-            double b0 = fma(t2, b1[f], c[k * S::NS + f] - b2[f]);
-            b2[f] = b1[f];
-            b1[f] = b0;
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < N; r++) {
-        s[r] = fma(t, b1[r], c[r] - b2[r]);
-        w[r] = fma(t, b1[N + r], c[N + r] - b2[N + r]);
-    }
+    rys_table_all<N>(tab, x, s, w);
 }
 
 // root r only (runtime r) from the shared-memory table
@@ -196,26 +218,16 @@ __device__ __forceinline__ void rys_root_one(const double* __restrict__ tab, dou
         return;
     }
     if (x >= S::XMAX) {
-        double rx = 1. / x;
-        s = tab[S::HERM + r] * rx;
-        w = tab[S::HERM + N + r] * sqrt(rx);
+        const double rx = rsqrt(x);
+        s = tab[S::HERM + r] * (rx * rx);
+        w = tab[S::HERM + N + r] * rx;
         return;
     }
-    int m = (int)(x * 0.5);
-    double t = x - (2 * m + 1), t2 = t + t;
+    const int m = (int)(x * 0.5);
+    const double t = x - (2 * m + 1);
     const double* c = tab + m * S::STRIDE;
-    double bs1 = 0., bs2 = 0., bw1 = 0., bw2 = 0.;
-#pragma unroll
-    for (int k = RYS_NC - 1; k >= 1; k--) {
-        double b0 = fma(t2, bs1, c[k * S::NS + r] - bs2);
-        bs2 = bs1;
-        bs1 = b0;
-        b0 = fma(t2, bw1, c[k * S::NS + N + r] - bw2);
-        bw2 = bw1;
-        bw1 = b0;
-    }
-    s = fma(t, bs1, c[r] - bs2);
-    w = fma(t, bw1, c[N + r] - bw2);
+    s = rys_series(c + r * RYS_NC, t);
+    w = rys_series(c + (N + r) * RYS_NC, t);
 }
 
 // root r straight from the global table (setup kernels)
@@ -230,55 +242,53 @@ __device__ __forceinline__ void rys_root(const double* __restrict__ rys_coef, do
         return;
     }
     if (x >= rys_xmax_c(N)) {
-        int b = N * (N - 1) / 2 + r;
-        double rx = 1. / x;
-        s = rys_herm_r[b] * rx;
-        w = rys_herm_w[b] * sqrt(rx);
+        const int b = N * (N - 1) / 2 + r;
+        const double rx = rsqrt(x);
+        s = rys_herm_r[b] * (rx * rx);
+        w = rys_herm_w[b] * rx;
         return;
     }
-    int m = (int)(x * 0.5);
-    double t = x - (2 * m + 1);
+    const int m = (int)(x * 0.5);
+    const double t = x - (2 * m + 1);
     const double* c = rys_coef + rys_off_c(N) + (m * 2 * N) * RYS_NC;
-    double b1 = 0., b2 = 0., v1 = 0., v2 = 0., tt = t + t;
-    const double* cs = c + r * RYS_NC;
-    const double* cw = c + (N + r) * RYS_NC;
-#pragma unroll
-    for (int k = RYS_NC - 1; k >= 1; k--) {
-        double b0 = fma(tt, b1, __ldg(cs + k) - b2);
-        b2 = b1;
-        b1 = b0;
-        b0 = fma(tt, v1, __ldg(cw + k) - v2);
-        v2 = v1;
-        v1 = b0;
-    }
-    s = fma(t, b1, __ldg(cs) - b2);
-    w = fma(t, v1, __ldg(cw) - v2);
+    s = rys_series_g(c + r * RYS_NC, t);
+    w = rys_series_g(c + (N + r) * RYS_NC, t);
 }
 
 // ---------------------------------------------------------------------------
 // Single-precision nodes and weights for the FP32 quartets of the mixed mode
 // at low order (n <= JK_F32_ROOTS): the Boys function in float for n = 1, the
-// same Chebyshev tables rounded to float for n = 2, 3.  Higher orders keep
-// the double evaluation above.  Same shared-memory layout as the double copy
-// (the stride is odd in floats too).
+// same tables rounded to float for n = 2, 3.  Higher orders keep the double
+// evaluation above.
 // ---------------------------------------------------------------------------
 #define JK_F32_ROOTS 3
 
 template <int N>
-__device__ __forceinline__ void rys_table_to_smem_f(const double* __restrict__ g, float* __restrict__ tab) {
-    using S = RysS<N>;
-    if (N == 1) return;
+struct RysF {
+    static constexpr int NS = 2 * N;
+    static constexpr int STRIDE = NS * RYS_NCF + 2;  // floats per interval, an odd number of 8-byte words
+    static constexpr int NINT = rys_nint_c(N);
+    static constexpr int HERM = NINT * STRIDE;
+    static constexpr int WORDS = HERM + NS;
+    static_assert((STRIDE / 2) % 2 == 1, "intervals start in different banks");
+};
+
+template <int N>
+__device__ __forceinline__ void rys_table_copy_f(const double* __restrict__ g, float* __restrict__ tab) {
+    using S = RysF<N>;
     const double* src = g + rys_off_c(N);
-    for (int e = threadIdx.x; e < S::NINT * S::NS * RYS_NC; e += blockDim.x) {
-        int m = e / (S::NS * RYS_NC);
-        int rem = e - m * (S::NS * RYS_NC);
-        int f = rem / RYS_NC, k = rem - f * RYS_NC;
-        tab[m * S::STRIDE + k * S::NS + f] = (float)__ldg(src + e);
+    for (int e = threadIdx.x; e < S::NINT * S::NS * RYS_NCF; e += blockDim.x) {
+        const int f = e / RYS_NCF, m = f / S::NS;
+        tab[e + 2 * m] = (float)__ldg(src + (size_t)f * RYS_NC + (e - f * RYS_NCF));
     }
     for (int r = threadIdx.x; r < N; r += blockDim.x) {
         tab[S::HERM + r] = (float)rys_herm_r[N * (N - 1) / 2 + r];
         tab[S::HERM + N + r] = (float)rys_herm_w[N * (N - 1) / 2 + r];
     }
+}
+template <int N>
+__device__ __forceinline__ void rys_table_to_smem_f(const double* __restrict__ g, float* __restrict__ tab) {
+    if (N > 1) rys_table_copy_f<N>(g, tab);
 }
 
 // F0 and F1 in float: the series below x = 0.75 (12 terms, truncation below
@@ -309,17 +319,10 @@ __device__ __forceinline__ void boys01_f(float x, float& f0, float& f1) {
 }
 
 template <int N>
-__device__ __forceinline__ void rys_roots_all_f(const float* __restrict__ tab, float x, float* s, float* w) {
-    using S = RysS<N>;
-    if (N == 1) {
-        float f0, f1;
-        boys01_f(x, f0, f1);
-        w[0] = f0;
-        s[0] = __fdividef(f1, f0);
-        return;
-    }
-    if (x >= (float)S::XMAX) {
-        float srx = rsqrtf(x), rx = srx * srx;
+__device__ __forceinline__ void rys_table_all_f(const float* __restrict__ tab, float x, float* s, float* w) {
+    using S = RysF<N>;
+    if (x >= (float)RysS<N>::XMAX) {
+        const float srx = rsqrtf(x), rx = srx * srx;
 #pragma unroll
         for (int r = 0; r < N; r++) {
             s[r] = tab[S::HERM + r] * rx;
@@ -327,32 +330,31 @@ __device__ __forceinline__ void rys_roots_all_f(const float* __restrict__ tab, f
         }
         return;
     }
-    int m = (int)(x * 0.5f);
-    float t = x - (float)(2 * m + 1), t2 = t + t;
+    const int m = (int)(x * 0.5f);
+    const float t = x - (float)(2 * m + 1);
     const float* c = tab + m * S::STRIDE;
-    float b1[S::NS], b2[S::NS];
-#pragma unroll
-    for (int f = 0; f < S::NS; f++) b1[f] = b2[f] = 0.f;
-#pragma unroll
-    for (int k = RYS_NC - 1; k >= 1; k--) {
-#pragma unroll
-        for (int f = 0; f < S::NS; f++) {
-            float b0 = fmaf(t2, b1[f], c[k * S::NS + f] - b2[f]);
-            b2[f] = b1[f];
-            b1[f] = b0;
-        }
-    }
 #pragma unroll
     for (int r = 0; r < N; r++) {
-        s[r] = fmaf(t, b1[r], c[r] - b2[r]);
-        w[r] = fmaf(t, b1[N + r], c[N + r] - b2[N + r]);
+        s[r] = rys_series_f(c + r * RYS_NCF, t);
+        w[r] = rys_series_f(c + (N + r) * RYS_NCF, t);
     }
+}
+template <int N>
+__device__ __forceinline__ void rys_roots_all_f(const float* __restrict__ tab, float x, float* s, float* w) {
+    if (N == 1) {
+        float f0, f1;
+        boys01_f(x, f0, f1);
+        w[0] = f0;
+        s[0] = __fdividef(f1, f0);
+        return;
+    }
+    rys_table_all_f<N>(tab, x, s, w);
 }
 
 // root r only (runtime r), single precision, from the float table copy
 template <int N>
 __device__ __forceinline__ void rys_root_one_f(const float* __restrict__ tab, float x, int r, float& s, float& w) {
-    using S = RysS<N>;
+    using S = RysF<N>;
     if (N == 1) {
         float f0, f1;
         boys01_f(x, f0, f1);
@@ -360,27 +362,17 @@ __device__ __forceinline__ void rys_root_one_f(const float* __restrict__ tab, fl
         s = __fdividef(f1, f0);
         return;
     }
-    if (x >= (float)S::XMAX) {
+    if (x >= (float)RysS<N>::XMAX) {
         const float srx = rsqrtf(x);
         s = tab[S::HERM + r] * srx * srx;
         w = tab[S::HERM + N + r] * srx;
         return;
     }
     const int m = (int)(x * 0.5f);
-    const float t = x - (float)(2 * m + 1), t2 = t + t;
+    const float t = x - (float)(2 * m + 1);
     const float* c = tab + m * S::STRIDE;
-    float bs1 = 0.f, bs2 = 0.f, bw1 = 0.f, bw2 = 0.f;
-#pragma unroll
-    for (int k = RYS_NC - 1; k >= 1; k--) {
-        float b0 = fmaf(t2, bs1, c[k * S::NS + r] - bs2);
-        bs2 = bs1;
-        bs1 = b0;
-        b0 = fmaf(t2, bw1, c[k * S::NS + N + r] - bw2);
-        bw2 = bw1;
-        bw1 = b0;
-    }
-    s = fmaf(t, bs1, c[r] - bs2);
-    w = fmaf(t, bw1, c[N + r] - bw2);
+    s = rys_series_f(c + r * RYS_NCF, t);
+    w = rys_series_f(c + (N + r) * RYS_NCF, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -425,6 +417,12 @@ struct JKClass {
     static constexpr int P = THREAD ? 0 : ((NF / NFI <= 64) ? 1 : 2);
     static constexpr int T = P == 0 ? 1 : (P == 1 ? NFI : NFI * NFJ);
     static constexpr int NACC = NF / T;
+    // team classes whose team (one lane per bra component i) lies in a warp
+    // and walks runs of bra pairs (jk_teams.cuh); the others (P = 2, or many
+    // ket components) take a quartet at a time
+    static constexpr bool TRUN = P == 1 && NFK * NFL <= 18;
+    static constexpr int TPW = P == 0 ? 32 : (TRUN ? 32 / T : 1);  // ket pairs a warp works on at once
+    static constexpr bool RUNS = P == 0 || TRUN;
     // resident 128-thread blocks asked of the register allocator (thread kernel)
     static constexpr int MINB = W <= 24 ? 4 : (W <= 40 ? 3 : 2);
 };
@@ -440,7 +438,9 @@ struct JKClass {
 // register arrays.  Output: I[i*XSI + j*XSJ + k*(LL+1) + l], by default the
 // packed layout I[((i*(LJ+1)+j)*(LK+1)+k)*(LL+1)+l].
 // ---------------------------------------------------------------------------
-template <typename R, class C, int XSI = C::SI, int XSJ = C::SJ, typename OutT>
+// KET = false stops after the bra transfer: I[i*XSI + j*XSJ + m], m up to
+// LK + LL (the reader does the ket transfer in registers).
+template <typename R, class C, int XSI = C::SI, int XSJ = C::SJ, bool KET = true, typename OutT>
 __device__ __forceinline__ void rys_2d(R seed, R c00, R c0p, R b10, R b01, R b00, R dij, R dkl,
                                        OutT* __restrict__ I) {
     constexpr int NM = C::NM, MM = C::MM;
@@ -458,6 +458,23 @@ __device__ __forceinline__ void rys_2d(R seed, R c00, R c0p, R b10, R b01, R b00
             G[n][m + 1] = v;
         }
     }
+    if constexpr (!KET) {
+#pragma unroll
+        for (int m = 0; m <= MM; m++) {
+            R A[NM + 1];
+#pragma unroll
+            for (int a = 0; a <= NM; a++) A[a] = G[a][m];
+#pragma unroll
+            for (int i = 0; i <= C::LI; i++) I[i * XSI + m] = A[i];
+#pragma unroll
+            for (int j = 1; j <= C::LJ; j++) {
+#pragma unroll
+                for (int a = 0; a + j <= NM; a++) A[a] = A[a + 1] + dij * A[a];
+#pragma unroll
+                for (int i = 0; i <= C::LI; i++) I[i * XSI + j * XSJ + m] = A[i];
+            }
+        }
+    } else {
     // bra transfer: H[i][j][m]
     R H[C::LI + 1][C::LJ + 1][MM + 1];
 #pragma unroll
@@ -493,18 +510,30 @@ __device__ __forceinline__ void rys_2d(R seed, R c00, R c0p, R b10, R b01, R b00
                 for (int k = 0; k <= C::LK; k++) I[i * XSI + j * XSJ + k * C::SK + l] = B[k];
             }
         }
+    }
 }
 
 // ---------------------------------------------------------------------------
-// Segment: one (molecule, class quartet) piece of work.  Tasks of a segment
-// are the screened contracted shell quartets (ij, kl), enumerated row by row:
-// row ij holds kl = 0 .. nkl(ij)-1 and qoff is the exclusive prefix of nkl.
+// Segment: one (molecule, class quartet) piece of work.  For the team and
+// generic kernels its tasks are the screened contracted shell quartets
+// (ij, kl), enumerated row by row: row ij holds kl = 0 .. nkl(ij)-1 and qoff
+// is the exclusive prefix of nkl.  For the run kernels (jk_runs.cuh) its
+// items are (run of bra pairs, chunk of 32 ket pairs), with the prefix ioff
+// over the runs.
 // ---------------------------------------------------------------------------
 struct JKSeg {
     const double* rys;      // Rys coefficient table (device)
     const long long* qoff;  // n_ij + 1 entries (device)
     const int* kl_base;     // first kl column of each row (FP32 part of the mixed mode), or null
     int n_ij;
+    // run kernels: entry e of the bra class is pair ent[e] (an index in the
+    // class), run r holds the entries run0[r] .. run0[r+1] (one shell i, at
+    // most 32 entries) and ioff[r+1] - ioff[r] items; entry e keeps the kets
+    // elo[e] .. ehi[e] (elo null: from 0)
+    int nrun;
+    const int *ent, *run0;
+    const int *elo, *ehi;
+    const long long* ioff;
     int pair_ij0, pair_kl0;  // first pair of each class in the pair arrays
     int prim_ij0, prim_kl0;  // first primitive pair of each class
     int nprim_ij, nprim_kl;
@@ -513,8 +542,6 @@ struct JKSeg {
     // lanes of a warp (consecutive kl pairs) load them coalesced
     int pst_ij, pst_kl;
     int nao, n_dm;
-    const int* pair2bra;
-    const int* pair2ket;
     const double* a12;
     const double* ia12;  // 1 / a12
     const double* e12;
@@ -533,43 +560,48 @@ struct JKSeg {
     const int* pao;
     int npt;
     // per pair: its leading primitive pairs that pass the exponent cutoff
-    // (the thread kernels loop over those only), or null
+    // (the run kernels loop over those only), or null
     const int* pnp;
-    const double* bas_x;  // shell centres, SoA x[nbas], y[nbas], z[nbas]
-    int nbas;
-    const int* ao_loc;
+    // run kernels, bra pairs in run-entry order (entry e of the class): one
+    // 64-byte record per entry and primitive at bprim + 8 (k * pst_ij + e)
+    // (a12 | 1/a12 | e12/a12 | P x y z | -), its single-precision twin
+    // (a12 | 1/a12 | e12/a12 | P - R_bra | -), and per entry the second
+    // shell's centre, first AO and primitive count (4 doubles)
+    const double* bprim;
+    const float* bprimf;
+    const double* bpair;
     const double* dm;
     double* vj;
     double* vk;
-    // Pair-packed J side (jk_build): the density blocks of the pairs of the
-    // two classes, component-major (element c of pair p of a class at
-    // c * np + p), and accumulators of the same layout for the J
-    // contributions, added to vj after the launches.  Null: the kernels
-    // gather D and add J straight into vj.
-    const double* dp_ij;
-    const double* dp_kl;
-    double* jp_ij;
-    double* jp_kl;
-    int np_ij, np_kl;        // pairs of each class (component stride)
+    // Pair-packed J side (builds of all class quartets): the density blocks
+    // of the pairs, component-major within a class (element c of pair p of
+    // the bra class at pk_ij + c * pst_ij + p), and accumulators of the same
+    // layout for the J contributions, added to vj after the launches.  Null:
+    // the kernels gather D and add J straight into vj.
+    // The run kernels keep the bra side of both per entry (dpb, jpb: element
+    // pk_ij + e * components + c), contiguous for the warp that works on e.
+    const double* dp;
+    double* jp;
+    const double* dpb;
+    double* jpb;
+    long long pk_ij, pk_kl;  // first packed element of each class
     long long pk_stride;     // packed elements per density
     int ls[4];               // angular momenta of the class (read by the generic kernel)
 };
 
-// launchers of one class: a single segment (by value) or a segment table
-typedef cudaError_t (*jk_launch_fn)(const JKSeg& seg, const long long* task0, long long max_tasks, int nsm,
-                                    cudaStream_t st);
-// Launch shape of one batched class launch (the knobs of the batch's
-// autotuner).  queue == nullptr: the tasks are split into equal contiguous
-// chunks over a grid sized by the unscreened task count.  Otherwise the
-// persistent mode: the grid is grid_mul x the kernel's resident blocks per
-// SM x the SMs, and the warps (thread kernels), teams (team kernels) or
-// blocks (generic kernel) take `grab` tasks at a time from the device
-// counter *queue, which the caller zeroes before the launch.
+// Launch shape of one class launch (the knobs of the batch's autotuner).
+// queue == nullptr: run kernels take items in turn over the grid, the others
+// split their tasks into equal contiguous chunks.  Otherwise the persistent
+// mode: the grid is grid_mul x the kernel's resident blocks per SM x the SMs,
+// and the warps (run kernels), teams (team kernels) or blocks (generic
+// kernel) take `grab` tasks at a time from the device counter *queue, which
+// the caller zeroes before the launch.
 struct JKBatchCfg {
     unsigned long long* queue;
     int grab;
     int grid_mul;
 };
-typedef cudaError_t (*jk_launch_batch_fn)(const JKSeg* segs, const long long* segt, int nseg, long long max_tasks,
-                                          int nsm, const JKBatchCfg& cfg, cudaStream_t st);
-
+// launcher of one class: a segment table with its task (or item) prefix;
+// max_tasks bounds the prefix's total
+typedef cudaError_t (*jk_launch_fn)(const JKSeg* segs, const long long* segt, int nseg, long long max_tasks, int n_dm,
+                                    int nsm, const JKBatchCfg& cfg, cudaStream_t st);

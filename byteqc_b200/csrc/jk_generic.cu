@@ -266,14 +266,7 @@ __device__ void jk_generic_body(const Src& src) {
 }
 
 template <int GL>
-__global__ void __launch_bounds__(JK_GEN_THREADS) jk_generic_kernel(const __grid_constant__ JKSeg sg,
-                                                                    const long long* __restrict__ task0) {
-    JKOneSeg src{sg, task0};
-    jk_generic_body<GL>(src);
-}
-
-template <int GL>
-__global__ void __launch_bounds__(JK_GEN_THREADS) jk_generic_kernel_batch(const JKSeg* __restrict__ segs,
+__global__ void __launch_bounds__(JK_GEN_THREADS) jk_generic_kernel(const JKSeg* __restrict__ segs,
                                                                           const long long* __restrict__ segt,
                                                                           int nseg, unsigned long long* queue,
                                                                           int grab) {
@@ -288,25 +281,14 @@ static int jk_generic_blocks(long long max_tasks, int nsm) {
 }
 
 template <int GL>
-static cudaError_t jk_launch_generic(const JKSeg& seg, const long long* task0, long long max_tasks, int nsm,
-                                     cudaStream_t st) {
-    if (max_tasks <= 0) return cudaSuccess;
-    static std::atomic<unsigned long long> attr_done{0};
-    if (cudaError_t e = jk_smem_attr(jk_generic_kernel<GL>, JKGen<GL>::SMEM, attr_done); e != cudaSuccess) return e;
-    jk_generic_kernel<GL><<<jk_generic_blocks<GL>(max_tasks, nsm), JK_GEN_THREADS, JKGen<GL>::SMEM, st>>>(seg,
-                                                                                                         task0);
-    return cudaGetLastError();
-}
-
-template <int GL>
-static cudaError_t jk_launch_generic_batch(const JKSeg* segs, const long long* segt, int nseg, long long max_tasks,
-                                           int nsm, const JKBatchCfg& cfg, cudaStream_t st) {
+static cudaError_t jk_launch_generic(const JKSeg* segs, const long long* segt, int nseg, long long max_tasks,
+                                     int n_dm, int nsm, const JKBatchCfg& cfg, cudaStream_t st) {
     if (max_tasks <= 0 || nseg <= 0) return cudaSuccess;
     static std::atomic<unsigned long long> attr_done{0};
-    if (cudaError_t e = jk_smem_attr(jk_generic_kernel_batch<GL>, JKGen<GL>::SMEM, attr_done); e != cudaSuccess)
+    if (cudaError_t e = jk_smem_attr(jk_generic_kernel<GL>, JKGen<GL>::SMEM, attr_done); e != cudaSuccess)
         return e;
     const int blocks = cfg.queue ? nsm * JKGen<GL>::CTAS * cfg.grid_mul : jk_generic_blocks<GL>(max_tasks, nsm);
-    jk_generic_kernel_batch<GL><<<blocks, JK_GEN_THREADS, JKGen<GL>::SMEM, st>>>(segs, segt, nseg, cfg.queue,
+    jk_generic_kernel<GL><<<blocks, JK_GEN_THREADS, JKGen<GL>::SMEM, st>>>(segs, segt, nseg, cfg.queue,
                                                                                 cfg.grab);
     return cudaGetLastError();
 }
@@ -461,7 +443,6 @@ void jk_register_generic(JKTables* T) {
                     const int c = JK_CLASS_INDEX(li, lj, lk, ll);
                     const bool six = li == 6 || lk == 6;  // li >= lj, lk >= ll
                     T->t64[c] = T->t32[c] = six ? jk_launch_generic<6> : jk_launch_generic<5>;
-                    T->b64[c] = T->b32[c] = six ? jk_launch_generic_batch<6> : jk_launch_generic_batch<5>;
                 }
 }
 

@@ -17,6 +17,8 @@
 #include "jk_launch.cuh"
 #include "jk_internal.h"
 
+static int class_index(const jk_basis* b, int cp_ij, int cp_kl);
+
 // primitive-pair screen of the thread kernels: exp(-mu r^2) below exp(-60)
 // (the default exponent cutoff of libcint's pair data) contributes nothing
 #define JK_PRIM_EXPCUT 60.0
@@ -167,30 +169,47 @@ static qcond_fn g_qcond[4][4] = {
 // per-call kernels: density condensation and quartet screening
 // ---------------------------------------------------------------------------
 // dm_cond[gi, gj] = max over the dms of max |D[p, q]|, p in group gi, q in gj
-// (lib.condense('absmax') over the group AO boundaries, cuobc/scf/hf.py:104-107)
-__global__ void jk_dm_cond_kernel(const double* __restrict__ dm, int nao, int n_dm, const int* __restrict__ gao,
-                                  int ngroups, double* __restrict__ out) {
-    int gi = blockIdx.x, gj = blockIdx.y;
-    int p0 = gao[gi], p1 = gao[gi + 1], q0 = gao[gj], q1 = gao[gj + 1];
-    int np = p1 - p0, nq = q1 - q0;
-    double mx = 0;
-    long long n = (long long)np * nq * n_dm;
-    for (long long e = threadIdx.x; e < n; e += blockDim.x) {
-        int idm = (int)(e / ((long long)np * nq));
-        int rem = (int)(e - (long long)idm * np * nq);
-        int p = p0 + rem / nq, qq = q0 + rem % nq;
-        mx = fmax(mx, fabs(dm[(size_t)idm * nao * nao + (size_t)p * nao + qq]));
-    }
-    __shared__ double red[256];
-    red[threadIdx.x] = mx;
+// (lib.condense('absmax') over the group AO boundaries, cuobc/scf/hf.py:104-107),
+// of one molecule (one) or many (tab, blockIdx.z).  A warp per row of D, the
+// rows of a group spread over gridDim.x blocks that meet in an atomic maximum
+// of the bit patterns (ordered as the non-negative values): one block per
+// group pair, as this kernel had, took 3.2 ms of the 220 ms build of (H2O)64 /
+// cc-pVDZ (5248 functions in 3 groups).  out starts at zero.
+#define JK_DMC_GROUPS 256
+__global__ void __launch_bounds__(256) jk_dm_cond_kernel(const JKDmCond one, const JKDmCond* __restrict__ tab) {
+    const JKDmCond m = tab ? tab[blockIdx.z] : one;
+    const int gi = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (gi >= m.ngroups) return;
+    __shared__ unsigned long long smax[JK_DMC_GROUPS];
+    const bool sh = m.ngroups <= JK_DMC_GROUPS;
+    unsigned long long* gout = reinterpret_cast<unsigned long long*>(m.out) + (size_t)gi * m.ngroups;
+    if (sh)
+        for (int g = threadIdx.x; g < m.ngroups; g += blockDim.x) smax[g] = 0;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-        __syncthreads();
+    const int p0 = m.gao[gi], np = m.gao[gi + 1] - p0;
+    const long long rows = (long long)np * m.n_dm;
+    for (long long r = (long long)blockIdx.x * 8 + warp; r < rows; r += (long long)gridDim.x * 8) {
+        const int idm = (int)(r / np), p = p0 + (int)(r - (long long)idm * np);
+        const double* row = m.dm + ((size_t)idm * m.nao + p) * m.nao;
+        for (int g = 0; g < m.ngroups; g++) {
+            double mx = 0;
+            for (int q = m.gao[g] + lane; q < m.gao[g + 1]; q += 32) mx = fmax(mx, fabs(row[q]));
+            for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            if (lane == 0)
+                atomicMax(sh ? smax + g : gout + g, (unsigned long long)__double_as_longlong(mx));
+        }
     }
-    if (threadIdx.x == 0) out[gi * ngroups + gj] = red[0];
+    if (!sh) return;
+    __syncthreads();
+    for (int g = threadIdx.x; g < m.ngroups; g += blockDim.x)
+        if (smax[g]) atomicMax(gout + g, smax[g]);
 }
 
+// clears every molecule's counters and condensed density (blockIdx.x = molecule)
+__global__ void jk_zero_kernel(const JKDmCond* __restrict__ tab) {
+    const JKDmCond m = tab[blockIdx.x];
+    for (int e = threadIdx.x; e < m.nzero; e += blockDim.x) m.zero[e] = 0;
+}
 
 // Block-wide inclusive scan of two counts (256 threads), with running carries.
 __device__ __forceinline__ void jk_block_scan2(long long a, long long b, long long& ia, long long& ib,
@@ -239,80 +258,89 @@ __device__ __forceinline__ double jk_cq_sub(const double* c, int ngroups, int gi
                 fmax(c[gi * ngroups + gl], c[gj * ngroups + gl]));
 }
 
-// One block (256 threads) per class quartet.  Reproduces the reference's
-// screening decision per contracted quartet (cuobc/scf/hf.py:136-145,
-// 567-578 and cuobc/lib/gvhf/nr_jk_driver.cu:252-280):
+// Screening of one class quartet, with the reference's decision per
+// contracted quartet (cuobc/scf/hf.py:136-145, 567-578 and
+// cuobc/lib/gvhf/nr_jk_driver.cu:252-280):
 //   skip the class quartet if prescreen and max(dm_cond over its 6 group
 //   pairs) < tol; else with scale = nbins / log(min(tol/sub, 0.1)) and
 //   s = floor(scale * log_q), keep (ij, kl) iff s_ij + s_kl < nbins (and
 //   kl <= ij inside a diagonal class quartet).
 // Because log_q is sorted descending inside a class, the kept kl of a row
-// form a prefix; its length is found by binary search and prefix-summed.
-// Mixed precision (fp32_cutoff > 0): the kept prefix of a row splits again
-// at the bound q_ij q_kl sub = fp32_cutoff (unclipped log q); the leading
-// part (larger bounds) runs in FP64, the tail in FP32.  qoff counts the FP64
-// part, qoff32 the FP32 part, whose first column per row is klb[ij].
+// form a prefix; its length is found by binary search.  Mixed precision
+// (fp32_cutoff > 0): the kept prefix of a row splits again at the bound
+// q_ij q_kl sub = fp32_cutoff (unclipped log q); the leading part (larger
+// bounds) runs in FP64, the tail in FP32.
+struct JKScreen {
+    bool skip, mixed, diag;
+    double scale, log_thr;
+    int nbins;
+    __device__ __forceinline__ JKScreen(const JKScreenCQ& cq, double tol, int nb, int prescreen, double fp32_cutoff) {
+        const double sub = jk_cq_sub(cq.dm_cond, cq.ngroups, cq.gi, cq.gj, cq.gk, cq.gl);
+        skip = prescreen && sub < tol;
+        nbins = nb;
+        scale = nb / log(fmin(tol / sub, 0.1));
+        mixed = fp32_cutoff > 0;
+        log_thr = mixed ? log(fp32_cutoff / sub) : 0.;  // q_ij q_kl >= fp32_cutoff / sub
+        diag = cq.cp_ij == cq.cp_kl;
+    }
+    // kept kets of row ij: [0, c64) in FP64, [c64, cnt) in FP32
+    __device__ __forceinline__ void row(const JKScreenCQ& cq, int ij, int& c64, int& cnt) const {
+        c64 = cnt = 0;
+        if (skip) return;
+        const int sij = (int)floor(scale * cq.lq_ij[ij]);
+        if (sij >= nbins) return;
+        const int b = nbins - sij;
+        // count kl with floor(scale * lq_kl) < b (non-decreasing in kl)
+        int lo = 0, hi = cq.n_kl;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if ((int)floor(scale * cq.lq_kl[mid]) < b) lo = mid + 1; else hi = mid;
+        }
+        cnt = lo;
+        if (diag && cnt > ij + 1) cnt = ij + 1;
+        c64 = cnt;
+        if (mixed && cnt > 0) {
+            // kl with rq_ij + rq_kl >= log_thr (non-increasing in kl)
+            const double need = log_thr - cq.rq_ij[ij];
+            lo = 0;
+            hi = cnt;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (cq.rq_kl[mid] >= need) lo = mid + 1; else hi = mid;
+            }
+            c64 = lo;
+        }
+    }
+};
+
+// Row classes (team and generic kernels): one block (256 threads) per class
+// quartet.  qoff counts the FP64 part, qoff32 the FP32 part, whose first
+// column per row is klb[ij].
 __global__ void jk_screen_kernel(const JKScreenCQ* __restrict__ cqs, double tol, int nbins, int prescreen,
                                  double fp32_cutoff) {
     const JKScreenCQ cq = cqs[blockIdx.x];
-    long long* qoff = cq.qoff;
-    long long* qoff32 = cq.qoff32;
-    int* klb = cq.klb;
-    const double* c = cq.dm_cond;
-    const int ngroups = cq.ngroups;
-    const double sub = jk_cq_sub(c, ngroups, cq.gi, cq.gj, cq.gk, cq.gl);
-    bool skip = prescreen && sub < tol;
-    double cutoff = tol / sub;
-    double scale = nbins / log(fmin(cutoff, 0.1));
-    const bool mixed = fp32_cutoff > 0;
-    const double log_thr = mixed ? log(fp32_cutoff / sub) : 0.;  // q_ij q_kl >= fp32_cutoff / sub
-    const double* lq_ij = cq.lq_ij;
-    const double* lq_kl = cq.lq_kl;
-    const double* rq_ij = cq.rq_ij;
-    const double* rq_kl = cq.rq_kl;
-    bool diag = cq.cp_ij == cq.cp_kl;
+    if (cq.runs) return;
+    const JKScreen sc(cq, tol, nbins, prescreen, fp32_cutoff);
     __shared__ long long carry, carry32;
     __shared__ long long wsum[32], wsum32[32];
     if (threadIdx.x == 0) {
         carry = carry32 = 0;
-        qoff[0] = 0;
-        qoff32[0] = 0;
+        cq.qoff[0] = 0;
+        cq.qoff32[0] = 0;
     }
     __syncthreads();
     for (int base = 0; base < cq.n_ij; base += blockDim.x) {
-        int ij = base + threadIdx.x;
-        long long cnt = 0, c64 = 0;
-        if (!skip && ij < cq.n_ij) {
-            int sij = (int)floor(scale * lq_ij[ij]);
-            if (sij < nbins) {
-                int b = nbins - sij;
-                // count kl with floor(scale * lq_kl) < b (non-decreasing in kl)
-                int lo = 0, hi = cq.n_kl;
-                while (lo < hi) {
-                    int mid = (lo + hi) >> 1;
-                    if ((int)floor(scale * lq_kl[mid]) < b) lo = mid + 1; else hi = mid;
-                }
-                cnt = lo;
-                if (diag && cnt > ij + 1) cnt = ij + 1;
-            }
+        const int ij = base + threadIdx.x;
+        int cnt = 0, c64 = 0;
+        if (ij < cq.n_ij) {
+            sc.row(cq, ij, c64, cnt);
+            cq.klb[ij] = c64;
         }
-        c64 = cnt;
-        if (mixed && cnt > 0) {
-            // kl with rq_ij + rq_kl >= log_thr (non-increasing in kl)
-            double need = log_thr - rq_ij[ij];
-            int lo = 0, hi = (int)cnt;
-            while (lo < hi) {
-                int mid = (lo + hi) >> 1;
-                if (rq_kl[mid] >= need) lo = mid + 1; else hi = mid;
-            }
-            c64 = lo;
-        }
-        if (ij < cq.n_ij) klb[ij] = (int)c64;
         long long i64, i32;
         jk_block_scan2(c64, cnt - c64, i64, i32, wsum, wsum32, carry, carry32);
         if (ij < cq.n_ij) {
-            qoff[ij + 1] = i64;
-            qoff32[ij + 1] = i32;
+            cq.qoff[ij + 1] = i64;
+            cq.qoff32[ij + 1] = i32;
         }
     }
     if (threadIdx.x == 0) {
@@ -323,50 +351,190 @@ __global__ void jk_screen_kernel(const JKScreenCQ* __restrict__ cqs, double tol,
     }
 }
 
-// Pair-packed J side of jk_build.  mode 0: gather the density blocks of
-// every pair into dp (element c of pair p of class k at off_k + c*np_k + p,
-// one copy per density); mode 1: add the packed J accumulators jp into vj.
-// Every (pair, component) is a distinct element of D and of vj.
-__device__ __forceinline__ void jk_pack_body(const JKPackCls* __restrict__ cls, int ncls, long long total,
-                                             const int* __restrict__ pair2bra, const int* __restrict__ pair2ket,
-                                             const int* __restrict__ ao_loc, const double* __restrict__ dm, int nao,
-                                             int n_dm, double* __restrict__ dp, const double* __restrict__ jp,
-                                             double* __restrict__ vj, int mode) {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        int lo = 0, hi = ncls - 1;
-        while (lo < hi) {
-            int mid = (lo + hi + 1) >> 1;
-            if (cls[mid].off <= t) lo = mid; else hi = mid - 1;
+// Run classes: a warp per run (blockIdx.x = class quartet), a lane per entry.
+// Writes the entries' bounds, adds up the quartet counts and leaves the
+// items of each run in ioff / ioff32 (made a prefix by jk_run_scan_kernel).
+__global__ void __launch_bounds__(256) jk_run_bounds_kernel(const JKScreenCQ* __restrict__ cqs, double tol, int nbins,
+                                                            int prescreen, double fp32_cutoff) {
+    const JKScreenCQ cq = cqs[blockIdx.x];
+    if (!cq.runs || (int)(blockIdx.y * 8) >= cq.nrun) return;
+    const JKScreen sc(cq, tol, nbins, prescreen, fp32_cutoff);
+    const int lane = threadIdx.x & 31;
+    long long n64 = 0, n32 = 0;
+    for (int run = blockIdx.y * 8 + (threadIdx.x >> 5); run < cq.nrun; run += gridDim.y * 8) {
+        const int e0 = cq.run0[run], ne = cq.run0[run + 1] - e0;
+        int c64 = 0, cnt = 0;
+        if (lane < ne) {
+            sc.row(cq, cq.ent[e0 + lane], c64, cnt);
+            cq.klb[e0 + lane] = c64;
+            cq.kle[e0 + lane] = cnt;
         }
-        const JKPackCls k = cls[lo];
-        const long long local = t - k.off;
-        const int comp = (int)(local / k.np), p = (int)(local - (long long)comp * k.np);
-        const int a = comp / k.nfj, bb = comp - a * k.nfj;
-        const int pair = k.pair0 + p;
-        const size_t e = (size_t)(ao_loc[pair2bra[pair]] + a) + (size_t)nao * (ao_loc[pair2ket[pair]] + bb);
-        for (int m = 0; m < n_dm; m++) {
-            const size_t mo = (size_t)m * nao * nao;
-            if (mode == 0) dp[m * total + t] = dm[mo + e];
-            else vj[mo + e] += jp[m * total + t];
+        n64 += c64;
+        n32 += cnt - c64;
+        const int h64 = __reduce_max_sync(0xffffffffu, c64);
+        const int l32 = __reduce_min_sync(0xffffffffu, c64 < cnt ? c64 : 0x7fffffff) / cq.runs * cq.runs;
+        const int h32 = __reduce_max_sync(0xffffffffu, c64 < cnt ? cnt : 0);
+        if (lane == 0) {
+            cq.ioff[run] = (h64 + cq.runs - 1) / cq.runs;
+            cq.ioff32[run] = h32 > 0 ? (h32 - l32 + cq.runs - 1) / cq.runs : 0;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        n64 += __shfl_xor_sync(0xffffffffu, n64, o);
+        n32 += __shfl_xor_sync(0xffffffffu, n32, o);
+    }
+    if (lane == 0 && (n64 | n32)) {
+        atomicAdd((unsigned long long*)cq.task0 + 1, (unsigned long long)n64);
+        atomicAdd((unsigned long long*)cq.task032 + 1, (unsigned long long)n32);
+    }
+}
+
+// items per run -> exclusive prefix in place, totals to tot[1] (one block)
+__device__ __forceinline__ void jk_run_scan_body(int nrun, long long* ioff, long long* ioff32, long long* tot,
+                                                 long long* tot32) {
+    __shared__ long long carry, carry32;
+    __shared__ long long wsum[32], wsum32[32];
+    if (threadIdx.x == 0) carry = carry32 = 0;
+    __syncthreads();
+    for (int base = 0; base < nrun; base += blockDim.x) {
+        const int r = base + threadIdx.x;
+        const long long a = r < nrun ? ioff[r] : 0, b = r < nrun && ioff32 ? ioff32[r] : 0;
+        long long ia, ib;
+        jk_block_scan2(a, b, ia, ib, wsum, wsum32, carry, carry32);
+        if (r < nrun) {
+            ioff[r] = ia - a;
+            if (ioff32) ioff32[r] = ib - b;
+        }
+    }
+    if (threadIdx.x == 0) {
+        tot[0] = 0;
+        tot[1] = carry;
+        if (tot32) {
+            tot32[0] = 0;
+            tot32[1] = carry32;
+        }
+    }
+}
+__global__ void __launch_bounds__(1024) jk_run_scan_kernel(const JKScreenCQ* __restrict__ cqs) {
+    const JKScreenCQ cq = cqs[blockIdx.x];
+    if (cq.runs) jk_run_scan_body(cq.nrun, cq.ioff, cq.ioff32, cq.itm, cq.itm32);
+}
+
+// per-class-pair entries: items of each run from the entries' ket ends
+__global__ void jk_run_items_kernel(int nrun, int chunk, const int* __restrict__ run0, const int* __restrict__ ehi,
+                                    long long* __restrict__ ioff) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrun; r += gridDim.x * blockDim.x) {
+        int h = 0;
+        for (int e = run0[r]; e < run0[r + 1]; e++) h = max(h, ehi[e]);
+        ioff[r] = (h + chunk - 1) / chunk;
+    }
+}
+__global__ void __launch_bounds__(1024) jk_run_scan1_kernel(int nrun, long long* ioff, long long* itm) {
+    jk_run_scan_body(nrun, ioff, nullptr, itm, nullptr);
+}
+
+// bra records of the run kernels (JKSeg::bprim, bprimf, bpair) of one class,
+// gathered in run-entry order
+__global__ void jk_bra_records_kernel(int np, int nprim, const int* __restrict__ ent, const double* __restrict__ prim,
+                                      const float* __restrict__ primf, long long n, const double* __restrict__ pgeo,
+                                      const int* __restrict__ pao, const int* __restrict__ pnp, int npt,
+                                      double* __restrict__ bprim, float* __restrict__ bprimf,
+                                      double* __restrict__ bpair) {
+    // prim, primf: first primitive of the class in the SoA arrays of stride n;
+    // pgeo, pao, pnp: its first pair in the arrays of stride npt
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < np * nprim; t += gridDim.x * blockDim.x) {
+        const int k = t / np, e = t - k * np, r = ent[e];
+        const double* s = prim + (size_t)k * np + r;
+        const float* f = primf + (size_t)k * np + r;
+        double* d = bprim + (size_t)t * 8;
+        float* g = bprimf + (size_t)t * 8;
+        d[0] = s[0];
+        d[1] = s[5 * n];
+        d[2] = s[n] * s[5 * n];
+        d[3] = s[2 * n];
+        d[4] = s[3 * n];
+        d[5] = s[4 * n];
+        d[6] = d[7] = 0.;
+        for (int x = 0; x < 6; x++) g[x] = f[x * n];
+        g[6] = g[7] = 0.f;
+        if (k == 0) {
+            double* b = bpair + (size_t)e * 4;
+            for (int x = 0; x < 3; x++) b[x] = pgeo[(size_t)(3 + x) * npt + r];
+            b[3] = __hiloint2double(pnp[r], pao[npt + r]);
         }
     }
 }
 
-__global__ void jk_pack_kernel(const JKPackCls* __restrict__ cls, int ncls, long long total,
-                               const int* __restrict__ pair2bra, const int* __restrict__ pair2ket,
-                               const int* __restrict__ ao_loc, const double* __restrict__ dm, int nao, int n_dm,
-                               double* __restrict__ dp, const double* __restrict__ jp, double* __restrict__ vj,
-                               int mode) {
-    jk_pack_body(cls, ncls, total, pair2bra, pair2ket, ao_loc, dm, nao, n_dm, dp, jp, vj, mode);
+__global__ void jk_put_seg_kernel(const __grid_constant__ JKSeg sg, JKSeg* __restrict__ dst) {
+    const int* a = reinterpret_cast<const int*>(&sg);
+    int* d = reinterpret_cast<int*>(dst);
+    for (int x = threadIdx.x; x < (int)(sizeof(JKSeg) / 4); x += blockDim.x) d[x] = a[x];
 }
+
+// the call's buffers into the segments of a plan
+struct JKCall {
+    const double* dm;
+    double *vj, *vk;
+    const double* dp;
+    double* jp;
+    const double* dpb;
+    double* jpb;
+    int n_dm;
+};
+__global__ void jk_set_call_kernel(JKSeg* __restrict__ s64, JKSeg* __restrict__ s32, int nseg, const JKCall c) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * nseg; i += gridDim.x * blockDim.x) {
+        JKSeg& s = i < nseg ? s64[i] : s32[i - nseg];
+        s.dm = c.dm;
+        s.vj = c.vj;
+        s.vk = c.vk;
+        s.dp = c.dp;
+        s.jp = c.jp;
+        s.dpb = c.dpb;
+        s.jpb = c.jpb;
+        s.n_dm = c.n_dm;
+    }
+}
+
+// Pair-packed J side.  mode 0: gather the density blocks of every pair into
+// dp (element c of pair p of class k at off_k + c*np_k + p, one copy per
+// density) and into dpb (entry-major: element c of entry e at off_k +
+// e*ncomp_k + c; inv gives a pair's entry); mode 1: add the packed J
+// accumulators jp and jpb into vj.  Every (pair, component) is a distinct
+// element of D and of vj.
+__device__ __forceinline__ void jk_pack_body(const JKPackMol& a, int mode) {
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < a.total;
+         t += (long long)gridDim.x * blockDim.x) {
+        int lo = 0, hi = a.ncls - 1;
+        while (lo < hi) {
+            int mid = (lo + hi + 1) >> 1;
+            if (a.cls[mid].off <= t) lo = mid; else hi = mid - 1;
+        }
+        const JKPackCls k = a.cls[lo];
+        const long long local = t - k.off;
+        const int comp = (int)(local / k.np), p = (int)(local - (long long)comp * k.np);
+        const int x = comp / k.nfj, y = comp - x * k.nfj;
+        const int pair = k.pair0 + p;
+        const long long tb = k.off + (long long)a.inv[pair] * (k.nfi * k.nfj) + comp;
+        const size_t e = (size_t)(a.ao_loc[a.pair2bra[pair]] + x) + (size_t)a.nao * (a.ao_loc[a.pair2ket[pair]] + y);
+        for (int m = 0; m < a.n_dm; m++) {
+            const size_t mo = (size_t)m * a.nao * a.nao;
+            if (mode == 0) {
+                const double v = a.dm[mo + e];
+                a.dp[m * a.total + t] = v;
+                a.dpb[m * a.total + tb] = v;
+            } else {
+                a.vj[mo + e] += a.jp[m * a.total + t] + a.jpb[m * a.total + tb];
+            }
+        }
+    }
+}
+
+__global__ void jk_pack_kernel(const JKPackMol one, int mode) { jk_pack_body(one, mode); }
 
 // one molecule per blockIdx.y
 __global__ void jk_pack_batch_kernel(const JKPackMol* __restrict__ mols, int mode) {
     const JKPackMol m = mols[blockIdx.y];
-    if (m.total <= 0) return;
-    jk_pack_body(m.cls, m.ncls, m.total, m.pair2bra, m.pair2ket, m.ao_loc, m.dm, m.nao, m.n_dm, m.dp, m.jp, m.vj,
-                 mode);
+    if (m.total > 0) jk_pack_body(m, mode);
 }
 
 // J = 2 (V + V^T), K = V + V^T in place on the working-basis buffers, where
@@ -401,14 +569,23 @@ static void free_basis(jk_basis* b) {
     cudaFree(b->d_log_q);
     cudaFree(b->d_log_q_raw);
     cudaFree(b->d_qoff32);
-    cudaFree(b->d_task032);
     cudaFree(b->d_klb);
+    cudaFree(b->d_kle);
+    cudaFree(b->d_ioff);
+    cudaFree(b->d_zero);
+    cudaFree(b->d_ent);
+    cudaFree(b->d_inv);
+    cudaFree(b->d_bprim);
+    cudaFree(b->d_bprimf);
+    cudaFree(b->d_bpair);
+    cudaFree(b->d_run0);
+    cudaFree(b->d_ehi1);
+    cudaFree(b->d_seg1);
+    jk_plan_free(b->plan);
     cudaFree(b->d_prim);
     cudaFree(b->d_primf);
     cudaFree(b->d_cq);
     cudaFree(b->d_qoff);
-    cudaFree(b->d_task0);
-    cudaFree(b->d_dm_cond);
     cudaFree(b->d_qoff1);
     cudaFree(b->d_task01);
     cudaFree(b->d_work);
@@ -455,6 +632,15 @@ static int rys_table_device(const double** out) {
     }
     *out = g_rys_dev[dev];
     return JK_OK;
+}
+
+// Run length of a class quartet's bra (an index of JK_RUN_LEN): the longest
+// that still gives a few items per resident warp before screening; a
+// molecule too small for that takes the shortest.
+static int run_level(const jk_basis* b, int cp_ij, int n_kl, int chunk) {
+    for (int v = 0; v < JK_RUN_LEVELS - 1; v++)
+        if ((long long)b->h_nrun[v][cp_ij] * ((n_kl + chunk - 1) / chunk) >= 40LL * b->nsm) return v;
+    return JK_RUN_LEVELS - 1;
 }
 
 static int create_impl(const int* atm, int natm, const int* bas, int nbas, const double* env, int nenv,
@@ -675,10 +861,60 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
     CUDA_TRY(upload(&b->d_pair2ket, b->h_pair2ket.data(), b->h_pair2ket.size()));
     CUDA_TRY(upload(&b->d_log_q, b->h_log_q.data(), b->h_log_q.size()));
     CUDA_TRY(upload(&b->d_log_q_raw, b->h_log_q_raw.data(), b->h_log_q_raw.size()));
-    // class quartets (cp_ij >= cp_kl), each with its slice of the qoff buffer
+    // runs of every class's pairs: the pairs of one first shell, in Schwarz
+    // order, cut at each run length
+    {
+        std::vector<int> ent(b->h_pair2bra.size()), inv(b->h_pair2bra.size()), run0;
+        for (int v = 0; v < JK_RUN_LEVELS; v++) {
+            b->h_nrun[v].assign(b->ncp, 0);
+            b->h_run_off[v].assign(b->ncp, 0);
+        }
+        for (int c = 0; c < b->ncp; c++) {
+            const int p0 = b->h_pair_locs[c], np = b->h_pair_locs[c + 1] - p0;
+            int* e = ent.data() + p0;
+            for (int x = 0; x < np; x++) e[x] = x;
+            std::stable_sort(e, e + np,
+                             [&](int x, int y) { return b->h_pair2bra[p0 + x] < b->h_pair2bra[p0 + y]; });
+            for (int x = 0; x < np; x++) inv[p0 + e[x]] = x;
+            for (int v = 0; v < JK_RUN_LEVELS; v++) {
+                b->h_run_off[v][c] = (int)run0.size();
+                int beg = 0;
+                for (int x = 0; x <= np; x++) {
+                    const bool cut = x == np || x - beg == JK_RUN_LEN[v] ||
+                                     b->h_pair2bra[p0 + e[x]] != b->h_pair2bra[p0 + e[beg]];
+                    if (!cut || x == beg) continue;
+                    run0.push_back(beg);
+                    b->h_nrun[v][c]++;
+                    beg = x;
+                }
+                run0.push_back(np);
+            }
+        }
+        CUDA_TRY(upload(&b->d_ent, ent.data(), ent.size()));
+        CUDA_TRY(upload(&b->d_run0, run0.data(), run0.size()));
+        CUDA_TRY(upload(&b->d_inv, inv.data(), inv.size()));
+        CUDA_TRY(cudaMalloc(&b->d_bprim, sizeof(double) * 8 * (size_t)std::max(npp, 1LL)));
+        CUDA_TRY(cudaMalloc(&b->d_bprimf, sizeof(float) * 8 * (size_t)std::max(npp, 1LL)));
+        CUDA_TRY(cudaMalloc(&b->d_bpair, sizeof(double) * 4 * std::max<size_t>(ent.size(), 1)));
+        for (int c = 0; c < b->ncp; c++) {
+            const int p0 = b->h_pair_locs[c], np = b->h_pair_locs[c + 1] - p0;
+            if (np == 0) continue;
+            const int nprim = b->h_group_nprim[b->h_cls_gi[c]] * b->h_group_nprim[b->h_cls_gj[c]];
+            const size_t q0 = b->h_prim_locs[c];
+            const int blocks = (int)std::min<long long>(((long long)np * nprim + 255) / 256, (long long)b->nsm * 16);
+            jk_bra_records_kernel<<<blocks, 256>>>(np, nprim, b->d_ent + p0, b->d_prim + q0, b->d_primf + q0, npp,
+                                                   b->d_pgeo + p0, b->d_pao + p0, b->d_pnp + p0,
+                                                   (int)b->h_pair2bra.size(), b->d_bprim + 8 * q0, b->d_bprimf + 8 * q0,
+                                                   b->d_bpair + 4 * (size_t)p0);
+            CUDA_TRY(cudaGetLastError());
+        }
+        CUDA_TRY(cudaStreamSynchronize(0));
+    }
+    // class quartets (cp_ij >= cp_kl), each with its slices of the screening buffers
+    std::vector<long long> qoff_at, ioff_at, ent_at;
     for (int cij = 0; cij < b->ncp; cij++)
         for (int ckl = 0; ckl <= cij; ckl++) {
-            JKScreenCQ c;
+            JKScreenCQ c{};
             c.cp_ij = cij;
             c.cp_kl = ckl;
             c.gi = b->h_cls_gi[cij];
@@ -690,8 +926,18 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             c.pair_kl0 = b->h_pair_locs[ckl];
             c.n_kl = b->h_pair_locs[ckl + 1] - c.pair_kl0;
             if (c.n_ij == 0 || c.n_kl == 0) continue;
-            c.qoff_off = b->qoff_total;
-            b->qoff_total += c.n_ij + 1;
+            c.runs = g_tabs.run[class_index(b, cij, ckl)];
+            qoff_at.push_back(b->qoff_total);
+            ioff_at.push_back(b->ioff_total);
+            ent_at.push_back(b->ent_total);
+            b->ent_total += c.n_ij;
+            if (c.runs) {
+                c.level = run_level(b, cij, c.n_kl, c.runs);
+                c.nrun = b->h_nrun[c.level][cij];
+                b->ioff_total += 2LL * c.nrun;
+            } else {
+                b->qoff_total += c.n_ij + 1;
+            }
             b->h_cq.push_back(c);
             // unscreened work for shard plans: quartets x primitive
             // quartets x roots x Cartesian components (+ the digestion)
@@ -704,12 +950,19 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             b->h_cq_cost.push_back(nq * (npq * ((l4[0] + l4[1] + l4[2] + l4[3]) / 2 + 1) * nf + 12. * nf));
         }
     b->ncq = (int)b->h_cq.size();
-    CUDA_TRY(cudaMalloc(&b->d_qoff, sizeof(long long) * (b->qoff_total ? b->qoff_total : 1)));
-    CUDA_TRY(cudaMalloc(&b->d_task0, sizeof(long long) * 2 * (b->ncq ? b->ncq : 1)));
-    CUDA_TRY(cudaMalloc(&b->d_qoff32, sizeof(long long) * (b->qoff_total ? b->qoff_total : 1)));
-    CUDA_TRY(cudaMalloc(&b->d_task032, sizeof(long long) * 2 * (b->ncq ? b->ncq : 1)));
-    CUDA_TRY(cudaMalloc(&b->d_klb, sizeof(int) * (b->qoff_total ? b->qoff_total : 1)));
-    CUDA_TRY(cudaMalloc(&b->d_dm_cond, sizeof(double) * ngroups * ngroups));
+    auto atleast1 = [](long long n) { return (size_t)(n > 0 ? n : 1); };
+    CUDA_TRY(cudaMalloc(&b->d_qoff, sizeof(long long) * atleast1(b->qoff_total)));
+    CUDA_TRY(cudaMalloc(&b->d_qoff32, sizeof(long long) * atleast1(b->qoff_total)));
+    CUDA_TRY(cudaMalloc(&b->d_ioff, sizeof(long long) * atleast1(b->ioff_total)));
+    CUDA_TRY(cudaMalloc(&b->d_klb, sizeof(int) * atleast1(b->ent_total)));
+    CUDA_TRY(cudaMalloc(&b->d_kle, sizeof(int) * atleast1(b->ent_total)));
+    // the buffers a build clears: condensed density, then {0, count} of the
+    // quartets and items of both parts
+    b->zero_bytes = sizeof(double) * ((size_t)ngroups * ngroups + 8 * (size_t)b->ncq);
+    CUDA_TRY(cudaMalloc(&b->d_zero, b->zero_bytes));
+    b->d_dm_cond = (double*)b->d_zero;
+    b->d_task0 = (long long*)(b->d_dm_cond + (size_t)ngroups * ngroups);
+    b->d_task032 = b->d_task0 + 2 * b->ncq;
     for (int c = 0; c < b->ncq; c++) {
         JKScreenCQ& q = b->h_cq[c];
         q.ngroups = ngroups;
@@ -718,20 +971,29 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         q.rq_ij = b->d_log_q_raw + q.pair_ij0;
         q.rq_kl = b->d_log_q_raw + q.pair_kl0;
         q.dm_cond = b->d_dm_cond;
-        q.qoff = b->d_qoff + q.qoff_off;
-        q.qoff32 = b->d_qoff32 + q.qoff_off;
-        q.klb = b->d_klb + q.qoff_off;
+        q.qoff = b->d_qoff + qoff_at[c];
+        q.qoff32 = b->d_qoff32 + qoff_at[c];
+        q.klb = b->d_klb + ent_at[c];
+        q.kle = b->d_kle + ent_at[c];
+        q.ioff = b->d_ioff + ioff_at[c];
+        q.ioff32 = q.ioff + q.nrun;
+        q.ent = b->d_ent + q.pair_ij0;
+        q.run0 = b->d_run0 + b->h_run_off[q.level][q.cp_ij];
         q.task0 = b->d_task0 + 2 * c;
         q.task032 = b->d_task032 + 2 * c;
+        q.itm = b->d_task0 + 4 * b->ncq + 2 * c;
+        q.itm32 = b->d_task0 + 6 * b->ncq + 2 * c;
     }
     CUDA_TRY(upload(&b->d_cq, b->h_cq.data(), b->h_cq.size()));
     CUDA_TRY(cudaMalloc(&b->d_task01, sizeof(long long) * 2));
+    CUDA_TRY(cudaMalloc(&b->d_seg1, sizeof(JKSeg)));
     // row prefixes of the per-class-pair entries: sized once for the largest
     // class, so those calls never free a buffer a queued kernel still reads
     {
         int mx = 1;
         for (int c = 0; c < b->ncp; c++) mx = std::max(mx, b->h_pair_locs[c + 1] - b->h_pair_locs[c]);
         CUDA_TRY(cudaMalloc(&b->d_qoff1, sizeof(long long) * (mx + 1)));
+        CUDA_TRY(cudaMalloc(&b->d_ehi1, sizeof(int) * mx));
         b->qoff1_cap = mx + 1;
     }
     // pair-packed layout of the J side (jk_build)
@@ -801,9 +1063,9 @@ extern "C" int jk_basis_pairs(const jk_basis_t* b, int* pair2shls, int* pair_loc
 
 static void fill_seg(const jk_basis* b, int cp_ij, int cp_kl, const long long* qoff, int n_ij, const double* dm,
                      int n_dm, double* vj, double* vk, JKSeg* s) {
+    *s = JKSeg{};
     s->rys = b->rys;
     s->qoff = qoff;
-    s->kl_base = nullptr;
     s->n_ij = n_ij;
     s->pair_ij0 = b->h_pair_locs[cp_ij];
     s->pair_kl0 = b->h_pair_locs[cp_kl];
@@ -815,8 +1077,6 @@ static void fill_seg(const jk_basis* b, int cp_ij, int cp_kl, const long long* q
     s->pst_kl = b->h_pair_locs[cp_kl + 1] - b->h_pair_locs[cp_kl];
     s->nao = b->nao;
     s->n_dm = n_dm;
-    s->pair2bra = b->d_pair2bra;
-    s->pair2ket = b->d_pair2ket;
     long long n = b->nprim_total;
     s->a12 = b->d_prim;
     s->e12 = b->d_prim + n;
@@ -826,27 +1086,25 @@ static void fill_seg(const jk_basis* b, int cp_ij, int cp_kl, const long long* q
     s->ia12 = b->d_prim + 5 * n;
     s->pf = b->d_primf;
     s->npf = n;
-    s->bas_x = b->d_bas_x;
     s->pgeo = b->d_pgeo;
     s->pnp = b->d_pnp;
+    s->bprim = b->d_bprim + 8 * (size_t)s->prim_ij0;
+    s->bprimf = b->d_bprimf + 8 * (size_t)s->prim_ij0;
+    s->bpair = b->d_bpair + 4 * (size_t)s->pair_ij0;
     s->pao = b->d_pao;
     s->npt = (int)b->h_pair2bra.size();
-    s->nbas = b->nbas;
-    s->ao_loc = b->d_ao_loc;
     s->dm = dm;
     s->vj = vj;
     s->vk = vk;
-    s->dp_ij = s->dp_kl = nullptr;
-    s->jp_ij = s->jp_kl = nullptr;
-    s->np_ij = s->np_kl = 0;
-    s->pk_stride = 0;
+    s->pk_ij = b->h_pack[cp_ij].off;
+    s->pk_kl = b->h_pack[cp_kl].off;
+    s->pk_stride = b->pack_total;
     s->ls[0] = b->h_group_l[b->h_cls_gi[cp_ij]];
     s->ls[1] = b->h_group_l[b->h_cls_gj[cp_ij]];
     s->ls[2] = b->h_group_l[b->h_cls_gi[cp_kl]];
     s->ls[3] = b->h_group_l[b->h_cls_gj[cp_kl]];
 }
 
-int jk_internal_class_index(const jk_basis_t* b, int cp_ij, int cp_kl);
 static int class_index(const jk_basis* b, int cp_ij, int cp_kl) {
     int li = b->h_group_l[b->h_cls_gi[cp_ij]], lj = b->h_group_l[b->h_cls_gj[cp_ij]];
     int lk = b->h_group_l[b->h_cls_gi[cp_kl]], ll = b->h_group_l[b->h_cls_gj[cp_kl]];
@@ -870,6 +1128,8 @@ extern "C" int jk_shard_plan(const double* cost, int n, int nshards, int* owner)
     return JK_OK;
 }
 
+static unsigned dm_cond_blocks(int nao) { return (unsigned)std::min(64, nao / 8 + 1); }
+
 // owner of every class quartet for nshards shards (cached per basis)
 static const int* shard_owners(jk_basis* b, int nshards) {
     if (b->cq_owner_n != nshards || (int)b->h_cq_owner.size() != b->ncq) {
@@ -880,6 +1140,25 @@ static const int* shard_owners(jk_basis* b, int nshards) {
     return b->h_cq_owner.data();
 }
 
+// class launches of jk_build for one shard (kept; rebuilt for another split)
+static int build_plan(jk_basis* b, int nshards, int shard) {
+    if (b->plan && b->plan->nshards == nshards && b->plan->shard == shard) return JK_OK;
+    jk_plan_free(b->plan);
+    b->plan = new JKPlan();
+    b->plan->nshards = nshards;
+    b->plan->shard = shard;
+    const int* owner = nshards > 1 ? shard_owners(b, nshards) : nullptr;
+    int rc = JK_OK;
+    for (int c = 0; c < b->ncq && !rc; c++)
+        if (!owner || owner[c] == shard) rc = jk_plan_add(b->plan, b, 0, c, false);
+    if (!rc) rc = jk_plan_finish(b->plan, {b});
+    if (rc) {
+        jk_plan_free(b->plan);
+        b->plan = nullptr;
+    }
+    return rc;
+}
+
 extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, double* vk, const jk_opts_t* opts,
                         void* stream) {
     if (!b || !dm || n_dm <= 0) return set_err(JK_ERR_ARG, "jk_build: invalid arguments");
@@ -888,70 +1167,58 @@ extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, d
     double tol = opts ? opts->direct_scf_tol : b->cutoff;
     int nbins = opts && opts->nbins > 0 ? opts->nbins : 10;
     int prescreen = opts ? opts->prescreen : 1;
-    dim3 gg(b->ngroups, b->ngroups);
-    jk_dm_cond_kernel<<<gg, 256, 0, st>>>(dm, b->nao, n_dm, b->d_group_ao, b->ngroups, b->d_dm_cond);
+    const int nshards = opts && opts->nshards > 1 ? opts->nshards : 1;
+    const int shard = nshards > 1 ? opts->shard : 0;
+    if (nshards > 1 && (shard < 0 || shard >= nshards)) return set_err(JK_ERR_ARG, "jk_build: shard out of range");
+    int rc = build_plan(b, nshards, shard);
+    if (rc) return rc;
+    CUDA_TRY(cudaMemsetAsync(b->d_zero, 0, b->zero_bytes, st));
+    const JKDmCond dc{dm, b->d_group_ao, b->d_dm_cond, b->nao, n_dm, b->ngroups, nullptr, 0};
+    jk_dm_cond_kernel<<<dim3(dm_cond_blocks(b->nao), b->ngroups), 256, 0, st>>>(dc, nullptr);
     CUDA_TRY(cudaGetLastError());
     if (b->ncq == 0) return JK_OK;
     double fp32_cutoff = opts ? opts->fp32_cutoff : 0.;
-    jk_screen_kernel<<<b->ncq, 256, 0, st>>>(b->d_cq, tol, nbins, prescreen, fp32_cutoff);
-    CUDA_TRY(cudaGetLastError());
-    // pair-packed density and J accumulators for the thread kernels
+    const bool mixed = fp32_cutoff > 0;
+    rc = jk_internal_screen(b->d_cq, b->ncq, tol, nbins, prescreen, fp32_cutoff, st);
+    if (!rc) rc = jk_plan_prefix(b->plan, mixed, st);
+    if (rc) return rc;
+    // pair-packed density and J accumulators for the run kernels
     const bool packed = vj && b->pack_total > 0;
-    double *dp = nullptr, *jp = nullptr;
+    JKCall call{dm, vj, vk, nullptr, nullptr, nullptr, nullptr, n_dm};
+    JKPackMol pm{};
     const int pk_blocks = (int)std::min<long long>((b->pack_total + 255) / 256, (long long)b->nsm * 8);
     if (packed) {
-        const size_t need = (size_t)2 * n_dm * b->pack_total;
+        const size_t need = (size_t)4 * n_dm * b->pack_total;
         if (need > b->pk_cap) {
             cudaFree(b->d_pk);
             b->d_pk = nullptr;
             CUDA_TRY(cudaMalloc(&b->d_pk, sizeof(double) * need));
             b->pk_cap = need;
         }
-        dp = b->d_pk;
-        jp = b->d_pk + (size_t)n_dm * b->pack_total;
-        jk_pack_kernel<<<pk_blocks, 256, 0, st>>>(b->d_pack, b->ncp, b->pack_total, b->d_pair2bra, b->d_pair2ket,
-                                                   b->d_ao_loc, dm, b->nao, n_dm, dp, nullptr, nullptr, 0);
+        pm = jk_internal_pack_mol(b, dm, n_dm, b->d_pk, b->d_pk + 2 * (size_t)n_dm * b->pack_total, vj);
+        call.dp = pm.dp;
+        call.jp = pm.jp;
+        call.dpb = pm.dpb;
+        call.jpb = pm.jpb;
+        jk_pack_kernel<<<pk_blocks, 256, 0, st>>>(pm, 0);
         CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaMemsetAsync(jp, 0, sizeof(double) * n_dm * b->pack_total, st));
+        CUDA_TRY(cudaMemsetAsync(pm.jp, 0, 2 * sizeof(double) * n_dm * b->pack_total, st));
     }
-    const int nshards = opts && opts->nshards > 1 ? opts->nshards : 1;
-    const int shard = opts ? opts->shard : 0;
-    if (nshards > 1 && (shard < 0 || shard >= nshards)) return set_err(JK_ERR_ARG, "jk_build: shard out of range");
-    const int* owner = nshards > 1 ? shard_owners(b, nshards) : nullptr;
+    if (b->plan->nseg) {
+        jk_set_call_kernel<<<(2 * b->plan->nseg + 255) / 256, 256, 0, st>>>(b->plan->d_seg[0], b->plan->d_seg[1],
+                                                                           b->plan->nseg, call);
+        CUDA_TRY(cudaGetLastError());
+    }
     CUDA_TRY(b->fan.begin(st));
-    for (int c = 0; c < b->ncq; c++) {
-        if (owner && owner[c] != shard) continue;
-        const JKScreenCQ& cq = b->h_cq[c];
-        JKSeg seg;
-        fill_seg(b, cq.cp_ij, cq.cp_kl, b->d_qoff + cq.qoff_off, cq.n_ij, dm, n_dm, vj, vk, &seg);
-        if (packed) {
-            const JKPackCls &ki = b->h_pack[cq.cp_ij], &kk = b->h_pack[cq.cp_kl];
-            seg.dp_ij = dp + ki.off;
-            seg.dp_kl = dp + kk.off;
-            seg.jp_ij = jp + ki.off;
-            seg.jp_kl = jp + kk.off;
-            seg.np_ij = ki.np;
-            seg.np_kl = kk.np;
-            seg.pk_stride = b->pack_total;
+    for (int k = 0; k < (int)b->plan->keys.size(); k++)
+        for (int part = 0; part < (mixed ? 2 : 1); part++) {
+            rc = jk_plan_launch(b->plan, k, part, b->plan->keys[k].cfg[part], n_dm, b->nsm,
+                                b->fan.pick(2 * k + part));
+            if (rc) return rc;
         }
-        long long maxt = cq.cp_ij == cq.cp_kl ? (long long)cq.n_ij * (cq.n_ij + 1) / 2
-                                              : (long long)cq.n_ij * cq.n_kl;
-        int ci = class_index(b, cq.cp_ij, cq.cp_kl);
-        jk_launch_fn fn = g_tab64[ci];
-        if (!fn) return set_err(JK_ERR_UNSUPPORTED, "no kernel for class quartet %d", c);
-        CUDA_TRY(fn(seg, b->d_task0 + 2 * c, maxt, b->nsm, b->fan.pick(2 * c)));
-        if (fp32_cutoff > 0) {
-            jk_launch_fn f32 = g_tab32[ci];
-            if (!f32) return set_err(JK_ERR_UNSUPPORTED, "no FP32 kernel for class quartet %d", c);
-            seg.qoff = b->d_qoff32 + cq.qoff_off;
-            seg.kl_base = b->d_klb + cq.qoff_off;
-            CUDA_TRY(f32(seg, b->d_task032 + 2 * c, maxt, b->nsm, b->fan.pick(2 * c + 1)));
-        }
-    }
     CUDA_TRY(b->fan.end(st));
     if (packed) {
-        jk_pack_kernel<<<pk_blocks, 256, 0, st>>>(b->d_pack, b->ncp, b->pack_total, b->d_pair2bra, b->d_pair2ket,
-                                                   b->d_ao_loc, dm, b->nao, n_dm, nullptr, jp, vj, 1);
+        jk_pack_kernel<<<pk_blocks, 256, 0, st>>>(pm, 1);
         CUDA_TRY(cudaGetLastError());
     }
     return JK_OK;
@@ -990,6 +1257,24 @@ __host__ __device__ inline long long jk_rowbins_tasks(const JKRowBins& b, long l
     return acc;
 }
 
+// columns row r keeps
+__device__ __forceinline__ int jk_rowbins_cols(const JKRowBins& b, int r) {
+    if (b.kl[0] != 0) return 0;
+    for (int s = 0; s < b.nbins; s++)
+        if (r >= b.ij[s] && r < b.ij[s + 1]) {
+            const int c = b.kl[b.nbins - s];
+            return b.diag && c > r + 1 ? r + 1 : c;
+        }
+    return 0;
+}
+
+// run classes: ket end of every entry
+__global__ void jk_run_rowbins_kernel(const __grid_constant__ JKRowBins rb, int n_ij, int n_kl,
+                                      const int* __restrict__ ent, int* __restrict__ ehi) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_ij; e += gridDim.x * blockDim.x)
+        ehi[e] = min(jk_rowbins_cols(rb, ent[e]), n_kl);
+}
+
 __global__ void jk_rowbins_kernel(const JKRowBins rb, int n_ij, long long* __restrict__ qoff,
                                   long long* __restrict__ task0) {
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r <= n_ij;
@@ -1001,20 +1286,22 @@ __global__ void jk_rowbins_kernel(const JKRowBins rb, int n_ij, long long* __res
     }
 }
 
-// bins of a per-class-pair call -> the basis's row prefix and task count, on
-// `st`; returns the task count through *tot
-static int class_pair_rows(jk_basis* b, const int* bins_ij, const int* bins_kl, int nbins, int n_ij, int diag,
-                           cudaStream_t st, long long* tot) {
+static int row_bins(const int* bins_ij, const int* bins_kl, int nbins, int diag, JKRowBins* rb) {
     if (nbins > JK_ROWBINS_MAX) return set_err(JK_ERR_ARG, "nbins %d above %d", nbins, JK_ROWBINS_MAX);
-    JKRowBins rb;
-    rb.nbins = nbins;
-    rb.diag = diag;
+    rb->nbins = nbins;
+    rb->diag = diag;
     for (int s = 0; s <= nbins; s++) {
-        rb.ij[s] = bins_ij[s];
-        rb.kl[s] = bins_kl[s];
+        rb->ij[s] = bins_ij[s];
+        rb->kl[s] = bins_kl[s];
         if (s && (bins_ij[s] < bins_ij[s - 1] || bins_kl[s] < bins_kl[s - 1]))
             return set_err(JK_ERR_ARG, "bins must not decrease");
     }
+    return JK_OK;
+}
+
+// bins of a per-class-pair call -> the basis's row prefix and task count, on
+// `st`; returns the task count through *tot
+static int class_pair_rows(jk_basis* b, const JKRowBins& rb, int n_ij, cudaStream_t st, long long* tot) {
     if (n_ij + 1 > (int)b->qoff1_cap) return set_err(JK_ERR_ARG, "class pair larger than the basis' classes");
     *tot = jk_rowbins_tasks(rb, n_ij);
     const int blocks = (int)std::min<long long>((n_ij + 256) / 256, (long long)b->nsm * 4);
@@ -1055,13 +1342,30 @@ extern "C" int jk_build_class_pair(jk_basis_t* b, double* vj, double* vk, const 
     // row ij (in bin sij) keeps kl < bins_kl[nbins - sij]; diagonal classes keep kl <= ij
     jk_launch_fn fn = g_tab64[class_index(b, cp_ij, cp_kl)];
     if (!fn) return set_err(JK_ERR_UNSUPPORTED, "no kernel for this class pair");
-    long long tot = 0;
-    int rc = class_pair_rows(b, bins_locs_ij, bins_locs_kl, nbins, n_ij, cp_ij == cp_kl, st, &tot);
+    JKRowBins rb;
+    int rc = row_bins(bins_locs_ij, bins_locs_kl, nbins, cp_ij == cp_kl, &rb);
     if (rc) return rc;
     JKSeg seg;
     fill_seg(b, cp_ij, cp_kl, b->d_qoff1, n_ij, dm, n_dm, vj, vk, &seg);
-    CUDA_TRY(fn(seg, b->d_task01, tot, b->nsm, st));
-    return JK_OK;
+    JKRunTab rt;
+    long long tot = 0;
+    if (jk_internal_run_table(b, cp_ij, cp_kl, &rt)) {
+        const int n_kl = seg.pst_kl;
+        if (n_ij == 0 || n_kl == 0) return JK_OK;
+        jk_run_rowbins_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(rb, n_ij, n_kl, rt.ent, b->d_ehi1);
+        CUDA_TRY(cudaGetLastError());
+        rc = jk_internal_run_items(rt, b->d_ehi1, b->d_qoff1, b->d_task01, st);
+        seg.nrun = rt.nrun;
+        seg.ent = rt.ent;
+        seg.run0 = rt.run0;
+        seg.ehi = b->d_ehi1;
+        seg.ioff = b->d_qoff1;
+        tot = (long long)rt.nrun * ((n_kl + rt.chunk - 1) / rt.chunk);
+    } else {
+        rc = class_pair_rows(b, rb, n_ij, st, &tot);
+    }
+    if (rc) return rc;
+    return jk_internal_launch(b, cp_ij, cp_kl, seg, b->d_seg1, b->d_task01, tot, stream);
 }
 
 // ERI tensor of one class pair (jk_generic.cu)
@@ -1081,8 +1385,10 @@ extern "C" int jk_fill_int2e(jk_basis_t* b, double* eri, int nao, const int* str
     const int n_ij = b->h_pair_locs[cp_ij + 1] - b->h_pair_locs[cp_ij];
     // kl bin kb pairs with ij in [bins_ij[0], bins_ij[nbins - kb]): row ij (in
     // bin sij) keeps kl < bins_kl[nbins - sij] (nr_fill_ao_ints.cu:519-545)
+    JKRowBins rb;
     long long tot = 0;
-    int rc = class_pair_rows(b, bins_locs_ij, bins_locs_kl, nbins, n_ij, 0, st, &tot);
+    int rc = row_bins(bins_locs_ij, bins_locs_kl, nbins, 0, &rb);
+    if (!rc) rc = class_pair_rows(b, rb, n_ij, st, &tot);
     if (rc) return rc;
     JKSeg seg;
     fill_seg(b, cp_ij, cp_kl, b->d_qoff1, n_ij, nullptr, 0, nullptr, nullptr, &seg);
@@ -1354,28 +1660,40 @@ void jk_internal_fill_seg(const jk_basis_t* b, int cp_ij, int cp_kl, const long 
     fill_seg(b, cp_ij, cp_kl, qoff, n_ij, dm, n_dm, vj, vk, out);
 }
 
-int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg& seg, const long long* d_task0,
-                       long long max_tasks, void* stream) {
+int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg& seg, JKSeg* d_seg,
+                       const long long* task0, long long max_tasks, void* stream) {
     jk_launch_fn fn = g_tab64[class_index(b, cp_ij, cp_kl)];
     if (!fn) return set_err(JK_ERR_UNSUPPORTED, "no kernel for class pair (%d, %d)", cp_ij, cp_kl);
-    CUDA_TRY(fn(seg, d_task0, max_tasks, b->nsm, (cudaStream_t)stream));
+    cudaStream_t st = (cudaStream_t)stream;
+    jk_put_seg_kernel<<<1, 128, 0, st>>>(seg, d_seg);
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(fn(d_seg, task0, 1, max_tasks, seg.n_dm, b->nsm, JKBatchCfg{nullptr, 0, 1}, st));
     return JK_OK;
 }
 
-int jk_internal_launch_part(int class_idx, int fp32, const JKSeg& seg, const long long* d_task0, long long max_tasks,
-                            int nsm, void* stream) {
-    init_tables();
-    jk_launch_fn fn = fp32 ? g_tab32[class_idx] : g_tab64[class_idx];
-    if (!fn) return set_err(JK_ERR_UNSUPPORTED, "no kernel for class %d", class_idx);
-    CUDA_TRY(fn(seg, d_task0, max_tasks, nsm, (cudaStream_t)stream));
+int jk_internal_run_table(const jk_basis_t* b, int cp_ij, int cp_kl, JKRunTab* out) {
+    if (!g_tabs.run[class_index(b, cp_ij, cp_kl)]) return 0;
+    out->chunk = g_tabs.run[class_index(b, cp_ij, cp_kl)];
+    const int v = run_level(b, cp_ij, b->h_pair_locs[cp_kl + 1] - b->h_pair_locs[cp_kl], out->chunk);
+    out->nrun = b->h_nrun[v][cp_ij];
+    out->ent = b->d_ent + b->h_pair_locs[cp_ij];
+    out->run0 = b->d_run0 + b->h_run_off[v][cp_ij];
+    return 1;
+}
+
+int jk_internal_run_items(const JKRunTab& rt, const int* ehi, long long* ioff, long long* itm, void* stream) {
+    cudaStream_t st = (cudaStream_t)stream;
+    if (rt.nrun > 0) jk_run_items_kernel<<<(rt.nrun + 255) / 256, 256, 0, st>>>(rt.nrun, rt.chunk, rt.run0, ehi, ioff);
+    jk_run_scan1_kernel<<<1, 1024, 0, st>>>(rt.nrun, ioff, itm);
+    CUDA_TRY(cudaGetLastError());
     return JK_OK;
 }
 
 int jk_internal_class_index(const jk_basis_t* b, int cp_ij, int cp_kl) { return class_index(b, cp_ij, cp_kl); }
 
-jk_launch_batch_fn jk_internal_batch_launcher(int class_idx, int fp32) {
+jk_launch_fn jk_internal_launcher(int class_idx, int fp32) {
     init_tables();
-    return fp32 ? g_tabs.b32[class_idx] : g_tabs.b64[class_idx];
+    return fp32 ? g_tab32[class_idx] : g_tab64[class_idx];
 }
 
 int jk_internal_class_team(int class_idx) {
@@ -1383,16 +1701,38 @@ int jk_internal_class_team(int class_idx) {
     return g_tabs.team[class_idx];
 }
 
+int jk_internal_class_run(int class_idx) {
+    init_tables();
+    return g_tabs.run[class_idx];
+}
+
 jk_fill_fn jk_internal_fill_launcher(int class_idx) {
     init_tables();
     return g_tabs.fill[class_idx];
 }
 
-void jk_internal_fill_seg_batch(const jk_basis_t* b, int c, const double* dm, int n_dm, double* vj, double* vk,
-                                int fp32, JKSeg* out) {
+void jk_internal_fill_seg_cq(const jk_basis_t* b, int c, int fp32, JKSeg* out) {
     const JKScreenCQ& cq = b->h_cq[c];
-    fill_seg(b, cq.cp_ij, cq.cp_kl, fp32 ? cq.qoff32 : cq.qoff, cq.n_ij, dm, n_dm, vj, vk, out);
-    if (fp32) out->kl_base = cq.klb;
+    fill_seg(b, cq.cp_ij, cq.cp_kl, cq.runs ? nullptr : (fp32 ? cq.qoff32 : cq.qoff), cq.n_ij, nullptr, 0, nullptr,
+             nullptr, out);
+    if (cq.runs) {
+        out->nrun = cq.nrun;
+        out->ent = cq.ent;
+        out->run0 = cq.run0;
+        out->elo = fp32 ? cq.klb : nullptr;
+        out->ehi = fp32 ? cq.kle : cq.klb;
+        out->ioff = fp32 ? cq.ioff32 : cq.ioff;
+    } else if (fp32) {
+        out->kl_base = cq.klb;
+    }
+}
+
+// pack record of one molecule: dens holds 2 n_dm packed densities (dp, dpb),
+// acc as many accumulators (jp, jpb)
+JKPackMol jk_internal_pack_mol(const jk_basis_t* b, const double* dm, int n_dm, double* dens, double* acc, double* vj) {
+    const size_t n = (size_t)n_dm * b->pack_total;
+    return JKPackMol{b->d_pack, b->ncp, b->pack_total, b->d_pair2bra, b->d_pair2ket, b->d_ao_loc, b->d_inv,
+                     dm,        b->nao, n_dm,          dens,          dens + n,      acc,         acc + n,  vj};
 }
 
 int jk_internal_pack_batch(const JKPackMol* d_mols, int nmol, long long max_total, int mode, void* stream) {
@@ -1406,7 +1746,23 @@ int jk_internal_pack_batch(const JKPackMol* d_mols, int nmol, long long max_tota
 int jk_internal_screen(const JKScreenCQ* d_cq, int ncq, double tol, int nbins, int prescreen, double fp32_cutoff,
                        void* stream) {
     if (ncq <= 0) return JK_OK;
-    jk_screen_kernel<<<ncq, 256, 0, (cudaStream_t)stream>>>(d_cq, tol, nbins, prescreen, fp32_cutoff);
+    cudaStream_t st = (cudaStream_t)stream;
+    jk_screen_kernel<<<ncq, 256, 0, st>>>(d_cq, tol, nbins, prescreen, fp32_cutoff);
+    // enough blocks for a large class, few enough that small ones (their
+    // surplus blocks leave at once) stay cheap
+    const unsigned by = ncq <= 64 ? 512 : (ncq <= 1024 ? 64 : 16);
+    jk_run_bounds_kernel<<<dim3(ncq, by), 256, 0, st>>>(d_cq, tol, nbins, prescreen, fp32_cutoff);
+    jk_run_scan_kernel<<<ncq, 1024, 0, st>>>(d_cq);
+    CUDA_TRY(cudaGetLastError());
+    return JK_OK;
+}
+
+int jk_internal_dm_cond(const JKDmCond* d_mols, int nmol, int max_groups, int max_nao, void* stream) {
+    if (nmol <= 0) return JK_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    jk_zero_kernel<<<nmol, 256, 0, st>>>(d_mols);
+    const unsigned bx = std::min(16u, dm_cond_blocks(max_nao));
+    jk_dm_cond_kernel<<<dim3(bx, max_groups, nmol), 256, 0, st>>>(JKDmCond{}, d_mols);
     CUDA_TRY(cudaGetLastError());
     return JK_OK;
 }

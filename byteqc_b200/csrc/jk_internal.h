@@ -3,39 +3,59 @@
 #pragma once
 #include <cublas_v2.h>
 
+#include <map>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "jk_common.cuh"
 #include "../../include/byteqc_jk.h"
 
-// One class quartet (cp_ij >= cp_kl) of one basis, as the screening kernel
-// sees it: pair counts, group indices and the device buffers it reads/writes.
+// One class quartet (cp_ij >= cp_kl) of one basis, as the screening kernels
+// see it: pair counts, group indices and the device buffers they read/write.
+// Classes of the run kernels (runs != 0) get per-entry ket bounds and an item
+// prefix over their runs, the others a task prefix over their rows.
 struct JKScreenCQ {
     int cp_ij, cp_kl;
     int gi, gj, gk, gl;
     int n_ij, n_kl;
     int ngroups;
+    int runs, nrun;               // ket pairs of an item (0: row class), runs
     const double *lq_ij, *lq_kl;  // clipped log q of the two classes
     const double *rq_ij, *rq_kl;  // unclipped log q (mixed-precision split)
     const double* dm_cond;        // ngroups x ngroups
-    long long *qoff, *qoff32;     // row prefixes, FP64 and FP32 parts
-    int* klb;                     // first FP32 column per row
-    long long *task0, *task032;   // {0, count} of each part
+    // rows: prefixes of the FP64 and FP32 parts and the first FP32 column
+    long long *qoff, *qoff32;
+    int* klb;                     // (run classes: per entry, the end of the FP64 part)
+    // runs: the run table, the end of the FP32 part per entry, item prefixes
+    const int *ent, *run0;
+    int* kle;
+    long long *ioff, *ioff32;
+    long long *itm, *itm32;       // {0, items} of each part
+    long long *task0, *task032;   // {0, quartets} of each part
     // host bookkeeping
     int pair_ij0, pair_kl0;
-    long long qoff_off;
+    int level;                    // run length of the table (JK_RUN_LEVELS)
 };
-
 
 int jk_internal_set_err(int code, const char* msg);
 // pair counts of the two classes and the working-basis size
 int jk_internal_class_info(const jk_basis_t* b, int cp_ij, int cp_kl, int* n_ij, int* n_kl, int* nao);
-void jk_internal_fill_seg(const jk_basis_t* b, int cp_ij, int cp_kl, const long long* qoff, int n_ij,
-                          const double* dm, int n_dm, double* vj, double* vk, JKSeg* out);
-// launch the class kernel of (cp_ij, cp_kl) on a device segment table of one entry
-int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg& seg, const long long* d_task0,
-                       long long max_tasks, void* stream);
+// Per-class-pair launch with caller-owned scratch: the segment goes by value
+// to *d_seg, then the class kernel runs on it.  task0: {0, count} as written
+// by the row-prefix kernel (row classes) or the run scan (run classes).
+int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg& seg, JKSeg* d_seg,
+                       const long long* task0, long long max_tasks, void* stream);
+// run table of the class pair as bra at the per-class-pair entries' run
+// length; 0 rows if the class quartet does not run a run kernel
+struct JKRunTab {
+    int nrun, chunk;  // runs, ket pairs of an item
+    const int *ent, *run0;
+};
+int jk_internal_run_table(const jk_basis_t* b, int cp_ij, int cp_kl, JKRunTab* out);
+// item counts per run from the entries' ket ends (ioff[0..nrun)), then their
+// exclusive prefix in place and itm = {0, total}
+int jk_internal_run_items(const JKRunTab& rt, const int* ehi, long long* ioff, long long* itm, void* stream);
 
 // Side streams of the class launches.  Every class kernel adds into J and K
 // with atomics, so launches of different class quartets (and the FP64 and
@@ -94,13 +114,51 @@ struct JKPackMol {
     const JKPackCls* cls;
     int ncls;
     long long total;
-    const int *pair2bra, *pair2ket, *ao_loc;
+    const int *pair2bra, *pair2ket, *ao_loc, *inv;
     const double* dm;
     int nao, n_dm;
-    double* dp;        // mode 0 output
-    const double* jp;  // mode 1 input
+    double *dp, *dpb;  // mode 0 output
+    double *jp, *jpb;  // mode 1 input
     double* vj;        // mode 1 output
 };
+
+// run lengths a run table exists for: long runs save more traffic, short ones
+// give a small molecule enough items to fill the device
+#define JK_RUN_LEVELS 3
+static const int JK_RUN_LEN[JK_RUN_LEVELS] = {32, 8, 2};
+
+// Class launches of a set of class quartets: one key per class (for the team
+// kernels per class and pair of primitive counts), its class quartets as
+// segments of one launch.
+struct JKPlanKey {
+    int cls, np_ij, np_kl;                  // np_* = -1: any primitive count
+    std::vector<std::pair<int, int>> segs;  // (molecule, class quartet)
+    std::vector<long long> seg_tasks;       // unscreened quartets of each segment
+    long long max_tasks = 0;                // their sum
+    long long max_items = 0;                // bound of the launch's task or item count
+    bool solo = false;                      // a class quartet launched on its own
+    JKBatchCfg cfg[2] = {{nullptr, 0, 1}, {nullptr, 0, 1}};  // FP64 part, FP32 part (queue set at launch)
+    float tuned_ms[2] = {-1.f, -1.f};
+};
+struct JKPlan {
+    std::vector<JKPlanKey> keys;
+    std::map<std::tuple<int, int, int>, int> index;  // key of a class while the plan is put together
+    std::vector<int> key_off;  // nkeys + 1 segment offsets
+    int nseg = 0, nshards = 1, shard = 0;
+    JKSeg* d_seg[2] = {nullptr, nullptr};        // FP64, FP32 parts
+    long long* d_segt[2] = {nullptr, nullptr};   // task prefix per key: nseg + nkeys entries
+    const long long** d_cnt[2] = {nullptr, nullptr};
+    int* d_key_off = nullptr;
+    unsigned long long* d_queue = nullptr;       // 2 work counters per key (persistent launches)
+};
+void jk_plan_free(JKPlan* p);
+// adds class quartet c of basis b (molecule m) to its key
+int jk_plan_add(JKPlan* p, const jk_basis* b, int m, int c, bool solo);
+// orders the keys (merged ones first) and segments, uploads the tables
+int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols);
+// exclusive prefixes of the segments' task counts (after the screening)
+int jk_plan_prefix(const JKPlan* p, bool mixed, cudaStream_t st);
+int jk_plan_launch(const JKPlan* p, int k, int part, const JKBatchCfg& cfg, int n_dm, int nsm, cudaStream_t st);
 
 // Per-geometry state (opaque to callers of the C-ABI)
 struct jk_basis {
@@ -116,8 +174,15 @@ struct jk_basis {
     std::vector<double> h_cq_cost;     // unscreened work of each class quartet (shard plans)
     std::vector<int> h_cq_owner;       // owner of each class quartet in the plan of
     int cq_owner_n = 0;                // cq_owner_n shards
-    std::vector<long long> h_qoff_off;
-    long long qoff_total = 0;
+    long long qoff_total = 0, ioff_total = 0, ent_total = 0;
+    // Runs of the bra pairs of each class (jk_runs.cuh): entry e of class c is
+    // pair d_ent[pair_locs[c] + e] of the class; run table v (run length
+    // JK_RUN_LEN[v]) of class c has h_nrun[v][c] runs at d_run0 + h_run_off[v][c]
+    std::vector<int> h_nrun[JK_RUN_LEVELS], h_run_off[JK_RUN_LEVELS];
+    int *d_ent = nullptr, *d_run0 = nullptr;
+    int* d_inv = nullptr;  // entry of a pair (the inverse of d_ent)
+    double *d_bprim = nullptr, *d_bpair = nullptr;  // bra records (JKSeg::bprim, bpair)
+    float* d_bprimf = nullptr;
     // device
     int *d_atm = nullptr, *d_bas = nullptr, *d_ao_loc = nullptr, *d_group_ao = nullptr;
     double *d_env = nullptr, *d_bas_x = nullptr, *d_qcond = nullptr;
@@ -126,13 +191,22 @@ struct jk_basis {
     float* d_primf = nullptr;  // FP32 path: a12|1/a12|e12/a12|P-R_bra (x, y, z)
     long long nprim_total = 0;
     JKScreenCQ* d_cq = nullptr;
-    long long *d_qoff = nullptr, *d_task0 = nullptr;
-    long long *d_qoff32 = nullptr, *d_task032 = nullptr;  // FP32 part of the mixed mode
+    long long *d_qoff = nullptr, *d_qoff32 = nullptr;  // FP64, FP32 part of the mixed mode
+    long long* d_ioff = nullptr;                       // item prefixes, both parts
     int* d_klb = nullptr;
+    int* d_kle = nullptr;
+    // zeroed at the start of a build, in one piece: the condensed density,
+    // then task0, task032, itm, itm32 of every class quartet
+    void* d_zero = nullptr;
+    size_t zero_bytes = 0;
     double* d_dm_cond = nullptr;
+    long long *d_task0 = nullptr, *d_task032 = nullptr;
+    JKPlan* plan = nullptr;  // class launches of jk_build
     // reference-compatible single class-pair path
     long long* d_qoff1 = nullptr;
     long long* d_task01 = nullptr;
+    int* d_ehi1 = nullptr;
+    JKSeg* d_seg1 = nullptr;
     long long qoff1_cap = 0;
     JKFanout fan;  // side streams of the class launches
     double* d_pgeo = nullptr;  // pair geometry (JKSeg::pgeo)
@@ -143,7 +217,7 @@ struct jk_basis {
     std::vector<JKPackCls> h_pack;
     JKPackCls* d_pack = nullptr;
     long long pack_total = 0;  // packed elements per density
-    double* d_pk = nullptr;    // n_dm x pack_total densities, then as many J accumulators
+    double* d_pk = nullptr;    // 2 n_dm x pack_total densities, then as many J accumulators
     size_t pk_cap = 0;
     // transform workspace
     cublasHandle_t blas = nullptr;
@@ -151,17 +225,27 @@ struct jk_basis {
     size_t work_cap = 0;
 };
 
-// launch one class quartet of basis b as a single segment
 int jk_internal_class_index(const jk_basis_t* b, int cp_ij, int cp_kl);
-// the single-segment launch of a class (FP64 part or FP32 part), as jk_build makes it
-int jk_internal_launch_part(int class_idx, int fp32, const JKSeg& seg, const long long* d_task0, long long max_tasks,
-                            int nsm, void* stream);
-jk_launch_batch_fn jk_internal_batch_launcher(int class_idx, int fp32);
+jk_launch_fn jk_internal_launcher(int class_idx, int fp32);
 // 1 if the class runs a team kernel (one primitive count per launch)
 int jk_internal_class_team(int class_idx);
-void jk_internal_fill_seg_batch(const jk_basis_t* b, int c, const double* dm, int n_dm, double* vj, double* vk,
-                                int fp32, JKSeg* out);
+int jk_internal_class_run(int class_idx);
+void jk_internal_fill_seg(const jk_basis_t* b, int cp_ij, int cp_kl, const long long* qoff, int n_ij,
+                          const double* dm, int n_dm, double* vj, double* vk, JKSeg* out);
+// segment of class quartet c, FP64 or FP32 part (no density, no outputs)
+void jk_internal_fill_seg_cq(const jk_basis_t* b, int c, int fp32, JKSeg* out);
+JKPackMol jk_internal_pack_mol(const jk_basis_t* b, const double* dm, int n_dm, double* dens, double* acc, double* vj);
 // pack (mode 0) or unpack (mode 1) the J side of nmol molecules (device table)
 int jk_internal_pack_batch(const JKPackMol* d_mols, int nmol, long long max_total, int mode, void* stream);
+// condensed densities (outputs zeroed first) of nmol molecules (device table)
+struct JKDmCond {
+    const double* dm;
+    const int* gao;  // group AO offsets (device)
+    double* out;     // ngroups x ngroups
+    int nao, n_dm, ngroups;
+    unsigned long long* zero;  // words cleared before the condensation (jk_basis::d_zero)
+    int nzero;
+};
+int jk_internal_dm_cond(const JKDmCond* d_mols, int nmol, int max_groups, int max_nao, void* stream);
 int jk_internal_screen(const JKScreenCQ* d_cq, int ncq, double tol, int nbins, int prescreen, double fp32_cutoff,
                        void* stream);

@@ -5,13 +5,12 @@
 //
 // Work unit: one screened contracted shell quartet (ij|kl) of one segment.
 // All primitive quartets and roots of it are summed in registers before the
-// quartet's contribution to J and K is formed, so every J/K element of the
-// quartet is written with one atomic, instead of one per primitive and root.
+// quartet's contribution to J and K is formed.
 //
 // Two execution shapes, fixed per class at compile time (JKClass::P):
 //   P = 0  one thread per quartet; the 2D integrals of one root live in
-//          registers and all NF Cartesian products accumulate in registers;
-//          the digestion goes straight to global atomics;
+//          registers and all NF Cartesian products accumulate in registers
+//          (the digestion is in jk_runs.cuh);
 //   P > 0  a team of T threads per quartet: the 3*NROOTS (axis, root) 2D
 //          blocks are built cooperatively in shared memory, each thread owns
 //          the leading P Cartesian indices (i, or i and j) and accumulates the
@@ -215,7 +214,7 @@ __device__ __forceinline__ JKPrim jk_prim2(const JKPP& b, const JKPP& k) {
 }
 
 // build the 2D block of (axis d, root r) into out (strides XSI, XSJ of i, j)
-template <class C, typename R, int XSI = C::SI, int XSJ = C::SJ, typename OutT>
+template <class C, typename R, int XSI = C::SI, int XSJ = C::SJ, bool KET = true, typename OutT>
 __device__ __forceinline__ void jk_unit(const JKPrim& p, double s, double w, int d, double norm, const double* ri,
                                         const double* rj, const double* rk, const double* rl, OutT* out) {
     // select by d without dynamic indexing (keeps everything in registers)
@@ -231,7 +230,7 @@ __device__ __forceinline__ void jk_unit(const JKPrim& p, double s, double w, int
     double c00 = (Pd - Rid) - bs * pq;
     double c0p = (Qd - Rkd) + as * pq;
     double seed = d == 0 ? norm : (d == 1 ? p.sy : w);
-    rys_2d<R, C, XSI, XSJ>((R)seed, (R)c00, (R)c0p, (R)b10, (R)b01, (R)b00, (R)(Rid - Rjd), (R)(Rkd - Rld), out);
+    rys_2d<R, C, XSI, XSJ, KET>((R)seed, (R)c00, (R)c0p, (R)b10, (R)b01, (R)b00, (R)(Rid - Rjd), (R)(Rkd - Rld), out);
 }
 
 // ---------------------------------------------------------------------------
@@ -283,7 +282,7 @@ __device__ __forceinline__ JKPrimF jk_prim_f2(const JKPPF& b, const JKPPF& k, co
     return p;
 }
 
-template <class C, int XSI = C::SI, int XSJ = C::SJ, typename OutT>
+template <class C, int XSI = C::SI, int XSJ = C::SJ, bool KET = true, typename OutT>
 __device__ __forceinline__ void jk_unit_f(const JKPrimF& p, float s, float w, int d, float norm, const float* dij,
                                           const float* dkl, OutT* out) {
     float siAB = s * p.iAB;
@@ -295,7 +294,7 @@ __device__ __forceinline__ void jk_unit_f(const JKPrimF& p, float s, float w, in
     float c00 = JK_PICK(p.PA) - bs * pq;
     float c0p = JK_PICK(p.QC) + as * pq;
     float seed = d == 0 ? norm : (d == 1 ? p.sy : w);
-    rys_2d<float, C, XSI, XSJ>(seed, c00, c0p, b10, b01, b00, JK_PICK(dij), JK_PICK(dkl), out);
+    rys_2d<float, C, XSI, XSJ, KET>(seed, c00, c0p, b10, b01, b00, JK_PICK(dij), JK_PICK(dkl), out);
 }
 #undef JK_PICK
 
@@ -323,177 +322,6 @@ __device__ __forceinline__ void load_pair_centres(const JKSeg& sg, int p, double
 // run NPASS passes over the primitive quartets (the 2D blocks are rebuilt
 // per pass, the accumulators of one pass only are live).
 // ===========================================================================
-// ---------------------------------------------------------------------------
-// Digestion of one quartet's Cartesian block (bra components ci in
-// [CI0, CI0 + NI)) into J and K through a sink:
-//   J_ij += (ij|kl) D_kl, J_kl += (ij|kl) D_ij,
-//   K_ik += (ij|kl) D_jl, K_il += (ij|kl) D_jk, K_jk += (ij|kl) D_il,
-//   K_jl += (ij|kl) D_ik
-// (cuobc/lib/gvhf/contract_jk.cu:225-316).  JKSinkGlobal adds every element
-// to the output buffers with one global atomic, element (a, b) at a + nao*b;
-// JKSinkSmem adds into the shared-memory blocks of a tile.
-// ---------------------------------------------------------------------------
-struct JKSinkGlobal {
-    double* vj;
-    double* vk;
-    int nao;
-    size_t nn;
-    __device__ __forceinline__ void jij(int idm, int a, int b, double v) const {
-        atomicAdd(vj + idm * nn + a + (size_t)nao * b, v);
-    }
-    __device__ __forceinline__ void jkl(int idm, int a, int b, double v) const {
-        atomicAdd(vj + idm * nn + a + (size_t)nao * b, v);
-    }
-    __device__ __forceinline__ void kik(int idm, int a, int b, double v) const {
-        atomicAdd(vk + idm * nn + a + (size_t)nao * b, v);
-    }
-    __device__ __forceinline__ void kil(int idm, int a, int b, double v) const { kik(idm, a, b, v); }
-    __device__ __forceinline__ void kjk(int idm, int a, int b, double v) const { kik(idm, a, b, v); }
-    __device__ __forceinline__ void kjl(int idm, int a, int b, double v) const { kik(idm, a, b, v); }
-};
-
-__device__ __forceinline__ JKSinkGlobal jk_sink_global(const JKSeg& sg) {
-    return JKSinkGlobal{sg.vj, sg.vk, sg.nao, (size_t)sg.nao * sg.nao};
-}
-
-template <class C, typename R, int NI, class Sink>
-__device__ __forceinline__ void jk_thread_digest(const JKSeg& sg, const JKQuartet& q, int CI0, const R* acc,
-                                                 const Sink& sink) {
-    const int nao = sg.nao;
-    const int i0 = q.i0 + CI0, j0 = q.j0;
-    const int k0 = q.k0, l0 = q.l0;
-    // the lanes of a warp usually share the ij pair (consecutive kl of one
-    // row): then the J_ij block is summed over the warp before it is added.
-    // In a batched launch a warp can straddle two molecules whose pairs
-    // carry the same indices, so the lanes must also share the output.
-    const unsigned am = __activemask();
-    bool wsame = false;
-    if (am == 0xffffffffu) {
-        const unsigned long long out = (unsigned long long)(sg.jp_ij ? (const void*)sg.jp_ij : (const void*)sg.vj);
-        const int p_0 = __shfl_sync(am, q.bij, 0);
-        unsigned long long o_0 = __shfl_sync(am, out, 0);
-        wsame = __all_sync(am, q.bij == p_0 && out == o_0);
-    }
-#define ACC(i, j, k, l) ((double)acc[(((i) * C::NFJ + (j)) * C::NFK + (k)) * C::NFL + (l)])
-    for (int idm = 0; idm < sg.n_dm; idm++) {
-        const double* D = sg.dm + (size_t)idm * nao * nao;
-        if (sg.vj && sg.dp_ij) {
-            // pair-packed: consecutive lanes hold consecutive kl pairs, so the
-            // D_kl loads and the J_kl additions are coalesced
-            const size_t po = (size_t)idm * sg.pk_stride;
-            const double* Dij = sg.dp_ij + po + q.row;
-            const double* Dkl = sg.dp_kl + po + q.col;
-#pragma unroll
-            for (int i = 0; i < NI; i++)
-#pragma unroll
-                for (int j = 0; j < C::NFJ; j++) {
-                    double v = 0;
-#pragma unroll
-                    for (int k = 0; k < C::NFK; k++)
-#pragma unroll
-                        for (int l = 0; l < C::NFL; l++)
-                            v += ACC(i, j, k, l) * __ldg(Dkl + (size_t)(k * C::NFL + l) * sg.np_kl);
-                    double* J = sg.jp_ij + po + (size_t)((CI0 + i) * C::NFJ + j) * sg.np_ij + q.row;
-                    if (wsame) {
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                        if ((threadIdx.x & 31) == 0) atomicAdd(J, v);
-                    } else {
-                        atomicAdd(J, v);
-                    }
-                }
-#pragma unroll
-            for (int k = 0; k < C::NFK; k++)
-#pragma unroll
-                for (int l = 0; l < C::NFL; l++) {
-                    double v = 0;
-#pragma unroll
-                    for (int i = 0; i < NI; i++)
-#pragma unroll
-                        for (int j = 0; j < C::NFJ; j++)
-                            v += ACC(i, j, k, l) * __ldg(Dij + (size_t)((CI0 + i) * C::NFJ + j) * sg.np_ij);
-                    atomicAdd(sg.jp_kl + po + (size_t)(k * C::NFL + l) * sg.np_kl + q.col, v);
-                }
-        } else if (sg.vj) {
-#pragma unroll
-            for (int i = 0; i < NI; i++)
-#pragma unroll
-                for (int j = 0; j < C::NFJ; j++) {
-                    double v = 0;
-#pragma unroll
-                    for (int k = 0; k < C::NFK; k++)
-#pragma unroll
-                        for (int l = 0; l < C::NFL; l++) v += ACC(i, j, k, l) * DM(k0 + k, l0 + l);
-                    if (wsame) {
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                        if ((threadIdx.x & 31) == 0) sink.jij(idm, i0 + i, j0 + j, v);
-                    } else {
-                        sink.jij(idm, i0 + i, j0 + j, v);
-                    }
-                }
-#pragma unroll
-            for (int k = 0; k < C::NFK; k++)
-#pragma unroll
-                for (int l = 0; l < C::NFL; l++) {
-                    double v = 0;
-#pragma unroll
-                    for (int i = 0; i < NI; i++)
-#pragma unroll
-                        for (int j = 0; j < C::NFJ; j++) v += ACC(i, j, k, l) * DM(i0 + i, j0 + j);
-                    sink.jkl(idm, k0 + k, l0 + l, v);
-                }
-        }
-        if (sg.vk) {
-#pragma unroll
-            for (int i = 0; i < NI; i++)
-#pragma unroll
-                for (int k = 0; k < C::NFK; k++) {
-                    double v = 0;
-#pragma unroll
-                    for (int j = 0; j < C::NFJ; j++)
-#pragma unroll
-                        for (int l = 0; l < C::NFL; l++) v += ACC(i, j, k, l) * DM(l0 + l, j0 + j);
-                    sink.kik(idm, i0 + i, k0 + k, v);
-                }
-#pragma unroll
-            for (int i = 0; i < NI; i++)
-#pragma unroll
-                for (int l = 0; l < C::NFL; l++) {
-                    double v = 0;
-#pragma unroll
-                    for (int j = 0; j < C::NFJ; j++)
-#pragma unroll
-                        for (int k = 0; k < C::NFK; k++) v += ACC(i, j, k, l) * DM(k0 + k, j0 + j);
-                    sink.kil(idm, i0 + i, l0 + l, v);
-                }
-#pragma unroll
-            for (int j = 0; j < C::NFJ; j++)
-#pragma unroll
-                for (int k = 0; k < C::NFK; k++) {
-                    double v = 0;
-#pragma unroll
-                    for (int i = 0; i < NI; i++)
-#pragma unroll
-                        for (int l = 0; l < C::NFL; l++) v += ACC(i, j, k, l) * DM(l0 + l, i0 + i);
-                    sink.kjk(idm, j0 + j, k0 + k, v);
-                }
-#pragma unroll
-            for (int j = 0; j < C::NFJ; j++)
-#pragma unroll
-                for (int l = 0; l < C::NFL; l++) {
-                    double v = 0;
-#pragma unroll
-                    for (int i = 0; i < NI; i++)
-#pragma unroll
-                        for (int k = 0; k < C::NFK; k++) v += ACC(i, j, k, l) * DM(k0 + k, i0 + i);
-                    sink.kjl(idm, j0 + j, l0 + l, v);
-                }
-        }
-    }
-#undef ACC
-}
-
 // acc[i][j][k][l] += Ix Iy Iz for the bra components ci in [CI0, CI0 + NI)
 template <class C, typename R, int CI0, int NI>
 __device__ __forceinline__ void jk_thread_products(R* acc, const R* Ix, const R* Iy, const R* Iz) {
@@ -515,190 +343,98 @@ __device__ __forceinline__ void jk_thread_products(R* acc, const R* Ix, const R*
                 }
 }
 
-template <class C, typename R, int CI0, int CI1, class Sink>
-__device__ __forceinline__ void jk_thread_pass(const JKSeg& sg, const JKQuartet& q, const double* __restrict__ tab,
-                                               const double* ri, const double* rj, const double* rk,
-                                               const double* rl, const Sink& sink, const JKFillOut* fo) {
+// one pass of the ERI-tensor fill (FP64): the bra components [CI0, CI1) of
+// the quartet's block go to the tensor
+template <class C, int CI0, int CI1>
+__device__ __forceinline__ void jk_thread_fill_pass(const JKSeg& sg, const JKQuartet& q,
+                                                    const double* __restrict__ tab, const double* ri, const double* rj,
+                                                    const double* rk, const double* rl, const JKFillOut& fo) {
     constexpr int NR = C::NROOTS;
     constexpr int NI = CI1 - CI0;
     constexpr int NA = NI * C::NFJ * C::NFK * C::NFL;
-    R acc[NA];
+    double acc[NA];
 #pragma unroll
-    for (int e = 0; e < NA; e++) acc[e] = R(0);
-    if constexpr (JKF32Prim<C, R>::value) {
-        const float* tabf = reinterpret_cast<const float*>(tab);
-        float dij[3], dkl[3], ac[3];
+    for (int e = 0; e < NA; e++) acc[e] = 0.;
+    const int npij = sg.pnp ? __ldg(sg.pnp + q.bij) : sg.nprim_ij;
+    const int npkl = sg.pnp ? __ldg(sg.pnp + q.bkl) : sg.nprim_kl;
+    JKPP kn = jk_pp(sg, q.prim_kl);
+    for (int kp = 0; kp < npkl; kp++) {
+        const JKPP kc = kn;
+        if (kp + 1 < npkl) kn = jk_pp(sg, q.prim_kl + (kp + 1) * sg.pst_kl);  // next ket primitive, in flight
+        for (int ip = 0; ip < npij; ip++) {
+            JKPrim p = jk_prim2(jk_pp(sg, q.prim_ij + ip * sg.pst_ij), kc);
+            double rs[NR], rw[NR];
+            rys_roots_all<NR>(tab, p.x, rs, rw);
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            dij[d] = (float)(ri[d] - rj[d]);
-            dkl[d] = (float)(rk[d] - rl[d]);
-            ac[d] = (float)(ri[d] - rk[d]);
-        }
-        const float normf = (float)q.norm;
-        const int npij = sg.pnp ? __ldg(sg.pnp + q.bij) : sg.nprim_ij;
-        const int npkl = sg.pnp ? __ldg(sg.pnp + q.bkl) : sg.nprim_kl;
-        JKPPF kn = jk_ppf(sg, q.prim_kl);
-        for (int kp = 0; kp < npkl; kp++) {
-            const JKPPF kc = kn;
-            if (kp + 1 < npkl) kn = jk_ppf(sg, q.prim_kl + (kp + 1) * sg.pst_kl);  // next ket primitive, in flight
-            for (int ip = 0; ip < npij; ip++) {
-                JKPrimF p = jk_prim_f2(jk_ppf(sg, q.prim_ij + ip * sg.pst_ij), kc, ac);
-                float rs[NR], rw[NR];
-                rys_roots_all_f<NR>(tabf, p.x, rs, rw);
-#pragma unroll
-                for (int r = 0; r < NR; r++) {
-                    float Ix[C::GS], Iy[C::GS], Iz[C::GS];
-                    jk_unit_f<C>(p, rs[r], rw[r], 0, normf, dij, dkl, Ix);
-                    jk_unit_f<C>(p, rs[r], rw[r], 1, normf, dij, dkl, Iy);
-                    jk_unit_f<C>(p, rs[r], rw[r], 2, normf, dij, dkl, Iz);
-                    jk_thread_products<C, R, CI0, NI>(acc, Ix, Iy, Iz);
-                }
-            }
-        }
-    } else {
-        const int npij = sg.pnp ? __ldg(sg.pnp + q.bij) : sg.nprim_ij;
-        const int npkl = sg.pnp ? __ldg(sg.pnp + q.bkl) : sg.nprim_kl;
-        JKPP kn = jk_pp(sg, q.prim_kl);
-        for (int kp = 0; kp < npkl; kp++) {
-            const JKPP kc = kn;
-            if (kp + 1 < npkl) kn = jk_pp(sg, q.prim_kl + (kp + 1) * sg.pst_kl);  // next ket primitive, in flight
-            for (int ip = 0; ip < npij; ip++) {
-                JKPrim p = jk_prim2(jk_pp(sg, q.prim_ij + ip * sg.pst_ij), kc);
-                double rs[NR], rw[NR];
-                rys_roots_all<NR>(tab, p.x, rs, rw);
-#pragma unroll
-                for (int r = 0; r < NR; r++) {
-                    const double s = rs[r], w = rw[r];
-                    R Ix[C::GS], Iy[C::GS], Iz[C::GS];
-                    jk_unit<C, R>(p, s, w, 0, q.norm, ri, rj, rk, rl, Ix);
-                    jk_unit<C, R>(p, s, w, 1, q.norm, ri, rj, rk, rl, Iy);
-                    jk_unit<C, R>(p, s, w, 2, q.norm, ri, rj, rk, rl, Iz);
-                    jk_thread_products<C, R, CI0, NI>(acc, Ix, Iy, Iz);
-                }
+            for (int r = 0; r < NR; r++) {
+                const double s = rs[r], w = rw[r];
+                double Ix[C::GS], Iy[C::GS], Iz[C::GS];
+                jk_unit<C, double>(p, s, w, 0, q.norm, ri, rj, rk, rl, Ix);
+                jk_unit<C, double>(p, s, w, 1, q.norm, ri, rj, rk, rl, Iy);
+                jk_unit<C, double>(p, s, w, 2, q.norm, ri, rj, rk, rl, Iz);
+                jk_thread_products<C, double, CI0, NI>(acc, Ix, Iy, Iz);
             }
         }
     }
-    if (fo) {  // ERI-tensor fill: the quartet's block goes to the tensor
-        const long long b0 = (long long)(q.i0 + CI0 - fo->off[0]) * fo->st[0] +
-                             (long long)(q.j0 - fo->off[1]) * fo->st[1] + (long long)(q.k0 - fo->off[2]) * fo->st[2] +
-                             (long long)(q.l0 - fo->off[3]) * fo->st[3];
+    const long long b0 = (long long)(q.i0 + CI0 - fo.off[0]) * fo.st[0] + (long long)(q.j0 - fo.off[1]) * fo.st[1] +
+                         (long long)(q.k0 - fo.off[2]) * fo.st[2] + (long long)(q.l0 - fo.off[3]) * fo.st[3];
 #pragma unroll
-        for (int i = 0; i < NI; i++)
+    for (int i = 0; i < NI; i++)
 #pragma unroll
-            for (int j = 0; j < C::NFJ; j++)
+        for (int j = 0; j < C::NFJ; j++)
 #pragma unroll
-                for (int k = 0; k < C::NFK; k++)
+            for (int k = 0; k < C::NFK; k++)
 #pragma unroll
-                    for (int l = 0; l < C::NFL; l++)
-                        atomicAdd(fo->eri + b0 + i * fo->st[0] + j * fo->st[1] + k * fo->st[2] + l * fo->st[3],
-                                  (double)acc[((i * C::NFJ + j) * C::NFK + k) * C::NFL + l]);
-        return;
-    }
-    jk_thread_digest<C, R, NI>(sg, q, CI0, acc, sink);
+                for (int l = 0; l < C::NFL; l++)
+                    atomicAdd(fo.eri + b0 + i * fo.st[0] + j * fo.st[1] + k * fo.st[2] + l * fo.st[3],
+                              acc[((i * C::NFJ + j) * C::NFK + k) * C::NFL + l]);
 }
 
-
-template <class C, typename R, int PASS, class Sink>
-__device__ __forceinline__ void jk_thread_passes(const JKSeg& sg, const JKQuartet& q, const double* __restrict__ tab,
-                                                 const double* ri, const double* rj, const double* rk,
-                                                 const double* rl, const Sink& sink, const JKFillOut* fo) {
+template <class C, int PASS>
+__device__ __forceinline__ void jk_thread_fill_passes(const JKSeg& sg, const JKQuartet& q,
+                                                      const double* __restrict__ tab, const double* ri,
+                                                      const double* rj, const double* rk, const double* rl,
+                                                      const JKFillOut& fo) {
     constexpr int CI0 = PASS * C::GI;
     if constexpr (CI0 < C::NFI) {
         constexpr int CI1 = CI0 + C::GI < C::NFI ? CI0 + C::GI : C::NFI;
-        jk_thread_pass<C, R, CI0, CI1>(sg, q, tab, ri, rj, rk, rl, sink, fo);
-        jk_thread_passes<C, R, PASS + 1>(sg, q, tab, ri, rj, rk, rl, sink, fo);
+        jk_thread_fill_pass<C, CI0, CI1>(sg, q, tab, ri, rj, rk, rl, fo);
+        jk_thread_fill_passes<C, PASS + 1>(sg, q, tab, ri, rj, rk, rl, fo);
     }
 }
 
-template <class C, typename R, class Sink>
-__device__ __forceinline__ void jk_thread_quartet(const JKSeg& sg, const JKQuartet& q, const double* __restrict__ tab,
-                                                  const Sink& sink, const JKFillOut* fo = nullptr) {
-    double ri[3], rj[3], rk[3], rl[3];
-    load_pair_centres(sg, q.bij, ri, rj);
-    load_pair_centres(sg, q.bkl, rk, rl);
-    jk_thread_passes<C, R, 0>(sg, q, tab, ri, rj, rk, rl, sink, fo);
-}
-
-// Resident 128-thread blocks asked of the register allocator (single-segment
-// kernel).  The FP32 quartets hold half-width values and spend more of their
-// time waiting on loads, so they get more resident warps; the batched kernel
-// keeps C::MINB (its segment cursor would spill).
-template <class C, typename R>
-struct JKThreadMinBlocks {
-    static constexpr int value = sizeof(R) == 4 ? (C::W <= 24 ? 8 : (C::W <= 40 ? 6 : 4)) : C::MINB;
-};
-
-template <class C, typename R, class Src>
-__device__ __forceinline__ void jk_thread_body(const Src& src, double* jk_tab, const JKFillOut* fo = nullptr) {
-    // each warp takes a contiguous chunk of tasks (a multiple of 32); lane i
-    // does tasks i, i+32, ... of it, so a warp covers consecutive kl of a row
-    const long long total = src.total();
-    const int lane = threadIdx.x & 31;
-    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-    const long long wid = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    unsigned long long* queue = src.queue();
-    const long long chunk = queue ? (long long)src.grab() : (((total + nwarps - 1) / nwarps) + 31) & ~31LL;
-    // static chunks: the grid is sized for the unscreened task count, and a
-    // block without any screened task leaves before it loads the Rys table
-    // (block-uniform test)
-    if (!queue && (long long)blockIdx.x * (blockDim.x >> 5) * chunk >= total) return;
-    if (queue && total == 0) return;
-    if constexpr (JKF32Prim<C, R>::value)
-        rys_table_to_smem_f<C::NROOTS>(src.first().rys, reinterpret_cast<float*>(jk_tab));
-    else
-        rys_table_to_smem<C::NROOTS>(src.first().rys, jk_tab);
-    __syncthreads();
-    long long c0 = wid * chunk;
-    for (;;) {
-        if (queue) {
-            unsigned long long g = 0;
-            if (lane == 0) g = atomicAdd(queue, (unsigned long long)chunk);
-            c0 = (long long)__shfl_sync(0xffffffffu, g, 0);
-        }
-        if (c0 >= total) break;
-        long long t = c0 + lane;
-        const long long tend = min(total, c0 + chunk);
-        if (t < tend) {
-            typename Src::Cursor cur;
-            cur.init(src, t);
-            for (; t < tend; t += 32) {
-                int row, col;
-                const JKSeg& sg = cur.seek(src, t, row, col);
-                JKQuartet q = jk_quartet_at(sg, row, col);
-                if (fo) q.norm = JK_FAC;  // the fill has no 1/2 on the ij == kl diagonal
-                jk_thread_quartet<C, R>(sg, q, jk_tab, jk_sink_global(sg), fo);
-            }
-        }
-        if (!queue) break;
-    }
-}
-
-template <class C, typename R>
-__global__ void __launch_bounds__(128, (JKThreadMinBlocks<C, R>::value)) jk_thread_kernel(const __grid_constant__ JKSeg sg,
-                                                                 const long long* __restrict__ task0) {
-    extern __shared__ __align__(16) double jk_tab[];
-    JKOneSeg src{sg, task0};
-    jk_thread_body<C, R>(src, jk_tab);
-}
-
-// ERI-tensor fill with the thread kernel's register recursion (FP64)
+// ERI-tensor fill, one thread per quartet.  Each warp takes a contiguous
+// chunk of tasks (a multiple of 32); lane i does tasks i, i+32, ... of it, so
+// a warp covers consecutive kl of a row.
 template <class C>
 __global__ void __launch_bounds__(128, C::MINB) jk_thread_fill_kernel(const __grid_constant__ JKSeg sg,
                                                                       const long long* __restrict__ task0,
                                                                       const __grid_constant__ JKFillOut out) {
     extern __shared__ __align__(16) double jk_tab[];
-    JKOneSeg src{sg, task0};
-    jk_thread_body<C, double>(src, jk_tab, &out);
-}
-
-template <class C, typename R>
-__global__ void __launch_bounds__(128, C::MINB) jk_thread_kernel_batch(const JKSeg* __restrict__ segs,
-                                                                       const long long* __restrict__ segt,
-                                                                       int nseg, unsigned long long* queue,
-                                                                       int grab) {
-    extern __shared__ __align__(16) double jk_tab[];
-    JKSegTable src{segs, segt, nseg, queue, grab};
-    jk_thread_body<C, R>(src, jk_tab);
+    const long long total = task0[1];
+    const int lane = threadIdx.x & 31;
+    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+    const long long wid = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const long long chunk = (((total + nwarps - 1) / nwarps) + 31) & ~31LL;
+    // the grid is sized for the unscreened task count, and a block without
+    // any task leaves before it loads the Rys table (block-uniform test)
+    if ((long long)blockIdx.x * (blockDim.x >> 5) * chunk >= total) return;
+    rys_table_to_smem<C::NROOTS>(sg.rys, jk_tab);
+    __syncthreads();
+    long long t = wid * chunk + lane;
+    const long long tend = min(total, (wid + 1) * chunk);
+    if (t >= tend) return;
+    JKTaskCursor cur;
+    cur.init(sg, t);
+    for (; t < tend; t += 32) {
+        const int col = cur.seek(sg, t);
+        JKQuartet q = jk_quartet_at(sg, cur.row, col);
+        q.norm = JK_FAC;  // the fill has no 1/2 on the ij == kl diagonal
+        double ri[3], rj[3], rk[3], rl[3];
+        load_pair_centres(sg, q.bij, ri, rj);
+        load_pair_centres(sg, q.bkl, rk, rl);
+        jk_thread_fill_passes<C, 0>(sg, q, jk_tab, ri, rj, rk, rl, out);
+    }
 }
 
 // ===========================================================================
@@ -1242,12 +978,6 @@ __device__ __forceinline__ void jk_team_body(const Src& src, const JKFillOut* fo
     if (!queue) break;
     }
 }
-template <class C, typename R>
-__global__ void jk_team_kernel(const __grid_constant__ JKSeg sg, const long long* __restrict__ task0) {
-    JKOneSeg src{sg, task0};
-    jk_team_body<C, R>(src);
-}
-
 // ERI-tensor fill with the team kernel's recursion (FP64)
 template <class C>
 __global__ void jk_team_fill_kernel(const __grid_constant__ JKSeg sg, const long long* __restrict__ task0,
@@ -1257,7 +987,7 @@ __global__ void jk_team_fill_kernel(const __grid_constant__ JKSeg sg, const long
 }
 
 template <class C, typename R>
-__global__ void jk_team_kernel_batch(const JKSeg* __restrict__ segs, const long long* __restrict__ segt, int nseg,
+__global__ void jk_team_kernel(const JKSeg* __restrict__ segs, const long long* __restrict__ segt, int nseg,
                                      unsigned long long* queue, int grab) {
     JKSegTable src{segs, segt, nseg, queue, grab};
     jk_team_body<C, R>(src);

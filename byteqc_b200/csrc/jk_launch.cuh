@@ -4,6 +4,7 @@
 #include <atomic>
 
 #include "jk_kernels.cuh"
+#include "jk_teams.cuh"
 
 // cudaFuncSetAttribute acts on the current device only, so the "already set"
 // flag of a kernel is kept per device (bit d of `done` for device d < 64;
@@ -20,33 +21,6 @@ cudaError_t jk_smem_attr(K kernel, size_t smem, std::atomic<unsigned long long>&
     return e;
 }
 
-
-// One class quartet (one segment): the segment descriptor goes by value into
-// the kernel's parameter space; task0[1] (device) holds the task count.
-template <int LI, int LJ, int LK, int LL, typename R>
-cudaError_t jk_launch(const JKSeg& seg, const long long* task0, long long max_tasks, int nsm, cudaStream_t st) {
-    using C = JKClass<LI, LJ, LK, LL>;
-    if (max_tasks <= 0) return cudaSuccess;
-    if constexpr (C::P == 0) {
-        constexpr size_t smem = RysS<C::NROOTS>::WORDS * sizeof(double);
-        static std::atomic<unsigned long long> attr_done{0};
-        if (cudaError_t e = jk_smem_attr(jk_thread_kernel<C, R>, smem, attr_done); e != cudaSuccess) return e;
-        long long want = (max_tasks + 127) / 128;
-        long long cap = (long long)nsm * 16;
-        int blocks = (int)(want < cap ? want : cap);
-        jk_thread_kernel<C, R><<<blocks, 128, smem, st>>>(seg, task0);
-    } else {
-        using S = JKTeamShape<C>;
-        constexpr size_t smem = jk_team_smem<C, R>();
-        static std::atomic<unsigned long long> attr_done{0};
-        if (cudaError_t e = jk_smem_attr(jk_team_kernel<C, R>, smem, attr_done); e != cudaSuccess) return e;
-        long long want = (max_tasks + S::QPB - 1) / S::QPB;
-        long long cap = (long long)nsm * 8;
-        int blocks = (int)(want < cap ? want : cap);
-        jk_team_kernel<C, R><<<blocks, S::THREADS, smem, st>>>(seg, task0);
-    }
-    return cudaGetLastError();
-}
 
 // resident blocks per SM of a kernel at a launch shape, looked up once per
 // device (bit d of `done`, the count in cnt[d])
@@ -65,46 +39,68 @@ int jk_resident_blocks(K kernel, int threads, size_t smem, std::atomic<unsigned 
     return nb;
 }
 
-// Batched launch: the segments of one class (same angular momenta and
-// primitive counts) of many molecules, task prefix segt[0..nseg] on the
-// device; static chunks or the persistent mode (JKBatchCfg).
+template <class C, typename R, bool MULTI>
+cudaError_t jk_launch_run(const JKSeg* segs, const long long* segt, int nseg, long long max_items, int n_dm, int nsm,
+                          const JKBatchCfg& cfg, cudaStream_t st) {
+    const size_t smem = MULTI ? jk_run_multi_smem<C>(n_dm) : JKRunShape<C>::SMEM;
+    static std::atomic<unsigned long long> attr_done{0}, occ_done{0};
+    static int occ[64];
+    if (cudaError_t e = jk_smem_attr(jk_run_kernel<C, R, MULTI>, MULTI ? JK_RUN_SMEM : smem, attr_done); e != cudaSuccess)
+        return e;
+    // resident grid (the most shared memory a MULTI launch may take)
+    const long long res = (long long)nsm * jk_resident_blocks(jk_run_kernel<C, R, MULTI>, JK_RUN_THREADS,
+                                                              MULTI ? (size_t)JK_RUN_SMEM : smem, occ_done, occ);
+    const long long want = (max_items + JK_RUN_THREADS / 32 - 1) / (JK_RUN_THREADS / 32);
+    const int blocks = (int)(cfg.queue ? res * cfg.grid_mul : (want < res ? want : res));
+    jk_run_kernel<C, R, MULTI><<<blocks, JK_RUN_THREADS, smem, st>>>(segs, segt, nseg, cfg.queue, cfg.grab);
+    return cudaGetLastError();
+}
+
+template <class C, typename R, bool MULTI>
+cudaError_t jk_launch_trun(const JKSeg* segs, const long long* segt, int nseg, long long max_items, int nsm,
+                           const JKBatchCfg& cfg, cudaStream_t st) {
+    constexpr size_t smem = JKTRunShape<C, R>::SMEM;
+    static_assert(smem <= 227 * 1024, "team run kernel shared memory");
+    static std::atomic<unsigned long long> attr_done{0}, occ_done{0};
+    static int occ[64];
+    if (cudaError_t e = jk_smem_attr(jk_trun_kernel<C, R, MULTI>, smem, attr_done); e != cudaSuccess) return e;
+    const long long res = (long long)nsm * jk_resident_blocks(jk_trun_kernel<C, R, MULTI>, JK_RUN_THREADS, smem,
+                                                              occ_done, occ);
+    const long long want = (max_items + JK_RUN_THREADS / 32 - 1) / (JK_RUN_THREADS / 32);
+    const int blocks = (int)(cfg.queue ? res * cfg.grid_mul : (want < res ? want : res));
+    jk_trun_kernel<C, R, MULTI><<<blocks, JK_RUN_THREADS, smem, st>>>(segs, segt, nseg, cfg.queue, cfg.grab);
+    return cudaGetLastError();
+}
+
+// The segments of one class (for the team kernels: of one class and one pair
+// of primitive counts), task or item prefix segt[0..nseg] on the device.
 template <int LI, int LJ, int LK, int LL, typename R>
-cudaError_t jk_launch_batch(const JKSeg* segs, const long long* segt, int nseg, long long max_tasks, int nsm,
-                            const JKBatchCfg& cfg, cudaStream_t st) {
+cudaError_t jk_launch(const JKSeg* segs, const long long* segt, int nseg, long long max_tasks, int n_dm, int nsm,
+                      const JKBatchCfg& cfg, cudaStream_t st) {
     using C = JKClass<LI, LJ, LK, LL>;
     if (max_tasks <= 0 || nseg <= 0) return cudaSuccess;
     if constexpr (C::P == 0) {
-        constexpr size_t smem = RysS<C::NROOTS>::WORDS * sizeof(double);
-        static std::atomic<unsigned long long> attr_done{0};
-        if (cudaError_t e = jk_smem_attr(jk_thread_kernel_batch<C, R>, smem, attr_done); e != cudaSuccess) return e;
-        int blocks;
-        if (cfg.queue) {
-            static std::atomic<unsigned long long> occ_done{0};
-            static int occ[64];
-            blocks = nsm * cfg.grid_mul * jk_resident_blocks(jk_thread_kernel_batch<C, R>, 128, smem, occ_done, occ);
-        } else {
-            long long want = (max_tasks + 127) / 128;
-            long long cap = (long long)nsm * 16;
-            blocks = (int)(want < cap ? want : cap);
-        }
-        jk_thread_kernel_batch<C, R><<<blocks, 128, smem, st>>>(segs, segt, nseg, cfg.queue, cfg.grab);
+        if (n_dm > 1) return jk_launch_run<C, R, true>(segs, segt, nseg, max_tasks, n_dm, nsm, cfg, st);
+        return jk_launch_run<C, R, false>(segs, segt, nseg, max_tasks, n_dm, nsm, cfg, st);
+    } else if constexpr (C::TRUN) {
+        if (n_dm > 1) return jk_launch_trun<C, R, true>(segs, segt, nseg, max_tasks, nsm, cfg, st);
+        return jk_launch_trun<C, R, false>(segs, segt, nseg, max_tasks, nsm, cfg, st);
     } else {
         using S = JKTeamShape<C>;
         constexpr size_t smem = jk_team_smem<C, R>();
         static std::atomic<unsigned long long> attr_done{0};
-        if (cudaError_t e = jk_smem_attr(jk_team_kernel_batch<C, R>, smem, attr_done); e != cudaSuccess) return e;
+        if (cudaError_t e = jk_smem_attr(jk_team_kernel<C, R>, smem, attr_done); e != cudaSuccess) return e;
         int blocks;
         if (cfg.queue) {
             static std::atomic<unsigned long long> occ_done{0};
             static int occ[64];
-            blocks = nsm * cfg.grid_mul *
-                     jk_resident_blocks(jk_team_kernel_batch<C, R>, S::THREADS, smem, occ_done, occ);
+            blocks = nsm * cfg.grid_mul * jk_resident_blocks(jk_team_kernel<C, R>, S::THREADS, smem, occ_done, occ);
         } else {
             long long want = (max_tasks + S::QPB - 1) / S::QPB;
             long long cap = (long long)nsm * 8;
             blocks = (int)(want < cap ? want : cap);
         }
-        jk_team_kernel_batch<C, R><<<blocks, S::THREADS, smem, st>>>(segs, segt, nseg, cfg.queue, cfg.grab);
+        jk_team_kernel<C, R><<<blocks, S::THREADS, smem, st>>>(segs, segt, nseg, cfg.queue, cfg.grab);
     }
     return cudaGetLastError();
 }
@@ -142,11 +138,11 @@ typedef cudaError_t (*jk_fill_fn)(const JKSeg& seg, const long long* task0, long
 // launcher tables indexed by JK_CLASS_INDEX(li, lj, lk, ll)
 struct JKTables {
     jk_launch_fn t64[JK_NCLASS], t32[JK_NCLASS];
-    jk_launch_batch_fn b64[JK_NCLASS], b32[JK_NCLASS];
     // team kernels need one primitive count per launch (their blocks loop
-    // over the primitives in step); thread and generic kernels read it per
+    // over the primitives in step); run and generic kernels read it per
     // segment
     unsigned char team[JK_NCLASS];
+    unsigned char run[JK_NCLASS];  // run kernels: ket pairs of an item (0: a row class, task prefix)
     jk_fill_fn fill[JK_NCLASS];  // templated ERI fill (classes up to f)
 };
 
@@ -158,14 +154,13 @@ void jk_register_generic(JKTables* T);
 
 #ifndef JK_NO_FP32
 #define JK_REG32(LI, LJ, LK, LL)                                         \
-    T->t32[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch<LI, LJ, LK, LL, float>; \
-    T->b32[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch_batch<LI, LJ, LK, LL, float>;
+    T->t32[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch<LI, LJ, LK, LL, float>;
 #else
 #define JK_REG32(LI, LJ, LK, LL)
 #endif
 #define JK_REG(LI, LJ, LK, LL)                                                       \
-    T->team[JK_CLASS_INDEX(LI, LJ, LK, LL)] = JKClass<LI, LJ, LK, LL>::P != 0;    \
+    T->team[JK_CLASS_INDEX(LI, LJ, LK, LL)] = !JKClass<LI, LJ, LK, LL>::RUNS;     \
     T->fill[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch_fill_t<LI, LJ, LK, LL>;   \
+    T->run[JK_CLASS_INDEX(LI, LJ, LK, LL)] = JKClass<LI, LJ, LK, LL>::RUNS ? JKClass<LI, LJ, LK, LL>::TPW : 0; \
     T->t64[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch<LI, LJ, LK, LL, double>;  \
-    T->b64[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch_batch<LI, LJ, LK, LL, double>; \
     JK_REG32(LI, LJ, LK, LL)

@@ -10,10 +10,11 @@
 // allocates its row-offset and segment buffers on first use and grows them
 // when a larger class pair comes; this entry point never does.
 //
-// How: the scratch (row offsets, task counts and the bins) lives in the
+// How: the scratch (row or item offsets, ket bounds, task counts, the bins and
+// the segment descriptor of the launch) lives in the
 // file-scope array jk_na_scratch below, sized for at most JK_NA_MAX_ROWS
 // shell pairs in the ij class and JK_NA_MAX_BINS bins.  Every GPU that loads
-// this module holds the array (about 1 MB) until the process exits.  Host
+// this module holds the array (about 1.6 MB) until the process exits.  Host
 // code cannot use the array's name as a device address (in host code it
 // names a host-side stand-in), so the first call on each device looks the
 // address up with cudaGetSymbolAddress, with that device current, and caches
@@ -38,11 +39,13 @@
 #define JK_NA_OFF_TASK0 0
 #define JK_NA_OFF_BINS 256
 #define JK_NA_OFF_QOFF (JK_NA_OFF_BINS + 2 * (JK_NA_MAX_BINS + 1) * 4 + 256)
-#define JK_NA_BYTES (JK_NA_OFF_QOFF + (JK_NA_MAX_ROWS + 1) * 8)
+#define JK_NA_OFF_EHI (JK_NA_OFF_QOFF + (JK_NA_MAX_ROWS + 1) * 8)
+#define JK_NA_OFF_SEG (JK_NA_OFF_EHI + JK_NA_MAX_ROWS * 4)
+#define JK_NA_BYTES (JK_NA_OFF_SEG + (int)sizeof(JKSeg))
 
 static __device__ __align__(256) unsigned char jk_na_scratch[JK_NA_BYTES];
 
-static_assert(JK_NA_OFF_QOFF % 8 == 0, "qoff alignment");
+static_assert(JK_NA_OFF_QOFF % 8 == 0 && JK_NA_OFF_SEG % 8 == 0, "scratch alignment");
 
 static std::mutex g_na_mu;
 static unsigned char* g_na_ptr[64];
@@ -64,12 +67,35 @@ static int na_scratch(unsigned char** out) {
     return JK_OK;
 }
 
-// Row offsets of one class pair from the reference's host bins
+// Columns row ij of one class pair keeps under the reference's host bins
 // (cuobc/lib/gvhf/nr_jk_driver.cu:252-280): row ij in bin s keeps
-// kl < bins_kl[nbins - s]; a diagonal class pair keeps kl <= ij.
-// One block; writes qoff[0..n_ij] and task0 = {0, total}.  A count is
+// kl < bins_kl[nbins - s]; a diagonal class pair keeps kl <= ij.  A count is
 // clamped to the n_kl pairs of the kl class, so bins beyond the class cannot
 // take the task total past the launch bound.
+__device__ __forceinline__ int na_cols(const int* __restrict__ bins_ij, const int* __restrict__ bins_kl, int nbins,
+                                       int n_kl, int diag, int ij) {
+    if (ij < bins_ij[0] || bins_kl[0] != 0) return 0;
+    int lo = 0, hi = nbins;  // smallest s with ij < bins_ij[s + 1]
+    while (lo < hi) {
+        int mid = (lo + hi) >> 1;
+        if (ij < bins_ij[mid + 1]) hi = mid; else lo = mid + 1;
+    }
+    if (lo >= nbins) return 0;
+    int cnt = bins_kl[nbins - lo];
+    if (cnt > n_kl) cnt = n_kl;
+    if (cnt < 0) cnt = 0;
+    if (diag && cnt > ij + 1) cnt = ij + 1;
+    return cnt;
+}
+
+// run classes: ket end of every entry
+__global__ void jk_na_ehi_kernel(const int* __restrict__ bins_ij, const int* __restrict__ bins_kl, int nbins, int n_ij,
+                                 int n_kl, int diag, const int* __restrict__ ent, int* __restrict__ ehi) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < n_ij) ehi[e] = na_cols(bins_ij, bins_kl, nbins, n_kl, diag, ent[e]);
+}
+
+// row classes: one block; writes qoff[0..n_ij] and task0 = {0, total}
 __global__ void jk_na_qoff_kernel(const int* __restrict__ bins_ij, const int* __restrict__ bins_kl, int nbins,
                                   int n_ij, int n_kl, int diag, long long* __restrict__ qoff,
                                   long long* __restrict__ task0) {
@@ -83,19 +109,7 @@ __global__ void jk_na_qoff_kernel(const int* __restrict__ bins_ij, const int* __
     for (int base = 0; base < n_ij; base += blockDim.x) {
         int ij = base + threadIdx.x;
         long long cnt = 0;
-        if (ij < n_ij && ij >= bins_ij[0] && bins_kl[0] == 0) {
-            int lo = 0, hi = nbins;  // smallest s with ij < bins_ij[s + 1]
-            while (lo < hi) {
-                int mid = (lo + hi) >> 1;
-                if (ij < bins_ij[mid + 1]) hi = mid; else lo = mid + 1;
-            }
-            if (lo < nbins) {
-                cnt = bins_kl[nbins - lo];
-                if (cnt > n_kl) cnt = n_kl;
-                if (cnt < 0) cnt = 0;
-                if (diag && cnt > ij + 1) cnt = ij + 1;
-            }
-        }
+        if (ij < n_ij) cnt = na_cols(bins_ij, bins_kl, nbins, n_kl, diag, ij);
         long long v = cnt;
         int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         for (int o = 1; o < 32; o <<= 1) {
@@ -155,11 +169,31 @@ extern "C" int jk_build_class_pair_noalloc(jk_basis_t* b, double* vj, double* vk
     JKSeg seg;
     jk_internal_fill_seg(b, cp_ij, cp_kl, d_qoff, n_ij, dm, n_dm, vj, vk, &seg);
     if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
-    jk_na_qoff_kernel<<<1, 1024, 0, st>>>(d_bins_ij, d_bins_kl, nbins, n_ij, n_kl, cp_ij == cp_kl, d_qoff, d_task0);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
-    long long max_tasks = cp_ij == cp_kl ? (long long)n_ij * (n_ij + 1) / 2 : (long long)n_ij * n_kl;
-    rc = jk_internal_launch(b, cp_ij, cp_kl, seg, d_task0, max_tasks, stream);
+    const int diag = cp_ij == cp_kl;
+    long long max_tasks;
+    JKRunTab rt;
+    if (jk_internal_run_table(b, cp_ij, cp_kl, &rt)) {
+        if (n_ij == 0 || n_kl == 0) return JK_OK;
+        int* d_ehi = (int*)(sc + JK_NA_OFF_EHI);
+        jk_na_ehi_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(d_bins_ij, d_bins_kl, nbins, n_ij, n_kl, diag, rt.ent,
+                                                             d_ehi);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
+        rc = jk_internal_run_items(rt, d_ehi, d_qoff, d_task0, stream);
+        if (rc) return rc;
+        seg.nrun = rt.nrun;
+        seg.ent = rt.ent;
+        seg.run0 = rt.run0;
+        seg.ehi = d_ehi;
+        seg.ioff = d_qoff;
+        max_tasks = (long long)rt.nrun * ((n_kl + rt.chunk - 1) / rt.chunk);
+    } else {
+        jk_na_qoff_kernel<<<1, 1024, 0, st>>>(d_bins_ij, d_bins_kl, nbins, n_ij, n_kl, diag, d_qoff, d_task0);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
+        max_tasks = diag ? (long long)n_ij * (n_ij + 1) / 2 : (long long)n_ij * n_kl;
+    }
+    rc = jk_internal_launch(b, cp_ij, cp_kl, seg, (JKSeg*)(sc + JK_NA_OFF_SEG), d_task0, max_tasks, stream);
     if (rc) return rc;
     // same synchronous contract as jk_build_class_pair
     e = cudaStreamSynchronize(st);

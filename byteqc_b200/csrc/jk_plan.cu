@@ -1,0 +1,146 @@
+// Class launches of a set of class quartets (one molecule for jk_build, many
+// for jk_batch_*): the class quartets that share a class become segments of
+// one launch.  A launch per class quartet, as jk_build made before, was 666
+// launches for a def2-TZVP molecule, most of them too small to fill the
+// device; merged they are 59, and the run kernels look a segment up once per
+// item (up to 32 x 32 quartets), so that merging costs the large ones nothing.
+#include <algorithm>
+
+#include "jk_internal.h"
+
+#define PCUDA(x)                                                                                 \
+    do {                                                                                         \
+        cudaError_t e_ = (x);                                                                    \
+        if (e_ != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e_));  \
+    } while (0)
+
+// exclusive prefix of the segments' counts of every key (blockIdx.x = key, one
+// warp); key k's prefix lives at segt[key_off[k] + k], n_k + 1 entries
+__global__ void jk_seg_prefix_kernel(const long long* const* __restrict__ cnt, const int* __restrict__ key_off,
+                                     long long* __restrict__ segt) {
+    const int k = blockIdx.x, lane = threadIdx.x;
+    const int s0 = key_off[k], n = key_off[k + 1] - s0;
+    long long* out = segt + s0 + k;
+    long long carry = 0;
+    if (lane == 0) out[0] = 0;
+    for (int base = 0; base < n; base += 32) {
+        const int i = base + lane;
+        long long v = i < n ? *cnt[s0 + i] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += y;
+        }
+        if (i < n) out[i + 1] = carry + v;
+        carry += __shfl_sync(0xffffffffu, v, 31);
+    }
+}
+
+void jk_plan_free(JKPlan* p) {
+    if (!p) return;
+    for (int i = 0; i < 2; i++) {
+        cudaFree(p->d_seg[i]);
+        cudaFree(p->d_segt[i]);
+        cudaFree((void*)p->d_cnt[i]);
+    }
+    cudaFree(p->d_key_off);
+    cudaFree(p->d_queue);
+    delete p;
+}
+
+int jk_plan_add(JKPlan* p, const jk_basis* b, int m, int c, bool solo) {
+    const JKScreenCQ& cq = b->h_cq[c];
+    const int cls = jk_internal_class_index(b, cq.cp_ij, cq.cp_kl);
+    if (!jk_internal_launcher(cls, 0)) return jk_internal_set_err(JK_ERR_UNSUPPORTED, "no kernel for a class quartet");
+    const long long n =
+        cq.cp_ij == cq.cp_kl ? (long long)cq.n_ij * (cq.n_ij + 1) / 2 : (long long)cq.n_ij * cq.n_kl;
+    int np_ij = b->h_group_nprim[cq.gi] * b->h_group_nprim[cq.gj];
+    int np_kl = b->h_group_nprim[cq.gk] * b->h_group_nprim[cq.gl];
+    if (!jk_internal_class_team(cls)) np_ij = np_kl = -1;
+    JKPlanKey* k = nullptr;
+    const auto id = std::make_tuple(cls, np_ij, np_kl);
+    if (!solo) {
+        auto it = p->index.find(id);
+        if (it != p->index.end()) k = &p->keys[it->second];
+        else p->index[id] = (int)p->keys.size();
+    }
+    if (!k) {
+        p->keys.emplace_back();
+        k = &p->keys.back();
+        k->cls = cls;
+        k->np_ij = np_ij;
+        k->np_kl = np_kl;
+        k->solo = solo;
+    }
+    k->segs.push_back({m, c});
+    k->seg_tasks.push_back(n);
+    k->max_tasks += n;
+    k->max_items += cq.runs ? (long long)cq.nrun * ((cq.n_kl + cq.runs - 1) / cq.runs + 1) : n;
+    return JK_OK;
+}
+
+int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols) {
+    p->index.clear();
+    std::stable_partition(p->keys.begin(), p->keys.end(), [](const JKPlanKey& k) { return !k.solo; });
+    // longest first within every key (stable: ties keep molecule order)
+    for (auto& k : p->keys) {
+        std::vector<int> ord(k.segs.size());
+        for (size_t i = 0; i < ord.size(); i++) ord[i] = (int)i;
+        std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return k.seg_tasks[a] > k.seg_tasks[b]; });
+        std::vector<std::pair<int, int>> segs(ord.size());
+        std::vector<long long> tasks(ord.size());
+        for (size_t i = 0; i < ord.size(); i++) {
+            segs[i] = k.segs[ord[i]];
+            tasks[i] = k.seg_tasks[ord[i]];
+        }
+        k.segs.swap(segs);
+        k.seg_tasks.swap(tasks);
+    }
+    const int nkeys = (int)p->keys.size();
+    p->key_off.assign(1, 0);
+    for (auto& k : p->keys) p->key_off.push_back(p->key_off.back() + (int)k.segs.size());
+    p->nseg = p->key_off.back();
+    const size_t ns = std::max(1, p->nseg);
+    PCUDA(cudaMalloc(&p->d_key_off, sizeof(int) * (nkeys + 1)));
+    PCUDA(cudaMemcpy(p->d_key_off, p->key_off.data(), sizeof(int) * (nkeys + 1), cudaMemcpyHostToDevice));
+    PCUDA(cudaMalloc(&p->d_queue, sizeof(unsigned long long) * 2 * std::max(1, nkeys)));
+    std::vector<JKSeg> seg(ns);
+    std::vector<const long long*> cnt(ns);
+    for (int part = 0; part < 2; part++) {
+        size_t i = 0;
+        for (auto& k : p->keys)
+            for (auto& s : k.segs) {
+                const jk_basis* b = mols[s.first];
+                const JKScreenCQ& cq = b->h_cq[s.second];
+                jk_internal_fill_seg_cq(b, s.second, part, &seg[i]);
+                cnt[i++] = (cq.runs ? (part ? cq.itm32 : cq.itm) : (part ? cq.task032 : cq.task0)) + 1;
+            }
+        PCUDA(cudaMalloc(&p->d_seg[part], sizeof(JKSeg) * ns));
+        PCUDA(cudaMalloc(&p->d_segt[part], sizeof(long long) * (ns + nkeys + 1)));
+        PCUDA(cudaMalloc((void**)&p->d_cnt[part], sizeof(long long*) * ns));
+        if (p->nseg) {
+            PCUDA(cudaMemcpy(p->d_seg[part], seg.data(), sizeof(JKSeg) * p->nseg, cudaMemcpyHostToDevice));
+            PCUDA(cudaMemcpy((void*)p->d_cnt[part], cnt.data(), sizeof(long long*) * p->nseg, cudaMemcpyHostToDevice));
+        }
+    }
+    return JK_OK;
+}
+
+int jk_plan_prefix(const JKPlan* p, bool mixed, cudaStream_t st) {
+    const int nkeys = (int)p->keys.size();
+    if (nkeys == 0) return JK_OK;
+    for (int part = 0; part < (mixed ? 2 : 1); part++)
+        jk_seg_prefix_kernel<<<nkeys, 32, 0, st>>>(p->d_cnt[part], p->d_key_off, p->d_segt[part]);
+    PCUDA(cudaGetLastError());
+    return JK_OK;
+}
+
+int jk_plan_launch(const JKPlan* p, int k, int part, const JKBatchCfg& cfg, int n_dm, int nsm, cudaStream_t st) {
+    const JKPlanKey& key = p->keys[k];
+    const int off = p->key_off[k], n = p->key_off[k + 1] - off;
+    jk_launch_fn f = jk_internal_launcher(key.cls, part);
+    if (!f) return jk_internal_set_err(JK_ERR_UNSUPPORTED, "no kernel for a class of the build");
+    JKBatchCfg c = cfg;
+    c.queue = c.grab > 0 ? p->d_queue + 2 * k + part : nullptr;
+    PCUDA(f(p->d_seg[part] + off, p->d_segt[part] + off + k, n, key.max_items, n_dm, nsm, c, st));
+    return JK_OK;
+}

@@ -8,14 +8,10 @@
 
 #include "../../include/byteqc_jk.h"
 
-static double cheb(const double* c, double t) {
-    double b1 = 0., b2 = 0., t2 = t + t;
-    for (int k = RYS_NC - 1; k >= 1; k--) {
-        double b0 = fma(t2, b1, c[k] - b2);
-        b2 = b1;
-        b1 = b0;
-    }
-    return fma(t, b1, c[0] - b2);
+static double horner(const double* c, double t) {
+    double v = c[RYS_NC - 1];
+    for (int k = RYS_NC - 2; k >= 0; k--) v = fma(v, t, c[k]);
+    return v;
 }
 
 extern "C" int jk_rys_roots_host(int n, double x, double* s, double* w) {
@@ -34,8 +30,8 @@ extern "C" int jk_rys_roots_host(int n, double x, double* s, double* w) {
     double t = (x - (m + 0.5) * h) / (0.5 * h);
     const double* c = rys_coef + rys_off[n] + (m * 2 * n) * RYS_NC;
     for (int r = 0; r < n; r++) {
-        s[r] = cheb(c + r * RYS_NC, t);
-        w[r] = cheb(c + (n + r) * RYS_NC, t);
+        s[r] = horner(c + r * RYS_NC, t);
+        w[r] = horner(c + (n + r) * RYS_NC, t);
     }
     return JK_OK;
 }

@@ -123,7 +123,7 @@ int jk_fill_int2e(jk_basis_t *basis, double *eri, int nao, const int *strides, c
  * host framework that owns all GPU memory through its own pool and cannot
  * have a library call cudaMalloc behind it).  No counterpart in the
  * reference.  It allocates nothing: its scratch is a fixed device array of
- * about 1 MB inside libjk.so, held on every GPU that loads the library.
+ * about 1.6 MB inside libjk.so, held on every GPU that loads the library.
  * Limits: at most 131072 shell pairs in the ij class and nbins <= 1024;
  * larger requests return JK_ERR_ARG.  The bins must be non-decreasing with
  * bins_locs_kl[nbins] <= the kl class's pair count (larger counts are
