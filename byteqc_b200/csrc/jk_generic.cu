@@ -9,13 +9,18 @@
 // l it serves, GL = 5 (every class up to (hh|hh), 86 KB of shared memory,
 // two CTAs per SM) or GL = 6 (classes with an i shell, 153 KB, one CTA):
 //
-//   one CTA per contracted quartet; for every primitive quartet and root the
-//   three (axis, root) 2D blocks are built in shared memory (threads 0-2),
-//   then every thread owns elements of the six J/K blocks of the quartet
-//   (J_ij, J_kl, K_ik, K_il, K_jk, K_jl), sums the integrals times the
-//   matching density elements over the other two indices into a shared-memory
-//   accumulator (no atomics: one owner per element), and the blocks are
-//   added to J and K with one atomic per element at the end.
+//   one CTA per contracted quartet.  The 2D blocks of a batch of roots (all
+//   of them for most classes) are built in three parallel steps: the vertical
+//   recursion by one thread per (root, axis), the bra transfer by one per
+//   (root, axis, m), the ket transfer by one per (root, axis, i, j).  The
+//   integrals of a range of (i, j) components are summed over primitives and
+//   roots in shared memory, once, and then digested from there: every thread
+//   owns elements of the six J/K blocks (J_ij, J_kl, K_ik, K_il, K_jk, K_jl)
+//   and sums integral times density over the other two indices (no atomics:
+//   one owner per element); the blocks are added to J and K with one atomic
+//   per element at the end.  Before, three threads of 128 built the blocks of
+//   one root at a time while the others waited, and each of the six blocks
+//   formed every integral again from three shared-memory loads.
 //
 // Digestion, index conventions and density orientation are those of the
 // templated kernels (cuobc/lib/gvhf/contract_jk.cu:225-316): output element
@@ -24,6 +29,8 @@
 
 #define JK_GEN_THREADS 128
 #define JK_FILL_CHUNK 4096
+#define JK_GEN_ACC 3072   // integrals of one pass of the J/K kernel
+#define JK_GEN_GRAB 4     // tasks a block takes in turn (static shape)
 
 // fixed sizes of the generic kernels serving shells up to l = GL
 template <int GL>
@@ -35,12 +42,9 @@ struct JKGen {
     static constexpr int G1 = 2 * GL + 1;                           // VRR range in n and m
     static constexpr int H1 = GL + 1;
     static constexpr int W = G1 * G1 + H1 * H1 * G1 + 2 * G1;       // recursion scratch of one unit
-    static constexpr size_t SMEM = (3 * GS + 12 * BLK + 3 * W) * sizeof(double);
     static constexpr size_t FILL_SMEM = (3 * GS + JK_FILL_CHUNK + 3 * W) * sizeof(double);
     static constexpr size_t QC_SMEM = (3 * GS + BLK + 3 * W) * sizeof(double);
-    static constexpr int CTAS = GL <= 5 ? 2 : 1;                    // resident CTAs per SM
 };
-static_assert(JKGen<5>::SMEM <= 227 * 1024 && JKGen<6>::SMEM <= 227 * 1024, "generic kernel shared memory");
 
 // One Rys 2D block at run-time angular momenta: the recursion of rys_2d,
 // output I[((i*(lj+1)+j)*(lk+1)+k)*(ll+1)+l].  The intermediate arrays live
@@ -112,156 +116,253 @@ __device__ void jk_cart_table(int l, int (*ex)[3]) {
     }
 }
 
+// Shared memory of the J/K kernel: integrals, density blocks, accumulator
+// blocks and the 2D blocks of as many roots at a time as fit.
+template <int GL>
+struct JKGenJK {
+    static constexpr int BLK = JKGen<GL>::BLK, NR = JKGen<GL>::NR;
+    // one (root, axis) unit of the largest class: H[i][j][m], then G or I
+    static constexpr int UNIT = (GL + 1) * (GL + 1) * (2 * GL + 1) + JKGen<GL>::GS;
+    static constexpr int ROOTS = GL <= 4 ? 2 : 1;  // roots of the largest class built at once
+    static constexpr int UNITS = 3 * ROOTS * UNIT;
+    static constexpr size_t SMEM = (JK_GEN_ACC + 12 * BLK + UNITS) * sizeof(double);
+    static constexpr int CTAS = GL <= 5 ? 2 : 1;   // resident CTAs per SM
+};
+static_assert(2 * JKGenJK<4>::SMEM <= 225 * 1024 && 2 * JKGenJK<5>::SMEM <= 225 * 1024 &&
+                  JKGenJK<6>::SMEM <= 225 * 1024, "generic J/K kernel shared memory");
+
 // ---------------------------------------------------------------------------
-// J/K of one class (one segment or a segment table), one quartet per CTA at
-// a time; each CTA takes a contiguous chunk of the tasks
+// J/K of one class, one quartet per CTA at a time
 // ---------------------------------------------------------------------------
 template <int GL, class Src>
 __device__ void jk_generic_body(const Src& src) {
     using G = JKGen<GL>;
+    using K = JKGenJK<GL>;
     extern __shared__ __align__(16) double gsm[];
-    double* gI = gsm;                  // 3 x G::GS: the blocks of one root
-    double* Dsm = gI + 3 * G::GS;      // density blocks
-    double* acc = Dsm + 6 * G::BLK;    // accumulator blocks
-    double* wk = acc + 6 * G::BLK;     // 3 x G::W: recursion scratch of threads 0-2
+    double* eri = gsm;                  // integrals of the current (i, j) components
+    double* Dsm = eri + JK_GEN_ACC;     // density blocks
+    double* acc = Dsm + 6 * K::BLK;     // accumulator blocks
+    double* units = acc + 6 * K::BLK;   // 2D blocks
     __shared__ JKQuartet s_q;
     __shared__ const JKSeg* s_sg;
     __shared__ double s_c[12];
     __shared__ JKPrim s_p;
-    __shared__ double s_rs[G::NR], s_rw[G::NR];
     __shared__ int s_ex[4][G::NF][3];  // Cartesian exponents of the four shells
     const int tid = threadIdx.x;
     const long long total = src.total();
     unsigned long long* queue = src.queue();
-    const long long chunk = queue ? (long long)src.grab() : (total + gridDim.x - 1) / gridDim.x;
+    const long long chunk = queue ? (long long)src.grab() : JK_GEN_GRAB;
     __shared__ long long s_grab;
-    long long tbeg = (long long)blockIdx.x * chunk;
-    for (;;) {
-    if (queue) {  // persistent mode: the block takes `chunk` tasks per round
-        __syncthreads();
-        if (tid == 0) s_grab = (long long)atomicAdd(queue, (unsigned long long)chunk);
-        __syncthreads();
-        tbeg = s_grab;
-    }
-    if (tbeg >= total) break;
-    const long long tend = min(total, tbeg + chunk);
-    typename Src::Cursor cur;
-    if (tid == 0 && tbeg < tend) cur.init(src, tbeg);
-    for (long long t = tbeg; t < tend; t++) {
-        if (tid == 0) {
-            int row, col;
-            s_sg = &cur.seek(src, t, row, col);
-            s_q = jk_quartet_at(*s_sg, row, col);
-            load_pair_centres(*s_sg, s_q.bij, s_c, s_c + 3);
-            load_pair_centres(*s_sg, s_q.bkl, s_c + 6, s_c + 9);
+    for (long long tbeg = (long long)blockIdx.x * chunk;; tbeg += (long long)gridDim.x * chunk) {
+        if (queue) {  // persistent mode: the block takes `chunk` tasks per round
+            __syncthreads();
+            if (tid == 0) s_grab = (long long)atomicAdd(queue, (unsigned long long)chunk);
+            __syncthreads();
+            tbeg = s_grab;
         }
-        __syncthreads();
-        const JKSeg& sg = *s_sg;
-        const JKQuartet q = s_q;
-        const int li = sg.ls[0], lj = sg.ls[1], lk = sg.ls[2], ll = sg.ls[3];
-        const int nfi = ncart(li), nfj = ncart(lj), nfk = ncart(lk), nfl = ncart(ll);
-        const int nr = (li + lj + lk + ll) / 2 + 1;
-        const int SK = ll + 1, SJ = (lk + 1) * SK, SI = (lj + 1) * SJ;
-        for (int sh = 0; sh < 4; sh++) jk_cart_table(sg.ls[sh], s_ex[sh]);
-        // accumulator blocks: [0, o1) J_ij, [o1, o2) J_kl, [o2, o3) K_ik,
-        // [o3, o4) K_il, [o4, o5) K_jk, [o5, E) K_jl
-        const int o1 = nfi * nfj, o2 = o1 + nfk * nfl, o3 = o2 + nfi * nfk, o4 = o3 + nfi * nfl,
-                  o5 = o4 + nfj * nfk, E = o5 + nfj * nfl;
-        // density blocks, each at the position of the accumulator it feeds:
-        // D_kl at 0, D_ij at d1, D_jl at d2, D_jk at d3, D_il at d4, D_ik at d5
-        const int d1 = nfk * nfl, d2 = d1 + nfi * nfj, d3 = d2 + nfj * nfl, d4 = d3 + nfj * nfk,
-                  d5 = d4 + nfi * nfl;
-        const int nao = sg.nao;
-        const int npij = sg.pnp ? __ldg(sg.pnp + q.bij) : sg.nprim_ij;
-        const int npkl = sg.pnp ? __ldg(sg.pnp + q.bkl) : sg.nprim_kl;
-        for (int idm = 0; idm < sg.n_dm; idm++) {
-            const double* D = sg.dm + (size_t)idm * nao * nao;
-            // densities in the orientation of the templated kernels: J side
-            // D[x + nao y], K side transposed, D[y + nao x]
-            for (int e = tid; e < E; e += JK_GEN_THREADS) {
-                int r, x0, y0, ny;
-                bool tr = true;
-                if (e < d1) { x0 = q.k0; y0 = q.l0; ny = nfl; r = e; tr = false; }
-                else if (e < d2) { x0 = q.i0; y0 = q.j0; ny = nfj; r = e - d1; tr = false; }
-                else if (e < d3) { x0 = q.j0; y0 = q.l0; ny = nfl; r = e - d2; }
-                else if (e < d4) { x0 = q.j0; y0 = q.k0; ny = nfk; r = e - d3; }
-                else if (e < d5) { x0 = q.i0; y0 = q.l0; ny = nfl; r = e - d4; }
-                else { x0 = q.i0; y0 = q.k0; ny = nfk; r = e - d5; }
-                const int a = r / ny, b = r - a * ny;
-                Dsm[e] = tr ? __ldg(D + (y0 + b) + (size_t)nao * (x0 + a))
-                            : __ldg(D + (x0 + a) + (size_t)nao * (y0 + b));
-                acc[e] = 0.;
+        if (tbeg >= total) break;
+        const long long tend = min(total, tbeg + chunk);
+        typename Src::Cursor cur;
+        if (tid == 0) cur.init(src, tbeg);
+        for (long long t = tbeg; t < tend; t++) {
+            if (tid == 0) {
+                int row, col;
+                s_sg = &cur.seek(src, t, row, col);
+                s_q = jk_quartet_at(*s_sg, row, col);
+                load_pair_centres(*s_sg, s_q.bij, s_c, s_c + 3);
+                load_pair_centres(*s_sg, s_q.bkl, s_c + 6, s_c + 9);
             }
             __syncthreads();
-            for (int kp = 0; kp < npkl; kp++)
-                for (int ip = 0; ip < npij; ip++) {
-                    if (tid == 0) s_p = jk_prim2(jk_pp(sg, q.prim_ij + ip * sg.pst_ij), jk_pp(sg, q.prim_kl + kp * sg.pst_kl));
-                    __syncthreads();
-                    if (tid < nr) rys_root_rt(sg.rys, nr, s_p.x, tid, s_rs[tid], s_rw[tid]);
-                    __syncthreads();
-                    for (int r = 0; r < nr; r++) {
-                        if (tid < 3)
-                            jk_unit_rt<GL>(s_p, s_rs[r], s_rw[r], tid, q.norm, s_c, s_c + 3, s_c + 6, s_c + 9, li,
-                                           lj, lk, ll, wk + tid * G::W, gI + tid * G::GS);
-                        __syncthreads();
-                        const double* gx = gI;
-                        const double* gy = gI + G::GS;
-                        const double* gz = gI + 2 * G::GS;
-#define JK_GEN_I(i, j, k, l)                                                                                  \
-    (gx[s_ex[0][i][0] * SI + s_ex[1][j][0] * SJ + s_ex[2][k][0] * SK + s_ex[3][l][0]] *                       \
-     gy[s_ex[0][i][1] * SI + s_ex[1][j][1] * SJ + s_ex[2][k][1] * SK + s_ex[3][l][1]] *                       \
-     gz[s_ex[0][i][2] * SI + s_ex[1][j][2] * SJ + s_ex[2][k][2] * SK + s_ex[3][l][2]])
-                        for (int e = tid; e < E; e += JK_GEN_THREADS) {
-                            double v = 0.;
-                            if (e < o1) {  // J_ij += (ij|kl) D_kl
-                                const int i = e / nfj, j = e - i * nfj;
-                                for (int k = 0; k < nfk; k++)
-                                    for (int l = 0; l < nfl; l++) v += JK_GEN_I(i, j, k, l) * Dsm[k * nfl + l];
-                            } else if (e < o2) {  // J_kl += (ij|kl) D_ij
-                                const int x = e - o1, k = x / nfl, l = x - k * nfl;
-                                for (int i = 0; i < nfi; i++)
-                                    for (int j = 0; j < nfj; j++) v += JK_GEN_I(i, j, k, l) * Dsm[d1 + i * nfj + j];
-                            } else if (e < o3) {  // K_ik += (ij|kl) D_jl
-                                const int x = e - o2, i = x / nfk, k = x - i * nfk;
-                                for (int j = 0; j < nfj; j++)
-                                    for (int l = 0; l < nfl; l++) v += JK_GEN_I(i, j, k, l) * Dsm[d2 + j * nfl + l];
-                            } else if (e < o4) {  // K_il += (ij|kl) D_jk
-                                const int x = e - o3, i = x / nfl, l = x - i * nfl;
-                                for (int j = 0; j < nfj; j++)
-                                    for (int k = 0; k < nfk; k++) v += JK_GEN_I(i, j, k, l) * Dsm[d3 + j * nfk + k];
-                            } else if (e < o5) {  // K_jk += (ij|kl) D_il
-                                const int x = e - o4, j = x / nfk, k = x - j * nfk;
-                                for (int i = 0; i < nfi; i++)
-                                    for (int l = 0; l < nfl; l++) v += JK_GEN_I(i, j, k, l) * Dsm[d4 + i * nfl + l];
-                            } else {  // K_jl += (ij|kl) D_ik
-                                const int x = e - o5, j = x / nfl, l = x - j * nfl;
-                                for (int i = 0; i < nfi; i++)
-                                    for (int k = 0; k < nfk; k++) v += JK_GEN_I(i, j, k, l) * Dsm[d5 + i * nfk + k];
-                            }
-                            acc[e] += v;
-                        }
-#undef JK_GEN_I
-                        __syncthreads();  // the next root rebuilds the blocks
-                    }
+            const JKSeg& sg = *s_sg;
+            const JKQuartet q = s_q;
+            const int li = sg.ls[0], lj = sg.ls[1], lk = sg.ls[2], ll = sg.ls[3];
+            const int nfi = ncart(li), nfj = ncart(lj), nfk = ncart(lk), nfl = ncart(ll);
+            const int nr = (li + lj + lk + ll) / 2 + 1;
+            const int nm = li + lj, mm = lk + ll;
+            const int SK = ll + 1, SJ = (lk + 1) * SK, SI = (lj + 1) * SJ;
+            const int nh = (li + 1) * (lj + 1) * (mm + 1);                     // H of one unit
+            const int ng = max((nm + 1) * (mm + 1), (li + 1) * SI), un = nh + ng;  // G and I share a place
+            const int rb = min(nr, K::UNITS / (3 * un));                       // roots at a time
+            for (int sh = 0; sh < 4; sh++) jk_cart_table(sg.ls[sh], s_ex[sh]);
+            // accumulator blocks: [0, o1) J_ij, [o1, o2) J_kl, [o2, o3) K_ik,
+            // [o3, o4) K_il, [o4, o5) K_jk, [o5, E) K_jl
+            const int o1 = nfi * nfj, o2 = o1 + nfk * nfl, o3 = o2 + nfi * nfk, o4 = o3 + nfi * nfl,
+                      o5 = o4 + nfj * nfk, E = o5 + nfj * nfl;
+            // density blocks, each at the position of the accumulator it feeds:
+            // D_kl at 0, D_ij at d1, D_jl at d2, D_jk at d3, D_il at d4, D_ik at d5
+            const int d1 = nfk * nfl, d2 = d1 + nfi * nfj, d3 = d2 + nfj * nfl, d4 = d3 + nfj * nfk,
+                      d5 = d4 + nfi * nfl;
+            const int nao = sg.nao, nkl = nfk * nfl;
+            const int npij = sg.pnp ? __ldg(sg.pnp + q.bij) : sg.nprim_ij;
+            const int npkl = sg.pnp ? __ldg(sg.pnp + q.bkl) : sg.nprim_kl;
+            // whole rows i of (i, j) components per pass where they fit, else
+            // parts of a row
+            const int per = max(1, min(nfi * nfj, JK_GEN_ACC / nkl));
+            const int nij = per >= nfj ? per / nfj * nfj : per;
+            for (int idm = 0; idm < sg.n_dm; idm++) {
+                const double* D = sg.dm + (size_t)idm * nao * nao;
+                __syncthreads();
+                // densities in the orientation of the templated kernels: J side
+                // D[x + nao y], K side transposed, D[y + nao x]
+                for (int e = tid; e < E; e += JK_GEN_THREADS) {
+                    int r, x0, y0, ny;
+                    bool tr = true;
+                    if (e < d1) { x0 = q.k0; y0 = q.l0; ny = nfl; r = e; tr = false; }
+                    else if (e < d2) { x0 = q.i0; y0 = q.j0; ny = nfj; r = e - d1; tr = false; }
+                    else if (e < d3) { x0 = q.j0; y0 = q.l0; ny = nfl; r = e - d2; }
+                    else if (e < d4) { x0 = q.j0; y0 = q.k0; ny = nfk; r = e - d3; }
+                    else if (e < d5) { x0 = q.i0; y0 = q.l0; ny = nfl; r = e - d4; }
+                    else { x0 = q.i0; y0 = q.k0; ny = nfk; r = e - d5; }
+                    const int a = r / ny, b = r - a * ny;
+                    Dsm[e] = tr ? __ldg(D + (y0 + b) + (size_t)nao * (x0 + a))
+                                : __ldg(D + (x0 + a) + (size_t)nao * (y0 + b));
+                    acc[e] = 0.;
                 }
-            // add the blocks to J and K
-            for (int e = tid; e < E; e += JK_GEN_THREADS) {
-                double* V;
-                int r, x0, y0, ny;
-                if (e < o1) { V = sg.vj; x0 = q.i0; y0 = q.j0; ny = nfj; r = e; }
-                else if (e < o2) { V = sg.vj; x0 = q.k0; y0 = q.l0; ny = nfl; r = e - o1; }
-                else if (e < o3) { V = sg.vk; x0 = q.i0; y0 = q.k0; ny = nfk; r = e - o2; }
-                else if (e < o4) { V = sg.vk; x0 = q.i0; y0 = q.l0; ny = nfl; r = e - o3; }
-                else if (e < o5) { V = sg.vk; x0 = q.j0; y0 = q.k0; ny = nfk; r = e - o4; }
-                else { V = sg.vk; x0 = q.j0; y0 = q.l0; ny = nfl; r = e - o5; }
-                if (!V) continue;
-                const int a = r / ny, b = r - a * ny;
-                atomicAdd(V + (size_t)idm * nao * nao + (x0 + a) + (size_t)nao * (y0 + b), acc[e]);
+                for (int ij0 = 0; ij0 < nfi * nfj; ij0 += nij) {
+                    const int ij1 = min(nfi * nfj, ij0 + nij), ne = (ij1 - ij0) * nkl;
+                    for (int e = tid; e < ne; e += JK_GEN_THREADS) eri[e] = 0.;
+                    for (int kp = 0; kp < npkl; kp++)
+                        for (int ip = 0; ip < npij; ip++) {
+                            __syncthreads();
+                            if (tid == 0)
+                                s_p = jk_prim2(jk_pp(sg, q.prim_ij + ip * sg.pst_ij),
+                                               jk_pp(sg, q.prim_kl + kp * sg.pst_kl));
+                            __syncthreads();
+                            for (int r0 = 0; r0 < nr; r0 += rb) {
+                                const int nb = min(rb, nr - r0), nu = 3 * nb;
+                                if (r0) __syncthreads();  // the products of the last batch are done
+                                // vertical recursion: G[n][m] of unit (root, axis)
+                                for (int u = tid; u < nu; u += JK_GEN_THREADS) {
+                                    const int d = u % 3;
+                                    double s, w;
+                                    rys_root_rt(sg.rys, nr, s_p.x, r0 + u / 3, s, w);
+                                    const double siAB = s * s_p.iAB, bs = s_p.B * siAB, as = s_p.A * siAB;
+                                    const double b00 = 0.5 * siAB, b10 = 0.5 * s_p.iA * (1. - bs),
+                                                 b01 = 0.5 * s_p.iB * (1. - as);
+                                    const double pq = s_p.P[d] - s_p.Q[d];
+                                    const double c00 = (s_p.P[d] - s_c[d]) - bs * pq,
+                                                 c0p = (s_p.Q[d] - s_c[6 + d]) + as * pq;
+                                    double* g = units + u * un + nh;
+                                    const int M1 = mm + 1;
+                                    double prev = 0., v = d == 0 ? q.norm : (d == 1 ? s_p.sy : w);
+                                    g[0] = v;
+                                    for (int n = 0; n < nm; n++) {
+                                        const double nx = c00 * v + n * b10 * prev;
+                                        prev = v;
+                                        v = nx;
+                                        g[(n + 1) * M1] = v;
+                                    }
+                                    for (int m = 0; m < mm; m++)
+                                        for (int n = 0; n <= nm; n++) {
+                                            double x = c0p * g[n * M1 + m];
+                                            if (m) x += m * b01 * g[n * M1 + m - 1];
+                                            if (n) x += n * b00 * g[(n - 1) * M1 + m];
+                                            g[n * M1 + m + 1] = x;
+                                        }
+                                }
+                                __syncthreads();
+                                // bra transfer: H[i][j][m], one column m per item
+                                for (int x = tid; x < nu * (mm + 1); x += JK_GEN_THREADS) {
+                                    const int u = x / (mm + 1), m = x - u * (mm + 1), d = u % 3;
+                                    const double ab = s_c[d] - s_c[3 + d];
+                                    double* H = units + u * un + m;
+                                    const double* g = units + u * un + nh + m;
+                                    double A[2 * GL + 1];
+                                    for (int a = 0; a <= nm; a++) A[a] = g[a * (mm + 1)];
+                                    for (int j = 0; j <= lj; j++) {
+                                        for (int i = 0; i <= li; i++) H[(i * (lj + 1) + j) * (mm + 1)] = A[i];
+                                        for (int a = 0; a + j < nm; a++) A[a] = A[a + 1] + ab * A[a];
+                                    }
+                                }
+                                __syncthreads();
+                                // ket transfer: I[i][j][k][l], one (i, j) per item
+                                const int hij = (li + 1) * (lj + 1);
+                                for (int x = tid; x < nu * hij; x += JK_GEN_THREADS) {
+                                    const int u = x / hij, ij = x - u * hij, d = u % 3;
+                                    const double cd = s_c[6 + d] - s_c[9 + d];
+                                    const double* H = units + u * un + ij * (mm + 1);
+                                    double* I = units + u * un + nh + ij * SJ;
+                                    double B[2 * GL + 1];
+                                    for (int c = 0; c <= mm; c++) B[c] = H[c];
+                                    for (int l = 0; l <= ll; l++) {
+                                        for (int k = 0; k <= lk; k++) I[k * SK + l] = B[k];
+                                        for (int c = 0; c + l < mm; c++) B[c] = B[c + 1] + cd * B[c];
+                                    }
+                                }
+                                __syncthreads();
+                                // products of the batch
+                                for (int e = tid; e < ne; e += JK_GEN_THREADS) {
+                                    const int ij = e / nkl, kl = e - ij * nkl;
+                                    const int i = (ij0 + ij) / nfj, j = ij0 + ij - i * nfj;
+                                    const int k = kl / nfl, l = kl - k * nfl;
+                                    int o[3];
+#pragma unroll
+                                    for (int d = 0; d < 3; d++)
+                                        o[d] = d * un + nh + s_ex[0][i][d] * SI + s_ex[1][j][d] * SJ +
+                                               s_ex[2][k][d] * SK + s_ex[3][l][d];
+                                    double v = 0.;
+                                    const double* U = units;
+                                    for (int r = 0; r < nb; r++, U += 3 * un) v += U[o[0]] * U[o[1]] * U[o[2]];
+                                    eri[e] += v;
+                                }
+                            }
+                        }
+                    __syncthreads();
+                    // digest the components [ij0, ij1)
+                    const int i_0 = ij0 / nfj, i_1 = (ij1 - 1) / nfj;
+                    for (int e = tid; e < E; e += JK_GEN_THREADS) {
+                        double v = 0.;
+                        if (e < o1) {  // J_ij += (ij|kl) D_kl
+                            if (e >= ij0 && e < ij1)
+                                for (int x = 0; x < nkl; x++) v += eri[(e - ij0) * nkl + x] * Dsm[x];
+                        } else if (e < o2) {  // J_kl += (ij|kl) D_ij
+                            const int x = e - o1;
+                            for (int ij = ij0; ij < ij1; ij++) v += eri[(ij - ij0) * nkl + x] * Dsm[d1 + ij];
+                        } else if (e < o4) {  // K_ik += (ij|kl) D_jl, K_il += (ij|kl) D_jk
+                            const bool ik = e < o3;
+                            const int x = e - (ik ? o2 : o3), nb = ik ? nfk : nfl, nc = ik ? nfl : nfk;
+                            const int i = x / nb, b = x - i * nb;
+                            const int j0 = max(0, ij0 - i * nfj), j1 = min(nfj, ij1 - i * nfj);
+                            const int sb = ik ? nfl : 1, sc = ik ? 1 : nfl;
+                            const double* dd = Dsm + (ik ? d2 : d3);
+                            for (int j = j0; j < j1; j++) {
+                                const double* g = eri + (i * nfj + j - ij0) * nkl + b * sb;
+                                for (int c = 0; c < nc; c++) v += g[c * sc] * dd[j * nc + c];
+                            }
+                        } else {  // K_jk += (ij|kl) D_il, K_jl += (ij|kl) D_ik
+                            const bool jk = e < o5;
+                            const int x = e - (jk ? o4 : o5), nb = jk ? nfk : nfl, nc = jk ? nfl : nfk;
+                            const int j = x / nb, b = x - j * nb;
+                            const int sb = jk ? nfl : 1, sc = jk ? 1 : nfl;
+                            const double* dd = Dsm + (jk ? d4 : d5);
+                            for (int i = i_0; i <= i_1; i++) {
+                                const int ij = i * nfj + j;
+                                if (ij < ij0 || ij >= ij1) continue;
+                                const double* g = eri + (ij - ij0) * nkl + b * sb;
+                                for (int c = 0; c < nc; c++) v += g[c * sc] * dd[i * nc + c];
+                            }
+                        }
+                        acc[e] += v;
+                    }
+                    __syncthreads();  // the next pass clears the integrals
+                }
+                // add the blocks to J and K
+                for (int e = tid; e < E; e += JK_GEN_THREADS) {
+                    double* V;
+                    int r, x0, y0, ny;
+                    if (e < o1) { V = sg.vj; x0 = q.i0; y0 = q.j0; ny = nfj; r = e; }
+                    else if (e < o2) { V = sg.vj; x0 = q.k0; y0 = q.l0; ny = nfl; r = e - o1; }
+                    else if (e < o3) { V = sg.vk; x0 = q.i0; y0 = q.k0; ny = nfk; r = e - o2; }
+                    else if (e < o4) { V = sg.vk; x0 = q.i0; y0 = q.l0; ny = nfl; r = e - o3; }
+                    else if (e < o5) { V = sg.vk; x0 = q.j0; y0 = q.k0; ny = nfk; r = e - o4; }
+                    else { V = sg.vk; x0 = q.j0; y0 = q.l0; ny = nfl; r = e - o5; }
+                    if (!V) continue;
+                    const int a = r / ny, b = r - a * ny;
+                    atomicAdd(V + (size_t)idm * nao * nao + (x0 + a) + (size_t)nao * (y0 + b), acc[e]);
+                }
             }
-            __syncthreads();  // the shared buffers are reused by the next density / quartet
+            __syncthreads();  // the shared buffers are reused by the next quartet
         }
-    }
-    if (!queue) break;
     }
 }
 
@@ -276,8 +377,8 @@ __global__ void __launch_bounds__(JK_GEN_THREADS) jk_generic_kernel(const JKSeg*
 
 template <int GL>
 static int jk_generic_blocks(long long max_tasks, int nsm) {
-    const long long cap = (long long)nsm * JKGen<GL>::CTAS;
-    return (int)(max_tasks < cap ? max_tasks : cap);
+    const long long cap = (long long)nsm * JKGenJK<GL>::CTAS, want = (max_tasks + JK_GEN_GRAB - 1) / JK_GEN_GRAB;
+    return (int)(want < cap ? want : cap);
 }
 
 template <int GL>
@@ -285,10 +386,10 @@ static cudaError_t jk_launch_generic(const JKSeg* segs, const long long* segt, i
                                      int n_dm, int nsm, const JKBatchCfg& cfg, cudaStream_t st) {
     if (max_tasks <= 0 || nseg <= 0) return cudaSuccess;
     static std::atomic<unsigned long long> attr_done{0};
-    if (cudaError_t e = jk_smem_attr(jk_generic_kernel<GL>, JKGen<GL>::SMEM, attr_done); e != cudaSuccess)
+    if (cudaError_t e = jk_smem_attr(jk_generic_kernel<GL>, JKGenJK<GL>::SMEM, attr_done); e != cudaSuccess)
         return e;
-    const int blocks = cfg.queue ? nsm * JKGen<GL>::CTAS * cfg.grid_mul : jk_generic_blocks<GL>(max_tasks, nsm);
-    jk_generic_kernel<GL><<<blocks, JK_GEN_THREADS, JKGen<GL>::SMEM, st>>>(segs, segt, nseg, cfg.queue,
+    const int blocks = cfg.queue ? nsm * JKGenJK<GL>::CTAS * cfg.grid_mul : jk_generic_blocks<GL>(max_tasks, nsm);
+    jk_generic_kernel<GL><<<blocks, JK_GEN_THREADS, JKGenJK<GL>::SMEM, st>>>(segs, segt, nseg, cfg.queue,
                                                                                 cfg.grab);
     return cudaGetLastError();
 }
@@ -441,8 +542,9 @@ void jk_register_generic(JKTables* T) {
                 for (int ll = 0; ll <= lk; ll++) {
                     if (li <= JK_LMAX && lk <= JK_LMAX) continue;
                     const int c = JK_CLASS_INDEX(li, lj, lk, ll);
-                    const bool six = li == 6 || lk == 6;  // li >= lj, lk >= ll
-                    T->t64[c] = T->t32[c] = six ? jk_launch_generic<6> : jk_launch_generic<5>;
+                    const int lx = li > lk ? li : lk;  // li >= lj, lk >= ll
+                    T->t64[c] = T->t32[c] = lx == 6 ? jk_launch_generic<6>
+                                                    : (lx == 5 ? jk_launch_generic<5> : jk_launch_generic<4>);
                 }
 }
 
