@@ -1,8 +1,8 @@
 """Dense two-electron integral tensor of the working basis on the GPU, the
 counterpart of the reference's ``cuobc/lib/int4c.py`` (``get_int4c``,
 ``get_int4c_slice``): per class pair the screened shell quartets are filled
-by ``jk_fill_int2e`` (libjk.so) into a block, and the eight index
-permutations of each block fill the tensor.  The tensor is in the working
+by ``jk_fill_int2e`` (libjk.so) into a block, or straight into the tensor,
+whose other index permutations ``jk_expand_int2e`` then fills.  The tensor is in the working
 basis of the ``_VHFOpt`` (decontracted, Cartesian, shells sorted into
 (l, nprim) groups), as the reference's; build the ``_VHFOpt`` with
 ``diag_block_with_triu=True`` (the default here, as in the reference's
@@ -73,11 +73,31 @@ def get_int4c(mol, blksize=None, vhfopt=None, batch=1, buf_size=0, nbins=1):
     reference's multi-GPU task batching) and ``buf_size`` (a staging-buffer
     size of its basis set-up) are accepted for call compatibility; one GPU
     per process fills the whole tensor."""
-    from byteqc_b200.cuobc.scf.hf import _torch
+    from byteqc_b200.cuobc.scf.hf import _make_s_index_offsets, _torch
     torch = _torch()
     vhfopt = _opt(mol, blksize, vhfopt)
     nao = vhfopt.nao
     out = torch.zeros((nao, nao, nao, nao), dtype=torch.float64, device='cuda')
+    if vhfopt.diag_fac == 1.:
+        # every class pair straight into the tensor, the permuted elements by
+        # one pass over it (both orders of a pair inside a group are filled)
+        lib = _lib.load_library()
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        ptr = ctypes.c_void_p(out.data_ptr())
+        offsets = np.zeros(4, dtype=np.int32)
+        strides = np.array([nao ** 3, nao ** 2, nao, 1], dtype=np.int32)
+        bins = [_make_s_index_offsets(q, nbins, vhfopt.direct_scf_tol)
+                for q in vhfopt.log_qs]
+        for cp_ij in range(len(bins)):
+            for cp_kl in range(cp_ij + 1):
+                _lib.check(lib.jk_fill_int2e(
+                    vhfopt.handle, ptr, nao, strides.ctypes.data,
+                    offsets.ctypes.data, bins[cp_ij].ctypes.data,
+                    bins[cp_kl].ctypes.data, nbins, cp_ij, cp_kl, stream),
+                    'jk_fill_int2e')
+        _lib.check(lib.jk_expand_int2e(vhfopt.handle, ptr, nao, stream),
+                   'jk_expand_int2e')
+        return out
     for cp_ij, cp_kl in zip(*np.tril_indices(len(vhfopt.log_qs))):
         si, sj, sk, sl, b = get_int4c_slice(int(cp_ij), int(cp_kl), vhfopt,
                                             nbins=nbins)

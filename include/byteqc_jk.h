@@ -118,6 +118,17 @@ int jk_fill_int2e(jk_basis_t *basis, double *eri, int nao, const int *strides, c
                   const int *bins_locs_ij, const int *bins_locs_kl, int nbins, int cp_ij, int cp_kl, void *stream);
 
 /*
+ * The remaining elements of the dense (nao, nao, nao, nao) tensor of the
+ * working basis, row-major on the device, from its canonical ones: those with
+ * group(a) >= group(b), group(c) >= group(d) and the class pair of (a, b) not
+ * below that of (c, d), as jk_fill_int2e leaves them when it fills every class
+ * pair cp_ij >= cp_kl at the tensor's own strides.  The basis must hold both
+ * orders of the pairs inside a group (diag_block_with_triu).  Replaces the
+ * eight permuted block copies of cuobc/lib/int4c.py:53-70.  nao <= 8160.
+ */
+int jk_expand_int2e(jk_basis_t *basis, double *eri, int nao, void *stream);
+
+/*
  * Same computation and buffer contract as jk_build_class_pair, for callers
  * that must not allocate device memory while they run (a serving process or
  * host framework that owns all GPU memory through its own pool and cannot
