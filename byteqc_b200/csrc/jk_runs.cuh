@@ -36,6 +36,7 @@
 // zeros.
 #pragma once
 #include "jk_kernels.cuh"
+#include "jk_os.cuh"
 
 #define JK_RUN_MAX 32      // bra pairs of a run: one per lane
 #define JK_RUN_THREADS 128
@@ -48,7 +49,10 @@ struct JKRunShape {
     static constexpr int NJ = C::NFK * C::NFL;             // J_kl elements
     static constexpr int NE = NK + NJ;
     static constexpr int NV = C::NFI * C::NFJ;             // J_ij elements
-    static constexpr size_t TAB = ((size_t)RysS<C::NROOTS>::TWORDS * sizeof(double) + 15) & ~(size_t)15;
+    // Boys table (L <= 3, JKOS) or Rys table; the FP32 tables are smaller
+    static constexpr size_t TABW = JKOS<C>::USE ? BoysS::WORDS : RysS<C::NROOTS>::TWORDS;
+    static constexpr size_t TAB = (TABW * sizeof(double) + 15) & ~(size_t)15;
+    static_assert(RysF<C::NROOTS>::WORDS * sizeof(float) <= TAB || C::NROOTS > JK_F32_ROOTS, "FP32 table");
     static constexpr size_t SLOT = (size_t)NE * JK_RUN_THREADS * sizeof(double);
     static constexpr size_t JBUF = (size_t)JK_RUN_THREADS * 16 * sizeof(double);
     // staged records (12 doubles per entry) and D_ij
@@ -275,6 +279,30 @@ struct JKRunItem {
                     }
                 }
             }
+        } else if constexpr (JKOS<C>::USE) {
+            using OS = JKOS<C>;
+            static_assert(CI0 == 0 && NI == NFI && sizeof(R) == 8, "one pass");
+            double E[OS::NE * OS::NF];
+#pragma unroll
+            for (int e = 0; e < OS::NE * OS::NF; e++) E[e] = 0.;
+            for (int q = 0; q < npkl; q++) {
+                if (npkl > 1) kp = jk_pp(sg, prim_kl + q * sg.pst_kl);
+                for (int p = 0; p < npij; p++) {
+                    const JKPrim pr = jk_prim2(bra(p), kp);
+                    double F[OS::L + 1], PA[3], QC[3], PQ[3];
+                    boys_all<OS::L>(tab, pr.x, F);
+#pragma unroll
+                    for (int d = 0; d < 3; d++) {
+                        PA[d] = pr.P[d] - ri[d];
+                        QC[d] = pr.Q[d] - rk[d];
+                        PQ[d] = pr.P[d] - pr.Q[d];
+                    }
+                    OS::prim(F, norm * pr.sy, pr, PA, QC, PQ, E);
+                }
+            }
+            const double AB[3] = {ri[0] - rj[0], ri[1] - rj[1], ri[2] - rj[2]};
+            const double CD[3] = {rk[0] - rl[0], rk[1] - rl[1], rk[2] - rl[2]};
+            OS::transfer(E, AB, CD, acc);
         } else {
             for (int q = 0; q < npkl; q++) {
                 if (npkl > 1) kp = jk_pp(sg, prim_kl + q * sg.pst_kl);
@@ -661,6 +689,7 @@ __global__ void __launch_bounds__(JK_RUN_THREADS, (JKRunMinBlocks<C, R>::value))
     if (!queue && (long long)blockIdx.x * (JK_RUN_THREADS / 32) >= total) return;  // block-uniform
     if (total == 0) return;
     if constexpr (JKF32Prim<C, R>::value) rys_table_copy_f<C::NROOTS>(segs[0].rys, reinterpret_cast<float*>(jk_tab));
+    else if constexpr (JKOS<C>::USE) boys_table_copy<JKOS<C>::L>(segs[0].rys, jk_tab);
     else rys_table_copy<C::NROOTS>(segs[0].rys, jk_tab);
     __syncthreads();
     double* stage = jk_tab + S::TAB / sizeof(double);

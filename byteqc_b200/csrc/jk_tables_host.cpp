@@ -44,6 +44,6 @@ extern "C" int jk_rys_table_uniform(void) {
 
 // the coefficient table, uploaded to each device by the engine
 extern "C" const double* jk_rys_coef_host(long long* count) {
-    if (count) *count = RYS_TOTAL;
+    if (count) *count = RYS_ALL;
     return rys_coef;
 }

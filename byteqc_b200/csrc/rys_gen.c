@@ -26,6 +26,9 @@
  *      w_i = H_i / sqrt(x) (2n-point Gauss-Hermite, positive nodes), with
  *      X_n the smallest point from which that limit is exact to 2e-17.
  *
+ *   6. the Boys functions F_0 .. F_3 themselves as power series of 10 terms on
+ *      intervals of width 1/2 up to x = 46, for the classes that need no roots.
+ *
  * Output: a C header with hex-float literals (exact doubles).
  * Usage: rys_gen <nmax> <out.h>
  */
@@ -157,6 +160,30 @@ static void fit(int n, qf x0, qf h, double *coef /* [2n][NC] */) {
     }
 }
 
+/* F_m on [x0, x0 + 1/2]: NB powers of t = (x - centre) / (1/4) */
+#define NB 10
+static void boys_fit(int m, qf x0, double *coef) {
+    qf f[NB], ch[NB], ta[NB] = {0}, tb[NB] = {0}, mono[NB] = {0}, b[8];
+    for (int j = 0; j < NB; j++) {
+        boys_q(m + 2, x0 + 0.25Q + 0.25Q * cosq(M_PIq * (j + 0.5Q) / NB), b);
+        f[j] = b[m];
+    }
+    ta[0] = 1;
+    tb[1] = 1;
+    for (int k = 0; k < NB; k++) {
+        qf acc = 0, tc[NB];
+        for (int j = 0; j < NB; j++) acc += f[j] * cosq(M_PIq * k * (j + 0.5Q) / NB);
+        ch[k] = acc * (k ? 2.0Q : 1.0Q) / NB;
+        for (int e = 0; e < NB; e++) {
+            mono[e] += ch[k] * ta[e];
+            tc[e] = 2 * (e ? tb[e - 1] : 0) - ta[e];
+        }
+        memcpy(ta, tb, sizeof(ta));
+        memcpy(tb, tc, sizeof(tb));
+    }
+    for (int e = 0; e < NB; e++) coef[e] = (double)mono[e];
+}
+
 static double horner(const double *c, double t) {
     double v = c[NC - 1];
     for (int k = NC - 2; k >= 0; k--) v = fma(v, t, c[k]);
@@ -278,12 +305,22 @@ int main(int argc, char **argv) {
     fprintf(fo, "0; }\nRYS_HD constexpr double rys_xmax_c(int n) { return ");
     for (int n = 1; n <= nmax; n++) fprintf(fo, "n == %d ? %a : ", n, xas[n]);
     fprintf(fo, "0.; }\n");
-    fprintf(fo, "#ifdef RYS_WANT_COEF\nstatic const double rys_coef[%d] = {\n", off[nmax + 1]);
+    /* Boys functions F_0 .. F_3 on [0, 46), appended to the coefficients */
+    const int nb = 92;
+    fprintf(fo, "#define BOYS_NC %d\n#define BOYS_NINT %d\n#define BOYS_OFF %d\n#define RYS_ALL %d\n", NB, nb, off[nmax + 1],
+            off[nmax + 1] + 4 * nb * NB);
+    fprintf(fo, "#ifdef RYS_WANT_COEF\nstatic const double rys_coef[%d] = {\n", off[nmax + 1] + 4 * nb * NB);
     for (int n = 1; n <= nmax; n++) {
         size_t cnt = (size_t)nint[n] * 2 * n * NC;
         for (size_t k = 0; k < cnt; k++)
             fprintf(fo, "%a,%s", tables[n][k], (k % 4 == 3) ? "\n" : " ");
     }
+    for (int m = 0; m < 4; m++)
+        for (int i = 0; i < nb; i++) {
+            double c[NB];
+            boys_fit(m, 0.5Q * i, c);
+            for (int e = 0; e < NB; e++) fprintf(fo, "%a,%s", c[e], e == NB - 1 ? "\n" : " ");
+        }
     fprintf(fo, "};\n#endif\n");
     fclose(fo);
     return 0;
