@@ -313,14 +313,9 @@ struct JKScreen {
     }
 };
 
-// Row classes (team and generic kernels): one block (256 threads) per class
-// quartet.  qoff counts the FP64 part, qoff32 the FP32 part, whose first
+// Row classes (team and generic kernels): one block of 256 threads.  qoff counts the FP64 part, qoff32 the FP32 part, whose first
 // column per row is klb[ij].
-__global__ void jk_screen_kernel(const JKScreenCQ* __restrict__ cqs, double tol, int nbins, int prescreen,
-                                 double fp32_cutoff) {
-    const JKScreenCQ cq = cqs[blockIdx.x];
-    if (cq.runs) return;
-    const JKScreen sc(cq, tol, nbins, prescreen, fp32_cutoff);
+__device__ __forceinline__ void jk_screen_rows(const JKScreenCQ& cq, const JKScreen& sc) {
     __shared__ long long carry, carry32;
     __shared__ long long wsum[32], wsum32[32];
     if (threadIdx.x == 0) {
@@ -351,14 +346,19 @@ __global__ void jk_screen_kernel(const JKScreenCQ* __restrict__ cqs, double tol,
     }
 }
 
-// Run classes: a warp per run (blockIdx.x = class quartet), a lane per entry.
+// Screening of a build, blockIdx.x = class quartet.  Row classes: the first
+// block, as above.  Run classes: a warp per run, a lane per entry.
 // Writes the entries' bounds, adds up the quartet counts and leaves the
 // items of each run in ioff / ioff32 (made a prefix by jk_run_scan_kernel).
-__global__ void __launch_bounds__(256) jk_run_bounds_kernel(const JKScreenCQ* __restrict__ cqs, double tol, int nbins,
+__global__ void __launch_bounds__(256) jk_screen_kernel(const JKScreenCQ* __restrict__ cqs, double tol, int nbins,
                                                             int prescreen, double fp32_cutoff) {
     const JKScreenCQ cq = cqs[blockIdx.x];
-    if (!cq.runs || (int)(blockIdx.y * 8) >= cq.nrun) return;
+    if (cq.runs ? (int)(blockIdx.y * 8) >= cq.nrun : blockIdx.y > 0) return;  // block-uniform
     const JKScreen sc(cq, tol, nbins, prescreen, fp32_cutoff);
+    if (!cq.runs) {
+        jk_screen_rows(cq, sc);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     long long n64 = 0, n32 = 0;
     for (int run = blockIdx.y * 8 + (threadIdx.x >> 5); run < cq.nrun; run += gridDim.y * 8) {
@@ -481,20 +481,6 @@ struct JKCall {
     double* jpb;
     int n_dm;
 };
-__global__ void jk_set_call_kernel(JKSeg* __restrict__ s64, JKSeg* __restrict__ s32, int nseg, const JKCall c) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * nseg; i += gridDim.x * blockDim.x) {
-        JKSeg& s = i < nseg ? s64[i] : s32[i - nseg];
-        s.dm = c.dm;
-        s.vj = c.vj;
-        s.vk = c.vk;
-        s.dp = c.dp;
-        s.jp = c.jp;
-        s.dpb = c.dpb;
-        s.jpb = c.jpb;
-        s.n_dm = c.n_dm;
-    }
-}
-
 // Pair-packed J side.  mode 0: gather the density blocks of every pair into
 // dp (element c of pair p of class k at off_k + c*np_k + p, one copy per
 // density) and into dpb (entry-major: element c of entry e at off_k +
@@ -531,23 +517,61 @@ __device__ __forceinline__ void jk_pack_body(const JKPackMol& a, int mode) {
 
 __global__ void jk_pack_kernel(const JKPackMol one, int mode) { jk_pack_body(one, mode); }
 
+// Start of a build, one launch: the call's buffers into the segments, the
+// counters and the J accumulators cleared, the densities packed.
+__global__ void __launch_bounds__(256) jk_begin_kernel(JKSeg* __restrict__ s64, JKSeg* __restrict__ s32, int nseg,
+                                                       const JKCall c, unsigned long long* __restrict__ zero,
+                                                       long long nzero, const JKPackMol pm) {
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    for (long long i = t0; i < 2 * nseg; i += step) {
+        JKSeg& s = i < nseg ? s64[i] : s32[i - nseg];
+        s.dm = c.dm;
+        s.vj = c.vj;
+        s.vk = c.vk;
+        s.dp = c.dp;
+        s.jp = c.jp;
+        s.dpb = c.dpb;
+        s.jpb = c.jpb;
+        s.n_dm = c.n_dm;
+    }
+    for (long long i = t0; i < nzero; i += step) zero[i] = 0;
+    if (pm.total > 0) {
+        const long long na = 2 * pm.n_dm * pm.total;  // jp and jpb lie together
+        for (long long i = t0; i < na; i += step) pm.jp[i] = 0.;
+        jk_pack_body(pm, 0);
+    }
+}
+
 // one molecule per blockIdx.y
 __global__ void jk_pack_batch_kernel(const JKPackMol* __restrict__ mols, int mode) {
     const JKPackMol m = mols[blockIdx.y];
     if (m.total > 0) jk_pack_body(m, mode);
 }
 
-// J = 2 (V + V^T), K = V + V^T in place on the working-basis buffers, where
-// V[i, j] = mem[i + nao j]; out_rm[p, q] = fac (mem[p nao + q] + mem[q nao + p])
-__global__ void jk_symmetrize_kernel(const double* __restrict__ in, double* __restrict__ out, int nao, int n_dm,
-                                     double fac) {
-    long long n = (long long)nao * nao * n_dm;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        long long m = e / ((long long)nao * nao);
-        long long r = e - m * nao * nao;
-        int p = (int)(r / nao), q = (int)(r % nao);
-        const double* b = in + m * nao * nao;
-        out[e] = fac * (b[(size_t)p * nao + q] + b[(size_t)q * nao + p]);
+// 2 (V + V^T) of the first nj matrices (J), V + V^T of the others (K), where
+// V[i, j] = mem[i + nao j]; out_rm[p, q] = fac (mem[p nao + q] + mem[q nao + p]).
+// 32 x 32 tiles, the transposed one through shared memory, so that both reads
+// and the write are whole rows (the element-wise kernel before read a column
+// per warp).
+__global__ void __launch_bounds__(256) jk_symmetrize_kernel(const double* __restrict__ in, double* __restrict__ out,
+                                                            int nao, int nmat, int nj) {
+    __shared__ double t[32][33];
+    const int nt = (nao + 31) / 32, x = threadIdx.x & 31, y0 = threadIdx.x >> 5;
+    const long long tiles = (long long)nmat * nt * nt;
+    for (long long b = blockIdx.x; b < tiles; b += gridDim.x) {
+        const int m = (int)(b / ((long long)nt * nt)), r = (int)(b - (long long)m * nt * nt);
+        const int p0 = r / nt * 32, q0 = r % nt * 32;
+        const double* v = in + (size_t)m * nao * nao;
+        const double fac = m < nj ? 2. : 1.;
+        for (int y = y0; y < 32; y += 8)
+            if (q0 + y < nao && p0 + x < nao) t[y][x] = v[(size_t)(q0 + y) * nao + p0 + x];
+        __syncthreads();
+        for (int y = y0; y < 32; y += 8)
+            if (p0 + y < nao && q0 + x < nao) {
+                const size_t e = (size_t)(p0 + y) * nao + q0 + x;
+                out[(size_t)m * nao * nao + e] = fac * (v[e] + t[x][y]);
+            }
+        __syncthreads();
     }
 }
 
@@ -1172,16 +1196,6 @@ extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, d
     if (nshards > 1 && (shard < 0 || shard >= nshards)) return set_err(JK_ERR_ARG, "jk_build: shard out of range");
     int rc = build_plan(b, nshards, shard);
     if (rc) return rc;
-    CUDA_TRY(cudaMemsetAsync(b->d_zero, 0, b->zero_bytes, st));
-    const JKDmCond dc{dm, b->d_group_ao, b->d_dm_cond, b->nao, n_dm, b->ngroups, nullptr, 0};
-    jk_dm_cond_kernel<<<dim3(dm_cond_blocks(b->nao), b->ngroups), 256, 0, st>>>(dc, nullptr);
-    CUDA_TRY(cudaGetLastError());
-    if (b->ncq == 0) return JK_OK;
-    double fp32_cutoff = opts ? opts->fp32_cutoff : 0.;
-    const bool mixed = fp32_cutoff > 0;
-    rc = jk_internal_screen(b->d_cq, b->ncq, tol, nbins, prescreen, fp32_cutoff, st);
-    if (!rc) rc = jk_plan_prefix(b->plan, mixed, st);
-    if (rc) return rc;
     // pair-packed density and J accumulators for the run kernels
     const bool packed = vj && b->pack_total > 0;
     JKCall call{dm, vj, vk, nullptr, nullptr, nullptr, nullptr, n_dm};
@@ -1192,6 +1206,7 @@ extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, d
         if (need > b->pk_cap) {
             cudaFree(b->d_pk);
             b->d_pk = nullptr;
+            b->pk_cap = 0;
             CUDA_TRY(cudaMalloc(&b->d_pk, sizeof(double) * need));
             b->pk_cap = need;
         }
@@ -1200,23 +1215,31 @@ extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, d
         call.jp = pm.jp;
         call.dpb = pm.dpb;
         call.jpb = pm.jpb;
-        jk_pack_kernel<<<pk_blocks, 256, 0, st>>>(pm, 0);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaMemsetAsync(pm.jp, 0, 2 * sizeof(double) * n_dm * b->pack_total, st));
     }
-    if (b->plan->nseg) {
-        jk_set_call_kernel<<<(2 * b->plan->nseg + 255) / 256, 256, 0, st>>>(b->plan->d_seg[0], b->plan->d_seg[1],
-                                                                           b->plan->nseg, call);
-        CUDA_TRY(cudaGetLastError());
-    }
-    CUDA_TRY(b->fan.begin(st));
+    jk_begin_kernel<<<std::max(pk_blocks, 8), 256, 0, st>>>(b->plan->d_seg[0], b->plan->d_seg[1], b->plan->nseg, call,
+                                                            (unsigned long long*)b->d_zero,
+                                                            (long long)(b->zero_bytes / 8), pm);
+    CUDA_TRY(cudaGetLastError());
+    const JKDmCond dc{dm, b->d_group_ao, b->d_dm_cond, b->nao, n_dm, b->ngroups, nullptr, 0};
+    jk_dm_cond_kernel<<<dim3(dm_cond_blocks(b->nao), b->ngroups), 256, 0, st>>>(dc, nullptr);
+    CUDA_TRY(cudaGetLastError());
+    if (b->ncq == 0) return JK_OK;
+    double fp32_cutoff = opts ? opts->fp32_cutoff : 0.;
+    const bool mixed = fp32_cutoff > 0;
+    rc = jk_internal_screen(b->d_cq, b->ncq, tol, nbins, prescreen, fp32_cutoff, st);
+    if (!rc) rc = jk_plan_prefix(b->plan, mixed, st);
+    if (rc) return rc;
+    // class launches on side streams: 4 of them, 8 with the FP32 parts or for
+    // a molecule whose launches leave most of the device idle
+    const int np = mixed ? 2 : 1, ns = mixed || b->h_pair2bra.size() < 4096 ? 8 : 4;
+    CUDA_TRY(b->fan.begin(st, ns));
     for (int k = 0; k < (int)b->plan->keys.size(); k++)
-        for (int part = 0; part < (mixed ? 2 : 1); part++) {
+        for (int part = 0; part < np; part++) {
             rc = jk_plan_launch(b->plan, k, part, b->plan->keys[k].cfg[part], n_dm, b->nsm,
-                                b->fan.pick(2 * k + part));
+                                b->fan.s[(np * k + part) % ns]);
             if (rc) return rc;
         }
-    CUDA_TRY(b->fan.end(st));
+    CUDA_TRY(b->fan.end(st, ns));
     if (packed) {
         jk_pack_kernel<<<pk_blocks, 256, 0, st>>>(pm, 1);
         CUDA_TRY(cudaGetLastError());
@@ -1521,11 +1544,12 @@ extern "C" int jk_get_jk(jk_basis_t* b, const double* coeff, int nao0, const dou
     if (!b || !coeff || !dm0 || n_dm <= 0 || nao0 <= 0) return set_err(JK_ERR_ARG, "jk_get_jk: invalid arguments");
     cudaStream_t st = (cudaStream_t)stream;
     int nao = b->nao;
-    size_t nn = (size_t)nao * nao * n_dm;
-    size_t need = 4 * nn + (size_t)nao * nao0;
+    size_t nn = (size_t)nao * nao * n_dm, nt = (size_t)nao * nao0 * n_dm;
+    size_t need = 5 * nn + 2 * nt;
     if (need > b->work_cap) {
         cudaFree(b->d_work);
         b->d_work = nullptr;
+        b->work_cap = 0;
         CUDA_TRY(cudaMalloc(&b->d_work, sizeof(double) * need));
         b->work_cap = need;
     }
@@ -1534,8 +1558,8 @@ extern "C" int jk_get_jk(jk_basis_t* b, const double* coeff, int nao0, const dou
     double* dms = b->d_work;
     double* vjw = dms + nn;
     double* vkw = vjw + nn;
-    double* sym = vkw + nn;
-    double* tmp = sym + nn;  // nao x nao0
+    double* sym = vkw + nn;      // J, then K
+    double* tmp = sym + 2 * nn;  // 2 n_dm x (nao x nao0)
     // dms = C D C^T (cuobc/scf/hf.py:73-74)
     for (int m = 0; m < n_dm; m++) {
         const double* D = dm0 + (size_t)m * nao0 * nao0;
@@ -1543,23 +1567,23 @@ extern "C" int jk_get_jk(jk_basis_t* b, const double* coeff, int nao0, const dou
         BLAS_TRY(gemm_rm(b->blas, false, true, nao, nao, nao0, 1.0, tmp, nao0, coeff, nao0, 0.0,
                          dms + (size_t)m * nao * nao, nao));
     }
-    if (vj0) CUDA_TRY(cudaMemsetAsync(vjw, 0, sizeof(double) * nn, st));
-    if (vk0) CUDA_TRY(cudaMemsetAsync(vkw, 0, sizeof(double) * nn, st));
+    if (!vj0 && !vk0) return JK_OK;
+    double* v0 = vj0 ? vjw : vkw;  // the outputs lie together
+    const size_t nv = vj0 && vk0 ? 2 * nn : nn;
+    CUDA_TRY(cudaMemsetAsync(v0, 0, sizeof(double) * nv, st));
     int rc = jk_build(b, dms, n_dm, vj0 ? vjw : nullptr, vk0 ? vkw : nullptr, opts, stream);
     if (rc) return rc;
-    // J = 2 C^T (V + V^T) C, K = C^T (V + V^T) C (cuobc/scf/hf.py:171-181)
-    for (int pass = 0; pass < 2; pass++) {
-        double* out = pass == 0 ? vj0 : vk0;
-        double* w = pass == 0 ? vjw : vkw;
-        if (!out) continue;
-        jk_symmetrize_kernel<<<b->nsm * 4, 256, 0, st>>>(w, sym, nao, n_dm, pass == 0 ? 2.0 : 1.0);
-        CUDA_TRY(cudaGetLastError());
-        for (int m = 0; m < n_dm; m++) {
-            BLAS_TRY(gemm_rm(b->blas, false, false, nao, nao0, nao, 1.0, sym + (size_t)m * nao * nao, nao, coeff,
-                             nao0, 0.0, tmp, nao0));
-            BLAS_TRY(gemm_rm(b->blas, true, false, nao0, nao0, nao, 1.0, coeff, nao0, tmp, nao0, 0.0,
-                             out + (size_t)m * nao0 * nao0, nao0));
-        }
+    // J = 2 C^T (V + V^T) C, K = C^T (V + V^T) C (cuobc/scf/hf.py:171-181):
+    // one symmetrisation, one product with C from the right for all matrices
+    const int nmat = (int)(nv / nn) * n_dm;
+    jk_symmetrize_kernel<<<b->nsm * 4, 256, 0, st>>>(v0, sym, nao, nmat, vj0 ? n_dm : 0);
+    CUDA_TRY(cudaGetLastError());
+    BLAS_TRY(gemm_rm(b->blas, false, false, nmat * nao, nao0, nao, 1.0, sym, nao, coeff, nao0, 0.0, tmp, nao0));
+    for (int m = 0; m < nmat; m++) {
+        double* out = vj0 && m < n_dm ? vj0 + (size_t)m * nao0 * nao0
+                                      : vk0 + (size_t)(vj0 ? m - n_dm : m) * nao0 * nao0;
+        BLAS_TRY(gemm_rm(b->blas, true, false, nao0, nao0, nao, 1.0, coeff, nao0, tmp + (size_t)m * nao * nao0, nao0,
+                         0.0, out, nao0));
     }
     return JK_OK;
 }
@@ -1852,11 +1876,10 @@ int jk_internal_screen(const JKScreenCQ* d_cq, int ncq, double tol, int nbins, i
                        void* stream) {
     if (ncq <= 0) return JK_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    jk_screen_kernel<<<ncq, 256, 0, st>>>(d_cq, tol, nbins, prescreen, fp32_cutoff);
     // enough blocks for a large class, few enough that small ones (their
     // surplus blocks leave at once) stay cheap
     const unsigned by = ncq <= 64 ? 512 : (ncq <= 1024 ? 64 : 16);
-    jk_run_bounds_kernel<<<dim3(ncq, by), 256, 0, st>>>(d_cq, tol, nbins, prescreen, fp32_cutoff);
+    jk_screen_kernel<<<dim3(ncq, by), 256, 0, st>>>(d_cq, tol, nbins, prescreen, fp32_cutoff);
     jk_run_scan_kernel<<<ncq, 1024, 0, st>>>(d_cq);
     CUDA_TRY(cudaGetLastError());
     return JK_OK;

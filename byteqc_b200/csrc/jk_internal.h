@@ -76,15 +76,16 @@ struct JKFanout {
         }
         return e;
     }
-    cudaError_t begin(cudaStream_t st) {
+    // fork the first n streams from st, join them back
+    cudaError_t begin(cudaStream_t st, int n = JK_SIDE_STREAMS) {
         cudaError_t e = cudaEventRecord(fork, st);
-        for (int i = 0; e == cudaSuccess && i < JK_SIDE_STREAMS; i++) e = cudaStreamWaitEvent(s[i], fork, 0);
+        for (int i = 0; e == cudaSuccess && i < n; i++) e = cudaStreamWaitEvent(s[i], fork, 0);
         return e;
     }
     cudaStream_t pick(int i) const { return s[i % JK_SIDE_STREAMS]; }
-    cudaError_t end(cudaStream_t st) {
+    cudaError_t end(cudaStream_t st, int n = JK_SIDE_STREAMS) {
         cudaError_t e = cudaSuccess;
-        for (int i = 0; e == cudaSuccess && i < JK_SIDE_STREAMS; i++) {
+        for (int i = 0; e == cudaSuccess && i < n; i++) {
             e = cudaEventRecord(join[i], s[i]);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(st, join[i], 0);
         }
@@ -146,7 +147,10 @@ struct JKPlan {
     std::vector<int> key_off;  // nkeys + 1 segment offsets
     int nseg = 0, nshards = 1, shard = 0;
     JKSeg* d_seg[2] = {nullptr, nullptr};        // FP64, FP32 parts
-    long long* d_segt[2] = {nullptr, nullptr};   // task prefix per key: nseg + nkeys entries
+    long long* d_segt[2] = {nullptr, nullptr};   // task prefix per key: nseg + nkeys entries (keys of one
+                                                 // segment use the screening's {0, count} itself)
+    std::vector<const long long*> one[2];        // that pair per key, or null
+    bool multi = false;                          // some key has several segments
     const long long** d_cnt[2] = {nullptr, nullptr};
     int* d_key_off = nullptr;
     unsigned long long* d_queue = nullptr;       // 2 work counters per key (persistent launches)

@@ -107,13 +107,20 @@ int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols) {
     std::vector<const long long*> cnt(ns);
     for (int part = 0; part < 2; part++) {
         size_t i = 0;
-        for (auto& k : p->keys)
+        for (auto& k : p->keys) {
+            if (k.segs.size() != 1) {
+                p->one[part].push_back(nullptr);
+                p->multi = true;
+            }
             for (auto& s : k.segs) {
                 const jk_basis* b = mols[s.first];
                 const JKScreenCQ& cq = b->h_cq[s.second];
                 jk_internal_fill_seg_cq(b, s.second, part, &seg[i]);
+                if (k.segs.size() == 1)
+                    p->one[part].push_back(cq.runs ? (part ? cq.itm32 : cq.itm) : (part ? cq.task032 : cq.task0));
                 cnt[i++] = (cq.runs ? (part ? cq.itm32 : cq.itm) : (part ? cq.task032 : cq.task0)) + 1;
             }
+        }
         PCUDA(cudaMalloc(&p->d_seg[part], sizeof(JKSeg) * ns));
         PCUDA(cudaMalloc(&p->d_segt[part], sizeof(long long) * (ns + nkeys + 1)));
         PCUDA(cudaMalloc((void**)&p->d_cnt[part], sizeof(long long*) * ns));
@@ -127,7 +134,7 @@ int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols) {
 
 int jk_plan_prefix(const JKPlan* p, bool mixed, cudaStream_t st) {
     const int nkeys = (int)p->keys.size();
-    if (nkeys == 0) return JK_OK;
+    if (nkeys == 0 || !p->multi) return JK_OK;
     for (int part = 0; part < (mixed ? 2 : 1); part++)
         jk_seg_prefix_kernel<<<nkeys, 32, 0, st>>>(p->d_cnt[part], p->d_key_off, p->d_segt[part]);
     PCUDA(cudaGetLastError());
@@ -141,6 +148,6 @@ int jk_plan_launch(const JKPlan* p, int k, int part, const JKBatchCfg& cfg, int 
     if (!f) return jk_internal_set_err(JK_ERR_UNSUPPORTED, "no kernel for a class of the build");
     JKBatchCfg c = cfg;
     c.queue = c.grab > 0 ? p->d_queue + 2 * k + part : nullptr;
-    PCUDA(f(p->d_seg[part] + off, p->d_segt[part] + off + k, n, key.max_items, n_dm, nsm, c, st));
+    PCUDA(f(p->d_seg[part] + off, p->one[part][k] ? p->one[part][k] : p->d_segt[part] + off + k, n, key.max_items, n_dm, nsm, c, st));
     return JK_OK;
 }
