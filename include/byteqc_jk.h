@@ -197,7 +197,7 @@ int jk_get_jk(jk_basis_t *basis, const double *coeff, int nao0, const double *dm
  * jk_build makes it; solo_tasks <= 0 merges everything.  jk_batch_create
  * uses JK_BATCH_SOLO_TASKS.
  */
-#define JK_BATCH_SOLO_TASKS (1LL << 14)
+#define JK_BATCH_SOLO_TASKS (1LL << 24)
 int jk_batch_create(jk_basis_t *const *bases, int nmol, jk_batch_t **out);
 int jk_batch_create_ex(jk_basis_t *const *bases, int nmol, long long solo_tasks, jk_batch_t **out);
 int jk_batch_destroy(jk_batch_t *batch);
