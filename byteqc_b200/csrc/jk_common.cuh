@@ -513,6 +513,19 @@ __device__ __forceinline__ void rys_2d(R seed, R c00, R c0p, R b10, R b01, R b00
     }
 }
 
+// Pairs of a class lie on the device in buckets of `bucket` consecutive Schwarz
+// ranks, ordered by shells inside a bucket.  End of the positions that hold
+// the ranks below h, and first position of an item grid of `chunk` pairs that
+// covers rank lo.
+__host__ __device__ __forceinline__ int jk_bucket_end(int h, int bucket, int n) {
+    if (h <= 0) return 0;
+    const int e = ((h - 1) / bucket + 1) * bucket;
+    return e < n ? e : n;
+}
+__host__ __device__ __forceinline__ int jk_item_base(int lo, int bucket, int chunk) {
+    return lo / bucket * bucket / chunk * chunk;
+}
+
 // ---------------------------------------------------------------------------
 // Segment: one (molecule, class quartet) piece of work.  For the team and
 // generic kernels its tasks are the screened contracted shell quartets
@@ -526,10 +539,14 @@ struct JKSeg {
     const long long* qoff;  // n_ij + 1 entries (device)
     const int* kl_base;     // first kl column of each row (FP32 part of the mixed mode), or null
     int n_ij;
-    // run kernels: entry e of the bra class is pair ent[e] (an index in the
+    // run kernels: entry e of the bra class is pair ent[e] (a position in the
     // class), run r holds the entries run0[r] .. run0[r+1] (one shell i, at
     // most 32 entries) and ioff[r+1] - ioff[r] items; entry e keeps the kets
-    // elo[e] .. ehi[e] (elo null: from 0)
+    // of Schwarz ranks elo[e] .. ehi[e] (elo null: from 0).  rank and pos,
+    // indexed by pair, give a position's rank in its class and the inverse
+    // (rows and columns of the other kernels are ranks).
+    const int *rank, *pos;
+    int bucket;  // Schwarz ranks per bucket of the ket class
     int nrun;
     const int *ent, *run0;
     const int *elo, *ehi;

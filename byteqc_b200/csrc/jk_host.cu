@@ -365,18 +365,18 @@ __global__ void __launch_bounds__(256) jk_screen_kernel(const JKScreenCQ* __rest
         const int e0 = cq.run0[run], ne = cq.run0[run + 1] - e0;
         int c64 = 0, cnt = 0;
         if (lane < ne) {
-            sc.row(cq, cq.ent[e0 + lane], c64, cnt);
+            sc.row(cq, cq.erank[e0 + lane], c64, cnt);
             cq.klb[e0 + lane] = c64;
             cq.kle[e0 + lane] = cnt;
         }
         n64 += c64;
         n32 += cnt - c64;
         const int h64 = __reduce_max_sync(0xffffffffu, c64);
-        const int l32 = __reduce_min_sync(0xffffffffu, c64 < cnt ? c64 : 0x7fffffff) / cq.runs * cq.runs;
+        const int l32 = jk_item_base(__reduce_min_sync(0xffffffffu, c64 < cnt ? c64 : 0x7fffffff), cq.bucket, cq.runs);
         const int h32 = __reduce_max_sync(0xffffffffu, c64 < cnt ? cnt : 0);
         if (lane == 0) {
-            cq.ioff[run] = (h64 + cq.runs - 1) / cq.runs;
-            cq.ioff32[run] = h32 > 0 ? (h32 - l32 + cq.runs - 1) / cq.runs : 0;
+            cq.ioff[run] = (jk_bucket_end(h64, cq.bucket, cq.n_kl) + cq.runs - 1) / cq.runs;
+            cq.ioff32[run] = h32 > 0 ? (jk_bucket_end(h32, cq.bucket, cq.n_kl) - l32 + cq.runs - 1) / cq.runs : 0;
         }
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -421,12 +421,12 @@ __global__ void __launch_bounds__(1024) jk_run_scan_kernel(const JKScreenCQ* __r
 }
 
 // per-class-pair entries: items of each run from the entries' ket ends
-__global__ void jk_run_items_kernel(int nrun, int chunk, const int* __restrict__ run0, const int* __restrict__ ehi,
+__global__ void jk_run_items_kernel(int nrun, int chunk, int bucket, int n_kl, const int* __restrict__ run0, const int* __restrict__ ehi,
                                     long long* __restrict__ ioff) {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrun; r += gridDim.x * blockDim.x) {
         int h = 0;
         for (int e = run0[r]; e < run0[r + 1]; e++) h = max(h, ehi[e]);
-        ioff[r] = (h + chunk - 1) / chunk;
+        ioff[r] = (jk_bucket_end(h, bucket, n_kl) + chunk - 1) / chunk;
     }
 }
 __global__ void __launch_bounds__(1024) jk_run_scan1_kernel(int nrun, long long* ioff, long long* itm) {
@@ -599,6 +599,9 @@ static void free_basis(jk_basis* b) {
     cudaFree(b->d_zero);
     cudaFree(b->d_ent);
     cudaFree(b->d_inv);
+    cudaFree(b->d_erank);
+    cudaFree(b->d_rank);
+    cudaFree(b->d_pos);
     cudaFree(b->d_bprim);
     cudaFree(b->d_bprimf);
     cudaFree(b->d_bpair);
@@ -657,6 +660,10 @@ static int rys_table_device(const double** out) {
     *out = g_rys_dev[dev];
     return JK_OK;
 }
+
+// Schwarz ranks per bucket of a class of n pairs: 16 buckets, of whole chunks
+// of 32 (a class up to 512 pairs is sorted inside its chunks only)
+static int sort_bucket(int n) { return std::max(32, (n / 16 + 31) / 32 * 32); }
 
 // Run length of a class quartet's bra (an index of JK_RUN_LEN): the longest
 // that still gives a few items per resident warp before screening; a
@@ -791,6 +798,31 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         }
     }
     b->ncp = (int)b->h_cls_gi.size();
+    // Device order of a class's pairs: buckets of sort_bucket(pairs)
+    // consecutive Schwarz ranks, inside a bucket by (bra shell, ket shell).
+    // The lanes of a run kernel's warp hold consecutive pairs, so the D_jk they
+    // read and the K_jk they add to lie on a few sectors instead of one each
+    // ((ps| pairs of (H2O)64 / cc-pVDZ: 5 sectors per 32 lanes for k and 23
+    // for l instead of 30 and 30), for at most one bucket of lanes idle at the
+    // end of a row (6 %).  The lists that the C-ABI gives out stay in rank
+    // order, as do log q and the screening.
+    const size_t npair = b->h_pair2bra.size();
+    std::vector<int> obra(npair), oket(npair), orank(npair), opos(npair);
+    for (int c = 0; c < b->ncp; c++) {
+        const int p0 = b->h_pair_locs[c], np = b->h_pair_locs[c + 1] - p0, S = sort_bucket(np);
+        int* r = orank.data() + p0;
+        for (int x = 0; x < np; x++) r[x] = x;
+        for (int x = 0; x < np; x += S)
+            std::sort(r + x, r + std::min(np, x + S), [&](int u, int v) {
+                const int a = b->h_pair2bra[p0 + u], d = b->h_pair2bra[p0 + v];
+                return a != d ? a < d : b->h_pair2ket[p0 + u] < b->h_pair2ket[p0 + v];
+            });
+        for (int x = 0; x < np; x++) {
+            opos[p0 + r[x]] = x;
+            obra[p0 + x] = b->h_pair2bra[p0 + r[x]];
+            oket[p0 + x] = b->h_pair2ket[p0 + r[x]];
+        }
+    }
     // primitive-pair data (cuobc/lib/gint/pair_data.c:83-141)
     long long npp = 0;
     b->h_prim_locs.push_back(0);
@@ -814,7 +846,7 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         // h_prim_locs[c] + k * (pairs in the class) + r
         const int p0 = b->h_pair_locs[c], pst = b->h_pair_locs[c + 1] - p0;
         for (int p = p0; p < p0 + pst; p++) {
-            int ish = b->h_pair2bra[p], jsh = b->h_pair2ket[p];
+            int ish = obra[p], jsh = oket[p];
             int npi = bas[ish * BAS_SLOTS + NPRIM_OF], npj = bas[jsh * BAS_SLOTS + NPRIM_OF];
             int li = bas[ish * BAS_SLOTS + ANG_OF], lj = bas[jsh * BAS_SLOTS + ANG_OF];
             const double* ai = env + bas[ish * BAS_SLOTS + PTR_EXP];
@@ -872,7 +904,7 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         std::vector<double> geo(6 * (np ? np : 1));
         std::vector<int> pao(2 * (np ? np : 1));
         for (size_t p = 0; p < np; p++) {
-            const int sh[2] = {b->h_pair2bra[p], b->h_pair2ket[p]};
+            const int sh[2] = {obra[p], oket[p]};
             for (int a = 0; a < 2; a++) {
                 for (int d = 0; d < 3; d++) geo[(3 * a + d) * np + p] = bx[(size_t)d * nbas + sh[a]];
                 pao[a * np + p] = b->h_ao_loc[sh[a]];
@@ -881,14 +913,16 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         CUDA_TRY(upload(&b->d_pgeo, geo.data(), geo.size()));
         CUDA_TRY(upload(&b->d_pao, pao.data(), pao.size()));
     }
-    CUDA_TRY(upload(&b->d_pair2bra, b->h_pair2bra.data(), b->h_pair2bra.size()));
-    CUDA_TRY(upload(&b->d_pair2ket, b->h_pair2ket.data(), b->h_pair2ket.size()));
+    CUDA_TRY(upload(&b->d_pair2bra, obra.data(), npair));
+    CUDA_TRY(upload(&b->d_pair2ket, oket.data(), npair));
+    CUDA_TRY(upload(&b->d_rank, orank.data(), npair));
+    CUDA_TRY(upload(&b->d_pos, opos.data(), npair));
     CUDA_TRY(upload(&b->d_log_q, b->h_log_q.data(), b->h_log_q.size()));
     CUDA_TRY(upload(&b->d_log_q_raw, b->h_log_q_raw.data(), b->h_log_q_raw.size()));
     // runs of every class's pairs: the pairs of one first shell, in Schwarz
     // order, cut at each run length
     {
-        std::vector<int> ent(b->h_pair2bra.size()), inv(b->h_pair2bra.size()), run0;
+        std::vector<int> ent(npair), erank(npair), inv(npair), run0;
         for (int v = 0; v < JK_RUN_LEVELS; v++) {
             b->h_nrun[v].assign(b->ncp, 0);
             b->h_run_off[v].assign(b->ncp, 0);
@@ -899,7 +933,7 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             for (int x = 0; x < np; x++) e[x] = x;
             std::stable_sort(e, e + np,
                              [&](int x, int y) { return b->h_pair2bra[p0 + x] < b->h_pair2bra[p0 + y]; });
-            for (int x = 0; x < np; x++) inv[p0 + e[x]] = x;
+            // e: ranks in run order, then the positions
             for (int v = 0; v < JK_RUN_LEVELS; v++) {
                 b->h_run_off[v][c] = (int)run0.size();
                 int beg = 0;
@@ -913,8 +947,14 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
                 }
                 run0.push_back(np);
             }
+            for (int x = 0; x < np; x++) {
+                erank[p0 + x] = e[x];
+                e[x] = opos[p0 + e[x]];
+                inv[p0 + e[x]] = x;
+            }
         }
         CUDA_TRY(upload(&b->d_ent, ent.data(), ent.size()));
+        CUDA_TRY(upload(&b->d_erank, erank.data(), erank.size()));
         CUDA_TRY(upload(&b->d_run0, run0.data(), run0.size()));
         CUDA_TRY(upload(&b->d_inv, inv.data(), inv.size()));
         CUDA_TRY(cudaMalloc(&b->d_bprim, sizeof(double) * 8 * (size_t)std::max(npp, 1LL)));
@@ -1002,6 +1042,8 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         q.ioff = b->d_ioff + ioff_at[c];
         q.ioff32 = q.ioff + q.nrun;
         q.ent = b->d_ent + q.pair_ij0;
+        q.erank = b->d_erank + q.pair_ij0;
+        q.bucket = sort_bucket(q.n_kl);
         q.run0 = b->d_run0 + b->h_run_off[q.level][q.cp_ij];
         q.task0 = b->d_task0 + 2 * c;
         q.task032 = b->d_task032 + 2 * c;
@@ -1112,6 +1154,9 @@ static void fill_seg(const jk_basis* b, int cp_ij, int cp_kl, const long long* q
     s->npf = n;
     s->pgeo = b->d_pgeo;
     s->pnp = b->d_pnp;
+    s->rank = b->d_rank;
+    s->pos = b->d_pos;
+    s->bucket = sort_bucket(s->pst_kl);
     s->bprim = b->d_bprim + 8 * (size_t)s->prim_ij0;
     s->bprimf = b->d_bprimf + 8 * (size_t)s->prim_ij0;
     s->bpair = b->d_bpair + 4 * (size_t)s->pair_ij0;
@@ -1293,9 +1338,9 @@ __device__ __forceinline__ int jk_rowbins_cols(const JKRowBins& b, int r) {
 
 // run classes: ket end of every entry
 __global__ void jk_run_rowbins_kernel(const __grid_constant__ JKRowBins rb, int n_ij, int n_kl,
-                                      const int* __restrict__ ent, int* __restrict__ ehi) {
+                                      const int* __restrict__ erank, int* __restrict__ ehi) {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_ij; e += gridDim.x * blockDim.x)
-        ehi[e] = min(jk_rowbins_cols(rb, ent[e]), n_kl);
+        ehi[e] = min(jk_rowbins_cols(rb, erank[e]), n_kl);
 }
 
 __global__ void jk_rowbins_kernel(const JKRowBins rb, int n_ij, long long* __restrict__ qoff,
@@ -1375,7 +1420,7 @@ extern "C" int jk_build_class_pair(jk_basis_t* b, double* vj, double* vk, const 
     if (jk_internal_run_table(b, cp_ij, cp_kl, &rt)) {
         const int n_kl = seg.pst_kl;
         if (n_ij == 0 || n_kl == 0) return JK_OK;
-        jk_run_rowbins_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(rb, n_ij, n_kl, rt.ent, b->d_ehi1);
+        jk_run_rowbins_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(rb, n_ij, n_kl, rt.erank, b->d_ehi1);
         CUDA_TRY(cudaGetLastError());
         rc = jk_internal_run_items(rt, b->d_ehi1, b->d_qoff1, b->d_task01, st);
         seg.nrun = rt.nrun;
@@ -1802,6 +1847,9 @@ int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg& s
 
 int jk_internal_run_table(const jk_basis_t* b, int cp_ij, int cp_kl, JKRunTab* out) {
     if (!g_tabs.run[class_index(b, cp_ij, cp_kl)]) return 0;
+    out->n_kl = b->h_pair_locs[cp_kl + 1] - b->h_pair_locs[cp_kl];
+    out->bucket = sort_bucket(out->n_kl);
+    out->erank = b->d_erank + b->h_pair_locs[cp_ij];
     out->chunk = g_tabs.run[class_index(b, cp_ij, cp_kl)];
     const int v = run_level(b, cp_ij, b->h_pair_locs[cp_kl + 1] - b->h_pair_locs[cp_kl], out->chunk);
     out->nrun = b->h_nrun[v][cp_ij];
@@ -1812,7 +1860,8 @@ int jk_internal_run_table(const jk_basis_t* b, int cp_ij, int cp_kl, JKRunTab* o
 
 int jk_internal_run_items(const JKRunTab& rt, const int* ehi, long long* ioff, long long* itm, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
-    if (rt.nrun > 0) jk_run_items_kernel<<<(rt.nrun + 255) / 256, 256, 0, st>>>(rt.nrun, rt.chunk, rt.run0, ehi, ioff);
+    if (rt.nrun > 0) jk_run_items_kernel<<<(rt.nrun + 255) / 256, 256, 0, st>>>(rt.nrun, rt.chunk, rt.bucket, rt.n_kl, rt.run0,
+                                                                                ehi, ioff);
     jk_run_scan1_kernel<<<1, 1024, 0, st>>>(rt.nrun, ioff, itm);
     CUDA_TRY(cudaGetLastError());
     return JK_OK;

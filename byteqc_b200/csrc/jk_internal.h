@@ -28,7 +28,8 @@ struct JKScreenCQ {
     long long *qoff, *qoff32;
     int* klb;                     // (run classes: per entry, the end of the FP64 part)
     // runs: the run table, the end of the FP32 part per entry, item prefixes
-    const int *ent, *run0;
+    const int *ent, *erank, *run0;  // positions and ranks of the entries
+    int bucket;                     // Schwarz ranks per bucket of the ket class
     int* kle;
     long long *ioff, *ioff32;
     long long *itm, *itm32;       // {0, items} of each part
@@ -50,7 +51,8 @@ int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg& s
 // length; 0 rows if the class quartet does not run a run kernel
 struct JKRunTab {
     int nrun, chunk;  // runs, ket pairs of an item
-    const int *ent, *run0;
+    int bucket, n_kl;
+    const int *ent, *erank, *run0;
 };
 int jk_internal_run_table(const jk_basis_t* b, int cp_ij, int cp_kl, JKRunTab* out);
 // item counts per run from the entries' ket ends (ioff[0..nrun)), then their
@@ -180,17 +182,19 @@ struct jk_basis {
     int cq_owner_n = 0;                // cq_owner_n shards
     long long qoff_total = 0, ioff_total = 0, ent_total = 0;
     // Runs of the bra pairs of each class (jk_runs.cuh): entry e of class c is
-    // pair d_ent[pair_locs[c] + e] of the class; run table v (run length
+    // pair d_ent[pair_locs[c] + e] (a position) of the class; run table v (run length
     // JK_RUN_LEN[v]) of class c has h_nrun[v][c] runs at d_run0 + h_run_off[v][c]
     std::vector<int> h_nrun[JK_RUN_LEVELS], h_run_off[JK_RUN_LEVELS];
     int *d_ent = nullptr, *d_run0 = nullptr;
     int* d_inv = nullptr;  // entry of a pair (the inverse of d_ent)
+    int* d_erank = nullptr;  // Schwarz rank of an entry
+    int *d_rank = nullptr, *d_pos = nullptr;  // rank of a position of the class, and the inverse
     double *d_bprim = nullptr, *d_bpair = nullptr;  // bra records (JKSeg::bprim, bpair)
     float* d_bprimf = nullptr;
     // device
     int *d_atm = nullptr, *d_bas = nullptr, *d_ao_loc = nullptr, *d_group_ao = nullptr;
     double *d_env = nullptr, *d_bas_x = nullptr, *d_qcond = nullptr;
-    int *d_pair2bra = nullptr, *d_pair2ket = nullptr;
+    int *d_pair2bra = nullptr, *d_pair2ket = nullptr;  // by position
     double *d_log_q = nullptr, *d_log_q_raw = nullptr, *d_prim = nullptr;  // prim: a12|e12|x12|y12|z12|1/a12
     float* d_primf = nullptr;  // FP32 path: a12|1/a12|e12/a12|P-R_bra (x, y, z)
     long long nprim_total = 0;

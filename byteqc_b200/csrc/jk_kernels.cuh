@@ -52,6 +52,8 @@ struct JKQuartet {
 __device__ __forceinline__ JKQuartet jk_quartet_at(const JKSeg& sg, int row, int col) {
     JKQuartet q;
     if (sg.kl_base) col += __ldg(sg.kl_base + row);
+    row = __ldg(sg.pos + sg.pair_ij0 + row);  // ranks to positions
+    col = __ldg(sg.pos + sg.pair_kl0 + col);
     const int bij = sg.pair_ij0 + row, bkl = sg.pair_kl0 + col;
     q.bij = bij;
     q.bkl = bkl;

@@ -90,9 +90,9 @@ __device__ __forceinline__ int na_cols(const int* __restrict__ bins_ij, const in
 
 // run classes: ket end of every entry
 __global__ void jk_na_ehi_kernel(const int* __restrict__ bins_ij, const int* __restrict__ bins_kl, int nbins, int n_ij,
-                                 int n_kl, int diag, const int* __restrict__ ent, int* __restrict__ ehi) {
+                                 int n_kl, int diag, const int* __restrict__ erank, int* __restrict__ ehi) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < n_ij) ehi[e] = na_cols(bins_ij, bins_kl, nbins, n_kl, diag, ent[e]);
+    if (e < n_ij) ehi[e] = na_cols(bins_ij, bins_kl, nbins, n_kl, diag, erank[e]);
 }
 
 // row classes: one block; writes qoff[0..n_ij] and task0 = {0, total}
@@ -175,7 +175,7 @@ extern "C" int jk_build_class_pair_noalloc(jk_basis_t* b, double* vj, double* vk
     if (jk_internal_run_table(b, cp_ij, cp_kl, &rt)) {
         if (n_ij == 0 || n_kl == 0) return JK_OK;
         int* d_ehi = (int*)(sc + JK_NA_OFF_EHI);
-        jk_na_ehi_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(d_bins_ij, d_bins_kl, nbins, n_ij, n_kl, diag, rt.ent,
+        jk_na_ehi_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(d_bins_ij, d_bins_kl, nbins, n_ij, n_kl, diag, rt.erank,
                                                              d_ehi);
         e = cudaGetLastError();
         if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));

@@ -9,7 +9,7 @@
 // some 150 FP64 operations, and the kernels waited on them.
 //
 // Work item: a run (up to 32 bra pairs ij that share the shell i, in Schwarz
-// order) x a chunk (32 consecutive ket pairs kl of the Schwarz-sorted list,
+// order) x a chunk (32 consecutive ket pairs kl of the class, in Schwarz buckets,
 // one per lane).  The warp walks the bra pairs of the run; a lane keeps its
 // ket pair's data, D_kl, D_ik, D_il and the sums for J_kl, K_ik and K_il
 // across the walk (in registers, or in lane-private shared memory where they
@@ -29,8 +29,8 @@
 // records and D_ij are staged in shared memory when the item starts, and the
 // D_jk, D_jl of small classes are asked for before the integrals.
 //
-// Screening: entry e of a run keeps the kets [lo_e, hi_e) (the reference's
-// decisions, from jk_run_bounds_kernel).  A warp loads the bounds of the
+// Screening: entry e of a run keeps the kets of Schwarz ranks [lo_e, hi_e) (the
+// reference's decisions, from jk_screen_kernel).  A warp loads the bounds of the
 // run's entries into its lanes, finds with one ballot the entries that meet
 // its chunk, and walks those; a lane outside an entry's range contributes
 // zeros.
@@ -498,11 +498,16 @@ struct JKRunItem {
             ehi = __ldg(sg.ehi + e0 + lane);
             ent = __ldg(sg.ent + e0 + lane);
         }
-        const int base = sg.elo ? (__reduce_min_sync(0xffffffffu, elo < ehi ? elo : 0x7fffffff) & ~31) : 0;
-        const int c0 = base + 32 * (int)(item - __ldg(sg.ioff + run));
-        unsigned mask = __ballot_sync(0xffffffffu, elo < ehi && elo < c0 + 32 && ehi > c0);
+        const int base =
+            sg.elo ? jk_item_base(__reduce_min_sync(0xffffffffu, elo < ehi ? elo : 0x7fffffff), sg.bucket, 32) : 0;
+        const int mycol = base + 32 * (int)(item - __ldg(sg.ioff + run)) + lane;
+        // Schwarz ranks of the chunk's pairs
+        const bool in = mycol < sg.pst_kl;
+        const int rank = in ? __ldg(sg.rank + sg.pair_kl0 + mycol) : -1;
+        const int rmin = __reduce_min_sync(0xffffffffu, in ? rank : 0x7fffffff),
+                  rmax = __reduce_max_sync(0xffffffffu, rank);
+        unsigned mask = __ballot_sync(0xffffffffu, elo < ehi && elo <= rmax && ehi > rmin);
         if (mask == 0) return;
-        const int mycol = c0 + lane;
         const int ent0 = __shfl_sync(0xffffffffu, ent, 0);
         pst_ij = sg.pst_ij;
         col = min(mycol, sg.pst_kl - 1);
@@ -585,7 +590,7 @@ struct JKRunItem {
             mask &= mask - 1;
             const int4 bound = *reinterpret_cast<const int4*>(rec + 6 * el + 5);
             const double2 pb = rec[6 * el + 4];
-            active = mycol >= bound.x && mycol < bound.y;
+            active = rank >= bound.x && rank < bound.y;
             used |= active;
             j0 = __double2loint(pb.y);
             npij = __double2hiint(pb.y);

@@ -320,13 +320,17 @@ struct JKTRunItem {
             ent = __ldg(sg.ent + e0 + lane);
         }
         const int base =
-            sg.elo ? __reduce_min_sync(0xffffffffu, elo < ehi ? elo : 0x7fffffff) / TPW * TPW : 0;
-        const int c0 = base + TPW * (int)(item - __ldg(sg.ioff + run));
-        unsigned mask = __ballot_sync(0xffffffffu, elo < ehi && elo < c0 + TPW && ehi > c0);
-        if (mask == 0) return;
+            sg.elo ? jk_item_base(__reduce_min_sync(0xffffffffu, elo < ehi ? elo : 0x7fffffff), sg.bucket, TPW) : 0;
         team = lane / T;
         ci = team < TPW ? lane - team * T : 0;
-        const int mycol = team < TPW ? c0 + team : -1;
+        const int mycol = team < TPW ? base + TPW * (int)(item - __ldg(sg.ioff + run)) + team : -1;
+        // Schwarz ranks of the item's ket pairs
+        const bool in = mycol >= 0 && mycol < sg.pst_kl;
+        const int rank = in ? __ldg(sg.rank + sg.pair_kl0 + mycol) : -1;
+        const int rmin = __reduce_min_sync(0xffffffffu, in ? rank : 0x7fffffff),
+                  rmax = __reduce_max_sync(0xffffffffu, rank);
+        unsigned mask = __ballot_sync(0xffffffffu, elo < ehi && elo <= rmax && ehi > rmin);
+        if (mask == 0) return;
         const int ent0 = __shfl_sync(0xffffffffu, ent, 0);
         pst_ij = sg.pst_ij;
         col = max(0, min(mycol, sg.pst_kl - 1));
@@ -383,7 +387,7 @@ struct JKTRunItem {
             mask &= mask - 1;
             const int4 bound = *reinterpret_cast<const int4*>(rec + 6 * el + 5);
             const double2 pa = rec[6 * el + 3], pb = rec[6 * el + 4];
-            active = mycol >= bound.x && mycol < bound.y;
+            active = rank >= bound.x && rank < bound.y;
             used |= active;
             rj[0] = pa.x;
             rj[1] = pa.y;
