@@ -69,6 +69,14 @@ struct JKRunShape {
     static constexpr size_t SLOTS = (KSM ? SLOT : 0) + (DSM ? SLOT : 0);
     static constexpr bool JT = NV <= 10 && FIX + SLOTS + JBUF <= JK_RUN_SMEM;
     static constexpr size_t SMEM = FIX + SLOTS + (JT ? JBUF : 0);
+    // One root at a time in a rolled loop where the code of all roots, times
+    // the passes, does not stay in the instruction cache: unrolled, (fp|ps)
+    // (4 passes, 3 roots) waited for instructions most (2.8 of 8.5 stalled
+    // warps per issue).  (H2O)32 / def2-TZVP, unrolled and rolled: (fp|ps) 14.9
+    // and 11.2 ms, (fs|pp) 7.4 and 5.7, (fs|fs) 4.9 and 3.2; at 2 and 3 passes
+    // (dp|ps) 9.7 and 9.7, (pp|pp) 7.1 and 6.3, but on a contracted basis 3.34
+    // and 3.63, 1.40 and 1.63.
+    static constexpr bool ROLL = C::NPASS >= 4;
     // elements numbered J_kl [0, NJ), K_ik [NJ, ..), K_il
     static constexpr int OIK = NJ, OIL = NJ + C::NFI * C::NFK;
 };
@@ -267,15 +275,25 @@ struct JKRunItem {
                 if (npkl > 1) kpf = jk_ppf(sg, prim_kl + q * sg.pst_kl);
                 for (int p = 0; p < npij; p++) {
                     const JKPrimF pr = jk_prim_f2(braf(p), kpf, ac);
-                    float rs[NR], rw[NR];
-                    rys_table_all_f<NR>(tabf, pr.x, rs, rw);
-#pragma unroll
-                    for (int r = 0; r < NR; r++) {
+                    auto root = [&](float s, float w) {
                         float Ix[C::GS], Iy[C::GS], Iz[C::GS];
-                        jk_unit_f<C>(pr, rs[r], rw[r], 0, normf, dij, dkl, Ix);
-                        jk_unit_f<C>(pr, rs[r], rw[r], 1, normf, dij, dkl, Iy);
-                        jk_unit_f<C>(pr, rs[r], rw[r], 2, normf, dij, dkl, Iz);
+                        jk_unit_f<C>(pr, s, w, 0, normf, dij, dkl, Ix);
+                        jk_unit_f<C>(pr, s, w, 1, normf, dij, dkl, Iy);
+                        jk_unit_f<C>(pr, s, w, 2, normf, dij, dkl, Iz);
                         jk_thread_products<C, R, CI0, NI>(acc, Ix, Iy, Iz);
+                    };
+                    if constexpr (S::ROLL) {
+#pragma unroll 1
+                        for (int r = 0; r < NR; r++) {
+                            float s, w;
+                            rys_root_one_f<NR>(tabf, pr.x, r, s, w);
+                            root(s, w);
+                        }
+                    } else {
+                        float rs[NR], rw[NR];
+                        rys_table_all_f<NR>(tabf, pr.x, rs, rw);
+#pragma unroll
+                        for (int r = 0; r < NR; r++) root(rs[r], rw[r]);
                     }
                 }
             }
@@ -308,15 +326,25 @@ struct JKRunItem {
                 if (npkl > 1) kp = jk_pp(sg, prim_kl + q * sg.pst_kl);
                 for (int p = 0; p < npij; p++) {
                     const JKPrim pr = jk_prim2(bra(p), kp);
-                    double rs[NR], rw[NR];
-                    rys_table_all<NR>(tab, pr.x, rs, rw);
-#pragma unroll
-                    for (int r = 0; r < NR; r++) {
+                    auto root = [&](double s, double w) {
                         R Ix[C::GS], Iy[C::GS], Iz[C::GS];
-                        jk_unit<C, R>(pr, rs[r], rw[r], 0, norm, ri, rj, rk, rl, Ix);
-                        jk_unit<C, R>(pr, rs[r], rw[r], 1, norm, ri, rj, rk, rl, Iy);
-                        jk_unit<C, R>(pr, rs[r], rw[r], 2, norm, ri, rj, rk, rl, Iz);
+                        jk_unit<C, R>(pr, s, w, 0, norm, ri, rj, rk, rl, Ix);
+                        jk_unit<C, R>(pr, s, w, 1, norm, ri, rj, rk, rl, Iy);
+                        jk_unit<C, R>(pr, s, w, 2, norm, ri, rj, rk, rl, Iz);
                         jk_thread_products<C, R, CI0, NI>(acc, Ix, Iy, Iz);
+                    };
+                    if constexpr (S::ROLL) {
+#pragma unroll 1
+                        for (int r = 0; r < NR; r++) {
+                            double s, w;
+                            rys_root_one<NR>(tab, pr.x, r, s, w);
+                            root(s, w);
+                        }
+                    } else {
+                        double rs[NR], rw[NR];
+                        rys_table_all<NR>(tab, pr.x, rs, rw);
+#pragma unroll
+                        for (int r = 0; r < NR; r++) root(rs[r], rw[r]);
                     }
                 }
             }
