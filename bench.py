@@ -797,12 +797,13 @@ def main():
     quartets = int(counts[:ncq].sum())
     flops = sum(int(c) * class_flops(*(int(v) for v in cq[i, 2:8]))
                 for i, c in enumerate(counts[:ncq]) if c)
-    # one FP64 atomic per element of the six J/K blocks of every quartet
-    atomics = 0
+    # elements of the six J/K blocks of every quartet (an FP64 atomic each in
+    # a kernel that kept no sums over its quartets)
+    block_elements = 0
     for i, c in enumerate(counts[:ncq]):
         fi, fj, fk, fl = (ncart(int(v)) for v in cq[i, 2:6])
-        atomics += int(c) * (fi * fj + fk * fl + fi * fk + fi * fl + fj * fk
-                             + fj * fl)
+        block_elements += int(c) * (fi * fj + fk * fl + fi * fk + fi * fl + fj * fk
+                                    + fj * fl)
     peak = ctypes.c_double()
     lib.jk_fma_peak(0, ctypes.byref(peak))
     peak32 = ctypes.c_double()
@@ -835,10 +836,11 @@ def main():
         'quartets_per_build': quartets,
         'quartets_per_s': world * quartets / (ms_step * 1e-3),
         'kernel_ms_per_build': ms_kern,
-        'atomics_per_build': atomics,
+        'block_elements_per_build': block_elements,
         'setup_s': setup_s,
-        # dm_cond + screen + one launch per class quartet + 2 symmetrize
-        'gpu_launches': 4 + ncq,
+        # begin, dm_cond, screen, scan, prefix, pack, symmetrize and at least
+        # one launch per class
+        'gpu_launches': 7 + len({tuple(r) for r in cq[:ncq, 2:6].tolist()}),
         'roofline': {'bound': 'fp64', 'achieved': achieved,
                      'peak': peak.value, 'unit': 'TFLOP/s',
                      'frac': achieved / peak.value if peak.value else None,

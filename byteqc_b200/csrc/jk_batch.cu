@@ -1,27 +1,23 @@
 // Batched J/K builds: many molecules (one jk_basis each) in one pass.
 //
-// The single-molecule path launches one kernel per class quartet; for small
-// molecules those launches are tiny and the GPU idles between them.  Here the
-// class quartets of all molecules that share a class key become segments of
-// ONE launch, so a batch of hundreds of molecules costs one launch per class
-// key plus three bookkeeping launches (density condensation, screening,
-// segment prefixes), with no host synchronisation; the whole sequence can be
-// captured into a CUDA graph and replayed every SCF iteration.  A key is the
-// class (four angular momenta), plus the two primitive counts for the team
-// kernels, whose blocks loop over the primitives in step.  Within a key the
-// segments are ordered by descending task count, so the largest molecules'
-// work is handed out first.
+// The class quartets of all molecules that share a class key become segments
+// of ONE launch (jk_plan.cu, as jk_build does for one molecule), so a batch of
+// hundreds of molecules costs one launch per class key plus the bookkeeping
+// (density condensation, screening, prefixes), with no host synchronisation;
+// the whole sequence can be captured into a CUDA graph and replayed every SCF
+// iteration.  A key is the class (four angular momenta), plus the two
+// primitive counts for the team kernels, whose blocks loop over the primitives
+// in step.  Within a key the segments are ordered by descending task count, so
+// the largest molecules' work is handed out first.
 //
 // Class quartets with at least `solo_tasks` unscreened tasks are not merged:
-// each runs as its own launch of the single-molecule kernel (segment in the
-// parameter bank, as jk_build launches it), in molecule order, fanned out
-// over the side streams ahead of the merged keys.  Such a launch fills the
-// device by itself, and merging it costs more than it saves (measured on
-// 6-31G* molecules of 276-588 functions: 13-36 % slower merged, while
-// molecules below 160 functions build 4.7x faster merged).
+// each is a launch of its own, in molecule order, fanned out over the side
+// streams ahead of the merged keys.  Merging costs the run kernels nothing (24
+// molecules of 3-30 atoms, 6-31G*: 80.4 ms with a threshold of 2^14, 76.7 at
+// 2^16, 75 merged; 12 of 3-60 atoms 260.6, 258.0 and 255.0), so the default
+// threshold, 2^24, leaves only launches that run for milliseconds on their own.
 //
-// Launch shape per key (JKBatchCfg): static contiguous chunks, or the
-// persistent mode in which a grid of the device's resident capacity takes
+// Launch shape per key (JKBatchCfg): static, or the persistent mode in which a grid of the device's resident capacity takes
 // chunks from a device counter.  jk_batch_tune times the candidate shapes of
 // every key on the batch itself and keeps the fastest; its choices can be
 // written to and read from a cache file.

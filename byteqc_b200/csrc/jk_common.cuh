@@ -423,7 +423,7 @@ struct JKClass {
     static constexpr bool TRUN = P == 1 && NFK * NFL <= 18;
     static constexpr int TPW = P == 0 ? 32 : (TRUN ? 32 / T : 1);  // ket pairs a warp works on at once
     static constexpr bool RUNS = P == 0 || TRUN;
-    // resident 128-thread blocks asked of the register allocator (thread kernel)
+    // resident 128-thread blocks asked of the register allocator (fill kernel)
     static constexpr int MINB = W <= 24 ? 4 : (W <= 40 ? 3 : 2);
 };
 

@@ -19,7 +19,7 @@
 
 static int class_index(const jk_basis* b, int cp_ij, int cp_kl);
 
-// primitive-pair screen of the thread kernels: exp(-mu r^2) below exp(-60)
+// primitive-pair screen of the run kernels: exp(-mu r^2) below exp(-60)
 // (the default exponent cutoff of libcint's pair data) contributes nothing
 #define JK_PRIM_EXPCUT 60.0
 
@@ -811,12 +811,14 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
     for (int c = 0; c < b->ncp; c++) {
         const int p0 = b->h_pair_locs[c], np = b->h_pair_locs[c + 1] - p0, S = sort_bucket(np);
         int* r = orank.data() + p0;
-        for (int x = 0; x < np; x++) r[x] = x;
-        for (int x = 0; x < np; x += S)
-            std::sort(r + x, r + std::min(np, x + S), [&](int u, int v) {
-                const int a = b->h_pair2bra[p0 + u], d = b->h_pair2bra[p0 + v];
-                return a != d ? a < d : b->h_pair2ket[p0 + u] < b->h_pair2ket[p0 + v];
-            });
+        std::vector<std::pair<long long, int>> key(S);  // (shells, rank) of one bucket
+        for (int x = 0; x < np; x += S) {
+            const int n = std::min(np - x, S);
+            for (int y = 0; y < n; y++)
+                key[y] = {(long long)b->h_pair2bra[p0 + x + y] * nbas + b->h_pair2ket[p0 + x + y], x + y};
+            std::sort(key.begin(), key.begin() + n);
+            for (int y = 0; y < n; y++) r[x + y] = key[y].second;
+        }
         for (int x = 0; x < np; x++) {
             opos[p0 + r[x]] = x;
             obra[p0 + x] = b->h_pair2bra[p0 + r[x]];
@@ -860,7 +862,7 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             double r2 = dx * dx + dy * dy + dz * dz;
             // primitive pairs whose Gaussian-product factor exp(-ai aj/(ai+aj) r^2)
             // is above exp(-JK_PRIM_EXPCUT) first, their count in h_pnp
-            // (the thread kernels loop over those only; the others carry a
+            // (the run kernels loop over those only; the others carry a
             // factor below 1e-26 and are kept after them for the kernels
             // that loop over all)
             std::vector<std::pair<int, int>> order;
@@ -930,10 +932,11 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         for (int c = 0; c < b->ncp; c++) {
             const int p0 = b->h_pair_locs[c], np = b->h_pair_locs[c + 1] - p0;
             int* e = ent.data() + p0;
-            for (int x = 0; x < np; x++) e[x] = x;
-            std::stable_sort(e, e + np,
-                             [&](int x, int y) { return b->h_pair2bra[p0 + x] < b->h_pair2bra[p0 + y]; });
-            // e: ranks in run order, then the positions
+            // e: ranks by first shell (counting sort, ranks ascending in a shell)
+            std::vector<int> at(nbas + 1, 0);
+            for (int x = 0; x < np; x++) at[b->h_pair2bra[p0 + x] + 1]++;
+            for (int x = 0; x < nbas; x++) at[x + 1] += at[x];
+            for (int x = 0; x < np; x++) e[at[b->h_pair2bra[p0 + x]]++] = x;
             for (int v = 0; v < JK_RUN_LEVELS; v++) {
                 b->h_run_off[v][c] = (int)run0.size();
                 int beg = 0;
@@ -1877,11 +1880,6 @@ jk_launch_fn jk_internal_launcher(int class_idx, int fp32) {
 int jk_internal_class_team(int class_idx) {
     init_tables();
     return g_tabs.team[class_idx];
-}
-
-int jk_internal_class_run(int class_idx) {
-    init_tables();
-    return g_tabs.run[class_idx];
 }
 
 jk_fill_fn jk_internal_fill_launcher(int class_idx) {

@@ -237,7 +237,6 @@ int jk_internal_class_index(const jk_basis_t* b, int cp_ij, int cp_kl);
 jk_launch_fn jk_internal_launcher(int class_idx, int fp32);
 // 1 if the class runs a team kernel (one primitive count per launch)
 int jk_internal_class_team(int class_idx);
-int jk_internal_class_run(int class_idx);
 void jk_internal_fill_seg(const jk_basis_t* b, int cp_ij, int cp_kl, const long long* qoff, int n_ij,
                           const double* dm, int n_dm, double* vj, double* vk, JKSeg* out);
 // segment of class quartet c, FP64 or FP32 part (no density, no outputs)

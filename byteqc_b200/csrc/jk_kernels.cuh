@@ -1,5 +1,6 @@
-// J/K kernels: Rys-quadrature ERIs of contracted shell quartets digested on
-// the fly into J and K (the work of the reference's GINTint2e_jk_kernel*,
+// Rys-quadrature ERIs of contracted shell quartets: the pieces the J/K kernels
+// share, the ERI-tensor fill and the team kernels, which digest a quartet at a
+// time into J and K (the work of the reference's GINTint2e_jk_kernel*,
 // cuobc/lib/gvhf/g2e.cu:998-1605, and GINTkernel_getjk,
 // cuobc/lib/gvhf/contract_jk.cu:28-635).
 //
@@ -7,11 +8,12 @@
 // All primitive quartets and roots of it are summed in registers before the
 // quartet's contribution to J and K is formed.
 //
-// Two execution shapes, fixed per class at compile time (JKClass::P):
+// Execution shapes, fixed per class at compile time (JKClass):
 //   P = 0  one thread per quartet; the 2D integrals of one root live in
 //          registers and all NF Cartesian products accumulate in registers
-//          (the digestion is in jk_runs.cuh);
-//   P > 0  a team of T threads per quartet: the 3*NROOTS (axis, root) 2D
+//          (J/K kernels in jk_runs.cuh);
+//   TRUN   a lane per bra component, runs of bra pairs (jk_teams.cuh);
+//   P > 0  otherwise: a team of T threads per quartet: the 3*NROOTS (axis, root) 2D
 //          blocks are built cooperatively in shared memory, each thread owns
 //          the leading P Cartesian indices (i, or i and j) and accumulates the
 //          remaining components in registers; the digestion reduces the
@@ -127,11 +129,12 @@ struct JKOneSeg {
 };
 
 // Persistent mode (queue != nullptr): the grid is the resident capacity of
-// the device and its warps (thread kernels) or blocks (team and generic
+// the device and its blocks (team and generic
 // kernels) take chunks of `grab` consecutive tasks from the device counter
 // *queue (zeroed before the launch) until the tasks run out; there is no
-// waiting on other blocks, only an atomic add per chunk.  Otherwise the
-// tasks are split into equal contiguous chunks over the grid.
+// waiting on other blocks, only an atomic add per chunk.  Otherwise the team
+// kernels split the tasks into equal contiguous chunks over the grid and the
+// generic kernel's blocks take small chunks in turn.
 struct JKSegTable {
     const JKSeg* segs;
     const long long* segt;

@@ -38,7 +38,6 @@
 #include "jk_kernels.cuh"
 #include "jk_os.cuh"
 
-#define JK_RUN_MAX 32      // bra pairs of a run: one per lane
 #define JK_RUN_THREADS 128
 #define JK_RUN_SMEM (110 * 1024)  // shared memory per block for two blocks per SM
 

@@ -35,11 +35,12 @@ from byteqc_b200.cuobc.scf.batch import JKBatch
 
 def _footprint(nbas, nao, nao0, npairs, nprim):
     """Device bytes of an admitted request from its basis sizes: shell-pair
-    Schwarz matrix, pair lists and primitive-pair cache (basis handle),
+    Schwarz matrix, pair lists, runs and primitive-pair caches (basis handle;
+    two orders of the primitive data in double and single precision),
     density / J / K work buffers in the working basis and the back
     transform, and the SCF state (S, H, orthogonaliser, density, DIIS
     history) in the caller's basis."""
-    words = (nbas * nbas + 4 * npairs + 6 * nprim + 6 * npairs  # basis
+    words = (nbas * nbas + 30 * npairs + 21 * nprim            # basis
              + 6 * nao * nao + nao * nao0                       # work buffers
              + 16 * nao0 * nao0)                                # SCF state
     return 8 * words

@@ -193,8 +193,8 @@ int jk_get_jk(jk_basis_t *basis, const double *coeff, int nao0, const double *dm
  * of the device's resident capacity taking chunks from a device counter),
  * as jk_batch_tune chose; untuned batches use static chunks.  A class
  * quartet with at least `solo_tasks` unscreened tasks (shell-pair rows x
- * columns) is not merged: it runs as its own single-molecule launch, as
- * jk_build makes it; solo_tasks <= 0 merges everything.  jk_batch_create
+ * columns) is not merged: it is a launch of its own; solo_tasks <= 0 merges
+ * everything.  jk_batch_create
  * uses JK_BATCH_SOLO_TASKS.
  */
 #define JK_BATCH_SOLO_TASKS (1LL << 24)
