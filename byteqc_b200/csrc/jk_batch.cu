@@ -56,6 +56,7 @@ struct jk_batch {
     std::vector<const double*> seg_dm;
     std::vector<double*> seg_vj, seg_vk;
     int seg_ndm = -1;
+    bool seg_krows = false;
     // transform workspace
     cublasHandle_t blas = nullptr;
     double* d_work = nullptr;
@@ -73,6 +74,8 @@ struct jk_batch {
     JKPackMol* d_pmol = nullptr;
     long long pk_max = 0;          // largest per-molecule packed size
     bool packed = false;
+    double* d_kt = nullptr;  // K by rows of jk_batch_build (JKPackMol::kt), every molecule's after the other
+    size_t kt_cap = 0, kt_len = 0;
 };
 
 // J = 2 (V + V^T), K = V + V^T per molecule (blockIdx.y = molecule)
@@ -95,6 +98,7 @@ static void free_batch(jk_batch* t) {
     t->fan.destroy();
     cudaFree(t->d_pk);
     cudaFree(t->d_pmol);
+    cudaFree(t->d_kt);
     cudaFree(t->d_cq);
     cudaFree(t->d_dmc);
     jk_plan_free(t->plan);
@@ -160,9 +164,10 @@ extern "C" int jk_batch_destroy(jk_batch_t* t) {
 }
 
 // (re)build the segment tables when the density / output buffers change
+// (krows as in jk_host.cu's build)
 static int batch_segments(jk_batch* t, const double* const* dms, double* const* vjs, double* const* vks, int n_dm,
-                          cudaStream_t st) {
-    bool same = t->seg_ndm == n_dm && (int)t->seg_dm.size() == t->nmol;
+                          bool krows, cudaStream_t st) {
+    bool same = t->seg_ndm == n_dm && t->seg_krows == krows && (int)t->seg_dm.size() == t->nmol;
     for (int m = 0; same && m < t->nmol; m++)
         same = t->seg_dm[m] == dms[m] && t->seg_vj[m] == (vjs ? vjs[m] : nullptr) &&
                t->seg_vk[m] == (vks ? vks[m] : nullptr);
@@ -187,10 +192,34 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
             BCUDA(cudaMalloc(&t->d_pk, sizeof(double) * std::max<size_t>(2 * tot, 1)));
             t->pk_cap = 2 * tot;
         }
+    }
+    // K by rows (jk_batch_build)
+    std::vector<size_t> kt_off(t->nmol, 0);
+    t->kt_len = 0;
+    if (vks && !krows) {
+        for (int m = 0; m < t->nmol; m++) {
+            kt_off[m] = t->kt_len;
+            t->kt_len += (size_t)n_dm * t->mols[m]->nao * t->mols[m]->nao;
+        }
+        if (t->kt_len > t->kt_cap) {
+            cudaFree(t->d_kt);
+            t->d_kt = nullptr;
+            t->kt_cap = 0;
+            BCUDA(cudaMalloc(&t->d_kt, sizeof(double) * t->kt_len));
+            t->kt_cap = t->kt_len;
+        }
+    }
+    if (t->packed || t->kt_len) {
         std::vector<JKPackMol> pm(t->nmol);
         for (int m = 0; m < t->nmol; m++) {
-            pm[m] = jk_internal_pack_mol(t->mols[m], dms[m], n_dm, t->d_pk + dp_off[m], t->d_pk + tot + dp_off[m],
-                                         vjs[m]);
+            const size_t o = dp_off[m];
+            pm[m] = jk_internal_pack_mol(t->mols[m], dms[m], n_dm, t->d_pk + o, t->d_pk + t->pk_jp + o,
+                                         vjs ? vjs[m] : nullptr);
+            if (!t->packed) pm[m].total = 0;
+            if (t->kt_len) {
+                pm[m].kt = t->d_kt + kt_off[m];
+                pm[m].vk = vks[m];
+            }
         }
         if (!t->d_pmol) BCUDA(cudaMalloc(&t->d_pmol, sizeof(JKPackMol) * t->nmol));
         BCUDA(cudaMemcpy(t->d_pmol, pm.data(), sizeof(JKPackMol) * t->nmol, cudaMemcpyHostToDevice));
@@ -208,6 +237,7 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
                 s.vj = vjs ? vjs[m] : nullptr;
                 s.vk = vks ? vks[m] : nullptr;
                 s.n_dm = n_dm;
+                if (t->kt_len && s.nrun > 0) s.vk = t->d_kt + kt_off[m];
                 if (t->packed) {
                     const size_t n = (size_t)n_dm * t->mols[m]->pack_total;
                     s.dp = t->d_pk + dp_off[m];
@@ -233,14 +263,15 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
         if (vks) t->seg_vk[m] = vks[m];
     }
     t->seg_ndm = n_dm;
+    t->seg_krows = krows;
     return JK_OK;
 }
 
 // everything before the class launches: segment tables, density
 // condensation, screening, task prefixes, pair-packed densities
 static int batch_prepare(jk_batch* t, const double* const* dms, double* const* vjs, double* const* vks, int n_dm,
-                         const jk_opts_t* opts, cudaStream_t st) {
-    int rc = batch_segments(t, dms, vjs, vks, n_dm, st);
+                         bool krows, const jk_opts_t* opts, cudaStream_t st) {
+    int rc = batch_segments(t, dms, vjs, vks, n_dm, krows, st);
     if (rc) return rc;
     double tol = opts ? opts->direct_scf_tol : t->mols[0]->cutoff;
     int nbins = opts && opts->nbins > 0 ? opts->nbins : 10;
@@ -256,15 +287,16 @@ static int batch_prepare(jk_batch* t, const double* const* dms, double* const* v
         if (rc) return rc;
         BCUDA(cudaMemsetAsync(t->d_pk + t->pk_jp, 0, sizeof(double) * t->pk_jp, st));
     }
+    if (t->kt_len) BCUDA(cudaMemsetAsync(t->d_kt, 0, sizeof(double) * t->kt_len, st));
     return JK_OK;
 }
 
-extern "C" int jk_batch_build(jk_batch_t* t, const double* const* dms, double* const* vjs, double* const* vks,
-                              int n_dm, const jk_opts_t* opts, void* stream) {
+static int batch_build(jk_batch* t, const double* const* dms, double* const* vjs, double* const* vks, int n_dm,
+                       bool krows, const jk_opts_t* opts, void* stream) {
     if (!t || !dms || n_dm <= 0) return jk_internal_set_err(JK_ERR_ARG, "jk_batch_build: invalid arguments");
     if (!vjs && !vks) return JK_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = batch_prepare(t, dms, vjs, vks, n_dm, opts, st);
+    int rc = batch_prepare(t, dms, vjs, vks, n_dm, krows, opts, st);
     if (rc || t->ncq == 0) return rc;
     const bool mixed = opts && opts->fp32_cutoff > 0;
     const int nkeys = (int)t->plan->keys.size();
@@ -282,11 +314,16 @@ extern "C" int jk_batch_build(jk_batch_t* t, const double* const* dms, double* c
         }
     }
     BCUDA(t->fan.end(st));
-    if (t->packed) {
-        rc = jk_internal_pack_batch(t->d_pmol, t->nmol, t->pk_max, 1, stream);
+    if (t->packed || t->kt_len) {
+        rc = jk_internal_pack_batch(t->d_pmol, t->nmol, std::max<long long>(t->pk_max, (long long)t->kt_len), 1, stream);
         if (rc) return rc;
     }
     return JK_OK;
+}
+
+extern "C" int jk_batch_build(jk_batch_t* t, const double* const* dms, double* const* vjs, double* const* vks,
+                              int n_dm, const jk_opts_t* opts, void* stream) {
+    return batch_build(t, dms, vjs, vks, n_dm, false, opts, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -338,7 +375,8 @@ extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* co
             fclose(f);
         }
     }
-    int rc = batch_prepare(t, dms, vjs, vks, n_dm, opts, st);
+    // as jk_batch_get_jk launches them
+    int rc = batch_prepare(t, dms, vjs, vks, n_dm, true, opts, st);
     if (rc) return rc;
     cudaEvent_t e0, e1;
     BCUDA(cudaEventCreate(&e0));
@@ -517,8 +555,8 @@ extern "C" int jk_batch_get_jk(jk_batch_t* t, const double* const* coeffs, const
         vjs[m] = w + t->w_vj[m];
         vks[m] = w + t->w_vk[m];
     }
-    int rc = jk_batch_build(t, dms.data(), vj0s ? vjs.data() : nullptr, vk0s ? vks.data() : nullptr, n_dm, opts,
-                            stream);
+    int rc = batch_build(t, dms.data(), vj0s ? vjs.data() : nullptr, vk0s ? vks.data() : nullptr, n_dm, true, opts,
+                         stream);
     if (rc) return rc;
     for (int pass = 0; pass < 2; pass++) {
         double* const* outs = pass == 0 ? vj0s : vk0s;

@@ -543,8 +543,8 @@ void jk_register_generic(JKTables* T) {
                     if (li <= JK_LMAX && lk <= JK_LMAX) continue;
                     const int c = JK_CLASS_INDEX(li, lj, lk, ll);
                     const int lx = li > lk ? li : lk;  // li >= lj, lk >= ll
-                    T->t64[c] = T->t32[c] = lx == 6 ? jk_launch_generic<6>
-                                                    : (lx == 5 ? jk_launch_generic<5> : jk_launch_generic<4>);
+                    T->t64[c] = T->t32[c] = T->pair[c] =
+                        lx == 6 ? jk_launch_generic<6> : (lx == 5 ? jk_launch_generic<5> : jk_launch_generic<4>);
                 }
 }
 

@@ -480,6 +480,8 @@ struct JKCall {
     const double* dpb;
     double* jpb;
     int n_dm;
+    double* kt;     // K of the run kernels (JKPackMol::kt), or null: they add into vk
+    long long nkt;  // its size
 };
 // Pair-packed J side.  mode 0: gather the density blocks of every pair into
 // dp (element c of pair p of class k at off_k + c*np_k + p, one copy per
@@ -515,7 +517,30 @@ __device__ __forceinline__ void jk_pack_body(const JKPackMol& a, int mode) {
     }
 }
 
-__global__ void jk_pack_kernel(const JKPackMol one, int mode) { jk_pack_body(one, mode); }
+// vk[a + nao b] += kt[a nao + b], 32 x 32 tiles through shared memory (256
+// threads); atomics, since builds of other handles may add into the same vk
+__device__ __forceinline__ void jk_kadd_body(const JKPackMol& a) {
+    __shared__ double t[32][33];
+    const int n = a.nao, nt = (n + 31) / 32, x = threadIdx.x & 31, y0 = threadIdx.x >> 5;
+    const long long tiles = (long long)a.n_dm * nt * nt;
+    for (long long b = blockIdx.x; b < tiles; b += gridDim.x) {
+        const int m = (int)(b / ((long long)nt * nt)), r = (int)(b - (long long)m * nt * nt);
+        const int p0 = r / nt * 32, q0 = r % nt * 32;
+        const size_t mo = (size_t)m * n * n;
+        for (int y = y0; y < 32; y += 8)
+            if (p0 + y < n && q0 + x < n) t[y][x] = a.kt[mo + (size_t)(p0 + y) * n + q0 + x];
+        __syncthreads();
+        for (int y = y0; y < 32; y += 8)
+            if (q0 + y < n && p0 + x < n) atomicAdd(a.vk + mo + (size_t)(q0 + y) * n + p0 + x, t[x][y]);
+        __syncthreads();
+    }
+}
+
+// end of a build: the J accumulators (total > 0) and kt (if any) to the outputs
+__global__ void __launch_bounds__(256) jk_finish_kernel(const JKPackMol one) {
+    if (one.total > 0) jk_pack_body(one, 1);
+    if (one.kt) jk_kadd_body(one);
+}
 
 // Start of a build, one launch: the call's buffers into the segments, the
 // counters and the J accumulators cleared, the densities packed.
@@ -527,7 +552,7 @@ __global__ void __launch_bounds__(256) jk_begin_kernel(JKSeg* __restrict__ s64, 
         JKSeg& s = i < nseg ? s64[i] : s32[i - nseg];
         s.dm = c.dm;
         s.vj = c.vj;
-        s.vk = c.vk;
+        s.vk = c.kt && s.nrun > 0 ? c.kt : c.vk;
         s.dp = c.dp;
         s.jp = c.jp;
         s.dpb = c.dpb;
@@ -535,6 +560,7 @@ __global__ void __launch_bounds__(256) jk_begin_kernel(JKSeg* __restrict__ s64, 
         s.n_dm = c.n_dm;
     }
     for (long long i = t0; i < nzero; i += step) zero[i] = 0;
+    for (long long i = t0; i < c.nkt; i += step) c.kt[i] = 0.;
     if (pm.total > 0) {
         const long long na = 2 * pm.n_dm * pm.total;  // jp and jpb lie together
         for (long long i = t0; i < na; i += step) pm.jp[i] = 0.;
@@ -543,9 +569,10 @@ __global__ void __launch_bounds__(256) jk_begin_kernel(JKSeg* __restrict__ s64, 
 }
 
 // one molecule per blockIdx.y
-__global__ void jk_pack_batch_kernel(const JKPackMol* __restrict__ mols, int mode) {
+__global__ void __launch_bounds__(256) jk_pack_batch_kernel(const JKPackMol* __restrict__ mols, int mode) {
     const JKPackMol m = mols[blockIdx.y];
     if (m.total > 0) jk_pack_body(m, mode);
+    if (mode == 1 && m.kt) jk_kadd_body(m);
 }
 
 // 2 (V + V^T) of the first nj matrices (J), V + V^T of the others (K), where
@@ -622,6 +649,7 @@ static void free_basis(jk_basis* b) {
     cudaFree(b->d_pao);
     b->fan.destroy();
     cudaFree(b->d_pk);
+    cudaFree(b->d_kt);
     if (b->blas) cublasDestroy(b->blas);
     delete b;
 }
@@ -1231,8 +1259,10 @@ static int build_plan(jk_basis* b, int nshards, int shard) {
     return rc;
 }
 
-extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, double* vk, const jk_opts_t* opts,
-                        void* stream) {
+// krows: the caller reads V + V^T of K only, which the run kernels may then
+// leave by rows; otherwise vk gets the layout of the C-ABI
+static int build(jk_basis* b, const double* dm, int n_dm, double* vj, double* vk, bool krows, const jk_opts_t* opts,
+                 void* stream) {
     if (!b || !dm || n_dm <= 0) return set_err(JK_ERR_ARG, "jk_build: invalid arguments");
     if (!vj && !vk) return JK_OK;
     cudaStream_t st = (cudaStream_t)stream;
@@ -1246,7 +1276,7 @@ extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, d
     if (rc) return rc;
     // pair-packed density and J accumulators for the run kernels
     const bool packed = vj && b->pack_total > 0;
-    JKCall call{dm, vj, vk, nullptr, nullptr, nullptr, nullptr, n_dm};
+    JKCall call{dm, vj, vk, nullptr, nullptr, nullptr, nullptr, n_dm, nullptr, 0};
     JKPackMol pm{};
     const int pk_blocks = (int)std::min<long long>((b->pack_total + 255) / 256, (long long)b->nsm * 8);
     if (packed) {
@@ -1263,6 +1293,28 @@ extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, d
         call.jp = pm.jp;
         call.dpb = pm.dpb;
         call.jpb = pm.jpb;
+    }
+    // K by rows into a buffer of the handle, added transposed at the end; a
+    // capture cannot allocate it, and lets the run kernels write vk itself
+    bool direct = false;
+    if (vk && !krows) {
+        const size_t need = (size_t)n_dm * b->nao * b->nao;
+        if (need > b->kt_cap) {
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            CUDA_TRY(cudaStreamIsCapturing(st, &cs));
+            direct = cs != cudaStreamCaptureStatusNone;
+            if (!direct) {
+                cudaFree(b->d_kt);
+                b->d_kt = nullptr;
+                b->kt_cap = 0;
+                CUDA_TRY(cudaMalloc(&b->d_kt, sizeof(double) * need));
+                b->kt_cap = need;
+            }
+        }
+        if (!direct) {
+            call.kt = b->d_kt;
+            call.nkt = (long long)need;
+        }
     }
     jk_begin_kernel<<<std::max(pk_blocks, 8), 256, 0, st>>>(b->plan->d_seg[0], b->plan->d_seg[1], b->plan->nseg, call,
                                                             (unsigned long long*)b->d_zero,
@@ -1284,15 +1336,30 @@ extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, d
     for (int k = 0; k < (int)b->plan->keys.size(); k++)
         for (int part = 0; part < np; part++) {
             rc = jk_plan_launch(b->plan, k, part, b->plan->keys[k].cfg[part], n_dm, b->nsm,
-                                b->fan.s[(np * k + part) % ns]);
+                                b->fan.s[(np * k + part) % ns], direct);
             if (rc) return rc;
         }
     CUDA_TRY(b->fan.end(st, ns));
-    if (packed) {
-        jk_pack_kernel<<<pk_blocks, 256, 0, st>>>(pm, 1);
+    if (call.kt) {
+        if (!packed) {
+            pm.nao = b->nao;
+            pm.n_dm = n_dm;
+        }
+        pm.kt = call.kt;
+        pm.vk = vk;
+    }
+    if (packed || pm.kt) {
+        const long long nt = (b->nao + 31) / 32, tiles = pm.kt ? n_dm * nt * nt : 0;
+        const int blocks = (int)std::min<long long>(std::max<long long>(tiles, pm.total ? pk_blocks : 1), b->nsm * 8LL);
+        jk_finish_kernel<<<blocks, 256, 0, st>>>(pm);
         CUDA_TRY(cudaGetLastError());
     }
     return JK_OK;
+}
+
+extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, double* vk, const jk_opts_t* opts,
+                        void* stream) {
+    return build(b, dm, n_dm, vj, vk, false, opts, stream);
 }
 
 // Row prefix of one class pair's task list from the host bins of the
@@ -1411,7 +1478,7 @@ extern "C" int jk_build_class_pair(jk_basis_t* b, double* vj, double* vk, const 
     int n_ij = b->h_pair_locs[cp_ij + 1] - b->h_pair_locs[cp_ij];
     // kl bin kb pairs with ij in [bins_ij[0], bins_ij[nbins - kb]) (nr_jk_driver.cu:252-280):
     // row ij (in bin sij) keeps kl < bins_kl[nbins - sij]; diagonal classes keep kl <= ij
-    jk_launch_fn fn = g_tab64[class_index(b, cp_ij, cp_kl)];
+    jk_launch_fn fn = g_tabs.pair[class_index(b, cp_ij, cp_kl)];
     if (!fn) return set_err(JK_ERR_UNSUPPORTED, "no kernel for this class pair");
     JKRowBins rb;
     int rc = row_bins(bins_locs_ij, bins_locs_kl, nbins, cp_ij == cp_kl, &rb);
@@ -1619,7 +1686,7 @@ extern "C" int jk_get_jk(jk_basis_t* b, const double* coeff, int nao0, const dou
     double* v0 = vj0 ? vjw : vkw;  // the outputs lie together
     const size_t nv = vj0 && vk0 ? 2 * nn : nn;
     CUDA_TRY(cudaMemsetAsync(v0, 0, sizeof(double) * nv, st));
-    int rc = jk_build(b, dms, n_dm, vj0 ? vjw : nullptr, vk0 ? vkw : nullptr, opts, stream);
+    int rc = build(b, dms, n_dm, vj0 ? vjw : nullptr, vk0 ? vkw : nullptr, true, opts, stream);
     if (rc) return rc;
     // J = 2 C^T (V + V^T) C, K = C^T (V + V^T) C (cuobc/scf/hf.py:171-181):
     // one symmetrisation, one product with C from the right for all matrices
@@ -1839,7 +1906,7 @@ void jk_internal_fill_seg(const jk_basis_t* b, int cp_ij, int cp_kl, const long 
 
 int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg& seg, JKSeg* d_seg,
                        const long long* task0, long long max_tasks, void* stream) {
-    jk_launch_fn fn = g_tab64[class_index(b, cp_ij, cp_kl)];
+    jk_launch_fn fn = g_tabs.pair[class_index(b, cp_ij, cp_kl)];
     if (!fn) return set_err(JK_ERR_UNSUPPORTED, "no kernel for class pair (%d, %d)", cp_ij, cp_kl);
     cudaStream_t st = (cudaStream_t)stream;
     jk_put_seg_kernel<<<1, 128, 0, st>>>(seg, d_seg);
@@ -1877,6 +1944,16 @@ jk_launch_fn jk_internal_launcher(int class_idx, int fp32) {
     return fp32 ? g_tab32[class_idx] : g_tab64[class_idx];
 }
 
+jk_launch_fn jk_internal_pair_launcher(int class_idx) {
+    init_tables();
+    return g_tabs.pair[class_idx];
+}
+
+int jk_internal_class_runs(int class_idx) {
+    init_tables();
+    return g_tabs.run[class_idx];
+}
+
 int jk_internal_class_team(int class_idx) {
     init_tables();
     return g_tabs.team[class_idx];
@@ -1908,12 +1985,13 @@ void jk_internal_fill_seg_cq(const jk_basis_t* b, int c, int fp32, JKSeg* out) {
 JKPackMol jk_internal_pack_mol(const jk_basis_t* b, const double* dm, int n_dm, double* dens, double* acc, double* vj) {
     const size_t n = (size_t)n_dm * b->pack_total;
     return JKPackMol{b->d_pack, b->ncp, b->pack_total, b->d_pair2bra, b->d_pair2ket, b->d_ao_loc, b->d_inv,
-                     dm,        b->nao, n_dm,          dens,          dens + n,      acc,         acc + n,  vj};
+                     dm,        b->nao, n_dm,          dens,          dens + n,      acc,         acc + n,  vj,
+                     nullptr,   nullptr};
 }
 
 int jk_internal_pack_batch(const JKPackMol* d_mols, int nmol, long long max_total, int mode, void* stream) {
-    if (nmol <= 0 || max_total <= 0) return JK_OK;
-    const unsigned bx = (unsigned)std::min<long long>((max_total + 255) / 256, 64);
+    if (nmol <= 0) return JK_OK;
+    const unsigned bx = (unsigned)std::max(1LL, std::min<long long>((max_total + 255) / 256, 64));
     jk_pack_batch_kernel<<<dim3(bx, nmol), 256, 0, (cudaStream_t)stream>>>(d_mols, mode);
     CUDA_TRY(cudaGetLastError());
     return JK_OK;

@@ -123,6 +123,10 @@ struct JKPackMol {
     double *dp, *dpb;  // mode 0 output
     double *jp, *jpb;  // mode 1 input
     double* vj;        // mode 1 output
+    // K of the run kernels by rows (n_dm x nao x nao, or null), added
+    // transposed into vk after the launches
+    const double* kt;
+    double* vk;
 };
 
 // run lengths a run table exists for: long runs save more traffic, short ones
@@ -164,7 +168,10 @@ int jk_plan_add(JKPlan* p, const jk_basis* b, int m, int c, bool solo);
 int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols);
 // exclusive prefixes of the segments' task counts (after the screening)
 int jk_plan_prefix(const JKPlan* p, bool mixed, cudaStream_t st);
-int jk_plan_launch(const JKPlan* p, int k, int part, const JKBatchCfg& cfg, int n_dm, int nsm, cudaStream_t st);
+// direct: the run kernels write K in the layout of the C-ABI (FP64 in both
+// parts), otherwise by rows
+int jk_plan_launch(const JKPlan* p, int k, int part, const JKBatchCfg& cfg, int n_dm, int nsm, cudaStream_t st,
+                   bool direct = false);
 
 // Per-geometry state (opaque to callers of the C-ABI)
 struct jk_basis {
@@ -227,6 +234,8 @@ struct jk_basis {
     long long pack_total = 0;  // packed elements per density
     double* d_pk = nullptr;    // 2 n_dm x pack_total densities, then as many J accumulators
     size_t pk_cap = 0;
+    double* d_kt = nullptr;    // K by rows of a jk_build (JKPackMol::kt)
+    size_t kt_cap = 0;
     // transform workspace
     cublasHandle_t blas = nullptr;
     double* d_work = nullptr;
@@ -235,14 +244,19 @@ struct jk_basis {
 
 int jk_internal_class_index(const jk_basis_t* b, int cp_ij, int cp_kl);
 jk_launch_fn jk_internal_launcher(int class_idx, int fp32);
+// launcher of the per-class-pair entries: K in the layout of the C-ABI
+jk_launch_fn jk_internal_pair_launcher(int class_idx);
 // 1 if the class runs a team kernel (one primitive count per launch)
 int jk_internal_class_team(int class_idx);
+// 1 if the class runs a run kernel
+int jk_internal_class_runs(int class_idx);
 void jk_internal_fill_seg(const jk_basis_t* b, int cp_ij, int cp_kl, const long long* qoff, int n_ij,
                           const double* dm, int n_dm, double* vj, double* vk, JKSeg* out);
 // segment of class quartet c, FP64 or FP32 part (no density, no outputs)
 void jk_internal_fill_seg_cq(const jk_basis_t* b, int c, int fp32, JKSeg* out);
 JKPackMol jk_internal_pack_mol(const jk_basis_t* b, const double* dm, int n_dm, double* dens, double* acc, double* vj);
-// pack (mode 0) or unpack (mode 1) the J side of nmol molecules (device table)
+// pack (mode 0) or unpack (mode 1) the J side of nmol molecules (device
+// table); mode 1 adds their kt too
 int jk_internal_pack_batch(const JKPackMol* d_mols, int nmol, long long max_total, int mode, void* stream);
 // condensed densities (outputs zeroed first) of nmol molecules (device table)
 struct JKDmCond {

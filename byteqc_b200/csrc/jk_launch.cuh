@@ -39,52 +39,52 @@ int jk_resident_blocks(K kernel, int threads, size_t smem, std::atomic<unsigned 
     return nb;
 }
 
-template <class C, typename R, bool MULTI>
+template <class C, typename R, bool MULTI, bool KROWS>
 cudaError_t jk_launch_run(const JKSeg* segs, const long long* segt, int nseg, long long max_items, int n_dm, int nsm,
                           const JKBatchCfg& cfg, cudaStream_t st) {
     const size_t smem = MULTI ? jk_run_multi_smem<C>(n_dm) : JKRunShape<C>::SMEM;
     static std::atomic<unsigned long long> attr_done{0}, occ_done{0};
     static int occ[64];
-    if (cudaError_t e = jk_smem_attr(jk_run_kernel<C, R, MULTI>, MULTI ? JK_RUN_SMEM : smem, attr_done); e != cudaSuccess)
+    if (cudaError_t e = jk_smem_attr(jk_run_kernel<C, R, MULTI, KROWS>, MULTI ? JK_RUN_SMEM : smem, attr_done); e != cudaSuccess)
         return e;
     // resident grid (the most shared memory a MULTI launch may take)
-    const long long res = (long long)nsm * jk_resident_blocks(jk_run_kernel<C, R, MULTI>, JK_RUN_THREADS,
+    const long long res = (long long)nsm * jk_resident_blocks(jk_run_kernel<C, R, MULTI, KROWS>, JK_RUN_THREADS,
                                                               MULTI ? (size_t)JK_RUN_SMEM : smem, occ_done, occ);
     const long long want = (max_items + JK_RUN_THREADS / 32 - 1) / (JK_RUN_THREADS / 32);
     const int blocks = (int)(cfg.queue ? res * cfg.grid_mul : (want < res ? want : res));
-    jk_run_kernel<C, R, MULTI><<<blocks, JK_RUN_THREADS, smem, st>>>(segs, segt, nseg, cfg.queue, cfg.grab);
+    jk_run_kernel<C, R, MULTI, KROWS><<<blocks, JK_RUN_THREADS, smem, st>>>(segs, segt, nseg, cfg.queue, cfg.grab);
     return cudaGetLastError();
 }
 
-template <class C, typename R, bool MULTI>
+template <class C, typename R, bool MULTI, bool KROWS>
 cudaError_t jk_launch_trun(const JKSeg* segs, const long long* segt, int nseg, long long max_items, int nsm,
                            const JKBatchCfg& cfg, cudaStream_t st) {
     constexpr size_t smem = JKTRunShape<C, R>::SMEM;
     static_assert(smem <= 227 * 1024, "team run kernel shared memory");
     static std::atomic<unsigned long long> attr_done{0}, occ_done{0};
     static int occ[64];
-    if (cudaError_t e = jk_smem_attr(jk_trun_kernel<C, R, MULTI>, smem, attr_done); e != cudaSuccess) return e;
-    const long long res = (long long)nsm * jk_resident_blocks(jk_trun_kernel<C, R, MULTI>, JK_RUN_THREADS, smem,
+    if (cudaError_t e = jk_smem_attr(jk_trun_kernel<C, R, MULTI, KROWS>, smem, attr_done); e != cudaSuccess) return e;
+    const long long res = (long long)nsm * jk_resident_blocks(jk_trun_kernel<C, R, MULTI, KROWS>, JK_RUN_THREADS, smem,
                                                               occ_done, occ);
     const long long want = (max_items + JK_RUN_THREADS / 32 - 1) / (JK_RUN_THREADS / 32);
     const int blocks = (int)(cfg.queue ? res * cfg.grid_mul : (want < res ? want : res));
-    jk_trun_kernel<C, R, MULTI><<<blocks, JK_RUN_THREADS, smem, st>>>(segs, segt, nseg, cfg.queue, cfg.grab);
+    jk_trun_kernel<C, R, MULTI, KROWS><<<blocks, JK_RUN_THREADS, smem, st>>>(segs, segt, nseg, cfg.queue, cfg.grab);
     return cudaGetLastError();
 }
 
 // The segments of one class (for the team kernels: of one class and one pair
 // of primitive counts), task or item prefix segt[0..nseg] on the device.
-template <int LI, int LJ, int LK, int LL, typename R>
+template <int LI, int LJ, int LK, int LL, typename R, bool KROWS>
 cudaError_t jk_launch(const JKSeg* segs, const long long* segt, int nseg, long long max_tasks, int n_dm, int nsm,
                       const JKBatchCfg& cfg, cudaStream_t st) {
     using C = JKClass<LI, LJ, LK, LL>;
     if (max_tasks <= 0 || nseg <= 0) return cudaSuccess;
     if constexpr (C::P == 0) {
-        if (n_dm > 1) return jk_launch_run<C, R, true>(segs, segt, nseg, max_tasks, n_dm, nsm, cfg, st);
-        return jk_launch_run<C, R, false>(segs, segt, nseg, max_tasks, n_dm, nsm, cfg, st);
+        if (n_dm > 1) return jk_launch_run<C, R, true, KROWS>(segs, segt, nseg, max_tasks, n_dm, nsm, cfg, st);
+        return jk_launch_run<C, R, false, KROWS>(segs, segt, nseg, max_tasks, n_dm, nsm, cfg, st);
     } else if constexpr (C::TRUN) {
-        if (n_dm > 1) return jk_launch_trun<C, R, true>(segs, segt, nseg, max_tasks, nsm, cfg, st);
-        return jk_launch_trun<C, R, false>(segs, segt, nseg, max_tasks, nsm, cfg, st);
+        if (n_dm > 1) return jk_launch_trun<C, R, true, KROWS>(segs, segt, nseg, max_tasks, nsm, cfg, st);
+        return jk_launch_trun<C, R, false, KROWS>(segs, segt, nseg, max_tasks, nsm, cfg, st);
     } else {
         using S = JKTeamShape<C>;
         constexpr size_t smem = jk_team_smem<C, R>();
@@ -137,7 +137,9 @@ typedef cudaError_t (*jk_fill_fn)(const JKSeg& seg, const long long* task0, long
 
 // launcher tables indexed by JK_CLASS_INDEX(li, lj, lk, ll)
 struct JKTables {
-    jk_launch_fn t64[JK_NCLASS], t32[JK_NCLASS];
+    // builds (the run kernels write K by rows, see JKRunItem), FP64 and FP32
+    // parts; the per-class-pair entries (K in the layout of the C-ABI)
+    jk_launch_fn t64[JK_NCLASS], t32[JK_NCLASS], pair[JK_NCLASS];
     // team kernels need one primitive count per launch (their blocks loop
     // over the primitives in step); run and generic kernels read it per
     // segment
@@ -154,7 +156,7 @@ void jk_register_generic(JKTables* T);
 
 #ifndef JK_NO_FP32
 #define JK_REG32(LI, LJ, LK, LL)                                         \
-    T->t32[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch<LI, LJ, LK, LL, float>;
+    T->t32[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch<LI, LJ, LK, LL, float, true>;
 #else
 #define JK_REG32(LI, LJ, LK, LL)
 #endif
@@ -162,5 +164,7 @@ void jk_register_generic(JKTables* T);
     T->team[JK_CLASS_INDEX(LI, LJ, LK, LL)] = !JKClass<LI, LJ, LK, LL>::RUNS;     \
     T->fill[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch_fill_t<LI, LJ, LK, LL>;   \
     T->run[JK_CLASS_INDEX(LI, LJ, LK, LL)] = JKClass<LI, LJ, LK, LL>::RUNS ? JKClass<LI, LJ, LK, LL>::TPW : 0; \
-    T->t64[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch<LI, LJ, LK, LL, double>;  \
+    T->t64[JK_CLASS_INDEX(LI, LJ, LK, LL)] = jk_launch<LI, LJ, LK, LL, double, true>;  \
+    T->pair[JK_CLASS_INDEX(LI, LJ, LK, LL)] =                                         \
+        jk_launch<LI, LJ, LK, LL, double, !JKClass<LI, LJ, LK, LL>::RUNS>;            \
     JK_REG32(LI, LJ, LK, LL)

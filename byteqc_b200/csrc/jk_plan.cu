@@ -141,10 +141,12 @@ int jk_plan_prefix(const JKPlan* p, bool mixed, cudaStream_t st) {
     return JK_OK;
 }
 
-int jk_plan_launch(const JKPlan* p, int k, int part, const JKBatchCfg& cfg, int n_dm, int nsm, cudaStream_t st) {
+int jk_plan_launch(const JKPlan* p, int k, int part, const JKBatchCfg& cfg, int n_dm, int nsm, cudaStream_t st,
+                   bool direct) {
     const JKPlanKey& key = p->keys[k];
     const int off = p->key_off[k], n = p->key_off[k + 1] - off;
-    jk_launch_fn f = jk_internal_launcher(key.cls, part);
+    jk_launch_fn f = direct && jk_internal_class_runs(key.cls) ? jk_internal_pair_launcher(key.cls)
+                                                               : jk_internal_launcher(key.cls, part);
     if (!f) return jk_internal_set_err(JK_ERR_UNSUPPORTED, "no kernel for a class of the build");
     JKBatchCfg c = cfg;
     c.queue = c.grab > 0 ? p->d_queue + 2 * k + part : nullptr;

@@ -173,7 +173,15 @@ __device__ __forceinline__ JKPPF jk_bra_ppf(const float* __restrict__ rec) {
 // element it is paired with (D_kl, D_ik, D_il) has the same number.  What the
 // loop over the bra pairs needs of the segment is copied here: the segment
 // itself (in shared memory) would be read again after every atomic.
-template <class C, typename R, bool MULTI>
+//
+// KROWS: element (a, b) of K goes to a * nao + b, so that the lanes of a warp,
+// whose ket shells are consecutive, add side by side; the caller reads V + V^T
+// only, or transposes.  Otherwise to a + nao * b, the layout of the C-ABI
+// (per-class-pair entries).  A template argument: with the two strides read
+// from the segment the builds took 1 to 2 % longer ((ps|ps) 332 bytes of
+// spill loads instead of 220); writing a + nao * b in every build, (H2O)64 /
+// cc-pVDZ took 146 instead of 95 ms and (H2O)32 / TZVP 288 instead of 256.
+template <class C, typename R, bool MULTI, bool KROWS>
 struct JKRunItem {
     using S = JKRunShape<C>;
     static constexpr int NFI = C::NFI, NFJ = C::NFJ, NFK = C::NFK, NFL = C::NFL, TS = JK_RUN_THREADS;
@@ -203,7 +211,11 @@ struct JKRunItem {
     double djk[DEARLY ? NJK : 1], djl[DEARLY ? NJL : 1];
 
     __device__ __forceinline__ const double* drow(int m, int a) const { return D + ((size_t)m * nao + a) * nao; }
-    __device__ __forceinline__ double* krow(int m, int a) const { return vk + ((size_t)m * nao + a) * nao; }
+    // K element (a, b) of density m at krow(m, a) + kcol(b)
+    __device__ __forceinline__ double* krow(int m, int a) const {
+        return KROWS ? vk + ((size_t)m * nao + a) * nao : vk + (size_t)m * nao * nao + a;
+    }
+    __device__ __forceinline__ size_t kcol(int b) const { return KROWS ? b : (size_t)b * nao; }
 
     // density element paired with element e of the state
     __device__ __forceinline__ double dload(int m, int e) const {
@@ -218,16 +230,15 @@ struct JKRunItem {
         else if constexpr (DSM) return sden[e * TS];
         else return dload(m, e);
     }
-    // element e of the state added to the output (the raw V may hold either
-    // orientation of an element: here the ket index runs fastest)
+    // element e of the state added to the output
     __device__ __forceinline__ void gadd(int m, int e, double v) const {
         if (e < S::OIK) {
             if (sg.jp) atomicAdd(sg.jp + sg.pk_kl + m * sg.pk_stride + (size_t)e * sg.pst_kl + col, v);
             else atomicAdd(sg.vj + (size_t)m * nao * nao + (k0 + e / NFL) + (size_t)nao * (l0 + e % NFL), v);
         } else if (e < S::OIL) {
-            atomicAdd(krow(m, i0 + (e - S::OIK) / NFK) + k0 + (e - S::OIK) % NFK, v);
+            atomicAdd(krow(m, i0 + (e - S::OIK) / NFK) + kcol(k0 + (e - S::OIK) % NFK), v);
         } else {
-            atomicAdd(krow(m, i0 + (e - S::OIL) / NFL) + l0 + (e - S::OIL) % NFL, v);
+            atomicAdd(krow(m, i0 + (e - S::OIL) / NFL) + kcol(l0 + (e - S::OIL) % NFL), v);
         }
     }
     __device__ __forceinline__ void add(int m, int e, double v) {
@@ -468,9 +479,9 @@ struct JKRunItem {
         for (int j = 0; j < NFJ; j++) {
             double* row = krow(m, j0 + j);
 #pragma unroll
-            for (int k = 0; k < NFK; k++) atomicAdd(row + k0 + k, vjk[j * NFK + k]);
+            for (int k = 0; k < NFK; k++) atomicAdd(row + kcol(k0 + k), vjk[j * NFK + k]);
 #pragma unroll
-            for (int l = 0; l < NFL; l++) atomicAdd(row + l0 + l, vjl[j * NFL + l]);
+            for (int l = 0; l < NFL; l++) atomicAdd(row + kcol(l0 + l), vjl[j * NFL + l]);
         }
     }
 
@@ -709,7 +720,7 @@ __device__ __forceinline__ void jk_run_items(const JKSeg* __restrict__ segs, con
     }
 }
 
-template <class C, typename R, bool MULTI>
+template <class C, typename R, bool MULTI, bool KROWS>
 __global__ void __launch_bounds__(JK_RUN_THREADS, (JKRunMinBlocks<C, R>::value))
     jk_run_kernel(const JKSeg* __restrict__ segs, const long long* __restrict__ segt, int nseg,
                   unsigned long long* queue, int grab) {
@@ -727,7 +738,7 @@ __global__ void __launch_bounds__(JK_RUN_THREADS, (JKRunMinBlocks<C, R>::value))
     double* stage = jk_tab + S::TAB / sizeof(double);
     double* dij = stage + S::STAGE / sizeof(double);
     double* slots = jk_tab + S::FIX / sizeof(double);
-    JKRunItem<C, R, MULTI> w{s_seg[warp],
+    JKRunItem<C, R, MULTI, KROWS> w{s_seg[warp],
                              jk_tab,
                              slots + threadIdx.x,
                              slots + S::SLOT / sizeof(double) + threadIdx.x,

@@ -55,7 +55,7 @@ struct JKTRunShape {
     static constexpr size_t SMEM = TAB + (JK_RUN_THREADS / 32) * WARP;
 };
 
-template <class C, typename R, bool MULTI>
+template <class C, typename R, bool MULTI, bool KROWS>
 struct JKTRunItem {
     using S = JKTRunShape<C, R>;
     static constexpr int NFI = C::NFI, NFJ = C::NFJ, NFK = C::NFK, NFL = C::NFL, T = C::T, TPW = C::TPW;
@@ -77,7 +77,11 @@ struct JKTRunItem {
     int ox, oy, oz;  // rows of component ci
 
     __device__ __forceinline__ const double* drow(int m, int a) const { return D + ((size_t)m * nao + a) * nao; }
-    __device__ __forceinline__ double* krow(int m, int a) const { return vk + ((size_t)m * nao + a) * nao; }
+    // K element (a, b) of density m at krow(m, a) + kcol(b), as in JKRunItem
+    __device__ __forceinline__ double* krow(int m, int a) const {
+        return KROWS ? vk + ((size_t)m * nao + a) * nao : vk + (size_t)m * nao * nao + a;
+    }
+    __device__ __forceinline__ size_t kcol(int b) const { return KROWS ? b : (size_t)b * nao; }
 
     __device__ __forceinline__ double dkl(int m, int e) const {
         return sg.dp ? __ldg(sg.dp + sg.pk_kl + m * sg.pk_stride + (size_t)e * sg.pst_kl + col)
@@ -174,9 +178,9 @@ struct JKTRunItem {
         if (dk && mine) {
             double* row = krow(m, i0 + ci);
 #pragma unroll
-            for (int k = 0; k < NFK; k++) atomicAdd(row + k0 + k, kik[k]);
+            for (int k = 0; k < NFK; k++) atomicAdd(row + kcol(k0 + k), kik[k]);
 #pragma unroll
-            for (int l = 0; l < NFL; l++) atomicAdd(row + l0 + l, kil[l]);
+            for (int l = 0; l < NFL; l++) atomicAdd(row + kcol(l0 + l), kil[l]);
         }
         if (dj) {  // J_kl: sum over the team
             __syncwarp();
@@ -288,8 +292,8 @@ struct JKTRunItem {
 #pragma unroll
                         for (int t = 0; t < T; t++) v += part[t * S::PS + e];
                         const int x = e - NJK;
-                        if (e < NJK) atomicAdd(krow(m, j0 + e / NFK) + k0 + e % NFK, v);
-                        else atomicAdd(krow(m, j0 + x / NFL) + l0 + x % NFL, v);
+                        if (e < NJK) atomicAdd(krow(m, j0 + e / NFK) + kcol(k0 + e % NFK), v);
+                        else atomicAdd(krow(m, j0 + x / NFL) + kcol(l0 + x % NFL), v);
                     }
                 __syncwarp();
             }
@@ -418,7 +422,7 @@ struct JKTRunItem {
 };
 
 // segt, queue and grab as in jk_run_kernel; warps work on their own items
-template <class C, typename R, bool MULTI>
+template <class C, typename R, bool MULTI, bool KROWS>
 __global__ void __launch_bounds__(JK_RUN_THREADS, 2)
     jk_trun_kernel(const JKSeg* __restrict__ segs, const long long* __restrict__ segt, int nseg,
                    unsigned long long* queue, int grab) {
@@ -436,7 +440,7 @@ __global__ void __launch_bounds__(JK_RUN_THREADS, 2)
     double* mem = jk_tab + (S::TAB + warp * S::WARP) / sizeof(double);
     const int team = min(lane / C::T, C::TPW - 1);
     double* reg = mem + 32 * 12 + (size_t)team * S::WORDS;
-    JKTRunItem<C, R, MULTI> w{s_seg[warp], S::SMEM_TAB ? jk_tab : rys, reinterpret_cast<R*>(reg), reg,
+    JKTRunItem<C, R, MULTI, KROWS> w{s_seg[warp], S::SMEM_TAB ? jk_tab : rys, reinterpret_cast<R*>(reg), reg,
                               reinterpret_cast<double2*>(mem)};
     jk_run_items(segs, segt, nseg, total, queue, grab, s_seg[warp], w);
 }

@@ -156,6 +156,10 @@ int jk_build_class_pair_noalloc(jk_basis_t *basis, double *vj, double *vk, const
  * per-group density condensation, the class-level density screen and the
  * log-Schwarz bin test per quartet, with the reference's decisions
  * (cuobc/scf/hf.py:104-160).  Same buffer contract as jk_build_class_pair.
+ * K goes through a buffer of n_dm nao^2 doubles that the handle keeps, made on
+ * first use and grown for more densities (a build inside a stream capture
+ * that would have to make it writes vk directly instead, up to 1.5 times
+ * slower, its FP32 quartets in FP64).
  * Replaces the task loop of get_jk (cuobc/scf/hf.py:111-166).
  */
 int jk_build(jk_basis_t *basis, const double *dm, int n_dm, double *vj, double *vk, const jk_opts_t *opts,
