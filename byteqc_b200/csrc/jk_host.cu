@@ -1483,6 +1483,7 @@ extern "C" int jk_build_class_pair(jk_basis_t* b, double* vj, double* vk, const 
     JKRowBins rb;
     int rc = row_bins(bins_locs_ij, bins_locs_kl, nbins, cp_ij == cp_kl, &rb);
     if (rc) return rc;
+    if (n_dm <= 0) return JK_OK;  // no densities (the launchers take n_dm <= 1 as one)
     JKSeg seg;
     fill_seg(b, cp_ij, cp_kl, b->d_qoff1, n_ij, dm, n_dm, vj, vk, &seg);
     JKRunTab rt;

@@ -87,6 +87,7 @@ int jk_basis_pairs(const jk_basis_t *basis, int *pair2shls, int *pair_locs, doub
  * (the host arrays may change once the call returns), the results are there
  * once `stream` reaches them.  The calls of one basis handle share a
  * row-prefix buffer: issue them on one stream (or order their streams).
+ * n_dm = 0 adds nothing.
  */
 int jk_build_class_pair(jk_basis_t *basis, double *vj, double *vk, const double *dm, int nao, int n_dm,
                         const int *bins_locs_ij, const int *bins_locs_kl, int nbins, int cp_ij, int cp_kl,

@@ -137,3 +137,17 @@ def test_raw_entries_agree(bas, n, cutoff):
         assert (vk - base - rk).abs().max().item() <= tol
     lib.jk_batch_destroy(h)
     opt.clear()
+
+
+def test_class_pair_without_densities_adds_nothing():
+    """n_dm = 0 is a call with nothing to do, on run and team classes alike
+    (full-size buffers: a kernel that took it for one density stays inside)."""
+    import torch
+    from byteqc_b200.cuobc import lib as jklib
+    lib = jklib.load_library()
+    opt, d = _setup(1, 'standin-def2-tzvp')
+
+    def fn(handle, vj, vk, dm, nao, n_dm, *a):
+        return lib.jk_build_class_pair(handle, vj, vk, dm, nao, 0, *a)
+    vj, vk = _class_pairs(opt, d, fn)
+    assert not vj.any().item() and not vk.any().item()
