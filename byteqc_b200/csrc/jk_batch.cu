@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <map>
+#include <set>
 #include <vector>
 
 #include "jk_internal.h"
@@ -46,6 +47,10 @@ struct JKSym {
 struct jk_batch {
     int device = 0, nsm = 148, nmol = 0, max_groups = 0, max_nao = 0;
     std::vector<jk_basis*> mols;
+    // screening records of every molecule: the basis's own, or those of a set
+    // of buffers of the batch where the basis occurred before
+    std::vector<const JKScreenCQ*> cqs;
+    std::vector<JKScreenSet> own;  // by molecule, empty (mem null) for a first occurrence
     JKPlan* plan = nullptr;  // merged keys, then the class quartets launched on their own
     int nmerged = 0;         // merged keys
     JKScreenCQ* d_cq = nullptr;
@@ -99,6 +104,7 @@ static void free_batch(jk_batch* t) {
     cudaFree(t->d_pk);
     cudaFree(t->d_pmol);
     cudaFree(t->d_kt);
+    for (auto& o : t->own) cudaFree(o.mem);
     cudaFree(t->d_cq);
     cudaFree(t->d_dmc);
     jk_plan_free(t->plan);
@@ -115,15 +121,20 @@ static int batch_create(jk_basis_t* const* bases, int nmol, long long solo_tasks
     t->nmol = nmol;
     t->plan = new JKPlan();
     std::vector<JKScreenCQ> cqs;
+    std::set<const jk_basis*> seen;
+    t->own.resize(nmol, JKScreenSet{});
     for (int m = 0; m < nmol; m++) {
         jk_basis* b = bases[m];
         if (!b) return jk_internal_set_err(JK_ERR_ARG, "jk_batch_create: null basis");
         if (b->device != t->device) return jk_internal_set_err(JK_ERR_ARG, "jk_batch_create: bases on other devices");
+        if (!seen.insert(b).second)
+            if (int rc = jk_internal_screen_set(b, &t->own[m])) return rc;
         t->mols.push_back(b);
+        t->cqs.push_back(t->own[m].mem ? t->own[m].cq.data() : b->h_cq.data());
         t->max_groups = std::max(t->max_groups, b->ngroups);
         t->max_nao = std::max(t->max_nao, b->nao);
         for (int c = 0; c < b->ncq; c++) {
-            const JKScreenCQ& cq = b->h_cq[c];
+            const JKScreenCQ& cq = t->cqs[m][c];
             cqs.push_back(cq);
             const long long n = cq.cp_ij == cq.cp_kl ? (long long)cq.n_ij * (cq.n_ij + 1) / 2
                                                      : (long long)cq.n_ij * cq.n_kl;
@@ -131,7 +142,7 @@ static int batch_create(jk_basis_t* const* bases, int nmol, long long solo_tasks
             if (rc) return rc;
         }
     }
-    int rc = jk_plan_finish(t->plan, t->mols);
+    int rc = jk_plan_finish(t->plan, t->mols, t->cqs);
     if (rc) return rc;
     for (const auto& k : t->plan->keys) t->nmerged += !k.solo;
     t->ncq = (int)cqs.size();
@@ -232,7 +243,7 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
             for (auto& sgi : k.segs) {
                 const int m = sgi.first;
                 JKSeg& s = seg[i++];
-                jk_internal_fill_seg_cq(t->mols[m], sgi.second, part, &s);
+                jk_internal_fill_seg_cq(t->mols[m], t->cqs[m][sgi.second], part, &s);
                 s.dm = dms[m];
                 s.vj = vjs ? vjs[m] : nullptr;
                 s.vk = vks ? vks[m] : nullptr;
@@ -251,8 +262,10 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
     t->h_dmc.resize(t->nmol);
     for (int m = 0; m < t->nmol; m++) {
         jk_basis* b = t->mols[m];
-        t->h_dmc[m] = JKDmCond{dms[m],     b->d_group_ao, b->d_dm_cond, b->nao, n_dm,
-                               b->ngroups, (unsigned long long*)b->d_zero, (int)(b->zero_bytes / 8)};
+        const JKScreenSet& o = t->own[m];
+        t->h_dmc[m] = JKDmCond{dms[m],     b->d_group_ao, o.mem ? o.dm_cond : b->d_dm_cond, b->nao, n_dm,
+                               b->ngroups, (unsigned long long*)(o.mem ? o.zero : b->d_zero),
+                               (int)(b->zero_bytes / 8)};
     }
     BCUDA(cudaMemcpy(t->d_dmc, t->h_dmc.data(), sizeof(JKDmCond) * t->nmol, cudaMemcpyHostToDevice));
     t->seg_dm.assign(dms, dms + t->nmol);

@@ -1251,7 +1251,7 @@ static int build_plan(jk_basis* b, int nshards, int shard) {
     int rc = JK_OK;
     for (int c = 0; c < b->ncq && !rc; c++)
         if (!owner || owner[c] == shard) rc = jk_plan_add(b->plan, b, 0, c, false);
-    if (!rc) rc = jk_plan_finish(b->plan, {b});
+    if (!rc) rc = jk_plan_finish(b->plan, {b}, {b->h_cq.data()});
     if (rc) {
         jk_plan_free(b->plan);
         b->plan = nullptr;
@@ -1965,8 +1965,7 @@ jk_fill_fn jk_internal_fill_launcher(int class_idx) {
     return g_tabs.fill[class_idx];
 }
 
-void jk_internal_fill_seg_cq(const jk_basis_t* b, int c, int fp32, JKSeg* out) {
-    const JKScreenCQ& cq = b->h_cq[c];
+void jk_internal_fill_seg_cq(const jk_basis_t* b, const JKScreenCQ& cq, int fp32, JKSeg* out) {
     fill_seg(b, cq.cp_ij, cq.cp_kl, cq.runs ? nullptr : (fp32 ? cq.qoff32 : cq.qoff), cq.n_ij, nullptr, 0, nullptr,
              nullptr, out);
     if (cq.runs) {
@@ -1979,6 +1978,33 @@ void jk_internal_fill_seg_cq(const jk_basis_t* b, int c, int fp32, JKSeg* out) {
     } else if (fp32) {
         out->kl_base = cq.klb;
     }
+}
+
+int jk_internal_screen_set(const jk_basis_t* b, JKScreenSet* out) {
+    // doubles and 64-bit words first, then the ints
+    const size_t w = b->zero_bytes / 8 + 2 * (size_t)b->qoff_total + (size_t)b->ioff_total;
+    CUDA_TRY(cudaMalloc(&out->mem, 8 * w + 2 * sizeof(int) * (size_t)b->ent_total + 8));
+    out->zero = out->mem;
+    out->dm_cond = (double*)out->mem;
+    long long* counts = (long long*)(out->dm_cond + (size_t)b->ngroups * b->ngroups);
+    long long *qoff = (long long*)((char*)out->mem + b->zero_bytes), *qoff32 = qoff + b->qoff_total,
+              *ioff = qoff32 + b->qoff_total;
+    int *klb = (int*)(ioff + b->ioff_total), *kle = klb + b->ent_total;
+    out->cq = b->h_cq;
+    for (JKScreenCQ& q : out->cq) {
+        q.dm_cond = out->dm_cond;
+        q.qoff = qoff + (q.qoff - b->d_qoff);
+        q.qoff32 = qoff32 + (q.qoff32 - b->d_qoff32);
+        q.ioff = ioff + (q.ioff - b->d_ioff);
+        q.ioff32 = ioff + (q.ioff32 - b->d_ioff);
+        q.klb = klb + (q.klb - b->d_klb);
+        q.kle = kle + (q.kle - b->d_kle);
+        q.task0 = counts + (q.task0 - b->d_task0);
+        q.task032 = counts + (q.task032 - b->d_task0);
+        q.itm = counts + (q.itm - b->d_task0);
+        q.itm32 = counts + (q.itm32 - b->d_task0);
+    }
+    return JK_OK;
 }
 
 // pack record of one molecule: dens holds 2 n_dm packed densities (dp, dpb),

@@ -164,8 +164,9 @@ struct JKPlan {
 void jk_plan_free(JKPlan* p);
 // adds class quartet c of basis b (molecule m) to its key
 int jk_plan_add(JKPlan* p, const jk_basis* b, int m, int c, bool solo);
-// orders the keys (merged ones first) and segments, uploads the tables
-int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols);
+// orders the keys (merged ones first) and segments, uploads the tables;
+// cqs[m]: the screening records of molecule m
+int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols, const std::vector<const JKScreenCQ*>& cqs);
 // exclusive prefixes of the segments' task counts (after the screening)
 int jk_plan_prefix(const JKPlan* p, bool mixed, cudaStream_t st);
 // direct: the run kernels write K in the layout of the C-ABI (FP64 in both
@@ -252,8 +253,18 @@ int jk_internal_class_team(int class_idx);
 int jk_internal_class_runs(int class_idx);
 void jk_internal_fill_seg(const jk_basis_t* b, int cp_ij, int cp_kl, const long long* qoff, int n_ij,
                           const double* dm, int n_dm, double* vj, double* vk, JKSeg* out);
-// segment of class quartet c, FP64 or FP32 part (no density, no outputs)
-void jk_internal_fill_seg_cq(const jk_basis_t* b, int c, int fp32, JKSeg* out);
+// segment of a class quartet, FP64 or FP32 part (no density, no outputs)
+void jk_internal_fill_seg_cq(const jk_basis_t* b, const JKScreenCQ& cq, int fp32, JKSeg* out);
+// buffers that a build's screening writes, apart from the basis's own ones: a
+// basis that occurs more than once in a batch is screened once per occurrence,
+// with other densities
+struct JKScreenSet {
+    std::vector<JKScreenCQ> cq;
+    double* dm_cond;
+    void* zero;  // jk_basis::d_zero
+    void* mem;   // one allocation, freed by the owner
+};
+int jk_internal_screen_set(const jk_basis_t* b, JKScreenSet* out);
 JKPackMol jk_internal_pack_mol(const jk_basis_t* b, const double* dm, int n_dm, double* dens, double* acc, double* vj);
 // pack (mode 0) or unpack (mode 1) the J side of nmol molecules (device
 // table); mode 1 adds their kt too

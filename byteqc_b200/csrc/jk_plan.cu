@@ -78,7 +78,7 @@ int jk_plan_add(JKPlan* p, const jk_basis* b, int m, int c, bool solo) {
     return JK_OK;
 }
 
-int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols) {
+int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols, const std::vector<const JKScreenCQ*>& cqs) {
     p->index.clear();
     std::stable_partition(p->keys.begin(), p->keys.end(), [](const JKPlanKey& k) { return !k.solo; });
     // longest first within every key (stable: ties keep molecule order)
@@ -113,9 +113,8 @@ int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols) {
                 p->multi = true;
             }
             for (auto& s : k.segs) {
-                const jk_basis* b = mols[s.first];
-                const JKScreenCQ& cq = b->h_cq[s.second];
-                jk_internal_fill_seg_cq(b, s.second, part, &seg[i]);
+                const JKScreenCQ& cq = cqs[s.first][s.second];
+                jk_internal_fill_seg_cq(mols[s.first], cq, part, &seg[i]);
                 if (k.segs.size() == 1)
                     p->one[part].push_back(cq.runs ? (part ? cq.itm32 : cq.itm) : (part ? cq.task032 : cq.task0));
                 cnt[i++] = (cq.runs ? (part ? cq.itm32 : cq.itm) : (part ? cq.task032 : cq.task0)) + 1;

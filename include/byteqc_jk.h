@@ -188,7 +188,8 @@ int jk_get_jk(jk_basis_t *basis, const double *coeff, int nao0, const double *dm
               double *vk0, const jk_opts_t *opts, void *stream);
 
 /*
- * Batched builds over many molecules (one jk_basis each, same device).  No
+ * Batched builds over many molecules (one jk_basis each, same device; a basis
+ * may occur more than once, with a density per occurrence).  No
  * single reference counterpart: the reference builds one molecule at a time
  * through the task loop of get_jk (cuobc/scf/hf.py:111-166); a batch runs
  * the class quartets of all molecules that share a class (angular momenta,

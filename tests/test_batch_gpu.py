@@ -46,6 +46,31 @@ def test_batch_matches_single_molecule_builds():
         assert abs(mres[m][1] - vk).max() <= 1e-9
 
 
+@pytest.mark.parametrize('solo', [None, 1])
+def test_batch_with_a_repeated_basis(solo):
+    """One basis handle several times in a batch, each time with a density of
+    its own (other screening decisions among them: the third is tiny): every
+    occurrence is screened into its own buffers."""
+    from byteqc_b200.cuobc.scf import hf
+    from byteqc_b200.cuobc.scf.batch import JKBatch
+    a, b = _mols()[:2]
+    oa, ob = hf._VHFOpt(a).build(), hf._VHFOpt(b).build()
+    mols = [a, b, a, a, b]
+    dms = _dms(mols)
+    dms[2] = 1e-11 * dms[2]
+    dms[3] = _dms([a], seed=9)[0]
+    batch = JKBatch(mols, vhfopts=[oa, ob, oa, oa, ob], solo_tasks=solo)
+    for cutoff in (None, 1e-6):
+        for rep in range(2):
+            res = batch.get_jk(dms, fp32_cutoff=cutoff)
+            for r, mol, dm, opt in zip(res, mols, dms, batch.opts):
+                vj, vk = hf.get_jk(mol, dm, vhfopt=opt, fp32_cutoff=cutoff)
+                tol = 1e-9 if cutoff else 1e-10
+                assert abs(r[0] - vj).max() <= tol * min(1., abs(dm).max())
+                assert abs(r[1] - vk).max() <= tol * min(1., abs(dm).max())
+    batch.close()
+
+
 def test_batch_graph_replay():
     from byteqc_b200.cuobc.scf.batch import JKBatch
     mols = _mols()
