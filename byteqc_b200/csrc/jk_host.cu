@@ -18,6 +18,7 @@
 #include "jk_internal.h"
 
 static int class_index(const jk_basis* b, int cp_ij, int cp_kl);
+static int make_plan(jk_basis* b, int nshards, int shard, JKPlan** out);
 
 // primitive-pair screen of the run kernels: exp(-mu r^2) below exp(-60)
 // (the default exponent cutoff of libcint's pair data) contributes nothing
@@ -636,6 +637,8 @@ static void free_basis(jk_basis* b) {
     cudaFree(b->d_ehi1);
     cudaFree(b->d_seg1);
     jk_plan_free(b->plan);
+    for (auto& p : b->shard_plans) jk_plan_free(p.second);
+    for (void* p : b->retired) cudaFree(p);
     cudaFree(b->d_prim);
     cudaFree(b->d_primf);
     cudaFree(b->d_cq);
@@ -1109,7 +1112,10 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
     }
     CUDA_TRY(upload(&b->d_pack, b->h_pack.data(), b->h_pack.size()));
     CUDA_TRY(b->fan.init());
-    return JK_OK;
+    // the class launches of jk_build (bases with classes that no J/K kernel
+    // serves, as the density fitting's, do without)
+    int rc = make_plan(b, 1, 0, &b->plan);
+    return rc == JK_ERR_UNSUPPORTED ? JK_OK : rc;
 }
 
 extern "C" int jk_basis_create(const int* atm, int natm, const int* bas, int nbas, const double* env, int nenv,
@@ -1240,23 +1246,41 @@ static const int* shard_owners(jk_basis* b, int nshards) {
     return b->h_cq_owner.data();
 }
 
-// class launches of jk_build for one shard (kept; rebuilt for another split)
-static int build_plan(jk_basis* b, int nshards, int shard) {
-    if (b->plan && b->plan->nshards == nshards && b->plan->shard == shard) return JK_OK;
-    jk_plan_free(b->plan);
-    b->plan = new JKPlan();
-    b->plan->nshards = nshards;
-    b->plan->shard = shard;
+// class launches of one shard of a build
+static int make_plan(jk_basis* b, int nshards, int shard, JKPlan** out) {
+    JKPlan* p = new JKPlan();
     const int* owner = nshards > 1 ? shard_owners(b, nshards) : nullptr;
     int rc = JK_OK;
     for (int c = 0; c < b->ncq && !rc; c++)
-        if (!owner || owner[c] == shard) rc = jk_plan_add(b->plan, b, 0, c, false);
-    if (!rc) rc = jk_plan_finish(b->plan, {b}, {b->h_cq.data()});
+        if (!owner || owner[c] == shard) rc = jk_plan_add(p, b, 0, c, false);
+    if (!rc) rc = jk_plan_finish(p, {b}, {b->h_cq.data()});
     if (rc) {
-        jk_plan_free(b->plan);
-        b->plan = nullptr;
+        jk_plan_free(p);
+        p = nullptr;
     }
+    *out = p;
     return rc;
+}
+
+static bool is_capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return cs != cudaStreamCaptureStatusNone;
+}
+
+// a workspace of the basis of at least `need` doubles
+static int grow(jk_basis* b, double** p, size_t* cap, size_t need) {
+    if (need <= *cap) return JK_OK;
+    if (b->captured && *p) b->retired.push_back(*p);
+    else cudaFree(*p);
+    *p = nullptr;
+    *cap = 0;
+    CUDA_TRY(cudaMalloc(p, sizeof(double) * need));
+    *cap = need;
+    return JK_OK;
 }
 
 // krows: the caller reads V + V^T of K only, which the run kernels may then
@@ -1272,22 +1296,38 @@ static int build(jk_basis* b, const double* dm, int n_dm, double* vj, double* vk
     const int nshards = opts && opts->nshards > 1 ? opts->nshards : 1;
     const int shard = nshards > 1 ? opts->shard : 0;
     if (nshards > 1 && (shard < 0 || shard >= nshards)) return set_err(JK_ERR_ARG, "jk_build: shard out of range");
-    int rc = build_plan(b, nshards, shard);
-    if (rc) return rc;
+    const bool capturing = is_capturing(st);
+    b->captured |= capturing;
+    // the plan of this split; the first build of a split inside a capture,
+    // which cannot make it, launches its class quartets one by one from the
+    // tables of the whole build
+    if (!b->plan) {  // a class without a kernel
+        int rc = make_plan(b, 1, 0, &b->plan);
+        if (rc) return rc;
+    }
+    JKPlan* plan = b->plan;
+    const int* singly = nullptr;
+    if (nshards > 1) {
+        auto it = b->shard_plans.find({nshards, shard});
+        if (it != b->shard_plans.end()) {
+            plan = it->second;
+        } else if (capturing) {
+            singly = shard_owners(b, nshards);
+        } else {
+            int rc = make_plan(b, nshards, shard, &plan);
+            if (rc) return rc;
+            b->shard_plans[{nshards, shard}] = plan;
+        }
+    }
+    int rc = JK_OK;
     // pair-packed density and J accumulators for the run kernels
     const bool packed = vj && b->pack_total > 0;
     JKCall call{dm, vj, vk, nullptr, nullptr, nullptr, nullptr, n_dm, nullptr, 0};
     JKPackMol pm{};
     const int pk_blocks = (int)std::min<long long>((b->pack_total + 255) / 256, (long long)b->nsm * 8);
     if (packed) {
-        const size_t need = (size_t)4 * n_dm * b->pack_total;
-        if (need > b->pk_cap) {
-            cudaFree(b->d_pk);
-            b->d_pk = nullptr;
-            b->pk_cap = 0;
-            CUDA_TRY(cudaMalloc(&b->d_pk, sizeof(double) * need));
-            b->pk_cap = need;
-        }
+        rc = grow(b, &b->d_pk, &b->pk_cap, (size_t)4 * n_dm * b->pack_total);
+        if (rc) return rc;
         pm = jk_internal_pack_mol(b, dm, n_dm, b->d_pk, b->d_pk + 2 * (size_t)n_dm * b->pack_total, vj);
         call.dp = pm.dp;
         call.jp = pm.jp;
@@ -1299,24 +1339,15 @@ static int build(jk_basis* b, const double* dm, int n_dm, double* vj, double* vk
     bool direct = false;
     if (vk && !krows) {
         const size_t need = (size_t)n_dm * b->nao * b->nao;
-        if (need > b->kt_cap) {
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-            CUDA_TRY(cudaStreamIsCapturing(st, &cs));
-            direct = cs != cudaStreamCaptureStatusNone;
-            if (!direct) {
-                cudaFree(b->d_kt);
-                b->d_kt = nullptr;
-                b->kt_cap = 0;
-                CUDA_TRY(cudaMalloc(&b->d_kt, sizeof(double) * need));
-                b->kt_cap = need;
-            }
-        }
+        direct = capturing && need > b->kt_cap;
         if (!direct) {
+            rc = grow(b, &b->d_kt, &b->kt_cap, need);
+            if (rc) return rc;
             call.kt = b->d_kt;
             call.nkt = (long long)need;
         }
     }
-    jk_begin_kernel<<<std::max(pk_blocks, 8), 256, 0, st>>>(b->plan->d_seg[0], b->plan->d_seg[1], b->plan->nseg, call,
+    jk_begin_kernel<<<std::max(pk_blocks, 8), 256, 0, st>>>(plan->d_seg[0], plan->d_seg[1], plan->nseg, call,
                                                             (unsigned long long*)b->d_zero,
                                                             (long long)(b->zero_bytes / 8), pm);
     CUDA_TRY(cudaGetLastError());
@@ -1327,16 +1358,21 @@ static int build(jk_basis* b, const double* dm, int n_dm, double* vj, double* vk
     double fp32_cutoff = opts ? opts->fp32_cutoff : 0.;
     const bool mixed = fp32_cutoff > 0;
     rc = jk_internal_screen(b->d_cq, b->ncq, tol, nbins, prescreen, fp32_cutoff, st);
-    if (!rc) rc = jk_plan_prefix(b->plan, mixed, st);
+    if (!rc && !singly) rc = jk_plan_prefix(plan, mixed, st);
     if (rc) return rc;
     // class launches on side streams: 4 of them, 8 with the FP32 parts or for
     // a molecule whose launches leave most of the device idle
     const int np = mixed ? 2 : 1, ns = mixed || b->h_pair2bra.size() < 4096 ? 8 : 4;
     CUDA_TRY(b->fan.begin(st, ns));
-    for (int k = 0; k < (int)b->plan->keys.size(); k++)
+    for (int k = 0; k < (int)plan->keys.size(); k++)
         for (int part = 0; part < np; part++) {
-            rc = jk_plan_launch(b->plan, k, part, b->plan->keys[k].cfg[part], n_dm, b->nsm,
-                                b->fan.s[(np * k + part) % ns], direct);
+            const JKPlanKey& key = plan->keys[k];
+            cudaStream_t side = b->fan.s[(np * k + part) % ns];
+            if (!singly) rc = jk_plan_launch(plan, k, part, key.cfg[part], n_dm, b->nsm, side, direct);
+            else
+                for (int x = 0; x < (int)key.segs.size() && !rc; x++)
+                    if (singly[key.segs[x].second] == shard)
+                        rc = jk_plan_launch_one(plan, k, x, part, b->h_cq[key.segs[x].second], n_dm, b->nsm, side, direct);
             if (rc) return rc;
         }
     CUDA_TRY(b->fan.end(st, ns));
@@ -1662,13 +1698,8 @@ extern "C" int jk_get_jk(jk_basis_t* b, const double* coeff, int nao0, const dou
     int nao = b->nao;
     size_t nn = (size_t)nao * nao * n_dm, nt = (size_t)nao * nao0 * n_dm;
     size_t need = 5 * nn + 2 * nt;
-    if (need > b->work_cap) {
-        cudaFree(b->d_work);
-        b->d_work = nullptr;
-        b->work_cap = 0;
-        CUDA_TRY(cudaMalloc(&b->d_work, sizeof(double) * need));
-        b->work_cap = need;
-    }
+    int rc = grow(b, &b->d_work, &b->work_cap, need);
+    if (rc) return rc;
     if (!b->blas) BLAS_TRY(cublasCreate(&b->blas));
     BLAS_TRY(cublasSetStream(b->blas, st));
     double* dms = b->d_work;
@@ -1687,7 +1718,7 @@ extern "C" int jk_get_jk(jk_basis_t* b, const double* coeff, int nao0, const dou
     double* v0 = vj0 ? vjw : vkw;  // the outputs lie together
     const size_t nv = vj0 && vk0 ? 2 * nn : nn;
     CUDA_TRY(cudaMemsetAsync(v0, 0, sizeof(double) * nv, st));
-    int rc = build(b, dms, n_dm, vj0 ? vjw : nullptr, vk0 ? vkw : nullptr, true, opts, stream);
+    rc = build(b, dms, n_dm, vj0 ? vjw : nullptr, vk0 ? vkw : nullptr, true, opts, stream);
     if (rc) return rc;
     // J = 2 C^T (V + V^T) C, K = C^T (V + V^T) C (cuobc/scf/hf.py:171-181):
     // one symmetrisation, one product with C from the right for all matrices

@@ -151,7 +151,7 @@ struct JKPlan {
     std::vector<JKPlanKey> keys;
     std::map<std::tuple<int, int, int>, int> index;  // key of a class while the plan is put together
     std::vector<int> key_off;  // nkeys + 1 segment offsets
-    int nseg = 0, nshards = 1, shard = 0;
+    int nseg = 0;
     JKSeg* d_seg[2] = {nullptr, nullptr};        // FP64, FP32 parts
     long long* d_segt[2] = {nullptr, nullptr};   // task prefix per key: nseg + nkeys entries (keys of one
                                                  // segment use the screening's {0, count} itself)
@@ -173,6 +173,9 @@ int jk_plan_prefix(const JKPlan* p, bool mixed, cudaStream_t st);
 // parts), otherwise by rows
 int jk_plan_launch(const JKPlan* p, int k, int part, const JKBatchCfg& cfg, int n_dm, int nsm, cudaStream_t st,
                    bool direct = false);
+// segment s of key k on its own, straight from the screening's counts
+int jk_plan_launch_one(const JKPlan* p, int k, int s, int part, const JKScreenCQ& cq, int n_dm, int nsm,
+                       cudaStream_t st, bool direct);
 
 // Per-geometry state (opaque to callers of the C-ABI)
 struct jk_basis {
@@ -217,7 +220,15 @@ struct jk_basis {
     size_t zero_bytes = 0;
     double* d_dm_cond = nullptr;
     long long *d_task0 = nullptr, *d_task032 = nullptr;
-    JKPlan* plan = nullptr;  // class launches of jk_build
+    // class launches of jk_build: of the whole build (made with the basis), and
+    // of every (nshards, shard) asked for.  All are kept, since CUDA graphs
+    // hold their tables.
+    JKPlan* plan = nullptr;
+    std::map<std::pair<int, int>, JKPlan*> shard_plans;
+    // a build of this basis was captured: buffers that grow are kept in
+    // `retired`, not freed, for the graph's sake
+    bool captured = false;
+    std::vector<void*> retired;
     // reference-compatible single class-pair path
     long long* d_qoff1 = nullptr;
     long long* d_task01 = nullptr;

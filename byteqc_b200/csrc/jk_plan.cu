@@ -47,6 +47,17 @@ void jk_plan_free(JKPlan* p) {
     delete p;
 }
 
+// bound of a class quartet's task or item count
+static long long cq_items(const JKScreenCQ& cq) {
+    if (cq.runs) return (long long)cq.nrun * ((cq.n_kl + cq.runs - 1) / cq.runs + 1);
+    return cq.cp_ij == cq.cp_kl ? (long long)cq.n_ij * (cq.n_ij + 1) / 2 : (long long)cq.n_ij * cq.n_kl;
+}
+// {0, count} of a class quartet's tasks or items
+static const long long* cq_count(const JKScreenCQ& cq, int part) {
+    if (cq.runs) return part ? cq.itm32 : cq.itm;
+    return part ? cq.task032 : cq.task0;
+}
+
 int jk_plan_add(JKPlan* p, const jk_basis* b, int m, int c, bool solo) {
     const JKScreenCQ& cq = b->h_cq[c];
     const int cls = jk_internal_class_index(b, cq.cp_ij, cq.cp_kl);
@@ -74,7 +85,7 @@ int jk_plan_add(JKPlan* p, const jk_basis* b, int m, int c, bool solo) {
     k->segs.push_back({m, c});
     k->seg_tasks.push_back(n);
     k->max_tasks += n;
-    k->max_items += cq.runs ? (long long)cq.nrun * ((cq.n_kl + cq.runs - 1) / cq.runs + 1) : n;
+    k->max_items += cq_items(cq);
     return JK_OK;
 }
 
@@ -116,8 +127,8 @@ int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols, const std::vec
                 const JKScreenCQ& cq = cqs[s.first][s.second];
                 jk_internal_fill_seg_cq(mols[s.first], cq, part, &seg[i]);
                 if (k.segs.size() == 1)
-                    p->one[part].push_back(cq.runs ? (part ? cq.itm32 : cq.itm) : (part ? cq.task032 : cq.task0));
-                cnt[i++] = (cq.runs ? (part ? cq.itm32 : cq.itm) : (part ? cq.task032 : cq.task0)) + 1;
+                    p->one[part].push_back(cq_count(cq, part));
+                cnt[i++] = cq_count(cq, part) + 1;
             }
         }
         PCUDA(cudaMalloc(&p->d_seg[part], sizeof(JKSeg) * ns));
@@ -140,15 +151,28 @@ int jk_plan_prefix(const JKPlan* p, bool mixed, cudaStream_t st) {
     return JK_OK;
 }
 
+static jk_launch_fn plan_launcher(int cls, int part, bool direct) {
+    return direct && jk_internal_class_runs(cls) ? jk_internal_pair_launcher(cls) : jk_internal_launcher(cls, part);
+}
+
 int jk_plan_launch(const JKPlan* p, int k, int part, const JKBatchCfg& cfg, int n_dm, int nsm, cudaStream_t st,
                    bool direct) {
     const JKPlanKey& key = p->keys[k];
     const int off = p->key_off[k], n = p->key_off[k + 1] - off;
-    jk_launch_fn f = direct && jk_internal_class_runs(key.cls) ? jk_internal_pair_launcher(key.cls)
-                                                               : jk_internal_launcher(key.cls, part);
+    jk_launch_fn f = plan_launcher(key.cls, part, direct);
     if (!f) return jk_internal_set_err(JK_ERR_UNSUPPORTED, "no kernel for a class of the build");
     JKBatchCfg c = cfg;
     c.queue = c.grab > 0 ? p->d_queue + 2 * k + part : nullptr;
-    PCUDA(f(p->d_seg[part] + off, p->one[part][k] ? p->one[part][k] : p->d_segt[part] + off + k, n, key.max_items, n_dm, nsm, c, st));
+    const long long* segt = p->one[part][k] ? p->one[part][k] : p->d_segt[part] + off + k;
+    PCUDA(f(p->d_seg[part] + off, segt, n, key.max_items, n_dm, nsm, c, st));
+    return JK_OK;
+}
+
+int jk_plan_launch_one(const JKPlan* p, int k, int s, int part, const JKScreenCQ& cq, int n_dm, int nsm,
+                       cudaStream_t st, bool direct) {
+    jk_launch_fn f = plan_launcher(p->keys[k].cls, part, direct);
+    if (!f) return jk_internal_set_err(JK_ERR_UNSUPPORTED, "no kernel for a class of the build");
+    PCUDA(f(p->d_seg[part] + p->key_off[k] + s, cq_count(cq, part), 1, cq_items(cq), n_dm, nsm,
+            JKBatchCfg{nullptr, 0, 1}, st));
     return JK_OK;
 }

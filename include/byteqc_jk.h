@@ -161,6 +161,11 @@ int jk_build_class_pair_noalloc(jk_basis_t *basis, double *vj, double *vk, const
  * first use and grown for more densities (a build inside a stream capture
  * that would have to make it writes vk directly instead, up to 1.5 times
  * slower, its FP32 quartets in FP64).
+ * A capture of a build holds the handle's tables and buffers: they live until
+ * the handle is destroyed, whatever is built in between.  Inside a capture
+ * nothing is allocated for the class launches (the first build of a split
+ * launches its class quartets one by one there); the J workspace has to be
+ * there from an earlier build with J of as many densities.
  * Replaces the task loop of get_jk (cuobc/scf/hf.py:111-166).
  */
 int jk_build(jk_basis_t *basis, const double *dm, int n_dm, double *vj, double *vk, const jk_opts_t *opts,
