@@ -149,6 +149,7 @@ static int batch_create(jk_basis_t* const* bases, int nmol, long long solo_tasks
     BCUDA(cudaMalloc(&t->d_cq, sizeof(JKScreenCQ) * std::max(1, t->ncq)));
     if (t->ncq) BCUDA(cudaMemcpy(t->d_cq, cqs.data(), sizeof(JKScreenCQ) * t->ncq, cudaMemcpyHostToDevice));
     BCUDA(cudaMalloc(&t->d_dmc, sizeof(JKDmCond) * nmol));
+    BCUDA(jk_internal_uploaded());
     return JK_OK;
 }
 
@@ -268,6 +269,7 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
                                (int)(b->zero_bytes / 8)};
     }
     BCUDA(cudaMemcpy(t->d_dmc, t->h_dmc.data(), sizeof(JKDmCond) * t->nmol, cudaMemcpyHostToDevice));
+    BCUDA(jk_internal_uploaded());
     t->seg_dm.assign(dms, dms + t->nmol);
     t->seg_vj.assign(t->nmol, nullptr);
     t->seg_vk.assign(t->nmol, nullptr);
@@ -545,6 +547,7 @@ extern "C" int jk_batch_get_jk(jk_batch_t* t, const double* const* coeffs, const
             sy[nmol + m] = JKSym{t->d_work + t->w_vk[m], t->d_work + t->w_sym[m], t->mols[m]->nao, n_dm};
         }
         BCUDA(cudaMemcpy(t->d_sym, sy.data(), sizeof(JKSym) * 2 * nmol, cudaMemcpyHostToDevice));
+        BCUDA(jk_internal_uploaded());
         t->w_ndm = n_dm;
     }
     if (!t->blas) BBLAS(cublasCreate(&t->blas));

@@ -682,6 +682,7 @@ static int rys_table_device(const double** out) {
         double* d;
         CUDA_TRY(cudaMalloc(&d, sizeof(double) * n));
         cudaError_t e = cudaMemcpy(d, h, sizeof(double) * n, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = jk_internal_uploaded();
         if (e != cudaSuccess) {
             cudaFree(d);
             CUDA_TRY(e);
@@ -1115,7 +1116,9 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
     // the class launches of jk_build (bases with classes that no J/K kernel
     // serves, as the density fitting's, do without)
     int rc = make_plan(b, 1, 0, &b->plan);
-    return rc == JK_ERR_UNSUPPORTED ? JK_OK : rc;
+    if (rc && rc != JK_ERR_UNSUPPORTED) return rc;
+    CUDA_TRY(jk_internal_uploaded());
+    return JK_OK;
 }
 
 extern "C" int jk_basis_create(const int* atm, int natm, const int* bas, int nbas, const double* env, int nenv,
@@ -1921,6 +1924,8 @@ extern "C" int jk_rys_roots_device(int n, const double* x, int count, double* s,
 // internal helpers for the other translation units
 // ---------------------------------------------------------------------------
 int jk_internal_set_err(int code, const char* msg) { return set_err(code, "%s", msg); }
+
+cudaError_t jk_internal_uploaded() { return cudaStreamSynchronize(cudaStreamLegacy); }
 
 int jk_internal_class_info(const jk_basis_t* b, int cp_ij, int cp_kl, int* n_ij, int* n_kl, int* nao) {
     if (!b || cp_ij < 0 || cp_ij >= b->ncp || cp_kl < 0 || cp_kl > cp_ij)

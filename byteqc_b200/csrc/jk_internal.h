@@ -40,6 +40,11 @@ struct JKScreenCQ {
 };
 
 int jk_internal_set_err(int code, const char* msg);
+// Waits until the tables that cudaMemcpy took from pageable memory lie on the
+// device.  It may return with the last transfer still under way on the legacy
+// stream, which a caller's non-blocking stream does not wait for; every function
+// that uploads tables ends with this.
+cudaError_t jk_internal_uploaded();
 // pair counts of the two classes and the working-basis size
 int jk_internal_class_info(const jk_basis_t* b, int cp_ij, int cp_kl, int* n_ij, int* n_kl, int* nao);
 // Per-class-pair launch with caller-owned scratch: the segment goes by value

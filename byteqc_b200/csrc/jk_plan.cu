@@ -139,6 +139,7 @@ int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols, const std::vec
             PCUDA(cudaMemcpy((void*)p->d_cnt[part], cnt.data(), sizeof(long long*) * p->nseg, cudaMemcpyHostToDevice));
         }
     }
+    PCUDA(jk_internal_uploaded());
     return JK_OK;
 }
 

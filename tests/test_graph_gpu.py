@@ -103,3 +103,42 @@ def test_first_builds_inside_a_capture(cutoff):
     torch.cuda.synchronize()
     assert (vj - rj).abs().max().item() <= tol
     assert (vk - rk).abs().max().item() <= tol
+
+
+def test_side_stream_right_after_set_up():
+    """Builds on a non-blocking stream right after the basis, the tables of a
+    split or those of a batch were made, with nothing in between that would
+    wait for their uploads."""
+    import torch
+    from byteqc_b200.cuobc.scf import hf
+    from byteqc_b200.cuobc.scf.batch import JKBatch
+    mol = Mole(atom=geom.water_cluster(2, box=5.0, seed=4),
+               basis='standin-def2-tzvp').build()
+    rng = np.random.default_rng(8)
+    dm = rng.standard_normal((mol.nao, mol.nao))
+    d = torch.as_tensor(dm + dm.T, device='cuda')
+    opt = hf._VHFOpt(mol).build()
+    rj, rk = hf.get_jk(mol, d, vhfopt=opt, out='device')
+    w = (opt.coeff_dev @ d @ opt.coeff_dev.T).contiguous()[None]
+    raw = torch.zeros_like(w), torch.zeros_like(w)
+    _build(opt, w, *raw)
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    sp = ctypes.c_void_p(s.cuda_stream)
+    for rep in range(10):
+        with torch.cuda.stream(s):
+            o = hf._VHFOpt(mol).build()
+            vj, vk = hf.get_jk(mol, d, vhfopt=o, out='device')
+            assert (vj - rj).abs().max().item() <= 1e-10
+            assert (vk - rk).abs().max().item() <= 1e-10
+            vj, vk = torch.zeros_like(w), torch.zeros_like(w)
+            for sh in range(2):
+                _build(o, w, vj, vk, sh, 2, sp)
+            assert (vj - raw[0]).abs().max().item() <= 1e-10
+            assert (vk - raw[1]).abs().max().item() <= 1e-10
+            b = JKBatch([mol, mol], vhfopts=[o, opt])
+            for vj, vk in b.get_jk([d, d], out='device'):
+                assert (vj - rj).abs().max().item() <= 1e-10
+                assert (vk - rk).abs().max().item() <= 1e-10
+            b.close()
+            o.clear()
