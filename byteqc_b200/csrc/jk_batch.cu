@@ -69,6 +69,7 @@ struct jk_batch {
     JKSym* d_sym = nullptr;
     std::vector<size_t> w_dms, w_vj, w_vk, w_sym, w_tmp;  // offsets per molecule
     int w_ndm = -1;
+    std::vector<int> w_nao0;  // caller basis sizes they were laid out for
     // captured graph
     cudaGraphExec_t graph = nullptr;
     JKFanout fan;  // side streams of the class launches
@@ -512,7 +513,9 @@ extern "C" int jk_batch_get_jk(jk_batch_t* t, const double* const* coeffs, const
         return jk_internal_set_err(JK_ERR_ARG, "jk_batch_get_jk: invalid arguments");
     cudaStream_t st = (cudaStream_t)stream;
     int nmol = t->nmol;
-    if (t->w_ndm != n_dm) {
+    bool fits = t->w_ndm == n_dm;
+    for (int m = 0; fits && m < nmol; m++) fits = nao0s[m] <= t->w_nao0[m];
+    if (!fits) {
         size_t off = 0;
         t->w_dms.resize(nmol);
         t->w_vj.resize(nmol);
@@ -549,6 +552,7 @@ extern "C" int jk_batch_get_jk(jk_batch_t* t, const double* const* coeffs, const
         BCUDA(cudaMemcpy(t->d_sym, sy.data(), sizeof(JKSym) * 2 * nmol, cudaMemcpyHostToDevice));
         BCUDA(jk_internal_uploaded());
         t->w_ndm = n_dm;
+        t->w_nao0.assign(nao0s, nao0s + nmol);
     }
     if (!t->blas) BBLAS(cublasCreate(&t->blas));
     BBLAS(cublasSetStream(t->blas, st));

@@ -71,6 +71,51 @@ def test_batch_with_a_repeated_basis(solo):
     batch.close()
 
 
+def test_batch_with_a_larger_caller_basis_later():
+    """jk_batch_get_jk at one n_dm with another caller basis than the first
+    call's: spherical, then Cartesian (more functions), then spherical."""
+    import ctypes
+    import torch
+    from byteqc_b200.cuobc import lib as jklib
+    from byteqc_b200.cuobc.scf import hf
+    from byteqc_b200.cuobc.scf.batch import JKBatch, _ptrs
+    lib = jklib.load_library()
+    mols = []
+    for i in range(3):
+        mols.append(Mole(atom=geom.water_cluster(1 + i, box=5.0, seed=i),
+                         basis='standin-def2-tzvp').build())
+    batch = JKBatch(mols)
+    rng = np.random.default_rng(2)
+    o = batch._opts(True, None, None)
+    for cart in (False, True, False):
+        coeff = [torch.eye(op.nao, dtype=torch.float64, device='cuda') if cart
+                 else op.coeff_dev for op in batch.opts]
+        dms = []
+        for c in coeff:
+            d = rng.standard_normal((c.shape[1], c.shape[1]))
+            dms.append(torch.as_tensor(d + d.T, device='cuda'))
+        vj, vk = ([torch.zeros_like(d) for d in dms] for _ in range(2))
+        assert lib.jk_batch_get_jk(
+            batch.handle, _ptrs([c.data_ptr() for c in coeff]),
+            (ctypes.c_int * 3)(*[c.shape[1] for c in coeff]),
+            *(_ptrs([x.data_ptr() for x in y]) for y in (dms, vj, vk)), 1,
+            ctypes.byref(o), None) == 0
+        torch.cuda.synchronize()
+        for m in range(3):
+            op = batch.opts[m]
+            rj, rk = torch.zeros_like(dms[m]), torch.zeros_like(dms[m])
+            so = jklib.JKOpts()
+            so.direct_scf_tol, so.nbins, so.prescreen = 1e-13, o.nbins, 1
+            assert lib.jk_get_jk(op.handle, coeff[m].data_ptr(),
+                                 coeff[m].shape[1], dms[m].data_ptr(), 1,
+                                 rj.data_ptr(), rk.data_ptr(),
+                                 ctypes.byref(so), None) == 0
+            torch.cuda.synchronize()
+            assert (vj[m] - rj).abs().max().item() <= 1e-10
+            assert (vk[m] - rk).abs().max().item() <= 1e-10
+    batch.close()
+
+
 def test_batch_graph_replay():
     from byteqc_b200.cuobc.scf.batch import JKBatch
     mols = _mols()
