@@ -367,6 +367,14 @@ static std::string tune_key_str(const JKPlanKey& k, int part) {
     return buf;
 }
 
+// First line of a cache file as the tuner writes it.  The number stands for
+// what a grab means: 2, items for the run kernels.  Files written before it
+// have the line without a number, and counted quartets there (grabs up to
+// 1024, which as items leave most of the device idle): they are not read.
+// Files without such a line (written by hand) are.
+static const char kTuneHead[] = "# byteqc_b200 batch launch shapes";
+static const char kTuneVersion[] = " 2: ";
+
 extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* const* vjs, double* const* vks,
                              int n_dm, const jk_opts_t* opts, const char* cache_path, void* stream) {
     if (!t || !dms || n_dm <= 0 || (!vjs && !vks))
@@ -381,9 +389,13 @@ extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* co
         if (f) {
             char line[256];
             while (fgets(line, sizeof(line), f)) {
+                if (!strncmp(line, kTuneHead, sizeof(kTuneHead) - 1) &&
+                    strncmp(line + sizeof(kTuneHead) - 1, kTuneVersion, sizeof(kTuneVersion) - 1))
+                    break;  // of another version
                 int cls, a, b, part, lg, grab, gm;
                 float ms;
                 if (sscanf(line, "%d %d %d %d %d %d %d %f", &cls, &a, &b, &part, &lg, &grab, &gm, &ms) != 8) continue;
+                if (grab < 0 || gm < 1 || gm > 64) continue;  // no launch shape
                 char key[96];
                 snprintf(key, sizeof(key), "%d %d %d %d %d", cls, a, b, part, lg);
                 cache[key] = {JKBatchCfg{nullptr, grab, gm}, ms};
@@ -451,7 +463,7 @@ extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* co
     if (cache_path) {
         FILE* f = fopen(cache_path, "w");
         if (!f) return jk_internal_set_err(JK_ERR_ARG, "jk_batch_tune: cannot write the cache file");
-        fprintf(f, "# byteqc_b200 batch launch shapes: cls np_ij np_kl part log2tasks grab grid_mul ms\n");
+        fprintf(f, "%s%scls np_ij np_kl part log2tasks grab grid_mul ms\n", kTuneHead, kTuneVersion);
         for (auto& kv : cache)
             fprintf(f, "%s %d %d %.4f\n", kv.first.c_str(), kv.second.first.grab, kv.second.first.grid_mul,
                     kv.second.second);

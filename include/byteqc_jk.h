@@ -233,7 +233,7 @@ int jk_batch_build(jk_batch_t *batch, const double *const *dms, double *const *v
  * jk_batch_build), and keeps the fastest.  cache_path (may be NULL): a text
  * file of earlier choices per (class, primitive counts, part, log2 task
  * count), read first (those launches are not timed again) and rewritten
- * with all choices.  The timing runs accumulate into vjs/vks, which are
+ * with all choices (a file that another version of the tuner wrote is not read).  The timing runs accumulate into vjs/vks, which are
  * zeroed before return; the call synchronises `stream`. */
 int jk_batch_tune(jk_batch_t *batch, const double *const *dms, double *const *vjs, double *const *vks, int n_dm,
                   const jk_opts_t *opts, const char *cache_path, void *stream);

@@ -266,6 +266,38 @@ def test_batch_persistent_shapes_match_static():
     batch.close()
 
 
+def test_batch_tune_leaves_files_of_before_alone(tmp_path):
+    """A cache file of the tuner whose grabs counted quartets (its first line
+    carries no version) is timed anew and rewritten; entries that are no launch
+    shape are passed over."""
+    from byteqc_b200.cuobc.scf.batch import JKBatch
+    mols = _mols()[:2]
+    dms = _dms(mols, seed=10)
+    batch = JKBatch(mols)
+    path = str(tmp_path / 'tune.txt')
+
+    def write(head, grab, gm):
+        with open(path, 'w') as f:
+            f.write(head)
+            for k in batch.info():
+                f.write('%d %d %d 0 %d %d %d 1.0\n' % (
+                    k['class'], k['np_ij'], k['np_kl'],
+                    max(0, int(k['tasks']).bit_length() - 1), grab, gm))
+    old = ('# byteqc_b200 batch launch shapes: cls np_ij np_kl part log2tasks '
+           'grab grid_mul ms\n')
+    for head, grab, gm in ((old, 1024, 1), ('', 4, 0), ('', -3, 1)):
+        write(head, grab, gm)
+        info = batch.tune(dms, cache=path)
+        assert all(k['fp64']['grab'] in (0, 1, 2, 4, 8, 16, 32)
+                   and k['fp64']['grid_mul'] in (1, 2) for k in info)
+        assert not any(k['fp64']['ms'] == 1.0 for k in info)
+    assert open(path).readline() != old
+    again = batch.tune(dms, cache=path)
+    for key in ('grab', 'grid_mul'):
+        assert [k['fp64'][key] for k in again] == [k['fp64'][key] for k in info]
+    batch.close()
+
+
 def test_batch_solo_class_quartets():
     """Class quartets above the solo threshold run as their own launches
     (the single-molecule kernels), the rest merged: every split gives the
