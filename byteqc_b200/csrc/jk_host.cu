@@ -16,6 +16,7 @@
 #include "../../include/byteqc_jk.h"
 #include "jk_launch.cuh"
 #include "jk_internal.h"
+#include "jk_pair.cuh"
 
 static int class_index(const jk_basis* b, int cp_ij, int cp_kl);
 static int make_plan(jk_basis* b, int nshards, int shard, JKPlan** out);
@@ -212,47 +213,6 @@ __global__ void jk_zero_kernel(const JKDmCond* __restrict__ tab) {
     for (int e = threadIdx.x; e < m.nzero; e += blockDim.x) m.zero[e] = 0;
 }
 
-// Block-wide inclusive scan of two counts (256 threads), with running carries.
-__device__ __forceinline__ void jk_block_scan2(long long a, long long b, long long& ia, long long& ib,
-                                               long long* wa, long long* wb, long long& carry_a,
-                                               long long& carry_b) {
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int o = 1; o < 32; o <<= 1) {
-        long long ya = __shfl_up_sync(0xffffffffu, a, o), yb = __shfl_up_sync(0xffffffffu, b, o);
-        if (lane >= o) {
-            a += ya;
-            b += yb;
-        }
-    }
-    if (lane == 31) {
-        wa[warp] = a;
-        wb[warp] = b;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        long long x = (lane < (int)(blockDim.x >> 5)) ? wa[lane] : 0;
-        long long y = (lane < (int)(blockDim.x >> 5)) ? wb[lane] : 0;
-        for (int o = 1; o < 32; o <<= 1) {
-            long long u = __shfl_up_sync(0xffffffffu, x, o), v = __shfl_up_sync(0xffffffffu, y, o);
-            if (lane >= o) {
-                x += u;
-                y += v;
-            }
-        }
-        wa[lane] = x;
-        wb[lane] = y;
-    }
-    __syncthreads();
-    ia = a + (warp ? wa[warp - 1] : 0) + carry_a;
-    ib = b + (warp ? wb[warp - 1] : 0) + carry_b;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) {
-        carry_a = ia;
-        carry_b = ib;
-    }
-    __syncthreads();
-}
-
 // max over the six group pairs of a class quartet of the condensed density
 __device__ __forceinline__ double jk_cq_sub(const double* c, int ngroups, int gi, int gj, int gk, int gl) {
     return fmax(fmax(fmax(c[gi * ngroups + gj], c[gk * ngroups + gl]), fmax(c[gi * ngroups + gk], c[gj * ngroups + gk])),
@@ -422,16 +382,17 @@ __global__ void __launch_bounds__(1024) jk_run_scan_kernel(const JKScreenCQ* __r
 }
 
 // per-class-pair entries: items of each run from the entries' ket ends
-__global__ void jk_run_items_kernel(int nrun, int chunk, int bucket, int n_kl, const int* __restrict__ run0, const int* __restrict__ ehi,
-                                    long long* __restrict__ ioff) {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrun; r += gridDim.x * blockDim.x) {
+__global__ void jk_run_items_kernel(const __grid_constant__ JKSeg sg, int chunk, long long* __restrict__ ioff) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < sg.nrun; r += gridDim.x * blockDim.x) {
         int h = 0;
-        for (int e = run0[r]; e < run0[r + 1]; e++) h = max(h, ehi[e]);
-        ioff[r] = (jk_bucket_end(h, bucket, n_kl) + chunk - 1) / chunk;
+        for (int e = sg.run0[r]; e < sg.run0[r + 1]; e++) h = max(h, sg.ehi[e]);
+        ioff[r] = (jk_bucket_end(h, sg.bucket, sg.pst_kl) + chunk - 1) / chunk;
     }
 }
-__global__ void __launch_bounds__(1024) jk_run_scan1_kernel(int nrun, long long* ioff, long long* itm) {
-    jk_run_scan_body(nrun, ioff, nullptr, itm, nullptr);
+__global__ void __launch_bounds__(1024) jk_run_scan1_kernel(const __grid_constant__ JKSeg sg, long long* ioff,
+                                                            long long* itm, JKSeg* dst) {
+    jk_seg_copy(sg, dst);
+    jk_run_scan_body(sg.nrun, ioff, nullptr, itm, nullptr);
 }
 
 // bra records of the run kernels (JKSeg::bprim, bprimf, bpair) of one class,
@@ -464,12 +425,6 @@ __global__ void jk_bra_records_kernel(int np, int nprim, const int* __restrict__
             b[3] = __hiloint2double(pnp[r], pao[npt + r]);
         }
     }
-}
-
-__global__ void jk_put_seg_kernel(const __grid_constant__ JKSeg sg, JKSeg* __restrict__ dst) {
-    const int* a = reinterpret_cast<const int*>(&sg);
-    int* d = reinterpret_cast<int*>(dst);
-    for (int x = threadIdx.x; x < (int)(sizeof(JKSeg) / 4); x += blockDim.x) d[x] = a[x];
 }
 
 // the call's buffers into the segments of a plan
@@ -700,10 +655,10 @@ static int sort_bucket(int n) { return std::max(32, (n / 16 + 31) / 32 * 32); }
 // Run length of a class quartet's bra (an index of JK_RUN_LEN): the longest
 // that still gives a few items per resident warp before screening; a
 // molecule too small for that takes the shortest.
-static int run_level(const jk_basis* b, int cp_ij, int n_kl, int chunk) {
-    for (int v = 0; v < JK_RUN_LEVELS - 1; v++)
+static int run_level(const jk_basis* b, int cp_ij, int n_kl, int chunk, int levels) {
+    for (int v = 0; v < levels - 1; v++)
         if ((long long)b->h_nrun[v][cp_ij] * ((n_kl + chunk - 1) / chunk) >= 40LL * b->nsm) return v;
-    return JK_RUN_LEVELS - 1;
+    return levels - 1;
 }
 
 static int create_impl(const int* atm, int natm, const int* bas, int nbas, const double* env, int nenv,
@@ -957,7 +912,7 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
     // order, cut at each run length
     {
         std::vector<int> ent(npair), erank(npair), inv(npair), run0;
-        for (int v = 0; v < JK_RUN_LEVELS; v++) {
+        for (int v = 0; v < JK_RUN_LEVELS_PAIR; v++) {
             b->h_nrun[v].assign(b->ncp, 0);
             b->h_run_off[v].assign(b->ncp, 0);
         }
@@ -969,7 +924,7 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             for (int x = 0; x < np; x++) at[b->h_pair2bra[p0 + x] + 1]++;
             for (int x = 0; x < nbas; x++) at[x + 1] += at[x];
             for (int x = 0; x < np; x++) e[at[b->h_pair2bra[p0 + x]]++] = x;
-            for (int v = 0; v < JK_RUN_LEVELS; v++) {
+            for (int v = 0; v < JK_RUN_LEVELS_PAIR; v++) {
                 b->h_run_off[v][c] = (int)run0.size();
                 int beg = 0;
                 for (int x = 0; x <= np; x++) {
@@ -1031,7 +986,7 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             ent_at.push_back(b->ent_total);
             b->ent_total += c.n_ij;
             if (c.runs) {
-                c.level = run_level(b, cij, c.n_kl, c.runs);
+                c.level = run_level(b, cij, c.n_kl, c.runs, JK_RUN_LEVELS);
                 c.nrun = b->h_nrun[c.level][cij];
                 b->ioff_total += 2LL * c.nrun;
             } else {
@@ -1435,25 +1390,31 @@ __host__ __device__ inline long long jk_rowbins_tasks(const JKRowBins& b, long l
 }
 
 // columns row r keeps
-__device__ __forceinline__ int jk_rowbins_cols(const JKRowBins& b, int r) {
-    if (b.kl[0] != 0) return 0;
-    for (int s = 0; s < b.nbins; s++)
-        if (r >= b.ij[s] && r < b.ij[s + 1]) {
-            const int c = b.kl[b.nbins - s];
-            return b.diag && c > r + 1 ? r + 1 : c;
-        }
-    return 0;
-}
+struct JKRowBinsCols {
+    JKRowBins b;
+    int n_kl;
+    __device__ __forceinline__ int operator()(int r) const {
+        if (b.kl[0] != 0) return 0;
+        for (int s = 0; s < b.nbins; s++)
+            if (r >= b.ij[s] && r < b.ij[s + 1]) {
+                const int c = min(b.kl[b.nbins - s], n_kl);
+                return b.diag && c > r + 1 ? r + 1 : c;
+            }
+        return 0;
+    }
+};
 
-// run classes: ket end of every entry
-__global__ void jk_run_rowbins_kernel(const __grid_constant__ JKRowBins rb, int n_ij, int n_kl,
+// run classes of many bra pairs: ket end of every entry
+__global__ void jk_run_rowbins_kernel(const __grid_constant__ JKRowBinsCols cols, int n_ij,
                                       const int* __restrict__ erank, int* __restrict__ ehi) {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_ij; e += gridDim.x * blockDim.x)
-        ehi[e] = min(jk_rowbins_cols(rb, erank[e]), n_kl);
+        ehi[e] = cols(erank[e]);
 }
 
+// row classes; the segment of a J/K call goes to *dst
 __global__ void jk_rowbins_kernel(const JKRowBins rb, int n_ij, long long* __restrict__ qoff,
-                                  long long* __restrict__ task0) {
+                                  long long* __restrict__ task0, const __grid_constant__ JKSeg sg, JKSeg* dst) {
+    if (dst && blockIdx.x == 0) jk_seg_copy(sg, dst);
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r <= n_ij;
          r += (long long)gridDim.x * blockDim.x)
         qoff[r] = jk_rowbins_tasks(rb, r);
@@ -1477,12 +1438,13 @@ static int row_bins(const int* bins_ij, const int* bins_kl, int nbins, int diag,
 }
 
 // bins of a per-class-pair call -> the basis's row prefix and task count, on
-// `st`; returns the task count through *tot
-static int class_pair_rows(jk_basis* b, const JKRowBins& rb, int n_ij, cudaStream_t st, long long* tot) {
+// `st`, and the segment to *dst (if any); returns the task count through *tot
+static int class_pair_rows(jk_basis* b, const JKRowBins& rb, int n_ij, const JKSeg& seg, JKSeg* dst, cudaStream_t st,
+                           long long* tot) {
     if (n_ij + 1 > (int)b->qoff1_cap) return set_err(JK_ERR_ARG, "class pair larger than the basis' classes");
     *tot = jk_rowbins_tasks(rb, n_ij);
     const int blocks = (int)std::min<long long>((n_ij + 256) / 256, (long long)b->nsm * 4);
-    jk_rowbins_kernel<<<blocks, 256, 0, st>>>(rb, n_ij, b->d_qoff1, b->d_task01);
+    jk_rowbins_kernel<<<blocks, 256, 0, st>>>(rb, n_ij, b->d_qoff1, b->d_task01, seg, dst);
     CUDA_TRY(cudaGetLastError());
     return JK_OK;
 }
@@ -1525,25 +1487,27 @@ extern "C" int jk_build_class_pair(jk_basis_t* b, double* vj, double* vk, const 
     if (n_dm <= 0) return JK_OK;  // no densities (the launchers take n_dm <= 1 as one)
     JKSeg seg;
     fill_seg(b, cp_ij, cp_kl, b->d_qoff1, n_ij, dm, n_dm, vj, vk, &seg);
-    JKRunTab rt;
     long long tot = 0;
-    if (jk_internal_run_table(b, cp_ij, cp_kl, &rt)) {
-        const int n_kl = seg.pst_kl;
-        if (n_ij == 0 || n_kl == 0) return JK_OK;
-        jk_run_rowbins_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(rb, n_ij, n_kl, rt.erank, b->d_ehi1);
-        CUDA_TRY(cudaGetLastError());
-        rc = jk_internal_run_items(rt, b->d_ehi1, b->d_qoff1, b->d_task01, st);
-        seg.nrun = rt.nrun;
-        seg.ent = rt.ent;
-        seg.run0 = rt.run0;
-        seg.ehi = b->d_ehi1;
-        seg.ioff = b->d_qoff1;
-        tot = (long long)rt.nrun * ((n_kl + rt.chunk - 1) / rt.chunk);
+    const int* erank;
+    int chunk;
+    if (jk_internal_pair_runs(b, cp_ij, cp_kl, &seg, b->d_ehi1, b->d_qoff1, &erank, &chunk)) {
+        const JKRowBinsCols cols{rb, seg.pst_kl};
+        if (n_ij == 0 || seg.pst_kl == 0) return JK_OK;
+        if (n_ij <= JK_PAIR_PREP_ROWS) {
+            jk_pair_prep_kernel<<<1, jk_pair_prep_threads(seg.nrun), 0, st>>>(cols, seg, b->d_seg1, erank, chunk, b->d_ehi1, b->d_qoff1,
+                                                    b->d_task01);
+            CUDA_TRY(cudaGetLastError());
+        } else {
+            jk_run_rowbins_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(cols, n_ij, erank, b->d_ehi1);
+            CUDA_TRY(cudaGetLastError());
+            rc = jk_internal_run_items(seg, chunk, b->d_task01, b->d_seg1, st);
+        }
+        tot = (long long)seg.nrun * ((seg.pst_kl + chunk - 1) / chunk);
     } else {
-        rc = class_pair_rows(b, rb, n_ij, st, &tot);
+        rc = class_pair_rows(b, rb, n_ij, seg, b->d_seg1, st, &tot);
     }
     if (rc) return rc;
-    return jk_internal_launch(b, cp_ij, cp_kl, seg, b->d_seg1, b->d_task01, tot, stream);
+    return jk_internal_launch(b, cp_ij, cp_kl, b->d_seg1, b->d_task01, tot, n_dm, stream);
 }
 
 // ERI tensor of one class pair (jk_generic.cu)
@@ -1587,10 +1551,10 @@ extern "C" int jk_fill_int2e(jk_basis_t* b, double* eri, int nao, const int* str
     JKRowBins rb;
     long long tot = 0;
     int rc = row_bins(bij, bkl, nbins, 0, &rb);
-    if (!rc) rc = class_pair_rows(b, rb, n_ij, st, &tot);
-    if (rc) return rc;
     JKSeg seg;
     fill_seg(b, cp_ij, cp_kl, b->d_qoff1, n_ij, nullptr, 0, nullptr, nullptr, &seg);
+    if (!rc) rc = class_pair_rows(b, rb, n_ij, seg, nullptr, st, &tot);
+    if (rc) return rc;
     CUDA_TRY(jk_launch_fill(seg, b->d_task01, tot, b->nsm, eri, s64, off, st));
     return JK_OK;
 }
@@ -1941,35 +1905,33 @@ void jk_internal_fill_seg(const jk_basis_t* b, int cp_ij, int cp_kl, const long 
     fill_seg(b, cp_ij, cp_kl, qoff, n_ij, dm, n_dm, vj, vk, out);
 }
 
-int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg& seg, JKSeg* d_seg,
-                       const long long* task0, long long max_tasks, void* stream) {
+int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg* d_seg, const long long* task0,
+                       long long max_tasks, int n_dm, void* stream) {
     jk_launch_fn fn = g_tabs.pair[class_index(b, cp_ij, cp_kl)];
     if (!fn) return set_err(JK_ERR_UNSUPPORTED, "no kernel for class pair (%d, %d)", cp_ij, cp_kl);
-    cudaStream_t st = (cudaStream_t)stream;
-    jk_put_seg_kernel<<<1, 128, 0, st>>>(seg, d_seg);
-    CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(fn(d_seg, task0, 1, max_tasks, seg.n_dm, b->nsm, JKBatchCfg{nullptr, 0, 1}, st));
+    CUDA_TRY(fn(d_seg, task0, 1, max_tasks, n_dm, b->nsm, JKBatchCfg{nullptr, 0, 1}, (cudaStream_t)stream));
     return JK_OK;
 }
 
-int jk_internal_run_table(const jk_basis_t* b, int cp_ij, int cp_kl, JKRunTab* out) {
-    if (!g_tabs.run[class_index(b, cp_ij, cp_kl)]) return 0;
-    out->n_kl = b->h_pair_locs[cp_kl + 1] - b->h_pair_locs[cp_kl];
-    out->bucket = sort_bucket(out->n_kl);
-    out->erank = b->d_erank + b->h_pair_locs[cp_ij];
-    out->chunk = g_tabs.run[class_index(b, cp_ij, cp_kl)];
-    const int v = run_level(b, cp_ij, b->h_pair_locs[cp_kl + 1] - b->h_pair_locs[cp_kl], out->chunk);
-    out->nrun = b->h_nrun[v][cp_ij];
-    out->ent = b->d_ent + b->h_pair_locs[cp_ij];
-    out->run0 = b->d_run0 + b->h_run_off[v][cp_ij];
-    return 1;
+bool jk_internal_pair_runs(const jk_basis_t* b, int cp_ij, int cp_kl, JKSeg* seg, int* ehi, long long* ioff,
+                           const int** erank, int* chunk) {
+    *chunk = g_tabs.run[class_index(b, cp_ij, cp_kl)];
+    if (!*chunk) return false;
+    const int v = run_level(b, cp_ij, seg->pst_kl, *chunk, JK_RUN_LEVELS_PAIR);
+    seg->nrun = b->h_nrun[v][cp_ij];
+    seg->ent = b->d_ent + b->h_pair_locs[cp_ij];
+    seg->run0 = b->d_run0 + b->h_run_off[v][cp_ij];
+    seg->ehi = ehi;
+    seg->ioff = ioff;
+    *erank = b->d_erank + b->h_pair_locs[cp_ij];
+    return true;
 }
 
-int jk_internal_run_items(const JKRunTab& rt, const int* ehi, long long* ioff, long long* itm, void* stream) {
+int jk_internal_run_items(const JKSeg& seg, int chunk, long long* itm, JKSeg* d_seg, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
-    if (rt.nrun > 0) jk_run_items_kernel<<<(rt.nrun + 255) / 256, 256, 0, st>>>(rt.nrun, rt.chunk, rt.bucket, rt.n_kl, rt.run0,
-                                                                                ehi, ioff);
-    jk_run_scan1_kernel<<<1, 1024, 0, st>>>(rt.nrun, ioff, itm);
+    long long* ioff = const_cast<long long*>(seg.ioff);
+    jk_run_items_kernel<<<(seg.nrun + 255) / 256, 256, 0, st>>>(seg, chunk, ioff);
+    jk_run_scan1_kernel<<<1, 1024, 0, st>>>(seg, ioff, itm, d_seg);
     CUDA_TRY(cudaGetLastError());
     return JK_OK;
 }

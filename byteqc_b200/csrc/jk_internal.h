@@ -47,22 +47,20 @@ int jk_internal_set_err(int code, const char* msg);
 cudaError_t jk_internal_uploaded();
 // pair counts of the two classes and the working-basis size
 int jk_internal_class_info(const jk_basis_t* b, int cp_ij, int cp_kl, int* n_ij, int* n_kl, int* nao);
-// Per-class-pair launch with caller-owned scratch: the segment goes by value
-// to *d_seg, then the class kernel runs on it.  task0: {0, count} as written
-// by the row-prefix kernel (row classes) or the run scan (run classes).
-int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg& seg, JKSeg* d_seg,
-                       const long long* task0, long long max_tasks, void* stream);
-// run table of the class pair as bra at the per-class-pair entries' run
-// length; 0 rows if the class quartet does not run a run kernel
-struct JKRunTab {
-    int nrun, chunk;  // runs, ket pairs of an item
-    int bucket, n_kl;
-    const int *ent, *erank, *run0;
-};
-int jk_internal_run_table(const jk_basis_t* b, int cp_ij, int cp_kl, JKRunTab* out);
-// item counts per run from the entries' ket ends (ioff[0..nrun)), then their
-// exclusive prefix in place and itm = {0, total}
-int jk_internal_run_items(const JKRunTab& rt, const int* ehi, long long* ioff, long long* itm, void* stream);
+// Class kernel of the per-class-pair entries on the segment at d_seg (device).
+// task0: {0, count} as the preparation kernels wrote it.
+int jk_internal_launch(const jk_basis_t* b, int cp_ij, int cp_kl, const JKSeg* d_seg, const long long* task0,
+                       long long max_tasks, int n_dm, void* stream);
+// completes the segment of a run class (seg->nrun > 0 on return, its ehi and
+// ioff in the caller's buffers) at the per-class-pair entries' run length, and
+// gives the ranks of the run entries; false for a row class
+bool jk_internal_pair_runs(const jk_basis_t* b, int cp_ij, int cp_kl, JKSeg* seg, int* ehi, long long* ioff,
+                           const int** erank, int* chunk);
+// for many bra pairs, in place of jk_pair_prep_kernel: item counts per run from
+// the entries' ket ends, their exclusive prefix, itm = {0, total}, and the
+// segment to *d_seg
+int jk_internal_run_items(const JKSeg& seg, int chunk, long long* itm, JKSeg* d_seg, void* stream);
+#define JK_PAIR_PREP_ROWS 8192  // bra pairs up to which one block prepares a call
 
 // Side streams of the class launches.  Every class kernel adds into J and K
 // with atomics, so launches of different class quartets (and the FP64 and
@@ -135,9 +133,11 @@ struct JKPackMol {
 };
 
 // run lengths a run table exists for: long runs save more traffic, short ones
-// give a small molecule enough items to fill the device
+// give a small molecule enough items to fill the device.  The per-class-pair
+// entries, whose launch has the device to itself, go down to single pairs.
 #define JK_RUN_LEVELS 3
-static const int JK_RUN_LEN[JK_RUN_LEVELS] = {32, 8, 2};
+#define JK_RUN_LEVELS_PAIR 4
+static const int JK_RUN_LEN[JK_RUN_LEVELS_PAIR] = {32, 8, 2, 1};
 
 // Class launches of a set of class quartets: one key per class (for the team
 // kernels per class and pair of primitive counts), its class quartets as
@@ -200,7 +200,7 @@ struct jk_basis {
     // Runs of the bra pairs of each class (jk_runs.cuh): entry e of class c is
     // pair d_ent[pair_locs[c] + e] (a position) of the class; run table v (run length
     // JK_RUN_LEN[v]) of class c has h_nrun[v][c] runs at d_run0 + h_run_off[v][c]
-    std::vector<int> h_nrun[JK_RUN_LEVELS], h_run_off[JK_RUN_LEVELS];
+    std::vector<int> h_nrun[JK_RUN_LEVELS_PAIR], h_run_off[JK_RUN_LEVELS_PAIR];
     int *d_ent = nullptr, *d_run0 = nullptr;
     int* d_inv = nullptr;  // entry of a pair (the inverse of d_ent)
     int* d_erank = nullptr;  // Schwarz rank of an entry

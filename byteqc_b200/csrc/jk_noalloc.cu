@@ -33,6 +33,7 @@
 #include <mutex>
 
 #include "jk_internal.h"
+#include "jk_pair.cuh"
 
 #define JK_NA_MAX_ROWS (1 << 17)  // shell pairs of the ij class
 #define JK_NA_MAX_BINS 1024
@@ -88,17 +89,25 @@ __device__ __forceinline__ int na_cols(const int* __restrict__ bins_ij, const in
     return cnt;
 }
 
-// run classes: ket end of every entry
-__global__ void jk_na_ehi_kernel(const int* __restrict__ bins_ij, const int* __restrict__ bins_kl, int nbins, int n_ij,
-                                 int n_kl, int diag, const int* __restrict__ erank, int* __restrict__ ehi) {
+struct JKNaCols {
+    const int *bins_ij, *bins_kl;
+    int nbins, n_kl, diag;
+    __device__ __forceinline__ int operator()(int ij) const {
+        return na_cols(bins_ij, bins_kl, nbins, n_kl, diag, ij);
+    }
+};
+
+// run classes of many bra pairs: ket end of every entry
+__global__ void jk_na_ehi_kernel(const JKNaCols cols, int n_ij, const int* __restrict__ erank, int* __restrict__ ehi) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < n_ij) ehi[e] = na_cols(bins_ij, bins_kl, nbins, n_kl, diag, erank[e]);
+    if (e < n_ij) ehi[e] = cols(erank[e]);
 }
 
-// row classes: one block; writes qoff[0..n_ij] and task0 = {0, total}
+// row classes: one block; writes qoff[0..n_ij], task0 = {0, total} and the segment
 __global__ void jk_na_qoff_kernel(const int* __restrict__ bins_ij, const int* __restrict__ bins_kl, int nbins,
                                   int n_ij, int n_kl, int diag, long long* __restrict__ qoff,
-                                  long long* __restrict__ task0) {
+                                  long long* __restrict__ task0, const __grid_constant__ JKSeg sg, JKSeg* dst) {
+    jk_seg_copy(sg, dst);
     __shared__ long long carry;
     __shared__ long long wsum[32];
     if (threadIdx.x == 0) {
@@ -171,29 +180,30 @@ extern "C" int jk_build_class_pair_noalloc(jk_basis_t* b, double* vj, double* vk
     if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
     const int diag = cp_ij == cp_kl;
     long long max_tasks;
-    JKRunTab rt;
-    if (jk_internal_run_table(b, cp_ij, cp_kl, &rt)) {
+    JKSeg* d_seg = (JKSeg*)(sc + JK_NA_OFF_SEG);
+    int* d_ehi = (int*)(sc + JK_NA_OFF_EHI);
+    const int* erank;
+    int chunk;
+    if (jk_internal_pair_runs(b, cp_ij, cp_kl, &seg, d_ehi, d_qoff, &erank, &chunk)) {
         if (n_ij == 0 || n_kl == 0) return JK_OK;
-        int* d_ehi = (int*)(sc + JK_NA_OFF_EHI);
-        jk_na_ehi_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(d_bins_ij, d_bins_kl, nbins, n_ij, n_kl, diag, rt.erank,
-                                                             d_ehi);
+        const JKNaCols cols{d_bins_ij, d_bins_kl, nbins, n_kl, diag};
+        if (n_ij <= JK_PAIR_PREP_ROWS)
+            jk_pair_prep_kernel<<<1, jk_pair_prep_threads(seg.nrun), 0, st>>>(cols, seg, d_seg, erank, chunk, d_ehi, d_qoff, d_task0);
+        else
+            jk_na_ehi_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(cols, n_ij, erank, d_ehi);
         e = cudaGetLastError();
         if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
-        rc = jk_internal_run_items(rt, d_ehi, d_qoff, d_task0, stream);
+        if (n_ij > JK_PAIR_PREP_ROWS) rc = jk_internal_run_items(seg, chunk, d_task0, d_seg, stream);
         if (rc) return rc;
-        seg.nrun = rt.nrun;
-        seg.ent = rt.ent;
-        seg.run0 = rt.run0;
-        seg.ehi = d_ehi;
-        seg.ioff = d_qoff;
-        max_tasks = (long long)rt.nrun * ((n_kl + rt.chunk - 1) / rt.chunk);
+        max_tasks = (long long)seg.nrun * ((n_kl + chunk - 1) / chunk);
     } else {
-        jk_na_qoff_kernel<<<1, 1024, 0, st>>>(d_bins_ij, d_bins_kl, nbins, n_ij, n_kl, diag, d_qoff, d_task0);
+        jk_na_qoff_kernel<<<1, 1024, 0, st>>>(d_bins_ij, d_bins_kl, nbins, n_ij, n_kl, diag, d_qoff, d_task0, seg,
+                                              d_seg);
         e = cudaGetLastError();
         if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
         max_tasks = diag ? (long long)n_ij * (n_ij + 1) / 2 : (long long)n_ij * n_kl;
     }
-    rc = jk_internal_launch(b, cp_ij, cp_kl, seg, (JKSeg*)(sc + JK_NA_OFF_SEG), d_task0, max_tasks, stream);
+    rc = jk_internal_launch(b, cp_ij, cp_kl, d_seg, d_task0, max_tasks, n_dm, stream);
     if (rc) return rc;
     // same synchronous contract as jk_build_class_pair
     e = cudaStreamSynchronize(st);

@@ -21,7 +21,7 @@ def _setup(n, bas, n_dm=1):
     if bas == 'tzvp+g':
         bas = {'O': basis.load('standin-def2-tzvp', 'O') + [[4, [1.2, 1.0]]],
                'H': basis.load('standin-def2-tzvp', 'H')}
-    mol = Mole(atom=geom.water_cluster(n, box=3.0 + n, seed=n),
+    mol = Mole(atom=geom.water_cluster(n, box=min(3.0 + n, 11.0), seed=n),
                basis=bas).build()
     opt = hf._VHFOpt(mol).build()
     rng = np.random.default_rng(5)
@@ -86,7 +86,9 @@ def test_class_pair_k_blocks(entry, n_dm):
     assert len(seen) > 20
 
 
-@pytest.mark.parametrize('bas,n', [('standin-cc-pvdz', 3), ('tzvp+g', 1)])
+@pytest.mark.parametrize('bas,n', [
+    ('standin-cc-pvdz', 3), ('tzvp+g', 1),
+    ('standin-cc-pvdz', 22)])  # classes of more than 8192 pairs
 @pytest.mark.parametrize('cutoff', [0., 1e-3])
 def test_raw_entries_agree(bas, n, cutoff):
     """jk_build, the same without J as a captured build whose K buffer was
@@ -96,6 +98,7 @@ def test_raw_entries_agree(bas, n, cutoff):
     from byteqc_b200.cuobc import lib as jklib
     lib = jklib.load_library()
     opt, d = _setup(n, bas, 2)
+    assert n < 22 or max(len(q) for q in opt.log_qs) > 8192
     rj, rk = _class_pairs(opt, d, lib.jk_build_class_pair)
     base = torch.randn_like(d)
     tol = 1e-10 if cutoff == 0. else 1e-4  # FP32 quartets up to 1e-3 each
@@ -151,3 +154,30 @@ def test_class_pair_without_densities_adds_nothing():
         return lib.jk_build_class_pair(handle, vj, vk, dm, nao, 0, *a)
     vj, vk = _class_pairs(opt, d, fn)
     assert not vj.any().item() and not vk.any().item()
+
+
+@pytest.mark.parametrize('bas', ['standin-cc-pvdz', 'tzvp+g'])
+def test_class_pair_call_is_two_launches(bas):
+    """A per-class-pair call of a small molecule is one preparation and one
+    class kernel: its latency is what such a call costs (five launches took
+    1.6 times as long for 13 atoms / TZVP)."""
+    import torch
+    from cuda.bindings import runtime as cudart
+    from byteqc_b200.cuobc import lib as jklib
+    lib = jklib.load_library()
+    opt, d = _setup(1, bas)
+    vj, vk = torch.zeros_like(d), torch.zeros_like(d)
+    _class_pairs(opt, d, lib.jk_build_class_pair)
+    for cij in range(len(opt.log_qs)):
+        bij = np.array([0, len(opt.log_qs[cij])], np.int32)
+        g, s = torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.graph(g, stream=s):
+            assert lib.jk_build_class_pair(
+                opt.handle, vj.data_ptr(), vk.data_ptr(), d.data_ptr(),
+                opt.nao, 1, bij.ctypes.data, bij.ctypes.data, 1, cij, cij,
+                ctypes.c_void_p(s.cuda_stream)) == 0
+        err, _, n = cudart.cudaGraphGetNodes(
+            cudart.cudaGraph_t(g.raw_cuda_graph()), 0)
+        assert err == cudart.cudaError_t.cudaSuccess
+        assert n == 2
