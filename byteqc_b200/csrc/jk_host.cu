@@ -395,35 +395,81 @@ __global__ void __launch_bounds__(1024) jk_run_scan1_kernel(const __grid_constan
     jk_run_scan_body(sg.nrun, ioff, nullptr, itm, nullptr);
 }
 
-// bra records of the run kernels (JKSeg::bprim, bprimf, bpair) of one class,
-// gathered in run-entry order
-__global__ void jk_bra_records_kernel(int np, int nprim, const int* __restrict__ ent, const double* __restrict__ prim,
-                                      const float* __restrict__ primf, long long n, const double* __restrict__ pgeo,
-                                      const int* __restrict__ pao, const int* __restrict__ pnp, int npt,
-                                      double* __restrict__ bprim, float* __restrict__ bprimf,
-                                      double* __restrict__ bpair) {
-    // prim, primf: first primitive of the class in the SoA arrays of stride n;
-    // pgeo, pao, pnp: its first pair in the arrays of stride npt
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < np * nprim; t += gridDim.x * blockDim.x) {
-        const int k = t / np, e = t - k * np, r = ent[e];
-        const double* s = prim + (size_t)k * np + r;
-        const float* f = primf + (size_t)k * np + r;
-        double* d = bprim + (size_t)t * 8;
-        float* g = bprimf + (size_t)t * 8;
-        d[0] = s[0];
-        d[1] = s[5 * n];
-        d[2] = s[n] * s[5 * n];
-        d[3] = s[2 * n];
-        d[4] = s[3 * n];
-        d[5] = s[4 * n];
-        d[6] = d[7] = 0.;
-        for (int x = 0; x < 6; x++) g[x] = f[x * n];
-        g[6] = g[7] = 0.f;
-        if (k == 0) {
-            double* b = bpair + (size_t)e * 4;
-            for (int x = 0; x < 3; x++) b[x] = pgeo[(size_t)(3 + x) * npt + r];
-            b[3] = __hiloint2double(pnp[r], pao[npt + r]);
-        }
+// last index i in [0, n] with off[i] <= t (off non-decreasing, off[0] <= t)
+__device__ __forceinline__ int jk_slot(const int* __restrict__ off, int n, int t) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(off + mid) <= t) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+// What follows of the uploaded lists per pair (set-up, one thread per pair): the
+// geometry, the inverses of the two orders, the entries' ranks and the log q
+// clipped at 0.  Uploaded, these were two thirds of the bytes of a set-up.
+__global__ void __launch_bounds__(256) jk_pair_tables_kernel(int npair, int ncp, const int* __restrict__ locs,
+                                                             const int* __restrict__ bra, const int* __restrict__ ket,
+                                                             const int* __restrict__ rank, const int* __restrict__ ent,
+                                                             const double* __restrict__ bx, int nbas,
+                                                             const int* __restrict__ ao_loc,
+                                                             const double* __restrict__ raw, double* __restrict__ lq,
+                                                             double* __restrict__ geo, int* __restrict__ pao,
+                                                             int* __restrict__ pos, int* __restrict__ inv,
+                                                             int* __restrict__ erank) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= npair) return;
+    const int p0 = __ldg(locs + jk_slot(locs, ncp, p)), x = p - p0, e = ent[p];
+    pos[p0 + rank[p]] = x;
+    inv[p0 + e] = x;
+    erank[p] = rank[p0 + e];
+    lq[p] = raw[p] > 0. ? 0. : raw[p];
+    const int sh[2] = {bra[p], ket[p]};
+    for (int a = 0; a < 2; a++) {
+        for (int d = 0; d < 3; d++) geo[(size_t)(3 * a + d) * npair + p] = bx[(size_t)d * nbas + sh[a]];
+        pao[(size_t)a * npair + p] = ao_loc[sh[a]];
+    }
+}
+
+// ... and per primitive pair: 1 / a12, the single-precision copy, and the bra
+// records of the run kernels (JKSeg::bprim, bprimf, bpair), gathered in
+// run-entry order.  prim: a12 | e12 | x12 | y12 | z12 | 1 / a12, stride n; primitive
+// k of position r of class c at plocs[c] + k * (pairs of c) + r.
+__global__ void __launch_bounds__(256) jk_prim_tables_kernel(int n, int npair, int ncp, const int* __restrict__ locs,
+                                                             const int* __restrict__ plocs, double* __restrict__ prim,
+                                                             float* __restrict__ primf, const int* __restrict__ inv,
+                                                             const double* __restrict__ geo,
+                                                             const int* __restrict__ pao, const int* __restrict__ pnp,
+                                                             double* __restrict__ bprim, float* __restrict__ bprimf,
+                                                             double* __restrict__ bpair) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const size_t N = n;
+    const int c = jk_slot(plocs, ncp, t), q0 = __ldg(plocs + c), p0 = __ldg(locs + c), np = __ldg(locs + c + 1) - p0;
+    const int k = (t - q0) / np, p = p0 + (t - q0) - k * np, e = inv[p];
+    const double a = prim[t], ia = 1. / a, e12 = prim[N + t];
+    prim[5 * N + t] = ia;
+    double* d = bprim + ((size_t)q0 + (size_t)k * np + e) * 8;
+    float* g = bprimf + ((size_t)q0 + (size_t)k * np + e) * 8;
+    d[0] = a;
+    d[1] = ia;
+    d[2] = e12 * ia;
+    primf[t] = g[0] = (float)a;
+    primf[N + t] = g[1] = (float)ia;
+    primf[2 * N + t] = g[2] = (float)(e12 / a);
+    for (int x = 0; x < 3; x++) {
+        // the product centre; single precision keeps it relative to the bra
+        // shell's, so that the small differences P - R_i keep their precision
+        const double P = prim[(2 + x) * N + t];
+        d[3 + x] = P;
+        primf[(3 + x) * N + t] = g[3 + x] = (float)(P - geo[(size_t)x * npair + p]);
+    }
+    d[6] = d[7] = 0.;
+    g[6] = g[7] = 0.f;
+    if (k == 0) {
+        double* b = bpair + ((size_t)p0 + e) * 4;
+        for (int x = 0; x < 3; x++) b[x] = geo[(size_t)(3 + x) * npair + p];
+        b[3] = __hiloint2double(pnp[p], pao[(size_t)npair + p]);
     }
 }
 
@@ -564,47 +610,12 @@ __global__ void __launch_bounds__(256) jk_symmetrize_kernel(const double* __rest
 
 static void free_basis(jk_basis* b) {
     if (!b) return;
-    cudaFree(b->d_atm);
-    cudaFree(b->d_bas);
-    cudaFree(b->d_ao_loc);
-    cudaFree(b->d_group_ao);
-    cudaFree(b->d_env);
-    cudaFree(b->d_bas_x);
-    cudaFree(b->d_qcond);
-    cudaFree(b->d_pair2bra);
-    cudaFree(b->d_pair2ket);
-    cudaFree(b->d_log_q);
-    cudaFree(b->d_log_q_raw);
-    cudaFree(b->d_qoff32);
-    cudaFree(b->d_klb);
-    cudaFree(b->d_kle);
-    cudaFree(b->d_ioff);
-    cudaFree(b->d_zero);
-    cudaFree(b->d_ent);
-    cudaFree(b->d_inv);
-    cudaFree(b->d_erank);
-    cudaFree(b->d_rank);
-    cudaFree(b->d_pos);
-    cudaFree(b->d_bprim);
-    cudaFree(b->d_bprimf);
-    cudaFree(b->d_bpair);
-    cudaFree(b->d_run0);
-    cudaFree(b->d_ehi1);
-    cudaFree(b->d_seg1);
+    cudaFree(b->mem_bas);
+    cudaFree(b->mem_pair);
     jk_plan_free(b->plan);
     for (auto& p : b->shard_plans) jk_plan_free(p.second);
     for (void* p : b->retired) cudaFree(p);
-    cudaFree(b->d_prim);
-    cudaFree(b->d_primf);
-    cudaFree(b->d_cq);
-    cudaFree(b->d_qoff);
-    cudaFree(b->d_qoff1);
-    cudaFree(b->d_task01);
     cudaFree(b->d_work);
-    cudaFree(b->d_pack);
-    cudaFree(b->d_pgeo);
-    cudaFree(b->d_pnp);
-    cudaFree(b->d_pao);
     b->fan.destroy();
     cudaFree(b->d_pk);
     cudaFree(b->d_kt);
@@ -612,13 +623,52 @@ static void free_basis(jk_basis* b) {
     delete b;
 }
 
-template <typename T>
-static cudaError_t upload(T** dst, const T* src, size_t n) {
-    cudaError_t e = cudaMalloc((void**)dst, sizeof(T) * (n ? n : 1));
-    if (e != cudaSuccess) return e;
-    if (n) e = cudaMemcpy(*dst, src, sizeof(T) * n, cudaMemcpyHostToDevice);
-    return e;
-}
+// Arrays of one set-up step in one device allocation: a request per array, the
+// ones with contents uploaded, small ones together (a basis made some forty
+// allocations and thirty copies, about 10 us each, and as many frees).
+struct JKArena {
+    struct Item {
+        void** dst;
+        const void* src;
+        size_t src_bytes, off;
+    };
+    std::vector<Item> items;
+    size_t total = 0;
+    // n elements at *dst, the first nsrc from src (all of them by default)
+    template <typename T>
+    void add(T** dst, size_t n, const T* src = nullptr, size_t nsrc = (size_t)-1) {
+        const size_t k = src ? std::min(n, nsrc) : 0;
+        items.push_back({(void**)dst, src, k * sizeof(T), total});
+        total += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
+    }
+    cudaError_t commit(void** mem) {
+        cudaError_t e = cudaMalloc(mem, total);
+        if (e != cudaSuccess) return e;
+        std::vector<char> stage;  // neighbouring small items
+        size_t at = 0;
+        auto flush = [&] {
+            if (!stage.empty())
+                e = cudaMemcpyAsync((char*)*mem + at, stage.data(), stage.size(), cudaMemcpyHostToDevice,
+                                    cudaStreamLegacy);
+            stage.clear();
+        };
+        for (const Item& it : items) {
+            *it.dst = (char*)*mem + it.off;
+            if (it.src_bytes == 0 || it.src_bytes > 65536) {
+                flush();
+                if (e == cudaSuccess && it.src_bytes)
+                    e = cudaMemcpyAsync(*it.dst, it.src, it.src_bytes, cudaMemcpyHostToDevice, cudaStreamLegacy);
+            } else {
+                if (stage.empty()) at = it.off;
+                stage.resize(it.off - at + it.src_bytes);
+                memcpy(stage.data() + (it.off - at), it.src, it.src_bytes);
+            }
+            if (e != cudaSuccess) return e;
+        }
+        flush();
+        return e == cudaSuccess ? jk_internal_uploaded() : e;
+    }
+};
 
 extern "C" int jk_rys_table_uniform(void);
 extern "C" const double* jk_rys_coef_host(long long* count);
@@ -706,13 +756,8 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         b->h_group_nprim.push_back(np);
     }
     // device copies of the basis
-    CUDA_TRY(upload(&b->d_atm, atm, (size_t)natm * ATM_SLOTS));
-    CUDA_TRY(upload(&b->d_bas, bas, (size_t)nbas * BAS_SLOTS));
-    CUDA_TRY(upload(&b->d_env, env, (size_t)nenv));
-    CUDA_TRY(upload(&b->d_ao_loc, b->h_ao_loc.data(), b->h_ao_loc.size()));
     std::vector<int> gao(ngroups + 1);
     for (int g = 0; g <= ngroups; g++) gao[g] = b->h_ao_loc[group_off[g]];
-    CUDA_TRY(upload(&b->d_group_ao, gao.data(), gao.size()));
     std::vector<double> bx(3 * (size_t)nbas);
     for (int i = 0; i < nbas; i++) {
         const double* r = env + atm[bas[i * BAS_SLOTS + ATOM_OF] * ATM_SLOTS + PTR_COORD];
@@ -720,11 +765,18 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         bx[nbas + i] = r[1];
         bx[2 * (size_t)nbas + i] = r[2];
     }
-    CUDA_TRY(upload(&b->d_bas_x, bx.data(), bx.size()));
+    CUDA_TRY(b->fan.init());
+    JKArena bas_mem;
+    bas_mem.add(&b->d_env, nenv, env);
+    bas_mem.add(&b->d_bas_x, bx.size(), bx.data());
+    bas_mem.add(&b->d_atm, (size_t)natm * ATM_SLOTS, atm);
+    bas_mem.add(&b->d_bas, (size_t)nbas * BAS_SLOTS, bas);
+    bas_mem.add(&b->d_ao_loc, b->h_ao_loc.size(), b->h_ao_loc.data());
+    bas_mem.add(&b->d_group_ao, gao.size(), gao.data());
+    CUDA_TRY(bas_mem.commit(&b->mem_bas));
 
-    // Schwarz matrix on the device
-    CUDA_TRY(cudaMalloc(&b->d_qcond, sizeof(double) * (size_t)nbas * nbas));
-    CUDA_TRY(cudaMemset(b->d_qcond, 0, sizeof(double) * (size_t)nbas * nbas));
+    // Schwarz matrix on the device, the pairs by their two l, a launch each
+    b->h_qcond.resize((size_t)nbas * nbas);
     {
         std::vector<int> pi[JK_LMAX_ALL + 1][JK_LMAX_ALL + 1], pj[JK_LMAX_ALL + 1][JK_LMAX_ALL + 1];
         for (int i = 0; i < nbas; i++)
@@ -733,56 +785,96 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
                 if (li >= lj) { pi[li][lj].push_back(i); pj[li][lj].push_back(j); }
                 else { pi[lj][li].push_back(j); pj[lj][li].push_back(i); }
             }
+        double* d_q;
+        int *dpi[JK_LMAX_ALL + 1][JK_LMAX_ALL + 1], *dpj[JK_LMAX_ALL + 1][JK_LMAX_ALL + 1];
+        JKArena mem;
+        mem.add(&d_q, (size_t)nbas * nbas);
         for (int a = 0; a <= JK_LMAX_ALL; a++)
             for (int c = 0; c <= a; c++) {
-                int n = (int)pi[a][c].size();
-                if (!n) continue;
-                int *dpi, *dpj;
-                CUDA_TRY(upload(&dpi, pi[a][c].data(), n));
-                CUDA_TRY(upload(&dpj, pj[a][c].data(), n));
-                if (a <= JK_LMAX)
-                    g_qcond[a][c](dpi, dpj, n, b->d_atm, b->d_bas, b->d_env, nbas, b->d_qcond, b->rys, 0);
-                else
-                    jk_qcond_generic(dpi, dpj, n, b->d_atm, b->d_bas, b->d_env, nbas, b->d_qcond, b->rys, a, 0);
-                cudaError_t e = cudaGetLastError();
-                if (e == cudaSuccess) e = cudaDeviceSynchronize();
-                cudaFree(dpi);
-                cudaFree(dpj);
-                CUDA_TRY(e);
+                if (pi[a][c].empty()) continue;
+                mem.add(&dpi[a][c], pi[a][c].size(), pi[a][c].data());
+                mem.add(&dpj[a][c], pj[a][c].size(), pj[a][c].data());
             }
-        b->h_qcond.resize((size_t)nbas * nbas);
-        CUDA_TRY(cudaMemcpy(b->h_qcond.data(), b->d_qcond, sizeof(double) * (size_t)nbas * nbas,
-                            cudaMemcpyDeviceToHost));
+        void* tmp = nullptr;
+        cudaError_t e = mem.commit(&tmp);
+        int k = 0;
+        for (int a = JK_LMAX_ALL; a >= 0 && e == cudaSuccess; a--)
+            for (int c = a; c >= 0 && e == cudaSuccess; c--) {
+                const int n = (int)pi[a][c].size();
+                if (!n) continue;
+                cudaStream_t st = b->fan.pick(k++);
+                if (a <= JK_LMAX)
+                    g_qcond[a][c](dpi[a][c], dpj[a][c], n, b->d_atm, b->d_bas, b->d_env, nbas, d_q, b->rys, st);
+                else
+                    jk_qcond_generic(dpi[a][c], dpj[a][c], n, b->d_atm, b->d_bas, b->d_env, nbas, d_q, b->rys, a, st);
+                e = cudaGetLastError();
+            }
+        for (int x = 0; x < JK_SIDE_STREAMS; x++) {  // also after an error: tmp is freed below
+            const cudaError_t es = cudaStreamSynchronize(b->fan.s[x]);
+            if (e == cudaSuccess) e = es;
+        }
+        if (e == cudaSuccess)
+            e = cudaMemcpy(b->h_qcond.data(), d_q, sizeof(double) * (size_t)nbas * nbas, cudaMemcpyDeviceToHost);
+        cudaFree(tmp);
+        CUDA_TRY(e);
     }
     // Schwarz-sorted pair lists per lower-triangular group pair, in the
     // reference's class order (cuobc/scf/hf.py:343-389)
     const std::vector<double>& q = b->h_qcond;
     b->h_pair_locs.push_back(0);
-    for (int gi = 0; gi < ngroups; gi++) {
-        for (int gj = 0; gj <= gi; gj++) {
-            std::vector<std::pair<double, long long>> lst;
-            int p0 = group_off[gi], p1 = group_off[gi + 1], q0 = group_off[gj], q1 = group_off[gj + 1];
-            for (int i = p0; i < p1; i++)
-                for (int j = q0; j < q1; j++) {
-                    if (gi == gj && !diag_block_with_triu && j > i) continue;
-                    double v = q[(size_t)i * nbas + j];
-                    if (v > cutoff) lst.push_back({v, (long long)i * nbas + j});
+    std::vector<int> obra, oket, orank, opos;  // device order, see below
+    {
+        struct Cand {
+            double q;
+            int at;  // place in (bra shell, ket shell) order
+        };
+        std::vector<Cand> lst;
+        std::vector<int> sh_i, sh_j, rank_of, fill;
+        for (int gi = 0; gi < ngroups; gi++)
+            for (int gj = 0; gj <= gi; gj++) {
+                lst.clear();
+                sh_i.clear();
+                sh_j.clear();
+                int p0 = group_off[gi], p1 = group_off[gi + 1], q0 = group_off[gj], q1 = group_off[gj + 1];
+                for (int i = p0; i < p1; i++)
+                    for (int j = q0; j < q1; j++) {
+                        if (gi == gj && !diag_block_with_triu && j > i) continue;
+                        double v = q[(size_t)i * nbas + j];
+                        if (v > cutoff) {
+                            lst.push_back({v, (int)sh_i.size()});
+                            sh_i.push_back(i);
+                            sh_j.push_back(j);
+                        }
+                    }
+                std::stable_sort(lst.begin(), lst.end(), [](const Cand& x, const Cand& y) { return x.q > y.q; });
+                const int np = (int)lst.size(), at0 = b->h_pair_locs.back(), S = sort_bucket(np);
+                rank_of.resize(np);
+                for (int x = 0; x < np; x++) {
+                    const Cand& c = lst[x];
+                    rank_of[c.at] = x;
+                    b->h_pair2bra.push_back(sh_i[c.at]);
+                    b->h_pair2ket.push_back(sh_j[c.at]);
+                    double lq = log(c.q);
+                    b->h_log_q.push_back(lq > 0 ? 0 : lq);
+                    b->h_log_q_raw.push_back(lq);
                 }
-            std::stable_sort(lst.begin(), lst.end(),
-                             [](const std::pair<double, long long>& x, const std::pair<double, long long>& y) {
-                                 return x.first > y.first;
-                             });
-            for (auto& e : lst) {
-                b->h_pair2bra.push_back((int)(e.second / nbas));
-                b->h_pair2ket.push_back((int)(e.second % nbas));
-                double lq = log(e.first);
-                b->h_log_q.push_back(lq > 0 ? 0 : lq);
-                b->h_log_q_raw.push_back(lq);
+                // the pairs in shell order, each to the end of its rank's bucket
+                fill.assign(np / S + 1, 0);
+                obra.resize(at0 + np);
+                oket.resize(at0 + np);
+                orank.resize(at0 + np);
+                opos.resize(at0 + np);
+                for (int y = 0; y < np; y++) {
+                    const int x = rank_of[y], k = x / S, pos = k * S + fill[k]++;
+                    orank[at0 + pos] = x;
+                    opos[at0 + x] = pos;
+                    obra[at0 + pos] = sh_i[y];
+                    oket[at0 + pos] = sh_j[y];
+                }
+                b->h_cls_gi.push_back(gi);
+                b->h_cls_gj.push_back(gj);
+                b->h_pair_locs.push_back(at0 + np);
             }
-            b->h_cls_gi.push_back(gi);
-            b->h_cls_gj.push_back(gj);
-            b->h_pair_locs.push_back((int)b->h_pair2bra.size());
-        }
     }
     b->ncp = (int)b->h_cls_gi.size();
     // Device order of a class's pairs: buckets of sort_bucket(pairs)
@@ -794,24 +886,6 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
     // end of a row (6 %).  The lists that the C-ABI gives out stay in rank
     // order, as do log q and the screening.
     const size_t npair = b->h_pair2bra.size();
-    std::vector<int> obra(npair), oket(npair), orank(npair), opos(npair);
-    for (int c = 0; c < b->ncp; c++) {
-        const int p0 = b->h_pair_locs[c], np = b->h_pair_locs[c + 1] - p0, S = sort_bucket(np);
-        int* r = orank.data() + p0;
-        std::vector<std::pair<long long, int>> key(S);  // (shells, rank) of one bucket
-        for (int x = 0; x < np; x += S) {
-            const int n = std::min(np - x, S);
-            for (int y = 0; y < n; y++)
-                key[y] = {(long long)b->h_pair2bra[p0 + x + y] * nbas + b->h_pair2ket[p0 + x + y], x + y};
-            std::sort(key.begin(), key.begin() + n);
-            for (int y = 0; y < n; y++) r[x + y] = key[y].second;
-        }
-        for (int x = 0; x < np; x++) {
-            opos[p0 + r[x]] = x;
-            obra[p0 + x] = b->h_pair2bra[p0 + r[x]];
-            oket[p0 + x] = b->h_pair2ket[p0 + r[x]];
-        }
-    }
     // primitive-pair data (cuobc/lib/gint/pair_data.c:83-141)
     long long npp = 0;
     b->h_prim_locs.push_back(0);
@@ -822,13 +896,9 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         b->h_prim_locs.push_back((int)npp);
     }
     b->nprim_total = npp;
-    std::vector<double> prim(6 * (size_t)(npp ? npp : 1));
+    std::vector<double> prim(5 * (size_t)(npp ? npp : 1));  // 1 / a12 and the rest of the tables: on the device
     double *a12 = prim.data(), *e12 = a12 + npp, *x12 = e12 + npp, *y12 = x12 + npp, *z12 = y12 + npp;
-    double* ia12 = z12 + npp;
-    // single-precision copy for the FP32 quartets of the mixed mode; the
-    // product centre is stored relative to the bra shell's centre so that
-    // the small differences P - R_i keep their relative precision
-    std::vector<float> primf(6 * (size_t)(npp ? npp : 1));
+    std::vector<std::pair<int, int>> order;
     b->h_pnp.assign(std::max<size_t>(b->h_pair2bra.size(), 1), 0);
     for (int c = 0; c < b->ncp; c++) {
         // primitive-major within the class: primitive k of pair r at
@@ -852,7 +922,7 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             // (the run kernels loop over those only; the others carry a
             // factor below 1e-26 and are kept after them for the kernels
             // that loop over all)
-            std::vector<std::pair<int, int>> order;
+            order.clear();
             for (int pass = 0; pass < 2; pass++)
                 for (int ip = 0; ip < npi; ip++)
                     for (int jp = 0; jp < npj; jp++) {
@@ -866,103 +936,49 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
                 {
                     double aij = ai[ip] + aj[jp];
                     a12[off] = aij;
-                    ia12[off] = 1. / aij;
                     e12[off] = norm * ci[ip] * cj[jp] * exp(-r2 * ai[ip] * aj[jp] / aij);
                     if (ish == jsh) e12[off] *= b->diag_fac;
                     x12[off] = (ai[ip] * ri[0] + aj[jp] * rj[0]) / aij;
                     y12[off] = (ai[ip] * ri[1] + aj[jp] * rj[1]) / aij;
                     z12[off] = (ai[ip] * ri[2] + aj[jp] * rj[2]) / aij;
-                    primf[off] = (float)aij;
-                    primf[npp + off] = (float)(1. / aij);
-                    primf[2 * npp + off] = (float)(e12[off] / aij);
-                    // P - R_i = aj (R_j - R_i) / (ai + aj)
-                    primf[3 * npp + off] = (float)(aj[jp] * (rj[0] - ri[0]) / aij);
-                    primf[4 * npp + off] = (float)(aj[jp] * (rj[1] - ri[1]) / aij);
-                    primf[5 * npp + off] = (float)(aj[jp] * (rj[2] - ri[2]) / aij);
                 }
                 off += pst;
             }
         }
     }
-    CUDA_TRY(upload(&b->d_pnp, b->h_pnp.data(), b->h_pnp.size()));
-    CUDA_TRY(upload(&b->d_prim, prim.data(), prim.size()));
-    CUDA_TRY(upload(&b->d_primf, primf.data(), primf.size()));
-    {
-        // pair geometry: the two shells' centres and first AOs per pair
-        const size_t np = b->h_pair2bra.size();
-        std::vector<double> geo(6 * (np ? np : 1));
-        std::vector<int> pao(2 * (np ? np : 1));
-        for (size_t p = 0; p < np; p++) {
-            const int sh[2] = {obra[p], oket[p]};
-            for (int a = 0; a < 2; a++) {
-                for (int d = 0; d < 3; d++) geo[(3 * a + d) * np + p] = bx[(size_t)d * nbas + sh[a]];
-                pao[a * np + p] = b->h_ao_loc[sh[a]];
-            }
-        }
-        CUDA_TRY(upload(&b->d_pgeo, geo.data(), geo.size()));
-        CUDA_TRY(upload(&b->d_pao, pao.data(), pao.size()));
-    }
-    CUDA_TRY(upload(&b->d_pair2bra, obra.data(), npair));
-    CUDA_TRY(upload(&b->d_pair2ket, oket.data(), npair));
-    CUDA_TRY(upload(&b->d_rank, orank.data(), npair));
-    CUDA_TRY(upload(&b->d_pos, opos.data(), npair));
-    CUDA_TRY(upload(&b->d_log_q, b->h_log_q.data(), b->h_log_q.size()));
-    CUDA_TRY(upload(&b->d_log_q_raw, b->h_log_q_raw.data(), b->h_log_q_raw.size()));
     // runs of every class's pairs: the pairs of one first shell, in Schwarz
     // order, cut at each run length
+    std::vector<int> ent(npair), run0;
     {
-        std::vector<int> ent(npair), erank(npair), inv(npair), run0;
         for (int v = 0; v < JK_RUN_LEVELS_PAIR; v++) {
             b->h_nrun[v].assign(b->ncp, 0);
             b->h_run_off[v].assign(b->ncp, 0);
         }
+        // single pairs: run r holds entry r, in every class
+        int mx = 0;
+        for (int c = 0; c < b->ncp; c++) mx = std::max(mx, b->h_pair_locs[c + 1] - b->h_pair_locs[c]);
+        run0.resize(mx + 1);
+        std::iota(run0.begin(), run0.end(), 0);
+        std::vector<int> at(nbas + 1), end(nbas + 1);
         for (int c = 0; c < b->ncp; c++) {
             const int p0 = b->h_pair_locs[c], np = b->h_pair_locs[c + 1] - p0;
+            const int s0 = group_off[b->h_cls_gi[c]], s1 = group_off[b->h_cls_gi[c] + 1];
             int* e = ent.data() + p0;
-            // e: ranks by first shell (counting sort, ranks ascending in a shell)
-            std::vector<int> at(nbas + 1, 0);
+            // e: positions by first shell (counting sort, ranks ascending in a shell)
+            for (int x = s0; x <= s1; x++) at[x] = 0;
             for (int x = 0; x < np; x++) at[b->h_pair2bra[p0 + x] + 1]++;
-            for (int x = 0; x < nbas; x++) at[x + 1] += at[x];
-            for (int x = 0; x < np; x++) e[at[b->h_pair2bra[p0 + x]]++] = x;
-            for (int v = 0; v < JK_RUN_LEVELS_PAIR; v++) {
+            for (int x = s0; x < s1; x++) at[x + 1] += at[x];
+            for (int x = s0; x <= s1; x++) end[x] = at[x];
+            for (int x = 0; x < np; x++) e[at[b->h_pair2bra[p0 + x]]++] = opos[p0 + x];
+            b->h_nrun[JK_RUN_LEVELS_PAIR - 1][c] = np;
+            for (int v = 0; v < JK_RUN_LEVELS_PAIR - 1; v++) {
                 b->h_run_off[v][c] = (int)run0.size();
-                int beg = 0;
-                for (int x = 0; x <= np; x++) {
-                    const bool cut = x == np || x - beg == JK_RUN_LEN[v] ||
-                                     b->h_pair2bra[p0 + e[x]] != b->h_pair2bra[p0 + e[beg]];
-                    if (!cut || x == beg) continue;
-                    run0.push_back(beg);
-                    b->h_nrun[v][c]++;
-                    beg = x;
-                }
+                for (int x = s0; x < s1; x++)
+                    for (int beg = end[x]; beg < end[x + 1]; beg += JK_RUN_LEN[v]) run0.push_back(beg);
+                b->h_nrun[v][c] = (int)run0.size() - b->h_run_off[v][c];
                 run0.push_back(np);
             }
-            for (int x = 0; x < np; x++) {
-                erank[p0 + x] = e[x];
-                e[x] = opos[p0 + e[x]];
-                inv[p0 + e[x]] = x;
-            }
         }
-        CUDA_TRY(upload(&b->d_ent, ent.data(), ent.size()));
-        CUDA_TRY(upload(&b->d_erank, erank.data(), erank.size()));
-        CUDA_TRY(upload(&b->d_run0, run0.data(), run0.size()));
-        CUDA_TRY(upload(&b->d_inv, inv.data(), inv.size()));
-        CUDA_TRY(cudaMalloc(&b->d_bprim, sizeof(double) * 8 * (size_t)std::max(npp, 1LL)));
-        CUDA_TRY(cudaMalloc(&b->d_bprimf, sizeof(float) * 8 * (size_t)std::max(npp, 1LL)));
-        CUDA_TRY(cudaMalloc(&b->d_bpair, sizeof(double) * 4 * std::max<size_t>(ent.size(), 1)));
-        for (int c = 0; c < b->ncp; c++) {
-            const int p0 = b->h_pair_locs[c], np = b->h_pair_locs[c + 1] - p0;
-            if (np == 0) continue;
-            const int nprim = b->h_group_nprim[b->h_cls_gi[c]] * b->h_group_nprim[b->h_cls_gj[c]];
-            const size_t q0 = b->h_prim_locs[c];
-            const int blocks = (int)std::min<long long>(((long long)np * nprim + 255) / 256, (long long)b->nsm * 16);
-            jk_bra_records_kernel<<<blocks, 256>>>(np, nprim, b->d_ent + p0, b->d_prim + q0, b->d_primf + q0, npp,
-                                                   b->d_pgeo + p0, b->d_pao + p0, b->d_pnp + p0,
-                                                   (int)b->h_pair2bra.size(), b->d_bprim + 8 * q0, b->d_bprimf + 8 * q0,
-                                                   b->d_bpair + 4 * (size_t)p0);
-            CUDA_TRY(cudaGetLastError());
-        }
-        CUDA_TRY(cudaStreamSynchronize(0));
     }
     // class quartets (cp_ij >= cp_kl), each with its slices of the screening buffers
     std::vector<long long> qoff_at, ioff_at, ent_at;
@@ -1004,16 +1020,74 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             b->h_cq_cost.push_back(nq * (npq * ((l4[0] + l4[1] + l4[2] + l4[3]) / 2 + 1) * nf + 12. * nf));
         }
     b->ncq = (int)b->h_cq.size();
-    auto atleast1 = [](long long n) { return (size_t)(n > 0 ? n : 1); };
-    CUDA_TRY(cudaMalloc(&b->d_qoff, sizeof(long long) * atleast1(b->qoff_total)));
-    CUDA_TRY(cudaMalloc(&b->d_qoff32, sizeof(long long) * atleast1(b->qoff_total)));
-    CUDA_TRY(cudaMalloc(&b->d_ioff, sizeof(long long) * atleast1(b->ioff_total)));
-    CUDA_TRY(cudaMalloc(&b->d_klb, sizeof(int) * atleast1(b->ent_total)));
-    CUDA_TRY(cudaMalloc(&b->d_kle, sizeof(int) * atleast1(b->ent_total)));
+    // pair-packed layout of the J side (jk_build)
+    b->h_pack.clear();
+    b->pack_total = 0;
+    int mx = 1;  // pairs of the largest class
+    for (int c = 0; c < b->ncp; c++) {
+        JKPackCls k;
+        k.off = b->pack_total;
+        k.pair0 = b->h_pair_locs[c];
+        k.np = b->h_pair_locs[c + 1] - k.pair0;
+        const int li = b->h_group_l[b->h_cls_gi[c]], lj = b->h_group_l[b->h_cls_gj[c]];
+        k.nfi = (li + 1) * (li + 2) / 2;
+        k.nfj = (lj + 1) * (lj + 2) / 2;
+        b->pack_total += (long long)k.np * k.nfi * k.nfj;
+        b->h_pack.push_back(k);
+        mx = std::max(mx, k.np);
+    }
     // the buffers a build clears: condensed density, then {0, count} of the
     // quartets and items of both parts
     b->zero_bytes = sizeof(double) * ((size_t)ngroups * ngroups + 8 * (size_t)b->ncq);
-    CUDA_TRY(cudaMalloc(&b->d_zero, b->zero_bytes));
+    int *d_locs, *d_plocs;
+    unsigned long long* zero;
+    JKArena mem;
+    mem.add(&b->d_prim, 6 * (size_t)npp, prim.data(), 5 * (size_t)npp);
+    mem.add(&b->d_log_q_raw, npair, b->h_log_q_raw.data());
+    mem.add(&b->d_pair2bra, npair, obra.data());
+    mem.add(&b->d_pair2ket, npair, oket.data());
+    mem.add(&b->d_rank, npair, orank.data());
+    mem.add(&b->d_ent, npair, ent.data());
+    mem.add(&b->d_pnp, b->h_pnp.size(), b->h_pnp.data());
+    mem.add(&b->d_run0, run0.size(), run0.data());
+    mem.add(&b->d_pack, b->h_pack.size(), b->h_pack.data());
+    mem.add(&d_locs, b->h_pair_locs.size(), b->h_pair_locs.data());
+    mem.add(&d_plocs, b->h_prim_locs.size(), b->h_prim_locs.data());
+    mem.add(&b->d_log_q, npair);
+    mem.add(&b->d_pos, npair);
+    mem.add(&b->d_inv, npair);
+    mem.add(&b->d_erank, npair);
+    mem.add(&b->d_pgeo, 6 * npair);
+    mem.add(&b->d_pao, 2 * npair);
+    mem.add(&b->d_primf, 6 * (size_t)npp);
+    mem.add(&b->d_bprim, 8 * (size_t)npp);
+    mem.add(&b->d_bprimf, 8 * (size_t)npp);
+    mem.add(&b->d_bpair, 4 * npair);
+    mem.add(&b->d_qoff, (size_t)b->qoff_total);
+    mem.add(&b->d_qoff32, (size_t)b->qoff_total);
+    mem.add(&b->d_ioff, (size_t)b->ioff_total);
+    mem.add(&b->d_klb, (size_t)b->ent_total);
+    mem.add(&b->d_kle, (size_t)b->ent_total);
+    mem.add(&zero, b->zero_bytes / 8);
+    mem.add(&b->d_cq, b->h_cq.size());
+    // the per-class-pair entries: row prefixes sized once for the largest
+    // class, so those calls never free a buffer a queued kernel still reads
+    mem.add(&b->d_task01, 2);
+    mem.add(&b->d_seg1, 1);
+    mem.add(&b->d_qoff1, (size_t)mx + 1);
+    mem.add(&b->d_ehi1, mx);
+    b->qoff1_cap = mx + 1;
+    CUDA_TRY(mem.commit(&b->mem_pair));
+    b->d_zero = zero;
+    if (npair) {
+        jk_pair_tables_kernel<<<(unsigned)((npair + 255) / 256), 256>>>(
+            (int)npair, b->ncp, d_locs, b->d_pair2bra, b->d_pair2ket, b->d_rank, b->d_ent, b->d_bas_x, nbas,
+            b->d_ao_loc, b->d_log_q_raw, b->d_log_q, b->d_pgeo, b->d_pao, b->d_pos, b->d_inv, b->d_erank);
+        jk_prim_tables_kernel<<<(unsigned)((npp + 255) / 256), 256>>>(
+            (int)npp, (int)npair, b->ncp, d_locs, d_plocs, b->d_prim, b->d_primf, b->d_inv, b->d_pgeo, b->d_pao,
+            b->d_pnp, b->d_bprim, b->d_bprimf, b->d_bpair);
+        CUDA_TRY(cudaGetLastError());
+    }
     b->d_dm_cond = (double*)b->d_zero;
     b->d_task0 = (long long*)(b->d_dm_cond + (size_t)ngroups * ngroups);
     b->d_task032 = b->d_task0 + 2 * b->ncq;
@@ -1040,34 +1114,9 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
         q.itm = b->d_task0 + 4 * b->ncq + 2 * c;
         q.itm32 = b->d_task0 + 6 * b->ncq + 2 * c;
     }
-    CUDA_TRY(upload(&b->d_cq, b->h_cq.data(), b->h_cq.size()));
-    CUDA_TRY(cudaMalloc(&b->d_task01, sizeof(long long) * 2));
-    CUDA_TRY(cudaMalloc(&b->d_seg1, sizeof(JKSeg)));
-    // row prefixes of the per-class-pair entries: sized once for the largest
-    // class, so those calls never free a buffer a queued kernel still reads
-    {
-        int mx = 1;
-        for (int c = 0; c < b->ncp; c++) mx = std::max(mx, b->h_pair_locs[c + 1] - b->h_pair_locs[c]);
-        CUDA_TRY(cudaMalloc(&b->d_qoff1, sizeof(long long) * (mx + 1)));
-        CUDA_TRY(cudaMalloc(&b->d_ehi1, sizeof(int) * mx));
-        b->qoff1_cap = mx + 1;
-    }
-    // pair-packed layout of the J side (jk_build)
-    b->h_pack.clear();
-    b->pack_total = 0;
-    for (int c = 0; c < b->ncp; c++) {
-        JKPackCls k;
-        k.off = b->pack_total;
-        k.pair0 = b->h_pair_locs[c];
-        k.np = b->h_pair_locs[c + 1] - k.pair0;
-        const int li = b->h_group_l[b->h_cls_gi[c]], lj = b->h_group_l[b->h_cls_gj[c]];
-        k.nfi = (li + 1) * (li + 2) / 2;
-        k.nfj = (lj + 1) * (lj + 2) / 2;
-        b->pack_total += (long long)k.np * k.nfi * k.nfj;
-        b->h_pack.push_back(k);
-    }
-    CUDA_TRY(upload(&b->d_pack, b->h_pack.data(), b->h_pack.size()));
-    CUDA_TRY(b->fan.init());
+    if (b->ncq)
+        CUDA_TRY(cudaMemcpyAsync(b->d_cq, b->h_cq.data(), sizeof(JKScreenCQ) * b->ncq, cudaMemcpyHostToDevice,
+                                 cudaStreamLegacy));
     // the class launches of jk_build (bases with classes that no J/K kernel
     // serves, as the density fitting's, do without)
     int rc = make_plan(b, 1, 0, &b->plan);

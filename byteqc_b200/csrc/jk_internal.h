@@ -164,6 +164,7 @@ struct JKPlan {
     bool multi = false;                          // some key has several segments
     const long long** d_cnt[2] = {nullptr, nullptr};
     int* d_key_off = nullptr;
+    void* mem = nullptr;                         // the tables' allocation
     unsigned long long* d_queue = nullptr;       // 2 work counters per key (persistent launches)
 };
 void jk_plan_free(JKPlan* p);
@@ -207,9 +208,10 @@ struct jk_basis {
     int *d_rank = nullptr, *d_pos = nullptr;  // rank of a position of the class, and the inverse
     double *d_bprim = nullptr, *d_bpair = nullptr;  // bra records (JKSeg::bprim, bpair)
     float* d_bprimf = nullptr;
-    // device
+    // device: the arrays of the basis and of its pairs lie in one allocation each
+    void *mem_bas = nullptr, *mem_pair = nullptr;
     int *d_atm = nullptr, *d_bas = nullptr, *d_ao_loc = nullptr, *d_group_ao = nullptr;
-    double *d_env = nullptr, *d_bas_x = nullptr, *d_qcond = nullptr;
+    double *d_env = nullptr, *d_bas_x = nullptr;
     int *d_pair2bra = nullptr, *d_pair2ket = nullptr;  // by position
     double *d_log_q = nullptr, *d_log_q_raw = nullptr, *d_prim = nullptr;  // prim: a12|e12|x12|y12|z12|1/a12
     float* d_primf = nullptr;  // FP32 path: a12|1/a12|e12/a12|P-R_bra (x, y, z)

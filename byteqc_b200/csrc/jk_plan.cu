@@ -4,6 +4,8 @@
 // launches for a def2-TZVP molecule, most of them too small to fill the
 // device; merged they are 59, and the run kernels look a segment up once per
 // item (up to 32 x 32 quartets), so that merging costs the large ones nothing.
+#include <string.h>
+
 #include <algorithm>
 
 #include "jk_internal.h"
@@ -37,13 +39,7 @@ __global__ void jk_seg_prefix_kernel(const long long* const* __restrict__ cnt, c
 
 void jk_plan_free(JKPlan* p) {
     if (!p) return;
-    for (int i = 0; i < 2; i++) {
-        cudaFree(p->d_seg[i]);
-        cudaFree(p->d_segt[i]);
-        cudaFree((void*)p->d_cnt[i]);
-    }
-    cudaFree(p->d_key_off);
-    cudaFree(p->d_queue);
+    cudaFree(p->mem);
     delete p;
 }
 
@@ -111,12 +107,18 @@ int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols, const std::vec
     for (auto& k : p->keys) p->key_off.push_back(p->key_off.back() + (int)k.segs.size());
     p->nseg = p->key_off.back();
     const size_t ns = std::max(1, p->nseg);
-    PCUDA(cudaMalloc(&p->d_key_off, sizeof(int) * (nkeys + 1)));
-    PCUDA(cudaMemcpy(p->d_key_off, p->key_off.data(), sizeof(int) * (nkeys + 1), cudaMemcpyHostToDevice));
-    PCUDA(cudaMalloc(&p->d_queue, sizeof(unsigned long long) * 2 * std::max(1, nkeys)));
-    std::vector<JKSeg> seg(ns);
-    std::vector<const long long*> cnt(ns);
+    // one allocation: what the host fills (segments and counts of both parts,
+    // key offsets) in front, uploaded as one piece
+    auto up = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+    const size_t seg_b = up(sizeof(JKSeg) * ns), cnt_b = up(sizeof(long long*) * ns),
+                 off_b = up(sizeof(int) * (nkeys + 1)), segt_b = up(sizeof(long long) * (ns + nkeys + 1));
+    const size_t host_b = 2 * (seg_b + cnt_b) + off_b;
+    PCUDA(cudaMalloc(&p->mem, host_b + 2 * segt_b + sizeof(unsigned long long) * 2 * std::max(1, nkeys)));
+    std::vector<char> host(host_b);
     for (int part = 0; part < 2; part++) {
+        const size_t seg_at = part * seg_b, cnt_at = 2 * seg_b + part * cnt_b;
+        JKSeg* seg = (JKSeg*)(host.data() + seg_at);
+        const long long** cnt = (const long long**)(host.data() + cnt_at);
         size_t i = 0;
         for (auto& k : p->keys) {
             if (k.segs.size() != 1) {
@@ -126,19 +128,18 @@ int jk_plan_finish(JKPlan* p, const std::vector<jk_basis*>& mols, const std::vec
             for (auto& s : k.segs) {
                 const JKScreenCQ& cq = cqs[s.first][s.second];
                 jk_internal_fill_seg_cq(mols[s.first], cq, part, &seg[i]);
-                if (k.segs.size() == 1)
-                    p->one[part].push_back(cq_count(cq, part));
+                if (k.segs.size() == 1) p->one[part].push_back(cq_count(cq, part));
                 cnt[i++] = cq_count(cq, part) + 1;
             }
         }
-        PCUDA(cudaMalloc(&p->d_seg[part], sizeof(JKSeg) * ns));
-        PCUDA(cudaMalloc(&p->d_segt[part], sizeof(long long) * (ns + nkeys + 1)));
-        PCUDA(cudaMalloc((void**)&p->d_cnt[part], sizeof(long long*) * ns));
-        if (p->nseg) {
-            PCUDA(cudaMemcpy(p->d_seg[part], seg.data(), sizeof(JKSeg) * p->nseg, cudaMemcpyHostToDevice));
-            PCUDA(cudaMemcpy((void*)p->d_cnt[part], cnt.data(), sizeof(long long*) * p->nseg, cudaMemcpyHostToDevice));
-        }
+        p->d_seg[part] = (JKSeg*)((char*)p->mem + seg_at);
+        p->d_cnt[part] = (const long long**)((char*)p->mem + cnt_at);
+        p->d_segt[part] = (long long*)((char*)p->mem + host_b + part * segt_b);
     }
+    memcpy(host.data() + 2 * (seg_b + cnt_b), p->key_off.data(), sizeof(int) * (nkeys + 1));
+    p->d_key_off = (int*)((char*)p->mem + 2 * (seg_b + cnt_b));
+    p->d_queue = (unsigned long long*)((char*)p->mem + host_b + 2 * segt_b);
+    PCUDA(cudaMemcpyAsync(p->mem, host.data(), host_b, cudaMemcpyHostToDevice, cudaStreamLegacy));
     PCUDA(jk_internal_uploaded());
     return JK_OK;
 }
