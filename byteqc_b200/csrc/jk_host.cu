@@ -1460,10 +1460,8 @@ __global__ void jk_run_rowbins_kernel(const __grid_constant__ JKRowBinsCols cols
         ehi[e] = cols(erank[e]);
 }
 
-// row classes; the segment of a J/K call goes to *dst
-__global__ void jk_rowbins_kernel(const JKRowBins rb, int n_ij, long long* __restrict__ qoff,
-                                  long long* __restrict__ task0, const __grid_constant__ JKSeg sg, JKSeg* dst) {
-    if (dst && blockIdx.x == 0) jk_seg_copy(sg, dst);
+__device__ __forceinline__ void jk_rowbins_body(const JKRowBins& rb, int n_ij, long long* __restrict__ qoff,
+                                                long long* __restrict__ task0) {
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r <= n_ij;
          r += (long long)gridDim.x * blockDim.x)
         qoff[r] = jk_rowbins_tasks(rb, r);
@@ -1471,6 +1469,16 @@ __global__ void jk_rowbins_kernel(const JKRowBins rb, int n_ij, long long* __res
         task0[0] = 0;
         task0[1] = jk_rowbins_tasks(rb, n_ij);
     }
+}
+__global__ void jk_rowbins_kernel(const JKRowBins rb, int n_ij, long long* __restrict__ qoff,
+                                  long long* __restrict__ task0) {
+    jk_rowbins_body(rb, n_ij, qoff, task0);
+}
+// ... and the segment of a J/K call (a row class) to *dst
+__global__ void jk_rowbins_seg_kernel(const JKRowBins rb, int n_ij, long long* __restrict__ qoff,
+                                      long long* __restrict__ task0, const __grid_constant__ JKSeg sg, JKSeg* dst) {
+    if (blockIdx.x == 0) jk_seg_copy(sg, dst);
+    jk_rowbins_body(rb, n_ij, qoff, task0);
 }
 
 static int row_bins(const int* bins_ij, const int* bins_kl, int nbins, int diag, JKRowBins* rb) {
@@ -1487,13 +1495,14 @@ static int row_bins(const int* bins_ij, const int* bins_kl, int nbins, int diag,
 }
 
 // bins of a per-class-pair call -> the basis's row prefix and task count, on
-// `st`, and the segment to *dst (if any); returns the task count through *tot
-static int class_pair_rows(jk_basis* b, const JKRowBins& rb, int n_ij, const JKSeg& seg, JKSeg* dst, cudaStream_t st,
+// `st`, and the segment (if any) to *dst; returns the task count through *tot
+static int class_pair_rows(jk_basis* b, const JKRowBins& rb, int n_ij, const JKSeg* seg, JKSeg* dst, cudaStream_t st,
                            long long* tot) {
     if (n_ij + 1 > (int)b->qoff1_cap) return set_err(JK_ERR_ARG, "class pair larger than the basis' classes");
     *tot = jk_rowbins_tasks(rb, n_ij);
     const int blocks = (int)std::min<long long>((n_ij + 256) / 256, (long long)b->nsm * 4);
-    jk_rowbins_kernel<<<blocks, 256, 0, st>>>(rb, n_ij, b->d_qoff1, b->d_task01, seg, dst);
+    if (seg) jk_rowbins_seg_kernel<<<blocks, 256, 0, st>>>(rb, n_ij, b->d_qoff1, b->d_task01, *seg, dst);
+    else jk_rowbins_kernel<<<blocks, 256, 0, st>>>(rb, n_ij, b->d_qoff1, b->d_task01);
     CUDA_TRY(cudaGetLastError());
     return JK_OK;
 }
@@ -1553,7 +1562,7 @@ extern "C" int jk_build_class_pair(jk_basis_t* b, double* vj, double* vk, const 
         }
         tot = (long long)seg.nrun * ((seg.pst_kl + chunk - 1) / chunk);
     } else {
-        rc = class_pair_rows(b, rb, n_ij, seg, b->d_seg1, st, &tot);
+        rc = class_pair_rows(b, rb, n_ij, &seg, b->d_seg1, st, &tot);
     }
     if (rc) return rc;
     return jk_internal_launch(b, cp_ij, cp_kl, b->d_seg1, b->d_task01, tot, n_dm, stream);
@@ -1600,10 +1609,10 @@ extern "C" int jk_fill_int2e(jk_basis_t* b, double* eri, int nao, const int* str
     JKRowBins rb;
     long long tot = 0;
     int rc = row_bins(bij, bkl, nbins, 0, &rb);
+    if (!rc) rc = class_pair_rows(b, rb, n_ij, nullptr, nullptr, st, &tot);
+    if (rc) return rc;
     JKSeg seg;
     fill_seg(b, cp_ij, cp_kl, b->d_qoff1, n_ij, nullptr, 0, nullptr, nullptr, &seg);
-    if (!rc) rc = class_pair_rows(b, rb, n_ij, seg, nullptr, st, &tot);
-    if (rc) return rc;
     CUDA_TRY(jk_launch_fill(seg, b->d_task01, tot, b->nsm, eri, s64, off, st));
     return JK_OK;
 }
