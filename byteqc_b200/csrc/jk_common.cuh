@@ -6,7 +6,7 @@
 #include <stdint.h>
 
 // The small per-n metadata is in constant memory of every module; the
-// Chebyshev coefficients (about 0.6 MB) are uploaded once per device into
+// coefficients (0.9 MB) are uploaded once per device into
 // global memory and reached through a pointer (JKSeg::rys), read with __ldg.
 #define RYS_META static __constant__
 #include "rys_table.h"
@@ -37,18 +37,18 @@
 // Rys nodes s_r = t_r^2 and weights w_r at x = rho |P-Q|^2.  The reference
 // evaluates the same quantities in the variable u = t^2/(1-t^2)
 // (cuobc/lib/gint/rys_roots.cu:1214-2176).
-//   n = 1:  w = F0(x), s = F1(x)/F0(x) from the Boys function itself
-//           (a Taylor series below x = 0.75, erf/exp above);
-//   n > 1:  the generated tables (power series in t on uniform intervals of
-//           width 2 up to rys_xmax[n], Gauss-Hermite limit beyond), evaluated
-//           by Horner's rule from a copy of the n-root table in shared memory
-//           (the run kernels take n = 1 from its table too: one series of 14
-//           terms for all lanes instead of three branches of erf and exp).
-//           Lanes of a warp read the intervals of their own x, two
-//           coefficients per 16-byte load; the copy's interval stride is an
-//           odd number of 16-byte words, so that different intervals start in
-//           different banks.  Clenshaw's rule on the Chebyshev form, as
-//           before, took twice the FP64 operations and 8-byte loads.
+//   tables: power series in t on uniform intervals of width 2 up to
+//           rys_xmax[n], the Gauss-Hermite limit beyond, evaluated by Horner's
+//           rule from a copy of the n-root table in shared memory.  Lanes of a
+//           warp read the intervals of their own x, two coefficients per
+//           16-byte load; the copy's interval stride is an odd number of
+//           16-byte words, so that different intervals start in different
+//           banks.  Clenshaw's rule on the Chebyshev form, as before, took
+//           twice the FP64 operations and 8-byte loads.
+//   n = 1:  in FP64 no J/K kernel needs a root: the classes of L <= 3 take the
+//           Boys functions (jk_os.cuh).  The ERI fill and the set-up kernels
+//           evaluate w = F0(x), s = F1(x)/F0(x) (a Taylor series below
+//           x = 0.75, erf/exp above); the FP32 quartets use the n = 1 table.
 // ---------------------------------------------------------------------------
 template <int N>
 struct RysS {
@@ -100,8 +100,10 @@ __device__ __forceinline__ double rys_series_g(const double* __restrict__ c, dou
     for (int k = RYS_NC - 2; k >= 0; k--) v = fma(v, t, __ldg(c + k));
     return v;
 }
-// the same in single precision (8-byte aligned); the terms from t^10 on are
-// below 1e-8 of the sum, under half a unit in the last place of a float
+// the same in single precision (8-byte aligned), 10 of the 14 terms: those from
+// t^10 on are at most 2.8e-8 (n = 1), 3.5e-8 (n = 2) and 8.5e-8 (n = 3) of the
+// sum, and the whole evaluation, rounding included, is off by at most 1.2e-7 of
+// it at any n (all intervals of the tables, t in steps of 0.01)
 #define RYS_NCF 10
 __device__ __forceinline__ float rys_series_f(const float* __restrict__ c, float t) {
     const float2* c2 = reinterpret_cast<const float2*>(c);
@@ -210,13 +212,6 @@ __device__ __forceinline__ void rys_roots_all(const double* __restrict__ tab, do
 template <int N>
 __device__ __forceinline__ void rys_root_one(const double* __restrict__ tab, double x, int r, double& s, double& w) {
     using S = RysS<N>;
-    if (N == 1) {
-        double f0, f1;
-        boys01(x, f0, f1);
-        w = f0;
-        s = f1 / f0;
-        return;
-    }
     if (x >= S::XMAX) {
         const double rx = rsqrt(x);
         s = tab[S::HERM + r] * (rx * rx);
@@ -257,9 +252,8 @@ __device__ __forceinline__ void rys_root(const double* __restrict__ rys_coef, do
 
 // ---------------------------------------------------------------------------
 // Single-precision nodes and weights for the FP32 quartets of the mixed mode
-// at low order (n <= JK_F32_ROOTS): the Boys function in float for n = 1, the
-// same tables rounded to float for n = 2, 3.  Higher orders keep the double
-// evaluation above.
+// at low order (n <= JK_F32_ROOTS): the tables rounded to float.  Higher orders
+// keep the double evaluation above.
 // ---------------------------------------------------------------------------
 #define JK_F32_ROOTS 3
 
@@ -287,38 +281,6 @@ __device__ __forceinline__ void rys_table_copy_f(const double* __restrict__ g, f
     }
 }
 template <int N>
-__device__ __forceinline__ void rys_table_to_smem_f(const double* __restrict__ g, float* __restrict__ tab) {
-    if (N > 1) rys_table_copy_f<N>(g, tab);
-}
-
-// F0 and F1 in float: the series below x = 0.75 (12 terms, truncation below
-// 1e-10), erf/exp above
-__device__ __forceinline__ void boys01_f(float x, float& f0, float& f1) {
-    if (x < 0.75f) {
-        float a0 = 0.f, a1 = 0.f;
-        double fk = 1.;
-        float c0[12], c1[12];
-#pragma unroll
-        for (int k = 0; k < 12; k++) {
-            if (k) fk *= k;
-            c0[k] = (float)(((k & 1) ? -1. : 1.) / (fk * (2 * k + 1)));
-            c1[k] = (float)(((k & 1) ? -1. : 1.) / (fk * (2 * k + 3)));
-        }
-#pragma unroll
-        for (int k = 11; k >= 0; k--) {
-            a0 = fmaf(a0, x, c0[k]);
-            a1 = fmaf(a1, x, c1[k]);
-        }
-        f0 = a0;
-        f1 = a1;
-    } else {
-        float rsx = rsqrtf(x);
-        f0 = 0.886226925f * erff(x * rsx) * rsx;  // sqrt(pi)/2 erf(sqrt x)/sqrt x
-        f1 = (f0 - expf(-x)) * (0.5f * rsx * rsx);
-    }
-}
-
-template <int N>
 __device__ __forceinline__ void rys_table_all_f(const float* __restrict__ tab, float x, float* s, float* w) {
     using S = RysF<N>;
     if (x >= (float)RysS<N>::XMAX) {
@@ -339,29 +301,10 @@ __device__ __forceinline__ void rys_table_all_f(const float* __restrict__ tab, f
         w[r] = rys_series_f(c + (N + r) * RYS_NCF, t);
     }
 }
-template <int N>
-__device__ __forceinline__ void rys_roots_all_f(const float* __restrict__ tab, float x, float* s, float* w) {
-    if (N == 1) {
-        float f0, f1;
-        boys01_f(x, f0, f1);
-        w[0] = f0;
-        s[0] = __fdividef(f1, f0);
-        return;
-    }
-    rys_table_all_f<N>(tab, x, s, w);
-}
-
 // root r only (runtime r), single precision, from the float table copy
 template <int N>
 __device__ __forceinline__ void rys_root_one_f(const float* __restrict__ tab, float x, int r, float& s, float& w) {
     using S = RysF<N>;
-    if (N == 1) {
-        float f0, f1;
-        boys01_f(x, f0, f1);
-        w = f0;
-        s = __fdividef(f1, f0);
-        return;
-    }
     if (x >= (float)RysS<N>::XMAX) {
         const float srx = rsqrtf(x);
         s = tab[S::HERM + r] * srx * srx;

@@ -6,15 +6,15 @@
 // (ii|ii)).  Basis sets such as cc-pVQZ or def2-QZVP carry g functions,
 // cc-pV5Z h and cc-pV6Z i.  These classes are rare, so the kernel aims at
 // correctness with bounded resources; its fixed sizes come from the largest
-// l it serves, GL = 5 (every class up to (hh|hh), 86 KB of shared memory,
-// two CTAs per SM) or GL = 6 (classes with an i shell, 153 KB, one CTA):
+// l it serves: GL = 4 (85 KB of shared memory), GL = 5 (105 KB; two CTAs per SM
+// for both) or GL = 6 (169 KB, one CTA):
 //
 //   one CTA per contracted quartet.  The 2D blocks of a batch of roots (all
 //   of them for most classes) are built in three parallel steps: the vertical
 //   recursion by one thread per (root, axis), the bra transfer by one per
 //   (root, axis, m), the ket transfer by one per (root, axis, i, j).  The
 //   integrals of a range of (i, j) components are summed over primitives and
-//   roots in shared memory, once, and then digested from there: every thread
+//   roots in shared memory, once per density, and then digested from there: every thread
 //   owns elements of the six J/K blocks (J_ij, J_kl, K_ik, K_il, K_jk, K_jl)
 //   and sums integral times density over the other two indices (no atomics:
 //   one owner per element); the blocks are added to J and K with one atomic

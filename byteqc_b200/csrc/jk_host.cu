@@ -1849,24 +1849,22 @@ extern "C" int jk_fma_peak(int fp32, double* tflops) {
     return JK_OK;
 }
 
-// device evaluation of the Rys tables at a batch of points, through the
-// paths the kernels use: mode 0 all roots from the shared-memory copy (thread
-// kernels), 1 one root at a time from it (team kernels), 2 one root from the
-// global table (setup kernels), 3 all roots in single precision (the FP32
-// quartets of the mixed mode, n <= JK_F32_ROOTS; thread kernels), 4 one root
-// at a time in single precision (team kernels)
+// device evaluation of the Rys tables and the Boys functions at a batch of
+// points, through the functions that the kernels call (modes in byteqc_jk.h)
 template <int N>
 __global__ void jk_rys_eval_kernel(const double* rys, const double* x, int count, double* s, double* w, int mode) {
     extern __shared__ __align__(16) double tab[];
-    if (mode >= 3) rys_table_to_smem_f<N>(rys, reinterpret_cast<float*>(tab));
-    else rys_table_to_smem<N>(rys, tab);
+    if (mode == 3 || mode == 4) rys_table_copy_f<N>(rys, reinterpret_cast<float*>(tab));
+    else if (mode == 7) {
+        if constexpr (N <= 4) boys_table_copy<N - 1>(rys, tab);
+    } else rys_table_copy<N>(rys, tab);
     __syncthreads();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     if (mode == 3) {
         if constexpr (N <= JK_F32_ROOTS) {
             float rs[N], rw[N];
-            rys_roots_all_f<N>(reinterpret_cast<const float*>(tab), (float)x[i], rs, rw);
+            rys_table_all_f<N>(reinterpret_cast<const float*>(tab), (float)x[i], rs, rw);
             for (int r = 0; r < N; r++) {
                 s[i * N + r] = rs[r];
                 w[i * N + r] = rw[r];
@@ -1881,16 +1879,16 @@ __global__ void jk_rys_eval_kernel(const double* rys, const double* x, int count
                 w[i * N + r] = rw;
             }
         }
-    } else if (mode == 5) {  // run-time root count (generic kernels), global table
-        for (int r = 0; r < N; r++) {
-            double rs, rw;
-            rys_root_rt(rys, N, x[i], r, rs, rw);
-            s[i * N + r] = rs;
-            w[i * N + r] = rw;
+    } else if (mode == 7) {
+        if constexpr (N <= 4) {
+            double F[N];
+            boys_all<N - 1>(tab, x[i], F);
+            for (int r = 0; r < N; r++) s[i * N + r] = w[i * N + r] = F[r];
         }
-    } else if (mode == 0) {
+    } else if (mode == 0 || mode == 6) {
         double rs[N], rw[N];
-        rys_roots_all<N>(tab, x[i], rs, rw);
+        if (mode == 0) rys_roots_all<N>(tab, x[i], rs, rw);
+        else rys_table_all<N>(tab, x[i], rs, rw);
         for (int r = 0; r < N; r++) {
             s[i * N + r] = rs[r];
             w[i * N + r] = rw[r];
@@ -1898,6 +1896,7 @@ __global__ void jk_rys_eval_kernel(const double* rys, const double* x, int count
     } else {
         for (int r = 0; r < N; r++) {
             if (mode == 1) rys_root_one<N>(tab, x[i], r, s[i * N + r], w[i * N + r]);
+            else if (mode == 5) rys_root_rt(rys, N, x[i], r, s[i * N + r], w[i * N + r]);
             else rys_root<N>(rys, x[i], r, s[i * N + r], w[i * N + r]);
         }
     }
@@ -1906,7 +1905,7 @@ __global__ void jk_rys_eval_kernel(const double* rys, const double* x, int count
 template <int N>
 static cudaError_t rys_eval_launch(const double* rys, const double* x, int count, double* s, double* w, int mode,
                                    cudaStream_t st) {
-    size_t smem = RysS<N>::WORDS * sizeof(double);
+    const size_t smem = std::max<size_t>(RysS<N>::TWORDS, N <= 4 ? (size_t)BoysS::WORDS : 0) * sizeof(double);
     cudaError_t e = cudaFuncSetAttribute(jk_rys_eval_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     jk_rys_eval_kernel<N><<<(count + 127) / 128, 128, smem, st>>>(rys, x, count, s, w, mode);
@@ -1914,8 +1913,8 @@ static cudaError_t rys_eval_launch(const double* rys, const double* x, int count
 }
 
 extern "C" int jk_rys_roots_device(int n, const double* x, int count, double* s, double* w, int mode, void* stream) {
-    if (n < 1 || n > RYS_NMAX || !x || !s || !w || count < 0 || mode < 0 || mode > 5 ||
-        ((mode == 3 || mode == 4) && n > JK_F32_ROOTS))
+    if (n < 1 || n > RYS_NMAX || !x || !s || !w || count < 0 || mode < 0 || mode > 7 ||
+        ((mode == 3 || mode == 4) && n > JK_F32_ROOTS) || (mode == 7 && n > 4))
         return set_err(JK_ERR_ARG, "jk_rys_roots_device: bad args");
     if (count == 0) return JK_OK;
     const double* rys;

@@ -624,7 +624,7 @@ __device__ __forceinline__ void jk_team_body(const Src& src, const JKFillOut* fo
     // table copy in shared memory is then single precision)
     constexpr bool F32P = JKF32Prim<C, R>::value && S::SMEM_TAB;
     if (S::SMEM_TAB) {
-        if constexpr (F32P) rys_table_to_smem_f<NR>(sg0.rys, reinterpret_cast<float*>(tab));
+        if constexpr (F32P) rys_table_copy_f<NR>(sg0.rys, reinterpret_cast<float*>(tab));
         else rys_table_to_smem<NR>(sg0.rys, tab);
     }
 

@@ -49,7 +49,8 @@ struct JKTRunShape {
     // different banks
     static constexpr int WORDS = ((WORDS0 + 1) & ~1) % 4 == 2 ? ((WORDS0 + 1) & ~1) : ((WORDS0 + 1) & ~1) + 2;
     static constexpr bool SMEM_TAB = NR <= 4;
-    static constexpr bool F32P = JKF32Prim<C, R>::value && SMEM_TAB;
+    static constexpr bool F32P = JKF32Prim<C, R>::value;
+    static_assert(!F32P || SMEM_TAB, "single-precision roots come from shared memory");
     static constexpr size_t TAB = SMEM_TAB ? ((size_t)RysS<NR>::TWORDS * sizeof(double) + 15) & ~(size_t)15 : 0;
     static constexpr size_t WARP = (size_t)TPW * WORDS * 8 + 32 * 12 * 8;  // team regions, staged records
     static constexpr size_t SMEM = TAB + (JK_RUN_THREADS / 32) * WARP;
@@ -117,8 +118,6 @@ struct JKTRunItem {
             JKPP b;
             if (p) {
                 b = jk_bra_pp(bprim + (size_t)p * pst_ij * 8);
-            } else if constexpr (JKF32Prim<C, R>::value) {
-                b = jk_bra_pp(bprim);  // the staged record is the single-precision one
             } else {
                 const double2 u = rec[6 * el], v = rec[6 * el + 1], w = rec[6 * el + 2];
                 b = JKPP{u.x, u.y, v.x, {v.y, w.x, w.y}};
@@ -369,7 +368,7 @@ struct JKTRunItem {
         __syncwarp();
         if ((mask >> lane) & 1) {  // stage the run
             double2* r = rec + 6 * lane;
-            if constexpr (JKF32Prim<C, R>::value) {
+            if constexpr (S::F32P) {
                 const float4* f = reinterpret_cast<const float4*>(bprimf0 + lane * 8);
                 reinterpret_cast<float4*>(r)[0] = __ldg(f);
                 reinterpret_cast<float4*>(r)[1] = __ldg(f + 1);

@@ -251,18 +251,20 @@ int jk_batch_get_jk(jk_batch_t *batch, const double *const *coeffs, const int *n
                     double *const *vj0s, double *const *vk0s, int n_dm, const jk_opts_t *opts, void *stream);
 
 /* Rys nodes s = t^2 and weights of the product tables, evaluated on the
- * host (for checking the tables).  Returns JK_ERR_ARG for n outside 1..11. */
+ * host (for checking the tables).  Returns JK_ERR_ARG for n outside 1..13. */
 int jk_rys_roots_host(int n, double x, double *s, double *w);
 
-/* The same tables evaluated by a device kernel through the paths the J/K
- * kernels use (mode 0: all roots from the shared-memory copy, 1: one root at
- * a time from it, 2: one root from the global copy, 3: all roots in single
- * precision as the FP32 quartets of the mixed mode use them, 4: one root at a
- * time in single precision; modes 3 and 4 for n <= 3 only; 5: one root at a
- * time with the root count known at run time, from the global copy, as the
- * generic kernels evaluate them; n = 1 is evaluated from the Boys function in
- * every mode; n <= 13).  x, s, w are device arrays (count,
- * count*n, count*n).  For checking the device evaluation. */
+/* The same evaluated by a device kernel through the functions that the kernels
+ * call: mode 0 all roots from the shared-memory copy, n = 1 from the Boys
+ * function (ERI fill); 1 one root at a time from the copy (team kernels, run
+ * kernels of four passes); 2 one root from the global copy, n = 1 from the Boys
+ * function (set-up, team kernels of many roots); 3 all roots and 4 one root at a
+ * time in single precision (FP32 quartets of the mixed mode, n <= 3); 5 one root
+ * with the root count known at run time, from the global copy (generic
+ * kernels); 6 all roots from the copy, n = 1 too (run kernels); 7 the Boys
+ * functions F_0 .. F_{n-1} (run kernels of L <= 3, n <= 4), the same in s and w.
+ * n <= 13.  x, s, w are device arrays (count, count*n, count*n).  For checking
+ * the device evaluation. */
 int jk_rys_roots_device(int n, const double *x, int count, double *s, double *w, int mode, void *stream);
 
 /* Per class quartet (8 ints each): cp_ij, cp_kl, li, lj, lk, ll, nprim_ij,

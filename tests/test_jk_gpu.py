@@ -108,6 +108,58 @@ def test_device_rys_tables_match_host():
                 np.testing.assert_allclose(w[i], hw, rtol=1e-14, atol=1e-300)
 
 
+def _boys(m, x):
+    """F_m(x) in extended precision: e^-x sum_k (2x)^k / ((2m+1) ... (2m+2k+1)),
+    all terms positive."""
+    x = np.longdouble(x)
+    t = np.longdouble(1) / (2 * m + 1)
+    s = t
+    for k in range(1, 400):
+        t = t * 2 * x / (2 * m + 2 * k + 1)
+        s += t
+    return float(s * np.exp(-x))
+
+
+def test_device_run_kernel_roots_and_boys():
+    """The evaluations of the run kernels: all roots from the shared-memory
+    tables (n = 1 too) against the host, and the Boys functions of the L <= 3
+    classes against the series, on interval edges, inside and beyond the table.
+    Tolerances: a Horner series of 10 or 14 terms in double, 1e-14 of the value;
+    beyond 46 F_m is the asymptotic term, off by e^-x."""
+    import torch
+    from byteqc_b200.cuobc import lib as jklib
+    lib = jklib.load_library()
+    rng = np.random.default_rng(3)
+    xs = np.concatenate([[0., 1e-13, 0.25, 0.5, 1.0, 1.5, 2.0, 41.9, 42., 45.5,
+                          45.999, 46.0, 46.5, 60., 97.9],
+                         rng.uniform(0, 60, 200)])
+    dx = torch.as_tensor(xs, device='cuda')
+
+    def eval_(n, mode):
+        ds = torch.zeros(len(xs) * n, dtype=torch.float64, device='cuda')
+        dw = torch.zeros_like(ds)
+        assert lib.jk_rys_roots_device(n, dx.data_ptr(), len(xs),
+                                       ds.data_ptr(), dw.data_ptr(), mode,
+                                       None) == 0
+        return (ds.cpu().numpy().reshape(-1, n), dw.cpu().numpy().reshape(-1, n))
+    for n in range(1, 6):
+        s, w = eval_(n, 6)
+        for i, x in enumerate(xs):
+            hs, hw = np.zeros(n), np.zeros(n)
+            lib.jk_rys_roots_host(n, x, hs.ctypes.data, hw.ctypes.data)
+            np.testing.assert_allclose(s[i], hs, rtol=1e-14, atol=1e-300)
+            np.testing.assert_allclose(w[i], hw, rtol=1e-14, atol=1e-300)
+    for n in range(1, 5):
+        f, _ = eval_(n, 7)
+        ref = np.array([[_boys(m, x) for m in range(n)] for x in xs])
+        np.testing.assert_allclose(f, ref, rtol=1e-14)
+    bad = torch.zeros(64, dtype=torch.float64, device='cuda')
+    assert lib.jk_rys_roots_device(5, bad.data_ptr(), 1, bad.data_ptr(),
+                                   bad.data_ptr(), 7, None) == 3
+    assert lib.jk_rys_roots_device(1, bad.data_ptr(), 1, bad.data_ptr(),
+                                   bad.data_ptr(), 8, None) == 3
+
+
 def test_device_rys_fp32_nodes():
     """Single-precision nodes and weights of the FP32 quartets (n <= 3):
     nodes s = t^2 in [0, 1) within 2e-6 absolute, weights within 2e-6 of
