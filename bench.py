@@ -63,9 +63,9 @@ def make_workload(name, oracle_overlap=False):
     return mol, dm
 
 
-# DRAM bytes (read + write) of one build's class-quartet launches, summed
+# DRAM bytes (read + write) of one build's class launches, summed
 # from an ncu launch list of `bench.py --profile-builds 2` on the workload
-PROFILED_TRAFFIC = {'h2o32-tzvp': 78.9e6, 'h2o12-tzvp': 5.7e6}
+PROFILED_TRAFFIC = {'h2o32-tzvp': 102.2e6, 'h2o12-tzvp': 7.2e6}
 
 
 def batch_workload(nmol=256, seed=4, basis='standin-6-31g*'):

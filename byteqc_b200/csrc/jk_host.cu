@@ -703,11 +703,18 @@ static int rys_table_device(const double** out) {
 static int sort_bucket(int n) { return std::max(32, (n / 16 + 31) / 32 * 32); }
 
 // Run length of a class quartet's bra (an index of JK_RUN_LEN): the longest
-// that still gives a few items per resident warp before screening; a
-// molecule too small for that takes the shortest.
-static int run_level(const jk_basis* b, int cp_ij, int n_kl, int chunk, int levels) {
+// that still gives `items` items per SM before screening; a molecule too small
+// for that takes the shortest.  In a build the launches of the classes share the
+// device, and 5 per SM do: at 5, 10, 20 and 40 (as it was) (H2O)8 / cc-pVDZ takes
+// 0.91, 0.96, 1.04 and 1.11 ms, 37 atoms in 6-31G* 31.4, 31.6, 32.4 and 33.4, (H2O)20
+// in 6-31G* 3.96, 4.15, 4.27 and 4.35, (H2O)32 / TZVP 254, 254, 254 and 255; at 160
+// (H2O)8 1.25 and (H2O)32 / TZVP 263.  A per-class-pair call has the device to
+// itself and keeps 40.
+#define JK_RUN_ITEMS 5
+#define JK_RUN_ITEMS_PAIR 40
+static int run_level(const jk_basis* b, int cp_ij, int n_kl, int chunk, int levels, int items) {
     for (int v = 0; v < levels - 1; v++)
-        if ((long long)b->h_nrun[v][cp_ij] * ((n_kl + chunk - 1) / chunk) >= 40LL * b->nsm) return v;
+        if ((long long)b->h_nrun[v][cp_ij] * ((n_kl + chunk - 1) / chunk) >= (long long)items * b->nsm) return v;
     return levels - 1;
 }
 
@@ -1002,7 +1009,7 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             ent_at.push_back(b->ent_total);
             b->ent_total += c.n_ij;
             if (c.runs) {
-                c.level = run_level(b, cij, c.n_kl, c.runs, JK_RUN_LEVELS);
+                c.level = run_level(b, cij, c.n_kl, c.runs, JK_RUN_LEVELS, JK_RUN_ITEMS);
                 c.nrun = b->h_nrun[c.level][cij];
                 b->ioff_total += 2LL * c.nrun;
             } else {
@@ -1367,8 +1374,10 @@ static int build(jk_basis* b, const double* dm, int n_dm, double* vj, double* vk
     rc = jk_internal_screen(b->d_cq, b->ncq, tol, nbins, prescreen, fp32_cutoff, st);
     if (!rc && !singly) rc = jk_plan_prefix(plan, mixed, st);
     if (rc) return rc;
-    // class launches on side streams: 4 of them, 8 with the FP32 parts or for
-    // a molecule whose launches leave most of the device idle
+    // class launches on side streams: 4 of them, 8 with the FP32 parts or for a
+    // molecule whose launches leave most of the device idle (8 and 4 streams: one
+    // water 186 and 220 us, 13 atoms / TZVP, 3662 pairs, 5.2 and 6.9 ms; from (H2O)8
+    // / cc-pVDZ, 6112 pairs, on the two are within 1 %, and 4 are cheaper to fork)
     const int np = mixed ? 2 : 1, ns = mixed || b->h_pair2bra.size() < 4096 ? 8 : 4;
     CUDA_TRY(b->fan.begin(st, ns));
     for (int k = 0; k < (int)plan->keys.size(); k++)
@@ -1974,7 +1983,7 @@ bool jk_internal_pair_runs(const jk_basis_t* b, int cp_ij, int cp_kl, JKSeg* seg
                            const int** erank, int* chunk) {
     *chunk = g_tabs.run[class_index(b, cp_ij, cp_kl)];
     if (!*chunk) return false;
-    const int v = run_level(b, cp_ij, seg->pst_kl, *chunk, JK_RUN_LEVELS_PAIR);
+    const int v = run_level(b, cp_ij, seg->pst_kl, *chunk, JK_RUN_LEVELS_PAIR, JK_RUN_ITEMS_PAIR);
     seg->nrun = b->h_nrun[v][cp_ij];
     seg->ent = b->d_ent + b->h_pair_locs[cp_ij];
     seg->run0 = b->d_run0 + b->h_run_off[v][cp_ij];
@@ -2084,8 +2093,10 @@ int jk_internal_screen(const JKScreenCQ* d_cq, int ncq, double tol, int nbins, i
     if (ncq <= 0) return JK_OK;
     cudaStream_t st = (cudaStream_t)stream;
     // enough blocks for a large class, few enough that small ones (their
-    // surplus blocks leave at once) stay cheap
-    const unsigned by = ncq <= 64 ? 512 : (ncq <= 1024 ? 64 : 16);
+    // surplus blocks leave at once) stay cheap: with 512 / 64 / 16 blocks, as it
+    // was, and with these, two waters / cc-pVDZ (21 class quartets) take 206 and
+    // 191 us, one water / TZVP (666) 1.42 and 1.37 ms, (H2O)64 / cc-pVDZ 98.4 ms both
+    const unsigned by = ncq <= 64 ? 128 : (ncq <= 1024 ? 16 : 4);
     jk_screen_kernel<<<dim3(ncq, by), 256, 0, st>>>(d_cq, tol, nbins, prescreen, fp32_cutoff);
     jk_run_scan_kernel<<<ncq, 1024, 0, st>>>(d_cq);
     CUDA_TRY(cudaGetLastError());

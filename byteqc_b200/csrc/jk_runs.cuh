@@ -676,7 +676,9 @@ struct JKRunItem {
     }
 };
 
-// Resident blocks asked of the register allocator.
+// Resident blocks asked of the register allocator.  One more of each in the
+// double kernels (6, 5, 4 for 5, 4, 3) spills: (H2O)32 / TZVP 212 instead of 206
+// ms, (H2O)64 / cc-pVDZ 143 instead of 112.
 template <class C, typename R>
 struct JKRunMinBlocks {
     static constexpr int value = sizeof(R) == 4 ? (C::W <= 10 ? 5 : (C::W <= 24 ? 4 : (C::W <= 40 ? 3 : 2)))
