@@ -44,6 +44,12 @@ def test_invalid_arguments_return_status():
     assert lib.jk_build_class_pair(None, None, None, None, 0, 1,
                                    bins.ctypes.data, bins.ctypes.data, 1, 0,
                                    0, None) == 3
+    assert lib.jk_expand_int2e(None, st.ctypes.data, 1, None) == 3
+    assert b'invalid' in lib.jk_last_error()
+    # no batch of no molecules, none of a null basis list
+    assert lib.jk_batch_create(None, 1, ctypes.byref(out)) == 3
+    assert lib.jk_batch_create((ctypes.c_void_p * 1)(), 0,
+                               ctypes.byref(out)) == 3
 
 
 def test_product_tables_match_oracle_tables():
