@@ -157,7 +157,7 @@ static int batch_create(jk_basis_t* const* bases, int nmol, long long solo_tasks
 extern "C" int jk_batch_create_ex(jk_basis_t* const* bases, int nmol, long long solo_tasks, jk_batch_t** out) {
     if (!bases || nmol <= 0 || !out) return jk_internal_set_err(JK_ERR_ARG, "jk_batch_create: invalid arguments");
     jk_batch* t = new jk_batch();
-    int rc = batch_create(bases, nmol, solo_tasks, t);
+    int rc = jk_guard([&] { return batch_create(bases, nmol, solo_tasks, t); });
     if (rc) {
         free_batch(t);
         *out = nullptr;
@@ -339,7 +339,7 @@ static int batch_build(jk_batch* t, const double* const* dms, double* const* vjs
 
 extern "C" int jk_batch_build(jk_batch_t* t, const double* const* dms, double* const* vjs, double* const* vks,
                               int n_dm, const jk_opts_t* opts, void* stream) {
-    return batch_build(t, dms, vjs, vks, n_dm, false, opts, stream);
+    return jk_guard([&] { return batch_build(t, dms, vjs, vks, n_dm, false, opts, stream); });
 }
 
 // ---------------------------------------------------------------------------
@@ -375,8 +375,8 @@ static std::string tune_key_str(const JKPlanKey& k, int part) {
 static const char kTuneHead[] = "# byteqc_b200 batch launch shapes";
 static const char kTuneVersion[] = " 2: ";
 
-extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* const* vjs, double* const* vks,
-                             int n_dm, const jk_opts_t* opts, const char* cache_path, void* stream) {
+static int batch_tune(jk_batch* t, const double* const* dms, double* const* vjs, double* const* vks, int n_dm,
+                      const jk_opts_t* opts, const char* cache_path, void* stream) {
     if (!t || !dms || n_dm <= 0 || (!vjs && !vks))
         return jk_internal_set_err(JK_ERR_ARG, "jk_batch_tune: invalid arguments");
     cudaStream_t st = (cudaStream_t)stream;
@@ -472,6 +472,11 @@ extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* co
     return JK_OK;
 }
 
+extern "C" int jk_batch_tune(jk_batch_t* t, const double* const* dms, double* const* vjs, double* const* vks,
+                             int n_dm, const jk_opts_t* opts, const char* cache_path, void* stream) {
+    return jk_guard([&] { return batch_tune(t, dms, vjs, vks, n_dm, opts, cache_path, stream); });
+}
+
 extern "C" int jk_batch_nsolo(const jk_batch_t* t, int* nsolo) {
     if (!t || !nsolo) return jk_internal_set_err(JK_ERR_ARG, "jk_batch_nsolo: invalid arguments");
     *nsolo = (int)t->plan->keys.size() - t->nmerged;
@@ -518,9 +523,8 @@ static cublasStatus_t gemm_rm_b(cublasHandle_t h, bool ta, bool tb, int M, int N
 // batched build, then J_m = 2 C_m^T (V + V^T) C_m, K_m = C_m^T (V + V^T) C_m.
 // coeffs[m] (nao_m, nao0s[m]) row-major device; dm0s/vj0s/vk0s device
 // (n_dm, nao0, nao0); vj0s/vk0s overwritten (either may be NULL).
-extern "C" int jk_batch_get_jk(jk_batch_t* t, const double* const* coeffs, const int* nao0s,
-                               const double* const* dm0s, double* const* vj0s, double* const* vk0s, int n_dm,
-                               const jk_opts_t* opts, void* stream) {
+static int batch_get_jk(jk_batch* t, const double* const* coeffs, const int* nao0s, const double* const* dm0s,
+                        double* const* vj0s, double* const* vk0s, int n_dm, const jk_opts_t* opts, void* stream) {
     if (!t || !coeffs || !nao0s || !dm0s || n_dm <= 0)
         return jk_internal_set_err(JK_ERR_ARG, "jk_batch_get_jk: invalid arguments");
     cudaStream_t st = (cudaStream_t)stream;
@@ -609,4 +613,10 @@ extern "C" int jk_batch_get_jk(jk_batch_t* t, const double* const* coeffs, const
         }
     }
     return JK_OK;
+}
+
+extern "C" int jk_batch_get_jk(jk_batch_t* t, const double* const* coeffs, const int* nao0s,
+                               const double* const* dm0s, double* const* vj0s, double* const* vk0s, int n_dm,
+                               const jk_opts_t* opts, void* stream) {
+    return jk_guard([&] { return batch_get_jk(t, coeffs, nao0s, dm0s, vj0s, vk0s, n_dm, opts, stream); });
 }

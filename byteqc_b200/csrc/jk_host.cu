@@ -8,6 +8,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <memory>
 #include <mutex>
 #include <numeric>
 #include <string>
@@ -1138,7 +1139,9 @@ extern "C" int jk_basis_create(const int* atm, int natm, const int* bas, int nba
     if (!atm || !bas || !env || !group_offsets || !out || natm <= 0 || nbas <= 0 || ngroups <= 0)
         return set_err(JK_ERR_ARG, "jk_basis_create: invalid arguments");
     jk_basis* b = new jk_basis();
-    int rc = create_impl(atm, natm, bas, nbas, env, nenv, group_offsets, ngroups, cutoff, diag_block_with_triu, b);
+    int rc = jk_guard([&] {
+        return create_impl(atm, natm, bas, nbas, env, nenv, group_offsets, ngroups, cutoff, diag_block_with_triu, b);
+    });
     if (rc != JK_OK) {
         free_basis(b);
         *out = nullptr;
@@ -1231,7 +1234,7 @@ static int class_index(const jk_basis* b, int cp_ij, int cp_kl) {
     return JK_CLASS_INDEX(li, lj, lk, ll);
 }
 
-extern "C" int jk_shard_plan(const double* cost, int n, int nshards, int* owner) {
+static int shard_plan(const double* cost, int n, int nshards, int* owner) {
     if (n < 0 || nshards < 1 || (n > 0 && (!cost || !owner)))
         return set_err(JK_ERR_ARG, "jk_shard_plan: invalid arguments");
     std::vector<int> ord(n);
@@ -1248,13 +1251,17 @@ extern "C" int jk_shard_plan(const double* cost, int n, int nshards, int* owner)
     return JK_OK;
 }
 
+extern "C" int jk_shard_plan(const double* cost, int n, int nshards, int* owner) {
+    return jk_guard([&] { return shard_plan(cost, n, nshards, owner); });
+}
+
 static unsigned dm_cond_blocks(int nao) { return (unsigned)std::min(64, nao / 8 + 1); }
 
 // owner of every class quartet for nshards shards (cached per basis)
 static const int* shard_owners(jk_basis* b, int nshards) {
     if (b->cq_owner_n != nshards || (int)b->h_cq_owner.size() != b->ncq) {
         b->h_cq_owner.assign(b->ncq, 0);
-        jk_shard_plan(b->h_cq_cost.data(), b->ncq, nshards, b->h_cq_owner.data());
+        shard_plan(b->h_cq_cost.data(), b->ncq, nshards, b->h_cq_owner.data());
         b->cq_owner_n = nshards;
     }
     return b->h_cq_owner.data();
@@ -1262,17 +1269,13 @@ static const int* shard_owners(jk_basis* b, int nshards) {
 
 // class launches of one shard of a build
 static int make_plan(jk_basis* b, int nshards, int shard, JKPlan** out) {
-    JKPlan* p = new JKPlan();
+    std::unique_ptr<JKPlan, void (*)(JKPlan*)> p(new JKPlan(), jk_plan_free);
     const int* owner = nshards > 1 ? shard_owners(b, nshards) : nullptr;
     int rc = JK_OK;
     for (int c = 0; c < b->ncq && !rc; c++)
-        if (!owner || owner[c] == shard) rc = jk_plan_add(p, b, 0, c, false);
-    if (!rc) rc = jk_plan_finish(p, {b}, {b->h_cq.data()});
-    if (rc) {
-        jk_plan_free(p);
-        p = nullptr;
-    }
-    *out = p;
+        if (!owner || owner[c] == shard) rc = jk_plan_add(p.get(), b, 0, c, false);
+    if (!rc) rc = jk_plan_finish(p.get(), {b}, {b->h_cq.data()});
+    *out = rc ? nullptr : p.release();
     return rc;
 }
 
@@ -1323,14 +1326,17 @@ static int build(jk_basis* b, const double* dm, int n_dm, double* vj, double* vk
     const int* singly = nullptr;
     if (nshards > 1) {
         auto it = b->shard_plans.find({nshards, shard});
-        if (it != b->shard_plans.end()) {
+        if (it != b->shard_plans.end() && it->second) {
             plan = it->second;
         } else if (capturing) {
             singly = shard_owners(b, nshards);
         } else {
-            int rc = make_plan(b, nshards, shard, &plan);
-            if (rc) return rc;
-            b->shard_plans[{nshards, shard}] = plan;
+            JKPlan*& slot = b->shard_plans[{nshards, shard}];
+            if (!slot) {
+                int rc = make_plan(b, nshards, shard, &slot);
+                if (rc) return rc;
+            }
+            plan = slot;
         }
     }
     int rc = JK_OK;
@@ -1411,7 +1417,7 @@ static int build(jk_basis* b, const double* dm, int n_dm, double* vj, double* vk
 
 extern "C" int jk_build(jk_basis_t* b, const double* dm, int n_dm, double* vj, double* vk, const jk_opts_t* opts,
                         void* stream) {
-    return build(b, dm, n_dm, vj, vk, false, opts, stream);
+    return jk_guard([&] { return build(b, dm, n_dm, vj, vk, false, opts, stream); });
 }
 
 // Row prefix of one class pair's task list from the host bins of the
@@ -1752,7 +1758,7 @@ extern "C" int jk_get_jk(jk_basis_t* b, const double* coeff, int nao0, const dou
     double* v0 = vj0 ? vjw : vkw;  // the outputs lie together
     const size_t nv = vj0 && vk0 ? 2 * nn : nn;
     CUDA_TRY(cudaMemsetAsync(v0, 0, sizeof(double) * nv, st));
-    rc = build(b, dms, n_dm, vj0 ? vjw : nullptr, vk0 ? vkw : nullptr, true, opts, stream);
+    rc = jk_guard([&] { return build(b, dms, n_dm, vj0 ? vjw : nullptr, vk0 ? vkw : nullptr, true, opts, stream); });
     if (rc) return rc;
     // J = 2 C^T (V + V^T) C, K = C^T (V + V^T) C (cuobc/scf/hf.py:171-181):
     // one symmetrisation, one product with C from the right for all matrices

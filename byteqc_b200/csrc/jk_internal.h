@@ -3,6 +3,7 @@
 #pragma once
 #include <cublas_v2.h>
 
+#include <exception>
 #include <map>
 #include <string>
 #include <tuple>
@@ -40,6 +41,15 @@ struct JKScreenCQ {
 };
 
 int jk_internal_set_err(int code, const char* msg);
+// The body of a C entry that allocates on the host: an exception becomes a status.
+template <class F>
+int jk_guard(F&& body) {
+    try {
+        return body();
+    } catch (const std::exception& e) {
+        return jk_internal_set_err(JK_ERR_CUDA, e.what());
+    }
+}
 // Waits until the tables that cudaMemcpy took from pageable memory lie on the
 // device.  It may return with the last transfer still under way on the legacy
 // stream, which a caller's non-blocking stream does not wait for; every function

@@ -97,6 +97,34 @@ def test_shard_plan_balances_and_is_deterministic():
     assert lib.jk_shard_plan(np.ones(1).ctypes.data, 1, 0, bad.ctypes.data) == 3
 
 
+def test_exceptions_do_not_leave_a_c_entry():
+    """A host allocation that fails inside an entry (16 GB of shard loads under
+    an address-space limit, in a child process) is a status and a message, not
+    the end of the process."""
+    import subprocess
+    import sys
+    code = """
+import ctypes, resource, sys
+import numpy as np
+lib = ctypes.CDLL(sys.argv[1])
+lib.jk_last_error.restype = ctypes.c_char_p
+own = np.zeros(1, dtype=np.int32)
+cost = np.ones(1)
+used = int(open('/proc/self/statm').read().split()[0]) * 4096
+resource.setrlimit(resource.RLIMIT_AS, (used + (1 << 30),) * 2)
+rc = lib.jk_shard_plan(ctypes.c_void_p(cost.ctypes.data), 1, 2147483647,
+                       ctypes.c_void_p(own.ctypes.data))
+assert rc == 1, rc
+assert b'alloc' in lib.jk_last_error()
+assert lib.jk_shard_plan(ctypes.c_void_p(cost.ctypes.data), 1, 2,
+                         ctypes.c_void_p(own.ctypes.data)) == 0
+print('status')
+"""
+    r = subprocess.run([sys.executable, '-c', code, jklib.LIBJK_PATH],
+                       capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == 'status', (r.stdout, r.stderr)
+
+
 def _ref_bin_loop_count(bins_ij, bins_kl, nbins, diag):
     """The reference's bin loop (gvhf/nr_jk_driver.cu:252-280): kl bin b
     pairs with the ij rows [bins_ij[0], bins_ij[nbins - b]); a diagonal
