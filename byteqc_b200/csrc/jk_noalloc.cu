@@ -205,7 +205,7 @@ extern "C" int jk_build_class_pair_noalloc(jk_basis_t* b, double* vj, double* vk
     }
     rc = jk_internal_launch(b, cp_ij, cp_kl, d_seg, d_task0, max_tasks, n_dm, stream);
     if (rc) return rc;
-    // same synchronous contract as jk_build_class_pair
+    // the scratch is free for the next call when this one returns
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
     return JK_OK;

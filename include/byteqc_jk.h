@@ -143,7 +143,7 @@ int jk_expand_int2e(jk_basis_t *basis, double *eri, int nao, void *stream);
  * address (make it before any stream capture); with CUDA's lazy module
  * loading that lookup is also when the array is placed on the device, so a
  * caller whose pool reserves most of the memory should make one call with
- * vj = vk = NULL (which does only the lookup) before the reservation.  Like
+ * vj = vk = NULL (which does only the lookup) before the reservation.  Unlike
  * jk_build_class_pair it returns after the GPU work has finished.  All calls
  * share the array: calls whose GPU work overlaps race and must be serialised
  * by the caller.
