@@ -228,8 +228,8 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
             const size_t o = dp_off[m];
             pm[m] = jk_internal_pack_mol(t->mols[m], dms[m], n_dm, t->d_pk + o, t->d_pk + t->pk_jp + o,
                                          vjs ? vjs[m] : nullptr);
-            if (!t->packed) pm[m].total = 0;
-            if (t->kt_len) {
+            if (!t->packed || !vjs[m]) pm[m].total = 0;  // no J wanted
+            if (t->kt_len && vks[m]) {
                 pm[m].kt = t->d_kt + kt_off[m];
                 pm[m].vk = vks[m];
             }
@@ -250,7 +250,7 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
                 s.vj = vjs ? vjs[m] : nullptr;
                 s.vk = vks ? vks[m] : nullptr;
                 s.n_dm = n_dm;
-                if (t->kt_len && s.nrun > 0) s.vk = t->d_kt + kt_off[m];
+                if (t->kt_len && s.vk && s.nrun > 0) s.vk = t->d_kt + kt_off[m];
                 if (t->packed) {
                     const size_t n = (size_t)n_dm * t->mols[m]->pack_total;
                     s.dp = t->d_pk + dp_off[m];

@@ -216,7 +216,8 @@ int jk_batch_destroy(jk_batch_t *batch);
 int jk_batch_nsolo(const jk_batch_t *batch, int *nsolo);
 
 /* Per molecule m: dms[m] device density in the working basis, vjs[m]/vks[m]
- * device buffers accumulated as in jk_build (either array may be NULL).  The
+ * device buffers accumulated as in jk_build (either array, and any entry of
+ * it, may be NULL).  The
  * segment tables follow the pointers: a call with new pointers synchronises
  * `stream` once to rebuild them; with the same pointers the call is fully
  * asynchronous. */

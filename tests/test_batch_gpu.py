@@ -116,6 +116,42 @@ def test_batch_with_a_larger_caller_basis_later():
     batch.close()
 
 
+def test_batch_build_with_outputs_left_out():
+    """jk_batch_build with null entries in the output arrays: J of the first
+    molecule only, K of the second only, both of the third."""
+    import ctypes
+    import torch
+    from byteqc_b200.cuobc import lib as jklib
+    from byteqc_b200.cuobc.scf.batch import JKBatch, _ptrs
+    lib = jklib.load_library()
+    mols = _mols()[:3]
+    batch = JKBatch(mols)
+    rng = np.random.default_rng(4)
+    dms = []
+    for op in batch.opts:
+        d = rng.standard_normal((op.nao, op.nao))
+        dms.append(torch.as_tensor(d + d.T, device='cuda'))
+    o = batch._opts(True, None, None)
+    full = None
+    for jn, kn in (((1, 1, 1), (1, 1, 1)), ((1, 0, 1), (0, 1, 1))):
+        vj, vk = ([torch.zeros_like(d) for d in dms] for _ in range(2))
+        assert lib.jk_batch_build(
+            batch.handle, _ptrs([d.data_ptr() for d in dms]),
+            _ptrs([v.data_ptr() if on else None for v, on in zip(vj, jn)]),
+            _ptrs([v.data_ptr() if on else None for v, on in zip(vk, kn)]), 1,
+            ctypes.byref(o), None) == 0
+        torch.cuda.synchronize()
+        if full is None:
+            full = vj, vk
+        for got, ref, on in ((vj, full[0], jn), (vk, full[1], kn)):
+            for g, r, want in zip(got, ref, on):
+                if want:
+                    assert (g - r).abs().max().item() <= 1e-10
+                else:
+                    assert not g.any().item()
+    batch.close()
+
+
 def test_batch_graph_replay():
     from byteqc_b200.cuobc.scf.batch import JKBatch
     mols = _mols()
