@@ -32,10 +32,10 @@
 
 #include "jk_internal.h"
 
-#define BCUDA(x)                                                                                   \
-    do {                                                                                           \
-        cudaError_t e_ = (x);                                                                      \
-        if (e_ != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e_));    \
+#define BCUDA(x)                                                  \
+    do {                                                          \
+        cudaError_t e_ = (x);                                     \
+        if (e_ != cudaSuccess) return jk_internal_cuda_err(e_);   \
     } while (0)
 
 struct JKSym {
@@ -187,6 +187,7 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
     if (same) return JK_OK;
     // earlier launches may still read the old tables and buffers
     BCUDA(cudaStreamSynchronize(st));
+    t->seg_ndm = -1;  // no tables until these are complete (an allocation may fail on the way)
     // pair-packed J side (with J only)
     t->packed = vjs != nullptr;
     std::vector<size_t> dp_off(t->nmol, 0);
@@ -202,6 +203,7 @@ static int batch_segments(jk_batch* t, const double* const* dms, double* const* 
         if (2 * tot > t->pk_cap) {
             cudaFree(t->d_pk);
             t->d_pk = nullptr;
+            t->pk_cap = 0;
             BCUDA(cudaMalloc(&t->d_pk, sizeof(double) * std::max<size_t>(2 * tot, 1)));
             t->pk_cap = 2 * tot;
         }
@@ -552,6 +554,7 @@ static int batch_get_jk(jk_batch* t, const double* const* coeffs, const int* nao
             off += (size_t)t->mols[m]->nao * nao0s[m];
         }
         BCUDA(cudaStreamSynchronize(st));
+        t->w_ndm = -1;  // until it is laid out
         cudaFree(t->d_work);
         t->d_work = nullptr;
         BCUDA(cudaMalloc(&t->d_work, sizeof(double) * std::max<size_t>(off, 1)));

@@ -44,7 +44,10 @@ static int set_err(int code, const char* fmt, ...) {
 #define CUDA_TRY(x)                                                                               \
     do {                                                                                          \
         cudaError_t e_ = (x);                                                                     \
-        if (e_ != cudaSuccess) return set_err(JK_ERR_CUDA, "%s: %s", #x, cudaGetErrorString(e_)); \
+        if (e_ != cudaSuccess) {                                                                  \
+            cudaGetLastError(); /* the check after the next call's launches would find it */      \
+            return set_err(JK_ERR_CUDA, "%s: %s", #x, cudaGetErrorString(e_));                    \
+        }                                                                                         \
     } while (0)
 
 extern "C" const char* jk_last_error(void) { return g_err.c_str(); }

@@ -41,6 +41,12 @@ struct JKScreenCQ {
 };
 
 int jk_internal_set_err(int code, const char* msg);
+// status of a failed CUDA call, taken off the runtime's last error too: the
+// check after the next call's launches would report it again
+inline int jk_internal_cuda_err(cudaError_t e) {
+    cudaGetLastError();
+    return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
+}
 // The body of a C entry that allocates on the host: an exception becomes a status.
 template <class F>
 int jk_guard(F&& body) {

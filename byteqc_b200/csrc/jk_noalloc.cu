@@ -55,13 +55,13 @@ static unsigned char* g_na_ptr[64];
 static int na_scratch(unsigned char** out) {
     int dev;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
+    if (e != cudaSuccess) return jk_internal_cuda_err(e);
     if (dev < 0 || dev >= 64) return jk_internal_set_err(JK_ERR_ARG, "device ordinal out of range");
     std::lock_guard<std::mutex> lk(g_na_mu);
     if (!g_na_ptr[dev]) {
         void* p = nullptr;
         e = cudaGetSymbolAddress(&p, jk_na_scratch);
-        if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
+        if (e != cudaSuccess) return jk_internal_cuda_err(e);
         g_na_ptr[dev] = (unsigned char*)p;
     }
     *out = g_na_ptr[dev];
@@ -177,7 +177,7 @@ extern "C" int jk_build_class_pair_noalloc(jk_basis_t* b, double* vj, double* vk
         e = cudaMemcpyAsync(d_bins_kl, bins_locs_kl, sizeof(int) * (nbins + 1), cudaMemcpyHostToDevice, st);
     JKSeg seg;
     jk_internal_fill_seg(b, cp_ij, cp_kl, d_qoff, n_ij, dm, n_dm, vj, vk, &seg);
-    if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
+    if (e != cudaSuccess) return jk_internal_cuda_err(e);
     const int diag = cp_ij == cp_kl;
     long long max_tasks;
     JKSeg* d_seg = (JKSeg*)(sc + JK_NA_OFF_SEG);
@@ -192,7 +192,7 @@ extern "C" int jk_build_class_pair_noalloc(jk_basis_t* b, double* vj, double* vk
         else
             jk_na_ehi_kernel<<<(n_ij + 255) / 256, 256, 0, st>>>(cols, n_ij, erank, d_ehi);
         e = cudaGetLastError();
-        if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
+        if (e != cudaSuccess) return jk_internal_cuda_err(e);
         if (n_ij > JK_PAIR_PREP_ROWS) rc = jk_internal_run_items(seg, chunk, d_task0, d_seg, stream);
         if (rc) return rc;
         max_tasks = (long long)seg.nrun * ((n_kl + chunk - 1) / chunk);
@@ -200,13 +200,13 @@ extern "C" int jk_build_class_pair_noalloc(jk_basis_t* b, double* vj, double* vk
         jk_na_qoff_kernel<<<1, 1024, 0, st>>>(d_bins_ij, d_bins_kl, nbins, n_ij, n_kl, diag, d_qoff, d_task0, seg,
                                               d_seg);
         e = cudaGetLastError();
-        if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
+        if (e != cudaSuccess) return jk_internal_cuda_err(e);
         max_tasks = diag ? (long long)n_ij * (n_ij + 1) / 2 : (long long)n_ij * n_kl;
     }
     rc = jk_internal_launch(b, cp_ij, cp_kl, d_seg, d_task0, max_tasks, n_dm, stream);
     if (rc) return rc;
     // the scratch is free for the next call when this one returns
     e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e));
+    if (e != cudaSuccess) return jk_internal_cuda_err(e);
     return JK_OK;
 }

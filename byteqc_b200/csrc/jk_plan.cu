@@ -10,10 +10,10 @@
 
 #include "jk_internal.h"
 
-#define PCUDA(x)                                                                                 \
-    do {                                                                                         \
-        cudaError_t e_ = (x);                                                                    \
-        if (e_ != cudaSuccess) return jk_internal_set_err(JK_ERR_CUDA, cudaGetErrorString(e_));  \
+#define PCUDA(x)                                                  \
+    do {                                                          \
+        cudaError_t e_ = (x);                                     \
+        if (e_ != cudaSuccess) return jk_internal_cuda_err(e_);   \
     } while (0)
 
 // exclusive prefix of the segments' counts of every key (blockIdx.x = key, one

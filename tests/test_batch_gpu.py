@@ -152,6 +152,41 @@ def test_batch_build_with_outputs_left_out():
     batch.close()
 
 
+def test_batch_build_after_one_that_did_not_fit():
+    """A build whose workspace cannot be allocated (4 million densities asked
+    for) is an error before any launch, and the next one of the old size makes
+    its tables again."""
+    import ctypes
+    import torch
+    from byteqc_b200.cuobc import lib as jklib
+    from byteqc_b200.cuobc.scf.batch import JKBatch, _ptrs
+    lib = jklib.load_library()
+    batch = JKBatch(_mols())
+    rng = np.random.default_rng(6)
+    dms = []
+    for op in batch.opts:
+        d = rng.standard_normal((op.nao, op.nao))
+        dms.append(torch.as_tensor(d + d.T, device='cuda'))
+    vj, vk = ([torch.zeros_like(d) for d in dms] for _ in range(2))
+    o = batch._opts(True, None, None)
+
+    def build(n_dm):
+        return lib.jk_batch_build(
+            batch.handle, *(_ptrs([x.data_ptr() for x in y])
+                            for y in (dms, vj, vk)), n_dm, ctypes.byref(o), None)
+    assert build(1) == 0
+    torch.cuda.synchronize()
+    ref = [v.clone() for v in vj + vk]
+    for v in vj + vk:
+        v.zero_()
+    assert build(1 << 22) == 1
+    assert build(1) == 0
+    torch.cuda.synchronize()
+    for v, r in zip(vj + vk, ref):
+        assert (v - r).abs().max().item() <= 1e-10
+    batch.close()
+
+
 def test_batch_graph_replay():
     from byteqc_b200.cuobc.scf.batch import JKBatch
     mols = _mols()
