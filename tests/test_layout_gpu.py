@@ -181,3 +181,34 @@ def test_class_pair_call_is_two_launches(bas):
             cudart.cudaGraph_t(g.raw_cuda_graph()), 0)
         assert err == cudart.cudaError_t.cudaSuccess
         assert n == 2
+
+
+def test_noalloc_entry_on_more_than_8192_bra_pairs():
+    """Above 8192 bra pairs a call is prepared by several launches instead of
+    one block: the no-alloc entry against the allocating one on the largest
+    class of (H2O)22, with itself (diagonal) and with the smallest class, the
+    bins cutting it off in the middle."""
+    import torch
+    from byteqc_b200.cuobc import lib as jklib
+    from byteqc_b200.cuobc.scf import hf
+    lib = jklib.load_library()
+    opt, d = _setup(22, 'standin-cc-pvdz')
+    sizes = [len(q) for q in opt.log_qs]
+    big = int(np.argmax(sizes))
+    assert sizes[big] > 8192
+    small = min((n, i) for i, n in enumerate(sizes) if n)[1]
+    for cij, ckl in ((big, big), (max(big, small), min(big, small))):
+        bij, bkl = (hf._make_s_index_offsets(opt.log_qs[c], 10, 1e-9)
+                    for c in (cij, ckl))
+        out = []
+        for fn in (lib.jk_build_class_pair, lib.jk_build_class_pair_noalloc):
+            vj, vk = torch.zeros_like(d), torch.zeros_like(d)
+            assert fn(opt.handle, vj.data_ptr(), vk.data_ptr(), d.data_ptr(),
+                      opt.nao, 1, bij.ctypes.data, bkl.ctypes.data, 10, cij,
+                      ckl, None) == 0
+            torch.cuda.synchronize()
+            out.append((vj, vk))
+        assert out[0][0].abs().max().item() > 0
+        for a, b in zip(*out):
+            assert (a - b).abs().max().item() <= 1e-10
+    opt.clear()
