@@ -14,13 +14,16 @@
 //   recursion by one thread per (root, axis), the bra transfer by one per
 //   (root, axis, m), the ket transfer by one per (root, axis, i, j).  The
 //   integrals of a range of (i, j) components are summed over primitives and
-//   roots in shared memory, once per density, and then digested from there: every thread
-//   owns elements of the six J/K blocks (J_ij, J_kl, K_ik, K_il, K_jk, K_jl)
-//   and sums integral times density over the other two indices (no atomics:
-//   one owner per element); the blocks are added to J and K with one atomic
-//   per element at the end.  Before, three threads of 128 built the blocks of
-//   one root at a time while the others waited, and each of the six blocks
-//   formed every integral again from three shared-memory loads.
+//   roots in shared memory, once per density, and then digested from there: every
+//   thread owns elements of the six J/K blocks (J_ij, J_kl, K_ik, K_il, K_jk, K_jl)
+//   and sums integral times density over the other two indices (no atomics: one
+//   owner per element); the blocks are added to J and K with one atomic per
+//   element at the end.  Classes whose integrals take many such ranges, (gg|gg)
+//   or (hh|hh), would build their 2D blocks again for each of them (up to 74
+//   times): there every element is summed from the blocks themselves.  One water,
+//   cc-pVDZ with added shells on the oxygen, ms, for a quartet at a time by three
+//   builders / ranges only / this rule: g 3.9 / 2.5 / 1.6, two g 5.2 / 8.0 / 4.6,
+//   h 9.1 / 16.9 / 4.6, i 21.7 / 85.7 / 11.5, contracted h 99 / 242 / 62.
 //
 // Digestion, index conventions and density orientation are those of the
 // templated kernels (cuobc/lib/gvhf/contract_jk.cu:225-316): output element
@@ -107,12 +110,12 @@ __device__ void jk_unit_rt(const JKPrim& p, double s, double w, int d, double no
     rys_2d_rt<GL>(li, lj, lk, ll, seed, c00, c0p, b10, b01, b00, ri[d] - rj[d], rk[d] - rl[d], W, out);
 }
 
-// Cartesian exponents of the components of shell l into ex[c][3]
-__device__ void jk_cart_table(int l, int (*ex)[3]) {
+// Cartesian exponents of the components of shell l, times a stride, into ex[c][3]
+__device__ void jk_cart_table(int l, int (*ex)[3], int stride = 1) {
     for (int c = threadIdx.x; c < ncart(l); c += blockDim.x) {
-        ex[c][0] = cart_lx(l, c);
-        ex[c][1] = cart_ly(l, c);
-        ex[c][2] = cart_lz(l, c);
+        ex[c][0] = stride * cart_lx(l, c);
+        ex[c][1] = stride * cart_ly(l, c);
+        ex[c][2] = stride * cart_lz(l, c);
     }
 }
 
@@ -147,7 +150,8 @@ __device__ void jk_generic_body(const Src& src) {
     __shared__ const JKSeg* s_sg;
     __shared__ double s_c[12];
     __shared__ JKPrim s_p;
-    __shared__ int s_ex[4][G::NF][3];  // Cartesian exponents of the four shells
+    __shared__ int s_of[4][G::NF][3];  // place of the four shells' components in a 2D block
+    __shared__ int s_nf[4];
     const int tid = threadIdx.x;
     const long long total = src.total();
     unsigned long long* queue = src.queue();
@@ -183,7 +187,10 @@ __device__ void jk_generic_body(const Src& src) {
             const int nh = (li + 1) * (lj + 1) * (mm + 1);                     // H of one unit
             const int ng = max((nm + 1) * (mm + 1), (li + 1) * SI), un = nh + ng;  // G and I share a place
             const int rb = min(nr, K::UNITS / (3 * un));                       // roots at a time
-            for (int sh = 0; sh < 4; sh++) jk_cart_table(sg.ls[sh], s_ex[sh]);
+            for (int sh = 0; sh < 4; sh++) {
+                jk_cart_table(sg.ls[sh], s_of[sh], sh == 0 ? SI : (sh == 1 ? SJ : (sh == 2 ? SK : 1)));
+                if (tid == 0) s_nf[sh] = ncart(sg.ls[sh]);
+            }
             // accumulator blocks: [0, o1) J_ij, [o1, o2) J_kl, [o2, o3) K_ik,
             // [o3, o4) K_il, [o4, o5) K_jk, [o5, E) K_jl
             const int o1 = nfi * nfj, o2 = o1 + nfk * nfl, o3 = o2 + nfi * nfk, o4 = o3 + nfi * nfl,
@@ -199,6 +206,21 @@ __device__ void jk_generic_body(const Src& src) {
             // parts of a row
             const int per = max(1, min(nfi * nfj, JK_GEN_ACC / nkl));
             const int nij = per >= nfj ? per / nfj * nfj : per;
+            const int npass = (nfi * nfj + nij - 1) / nij;
+            // batches of roots of all primitive quartets
+            const int nrb = (nr + rb - 1) / rb, nbat = npij * npkl * nrb;
+            // By passes (the integrals of a range of components at a time, the
+            // 2D blocks of every batch built again in every pass) or directly
+            // (the blocks built once, every J/K element from them, each
+            // integral formed six times).  Estimated cycles: a build waits on
+            // the serial recursion and four barriers, the digest of a pass on
+            // its longest sum.  Between 0.6 and 1.0 for the factor 0.8 nothing
+            // changes; at 0.3 and 1.5 two waters in TZVP + g take 13.9 and 15.1
+            // instead of 11.7 ms.
+            const long long by_pass = (long long)(npass - 1) * nbat * (60 * (nm + 1) * (mm + 1) + 1500) +
+                                      (long long)npass * (30 * nkl + 3000),
+                            at_once = (long long)nbat * rb * nfi * nfj * nkl * 4 / 5;
+            const bool direct = npass > 1 && by_pass > at_once;
             for (int idm = 0; idm < sg.n_dm; idm++) {
                 const double* D = sg.dm + (size_t)idm * nao * nao;
                 __syncthreads();
@@ -218,95 +240,121 @@ __device__ void jk_generic_body(const Src& src) {
                                 : __ldg(D + (x0 + a) + (size_t)nao * (y0 + b));
                     acc[e] = 0.;
                 }
-                for (int ij0 = 0; ij0 < nfi * nfj; ij0 += nij) {
-                    const int ij1 = min(nfi * nfj, ij0 + nij), ne = (ij1 - ij0) * nkl;
-                    for (int e = tid; e < ne; e += JK_GEN_THREADS) eri[e] = 0.;
-                    for (int kp = 0; kp < npkl; kp++)
-                        for (int ip = 0; ip < npij; ip++) {
-                            __syncthreads();
-                            if (tid == 0)
-                                s_p = jk_prim2(jk_pp(sg, q.prim_ij + ip * sg.pst_ij),
-                                               jk_pp(sg, q.prim_kl + kp * sg.pst_kl));
-                            __syncthreads();
-                            for (int r0 = 0; r0 < nr; r0 += rb) {
-                                const int nb = min(rb, nr - r0), nu = 3 * nb;
-                                if (r0) __syncthreads();  // the products of the last batch are done
-                                // vertical recursion: G[n][m] of unit (root, axis)
-                                for (int u = tid; u < nu; u += JK_GEN_THREADS) {
-                                    const int d = u % 3;
-                                    double s, w;
-                                    rys_root_rt(sg.rys, nr, s_p.x, r0 + u / 3, s, w);
-                                    const double siAB = s * s_p.iAB, bs = s_p.B * siAB, as = s_p.A * siAB;
-                                    const double b00 = 0.5 * siAB, b10 = 0.5 * s_p.iA * (1. - bs),
-                                                 b01 = 0.5 * s_p.iB * (1. - as);
-                                    const double pq = s_p.P[d] - s_p.Q[d];
-                                    const double c00 = (s_p.P[d] - s_c[d]) - bs * pq,
-                                                 c0p = (s_p.Q[d] - s_c[6 + d]) + as * pq;
-                                    double* g = units + u * un + nh;
-                                    const int M1 = mm + 1;
-                                    double prev = 0., v = d == 0 ? q.norm : (d == 1 ? s_p.sy : w);
-                                    g[0] = v;
-                                    for (int n = 0; n < nm; n++) {
-                                        const double nx = c00 * v + n * b10 * prev;
-                                        prev = v;
-                                        v = nx;
-                                        g[(n + 1) * M1] = v;
-                                    }
-                                    for (int m = 0; m < mm; m++)
-                                        for (int n = 0; n <= nm; n++) {
-                                            double x = c0p * g[n * M1 + m];
-                                            if (m) x += m * b01 * g[n * M1 + m - 1];
-                                            if (n) x += n * b00 * g[(n - 1) * M1 + m];
-                                            g[n * M1 + m + 1] = x;
-                                        }
+                for (int step = 0, built = -1; step < (direct ? nbat : npass * nbat); step++) {
+                    const int pass = direct ? 0 : step / nbat, bat = direct ? step : step % nbat;
+                    const int ij0 = pass * nij, ij1 = min(nfi * nfj, ij0 + nij), ne = (ij1 - ij0) * nkl;
+                    const int r0 = bat % nrb * rb, nb = min(rb, nr - r0), nu = 3 * nb;
+                    if (bat != built) {
+                        built = bat;
+                        __syncthreads();  // the products of the last batch are done
+                        if (tid == 0) {
+                            const int pr = bat / nrb, kp = pr / npij, ip = pr - kp * npij;
+                            s_p = jk_prim2(jk_pp(sg, q.prim_ij + ip * sg.pst_ij), jk_pp(sg, q.prim_kl + kp * sg.pst_kl));
+                        }
+                        __syncthreads();
+                        // vertical recursion: G[n][m] of unit (root, axis)
+                        for (int u = tid; u < nu; u += JK_GEN_THREADS) {
+                            const int d = u % 3;
+                            double s, w;
+                            rys_root_rt(sg.rys, nr, s_p.x, r0 + u / 3, s, w);
+                            const double siAB = s * s_p.iAB, bs = s_p.B * siAB, as = s_p.A * siAB;
+                            const double b00 = 0.5 * siAB, b10 = 0.5 * s_p.iA * (1. - bs),
+                                         b01 = 0.5 * s_p.iB * (1. - as);
+                            const double pq = s_p.P[d] - s_p.Q[d];
+                            const double c00 = (s_p.P[d] - s_c[d]) - bs * pq, c0p = (s_p.Q[d] - s_c[6 + d]) + as * pq;
+                            double* g = units + u * un + nh;
+                            const int M1 = mm + 1;
+                            double prev = 0., v = d == 0 ? q.norm : (d == 1 ? s_p.sy : w);
+                            g[0] = v;
+                            for (int n = 0; n < nm; n++) {
+                                const double nx = c00 * v + n * b10 * prev;
+                                prev = v;
+                                v = nx;
+                                g[(n + 1) * M1] = v;
+                            }
+                            for (int m = 0; m < mm; m++)
+                                for (int n = 0; n <= nm; n++) {
+                                    double x = c0p * g[n * M1 + m];
+                                    if (m) x += m * b01 * g[n * M1 + m - 1];
+                                    if (n) x += n * b00 * g[(n - 1) * M1 + m];
+                                    g[n * M1 + m + 1] = x;
                                 }
-                                __syncthreads();
-                                // bra transfer: H[i][j][m], one column m per item
-                                for (int x = tid; x < nu * (mm + 1); x += JK_GEN_THREADS) {
-                                    const int u = x / (mm + 1), m = x - u * (mm + 1), d = u % 3;
-                                    const double ab = s_c[d] - s_c[3 + d];
-                                    double* H = units + u * un + m;
-                                    const double* g = units + u * un + nh + m;
-                                    double A[2 * GL + 1];
-                                    for (int a = 0; a <= nm; a++) A[a] = g[a * (mm + 1)];
-                                    for (int j = 0; j <= lj; j++) {
-                                        for (int i = 0; i <= li; i++) H[(i * (lj + 1) + j) * (mm + 1)] = A[i];
-                                        for (int a = 0; a + j < nm; a++) A[a] = A[a + 1] + ab * A[a];
-                                    }
-                                }
-                                __syncthreads();
-                                // ket transfer: I[i][j][k][l], one (i, j) per item
-                                const int hij = (li + 1) * (lj + 1);
-                                for (int x = tid; x < nu * hij; x += JK_GEN_THREADS) {
-                                    const int u = x / hij, ij = x - u * hij, d = u % 3;
-                                    const double cd = s_c[6 + d] - s_c[9 + d];
-                                    const double* H = units + u * un + ij * (mm + 1);
-                                    double* I = units + u * un + nh + ij * SJ;
-                                    double B[2 * GL + 1];
-                                    for (int c = 0; c <= mm; c++) B[c] = H[c];
-                                    for (int l = 0; l <= ll; l++) {
-                                        for (int k = 0; k <= lk; k++) I[k * SK + l] = B[k];
-                                        for (int c = 0; c + l < mm; c++) B[c] = B[c + 1] + cd * B[c];
-                                    }
-                                }
-                                __syncthreads();
-                                // products of the batch
-                                for (int e = tid; e < ne; e += JK_GEN_THREADS) {
-                                    const int ij = e / nkl, kl = e - ij * nkl;
-                                    const int i = (ij0 + ij) / nfj, j = ij0 + ij - i * nfj;
-                                    const int k = kl / nfl, l = kl - k * nfl;
-                                    int o[3];
-#pragma unroll
-                                    for (int d = 0; d < 3; d++)
-                                        o[d] = d * un + nh + s_ex[0][i][d] * SI + s_ex[1][j][d] * SJ +
-                                               s_ex[2][k][d] * SK + s_ex[3][l][d];
-                                    double v = 0.;
-                                    const double* U = units;
-                                    for (int r = 0; r < nb; r++, U += 3 * un) v += U[o[0]] * U[o[1]] * U[o[2]];
-                                    eri[e] += v;
-                                }
+                        }
+                        __syncthreads();
+                        // bra transfer: H[i][j][m], one column m per item
+                        for (int x = tid; x < nu * (mm + 1); x += JK_GEN_THREADS) {
+                            const int u = x / (mm + 1), m = x - u * (mm + 1), d = u % 3;
+                            const double ab = s_c[d] - s_c[3 + d];
+                            double* H = units + u * un + m;
+                            const double* g = units + u * un + nh + m;
+                            double A[2 * GL + 1];
+                            for (int a = 0; a <= nm; a++) A[a] = g[a * (mm + 1)];
+                            for (int j = 0; j <= lj; j++) {
+                                for (int i = 0; i <= li; i++) H[(i * (lj + 1) + j) * (mm + 1)] = A[i];
+                                for (int a = 0; a + j < nm; a++) A[a] = A[a + 1] + ab * A[a];
                             }
                         }
+                        __syncthreads();
+                        // ket transfer: I[i][j][k][l], one (i, j) per item
+                        const int hij = (li + 1) * (lj + 1);
+                        for (int x = tid; x < nu * hij; x += JK_GEN_THREADS) {
+                            const int u = x / hij, ij = x - u * hij, d = u % 3;
+                            const double cd = s_c[6 + d] - s_c[9 + d];
+                            const double* H = units + u * un + ij * (mm + 1);
+                            double* I = units + u * un + nh + ij * SJ;
+                            double B[2 * GL + 1];
+                            for (int c = 0; c <= mm; c++) B[c] = H[c];
+                            for (int l = 0; l <= ll; l++) {
+                                for (int k = 0; k <= lk; k++) I[k * SK + l] = B[k];
+                                for (int c = 0; c + l < mm; c++) B[c] = B[c + 1] + cd * B[c];
+                            }
+                        }
+                        __syncthreads();
+                    }
+                    if (direct) {  // every element from the blocks themselves
+                        for (int e = tid; e < E; e += JK_GEN_THREADS) {
+                            // two shells (a, b) of the element fixed, the others (c, d) summed with D[c nd + d]
+                            int r, sa, sb, sc, sd;
+                            const double* dd = Dsm;
+                            if (e < o1) { r = e; sa = 0; sb = 1; sc = 2; sd = 3; }
+                            else if (e < o2) { r = e - o1; sa = 2; sb = 3; sc = 0; sd = 1; dd += d1; }
+                            else if (e < o3) { r = e - o2; sa = 0; sb = 2; sc = 1; sd = 3; dd += d2; }
+                            else if (e < o4) { r = e - o3; sa = 0; sb = 3; sc = 1; sd = 2; dd += d3; }
+                            else if (e < o5) { r = e - o4; sa = 1; sb = 2; sc = 0; sd = 3; dd += d4; }
+                            else { r = e - o5; sa = 1; sb = 3; sc = 0; sd = 2; dd += d5; }
+                            const int fb = s_nf[sb], fc = s_nf[sc], fd = s_nf[sd];
+                            const int a = r / fb, b = r - a * fb;
+                            const double *X = units + nh + s_of[sa][a][0] + s_of[sb][b][0],
+                                         *Y = units + un + nh + s_of[sa][a][1] + s_of[sb][b][1],
+                                         *Z = units + 2 * un + nh + s_of[sa][a][2] + s_of[sb][b][2];
+                            double v = 0.;
+                            for (int y = 0; y < nb; y++, X += 3 * un, Y += 3 * un, Z += 3 * un)
+                                for (int c = 0; c < fc; c++) {
+                                    const double *Xc = X + s_of[sc][c][0], *Yc = Y + s_of[sc][c][1],
+                                                 *Zc = Z + s_of[sc][c][2], *dc = dd + c * fd;
+#pragma unroll 4
+                                    for (int x = 0; x < fd; x++)
+                                        v += Xc[s_of[sd][x][0]] * Yc[s_of[sd][x][1]] * Zc[s_of[sd][x][2]] * dc[x];
+                                }
+                            acc[e] += v;
+                        }
+                        continue;
+                    }
+                    // products of the batch
+                    for (int e = tid; e < ne; e += JK_GEN_THREADS) {
+                        const int ij = e / nkl, kl = e - ij * nkl;
+                        const int i = (ij0 + ij) / nfj, j = ij0 + ij - i * nfj;
+                        const int k = kl / nfl, l = kl - k * nfl;
+                        int o[3];
+#pragma unroll
+                        for (int d = 0; d < 3; d++)
+                            o[d] = d * un + nh + s_of[0][i][d] + s_of[1][j][d] + s_of[2][k][d] + s_of[3][l][d];
+                        double v = 0.;
+                        const double* U = units;
+                        for (int r = 0; r < nb; r++, U += 3 * un) v += U[o[0]] * U[o[1]] * U[o[2]];
+                        eri[e] = bat ? eri[e] + v : v;
+                    }
+                    if (bat + 1 < nbat) continue;
                     __syncthreads();
                     // digest the components [ij0, ij1)
                     const int i_0 = ij0 / nfj, i_1 = (ij1 - 1) / nfj;
@@ -344,7 +392,7 @@ __device__ void jk_generic_body(const Src& src) {
                         }
                         acc[e] += v;
                     }
-                    __syncthreads();  // the next pass clears the integrals
+                    __syncthreads();  // the next pass overwrites the integrals
                 }
                 // add the blocks to J and K
                 for (int e = tid; e < E; e += JK_GEN_THREADS) {
