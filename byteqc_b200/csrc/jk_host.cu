@@ -716,6 +716,13 @@ static int sort_bucket(int n) { return std::max(32, (n / 16 + 31) / 32 * 32); }
 // itself and keeps 40.
 #define JK_RUN_ITEMS 5
 #define JK_RUN_ITEMS_PAIR 40
+// Contracted class quartets of at least this many primitive quartets go down to
+// single bra pairs in a build too: a lane's chain of two of them is what a small
+// molecule waits for.  Six waters in a six-fold contracted minimal basis 5.2 ms a
+// quartet per thread, 11.2 with runs of two at least, 6.4 now; 13 atoms in 6-31G*
+// 1.10 and 0.86 ms, 13 atoms / TZVP 5.2 and 4.95; 24 molecules in 6-31G* in a batch
+// 40.9 and 40.2 ms, but 42.3 with single pairs for every class quartet.
+#define JK_RUN_NPQ 64
 static int run_level(const jk_basis* b, int cp_ij, int n_kl, int chunk, int levels, int items) {
     for (int v = 0; v < levels - 1; v++)
         if ((long long)b->h_nrun[v][cp_ij] * ((n_kl + chunk - 1) / chunk) >= (long long)items * b->nsm) return v;
@@ -1007,13 +1014,15 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             c.pair_kl0 = b->h_pair_locs[ckl];
             c.n_kl = b->h_pair_locs[ckl + 1] - c.pair_kl0;
             if (c.n_ij == 0 || c.n_kl == 0) continue;
+            const double npq = (double)b->h_group_nprim[c.gi] * b->h_group_nprim[c.gj] * b->h_group_nprim[c.gk] *
+                               b->h_group_nprim[c.gl];
             c.runs = g_tabs.run[class_index(b, cij, ckl)];
             qoff_at.push_back(b->qoff_total);
             ioff_at.push_back(b->ioff_total);
             ent_at.push_back(b->ent_total);
             b->ent_total += c.n_ij;
             if (c.runs) {
-                c.level = run_level(b, cij, c.n_kl, c.runs, JK_RUN_LEVELS, JK_RUN_ITEMS);
+                c.level = run_level(b, cij, c.n_kl, c.runs, npq >= JK_RUN_NPQ ? JK_RUN_LEVELS_PAIR : JK_RUN_LEVELS, JK_RUN_ITEMS);
                 c.nrun = b->h_nrun[c.level][cij];
                 b->ioff_total += 2LL * c.nrun;
             } else {
@@ -1026,8 +1035,6 @@ static int create_impl(const int* atm, int natm, const int* bas, int nbas, const
             double nf = 1.;
             for (int a = 0; a < 4; a++) nf *= (l4[a] + 1) * (l4[a] + 2) / 2;
             const double nq = cij == ckl ? 0.5 * c.n_ij * (c.n_ij + 1.) : (double)c.n_ij * c.n_kl;
-            const double npq = (double)b->h_group_nprim[c.gi] * b->h_group_nprim[c.gj] * b->h_group_nprim[c.gk] *
-                               b->h_group_nprim[c.gl];
             b->h_cq_cost.push_back(nq * (npq * ((l4[0] + l4[1] + l4[2] + l4[3]) / 2 + 1) * nf + 12. * nf));
         }
     b->ncq = (int)b->h_cq.size();

@@ -150,7 +150,8 @@ struct JKPackMol {
 
 // run lengths a run table exists for: long runs save more traffic, short ones
 // give a small molecule enough items to fill the device.  The per-class-pair
-// entries, whose launch has the device to itself, go down to single pairs.
+// entries, whose launch has the device to itself, and contracted class quartets
+// go down to single pairs.
 #define JK_RUN_LEVELS 3
 #define JK_RUN_LEVELS_PAIR 4
 static const int JK_RUN_LEN[JK_RUN_LEVELS_PAIR] = {32, 8, 2, 1};

@@ -49,3 +49,24 @@ def test_run_kernels_vs_oracle(basis, nw, n_dm, group_size):
     assert abs(vj - rj).max() <= 1e-9
     assert abs(vk - rk).max() <= 1e-9
     opt.clear()
+
+
+def test_single_pair_runs_of_contracted_classes_vs_oracle():
+    """Two waters in a six-fold contracted minimal basis: 1296 primitive
+    quartets each, too few items for runs of more than one bra pair."""
+    from byteqc_b200.cuobc.scf import hf
+    from oracle import hf_oracle
+    six = [[a, 1. / (i + 1)] for i, a in enumerate((60., 20., 7., 2.5, .9, .3))]
+    mol = Mole(atom=geom.water_cluster(2, box=5.0, seed=2),
+               basis={'O': [[0] + six, [1] + six], 'H': [[0] + six]}).build()
+    dm = _dm(mol, 2, 3)
+    opt = hf._VHFOpt(mol).build()
+    rj, rk = zip(*(hf_oracle.get_jk(mol, d) for d in dm))
+    for d, j, k in zip(dm, rj, rk):
+        vj, vk = hf.get_jk(mol, d, vhfopt=opt)
+        assert abs(vj - j).max() <= 1e-10
+        assert abs(vk - k).max() <= 1e-10
+    vj, vk = hf.get_jk(mol, dm, vhfopt=opt)
+    assert abs(vj - np.stack(rj)).max() <= 1e-10
+    assert abs(vk - np.stack(rk)).max() <= 1e-10
+    opt.clear()
