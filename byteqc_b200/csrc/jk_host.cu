@@ -709,12 +709,13 @@ static int sort_bucket(int n) { return std::max(32, (n / 16 + 31) / 32 * 32); }
 // Run length of a class quartet's bra (an index of JK_RUN_LEN): the longest
 // that still gives `items` items per SM before screening; a molecule too small
 // for that takes the shortest.  In a build the launches of the classes share the
-// device, and 5 per SM do: at 5, 10, 20 and 40 (as it was) (H2O)8 / cc-pVDZ takes
-// 0.91, 0.96, 1.04 and 1.11 ms, 37 atoms in 6-31G* 31.4, 31.6, 32.4 and 33.4, (H2O)20
-// in 6-31G* 3.96, 4.15, 4.27 and 4.35, (H2O)32 / TZVP 254, 254, 254 and 255; at 160
-// (H2O)8 1.25 and (H2O)32 / TZVP 263.  A per-class-pair call has the device to
-// itself and keeps 40.
-#define JK_RUN_ITEMS 5
+// device, and 16 per SM do: at 5, 10, 16 and 40 (as it was) (H2O)8 / cc-pVDZ takes
+// 1.34, 1.34, 1.41 and 1.58 ms, 37 atoms in 6-31G* 31.4, 31.8, 31.8 and 33.3, (H2O)12 /
+// cc-pVDZ with an FP32 part 3.03, 3.02, 3.13 and 3.28, (H2O)9 / cc-pVDZ with one and
+// two densities 4.95, 4.69, 4.58 and 4.58: below 16 the last one is slower.  At 160
+// (H2O)32 / TZVP takes 263 ms instead of 255.  A per-class-pair call has the device
+// to itself and keeps 40.
+#define JK_RUN_ITEMS 16
 #define JK_RUN_ITEMS_PAIR 40
 // Contracted class quartets of at least this many primitive quartets go down to
 // single bra pairs in a build too: a lane's chain of two of them is what a small
